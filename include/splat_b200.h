@@ -225,6 +225,19 @@ int32_t splat_spmm_band(const void* p, const void* v, void* o, const float* sTod
                         int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
                         const int32_t* plan_i32, int32_t* status_word, void* stream);
 
+/* SDDMM / SpMM of fp32 operands on register tiles (true fp32 FMA), for patterns whose rows are bands
+ * of one stride (plan_i32 as from splat_acsr_classify); n_rows need not be a multiple of the stride.
+ * d = 32, 64 or 128, K as rows of d or as a contiguous (BH, d, n_cols) array.  Otherwise
+ * SPLAT_ERR_UNSUPPORTED_SHAPE / SPLAT_ERR_MISALIGNED without a launch: use splat_sddmm / splat_spmm. */
+int32_t splat_sddmm_tile(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
+                         int64_t k_stride_k, void* s_out, const float* sTod_lin, const float* sTod_tr,
+                         const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
+                         int64_t trailing_dim, int32_t dtype, const int32_t* plan_i32, void* stream);
+int32_t splat_spmm_tile(const void* p, const void* v, void* o, const float* sTod_lin,
+                        const float* sTod_tr, const float* nnzs, int64_t bh, int64_t n_rows,
+                        int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
+                        const int32_t* plan_i32, void* stream);
+
 /* Self-test of the bounded device-side wait used by the tensor-core kernels: one CTA waits on an
  * mbarrier that nothing arrives on, gives up after limit_cycles SM clocks (1 .. 2e9), stores code
  * 99 in *status_word (device int32, cleared by the caller) and ends normally; the context stays

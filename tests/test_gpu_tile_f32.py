@@ -1,0 +1,57 @@
+"""GPU: the fp32 register-tile kernels (fused, SDDMM, SpMM) against the CPU oracle at the edges of their
+tiles: lengths around multiples of 64, classes with a missing last row, both K layouts, rows with one or
+no non-zero."""
+import pytest
+import torch
+
+from conftest import assert_close
+from oracle import acsr_oracle as ao
+from oracle import attention_oracle as at
+
+pytestmark = pytest.mark.gpu
+
+#        kind, L, p0, p1, heads (32-row CTAs below 444 64-row tiles over all heads, 64-row CTAs from there)
+PATTERNS = [
+    (ao.PATTERN_CAUSAL_WINDOWED, 65, 63, 0, 3),      # one row in the second tile
+    (ao.PATTERN_CAUSAL_WINDOWED, 127, 126, 0, 3),    # dense causal, one row short of two tiles
+    (ao.PATTERN_CAUSAL_WINDOWED, 389, 64, 0, 64),    # L not a multiple of 4; 448 tiles
+    (ao.PATTERN_WINDOWED, 256, 37, 0, 111),          # 444 tiles
+    (ao.PATTERN_BLOCKED, 200, 48, 0, 3),
+    (ao.PATTERN_STRIDED, 203, 8, 0, 56),             # classes of 26 and 25 rows, single-element rows; 448 tiles
+    (ao.PATTERN_DILATED, 301, 40, 3, 3),             # classes of 101 and 100 rows
+    (ao.PATTERN_CAUSAL_WINDOWED, 3, 1, 0, 3),        # smallest
+]
+
+
+@pytest.mark.parametrize("contiguous", [False, True])
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_tile_kernels_against_oracle(d, contiguous):
+    import acsr_helpers as ah
+    import splat_native as n
+    for i, (kind, L, p0, p1, H) in enumerate(PATTERNS):
+        torch.manual_seed(700 + i)
+        acsr = ah.create_acsr(ah.PatternMask(kind, L, p0, p1), 16, 0)
+        meta = ao.metadata_from_pattern(kind, L, p0, p1, 16)
+        T, what = acsr[5], f"{(kind, L, p0, p1)} d={d}"
+        q, k, v = (torch.randn(1, H, L, d) for _ in range(3))
+        kt = k.cuda().transpose(2, 3)
+        kt = kt.contiguous() if contiguous else kt
+        scale = d ** -0.5
+        plan = n.classify(acsr[2], acsr[3], acsr[4])
+        assert plan[3] == 0 and (plan[7] == 0 or plan[1] == plan[2])     # a band pattern: the tile kernels run
+        o = torch.full((1, H, L, d), float("nan"), device="cuda")
+        lse = torch.full((1, H, L), float("nan"), device="cuda")
+        n.attention_fused(q.cuda(), kt, v.cuda(), o, acsr[2], acsr[3], acsr[4], scale, n.PATH_AUTO, lse=lse)
+        s_ref = at.sddmm_acsr(q, k.transpose(2, 3), meta, T)
+        assert_close(o, at.attention_acsr(q, k.transpose(2, 3), v, meta, T, scale), torch.float32, f"fused {what}")
+        assert_close(lse, at.lse_acsr(s_ref, meta, scale), torch.float32, f"lse {what}")
+        s = torch.full((1, H, L, T), float("nan"), device="cuda")
+        n.sddmm(q.cuda(), kt, s, acsr[2], acsr[3], acsr[4], T)
+        assert_close(s, s_ref, torch.float32, f"sddmm {what}")
+        _cols, valid = at._cols(meta, T)
+        assert torch.count_nonzero(s.cpu() * (~valid)) == 0, "padding slots must be zero"
+        p = torch.rand(1, H, L, T)
+        p_dev = torch.where(valid, p, torch.full_like(p, float("nan"))).cuda()     # padding is not read
+        o2 = torch.full((1, H, L, d), float("nan"), device="cuda")
+        n.spmm(p_dev, v.cuda(), o2, acsr[2], acsr[3], acsr[4], T)
+        assert_close(o2, at.spmm_acsr(p, v, meta), torch.float32, f"spmm {what}")

@@ -47,6 +47,9 @@ SIGNATURES = {
                          _i32, _vp, _vp, _vp],
     "splat_spmm_band": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp,
                         _vp],
+    "splat_sddmm_tile": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64,
+                         _i32, _vp, _vp],
+    "splat_spmm_tile": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp],
     "splat_selftest_bounded_wait": [_vp, _i64, _vp],
     "splat_debug_check_indices": [_vp],
     "splat_attention_noalloc": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _i64, _i64,
@@ -363,6 +366,16 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
     if x.dtype != torch.float32 and x.numel() > 0:
         _warn_cuda_core_16bit("sddmm")
     debug = _debug_before(dev)
+    if x.dtype == torch.float32 and path == PATH_AUTO and x.numel() > 0:
+        plan_arr = (ctypes.c_int32 * 8)(*classify(sTod_lin, sTod_tr, nnzs))
+        with _on(dev):
+            rc = _lib.splat_sddmm_tile(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
+                                       _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
+                                       _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, trailing_dim,
+                                       dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p), _stream(dev))
+        if rc not in _BAND_NOT_APPLICABLE:
+            check(rc, "splat_sddmm_tile")
+            return
     with _on(dev):
         check(_lib.splat_sddmm(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
                                _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
@@ -412,6 +425,16 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
     if x.dtype != torch.float32 and x.numel() > 0:
         _warn_cuda_core_16bit("spmm")
     debug = _debug_before(dev)
+    if x.dtype == torch.float32 and path == PATH_AUTO and x.numel() > 0:
+        plan_arr = (ctypes.c_int32 * 8)(*classify(sTod_lin, sTod_tr, nnzs))
+        with _on(dev):
+            rc = _lib.splat_spmm_tile(x.data_ptr(), y.data_ptr(), output.data_ptr(),
+                                      _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
+                                      _f32_vec(nnzs, L, "nnzs"), B * H, L, n_cols, d, T,
+                                      dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p), _stream(dev))
+        if rc not in _BAND_NOT_APPLICABLE:
+            check(rc, "splat_spmm_tile")
+            return
     with _on(dev):
         check(_lib.splat_spmm(x.data_ptr(), y.data_ptr(), output.data_ptr(),
                               _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),

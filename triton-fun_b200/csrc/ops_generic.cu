@@ -24,6 +24,7 @@ constexpr int kWarpsPerBlock = 4;
 // clamped to the nearest valid one before it is dereferenced and the kernel's code is recorded in
 // the word (the first code stays).  Off (null) the comparison is skipped.
 static int32_t* g_index_check = nullptr;
+bool index_check_on() { return g_index_check != nullptr; }
 enum : int32_t { kIndexSddmm = 71, kIndexSpmm = 72, kIndexFused = 73 };
 
 __device__ __forceinline__ int64_t slot_col(const RowAffine& ra, int j, int64_t n_cols, int32_t* check,
