@@ -238,6 +238,12 @@ int32_t splat_spmm_tile(const void* p, const void* v, void* o, const float* sTod
                         int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
                         const int32_t* plan_i32, void* stream);
 
+/* Host copy of a status word: host_copy is page-locked host memory (device-accessible, one int32, cleared
+ * by the caller).  A tensor-core kernel that is started while *status_word is non-zero does nothing but
+ * store that value in *host_copy, so a caller sees at a later launch that an earlier one gave up without
+ * copying or synchronising anything on the normal path.  NULL host_copy removes the pair; at most 64. */
+int32_t splat_set_status_mirror(int32_t* status_word, int32_t* host_copy);
+
 /* Self-test of the bounded device-side wait used by the tensor-core kernels: one CTA waits on an
  * mbarrier that nothing arrives on, gives up after limit_cycles SM clocks (1 .. 2e9), stores code
  * 99 in *status_word (device int32, cleared by the caller) and ends normally; the context stays

@@ -48,6 +48,7 @@ class RegularAttention(nn.Module):
          self.nnzs, self.acsr_trailing_dim,
          self.span_loop_start, self.span_loop_end) = create_acsr(mask, BLOCK_SIZE_Y, self.device)
         self.plan = _n.classify(self.sTod_linear_transformations, self.sTod_translations, self.nnzs)
+        _n.status_word(self.device)
 
         self.BLOCK_SIZE_Y = BLOCK_SIZE_Y
         self.BLOCK_SIZE_X = BLOCK_SIZE_X
@@ -80,6 +81,10 @@ class RegularAttention(nn.Module):
 
     ## Input x should already be in query/key/value post RoPe application.
     def forward(self, x):
+        if self.fused:
+            out = _n.module_forward(self.__dict__, x)
+            if out is not None:
+                return out
         q, k, v = x
         if self.fused:
             _n.attention_fused(q, k, v, self.rspmm_output, self.sTod_linear_transformations,

@@ -9,7 +9,6 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import os
-import time
 
 import torch
 
@@ -22,6 +21,11 @@ if not os.path.exists(LIB_PATH):
         "(this package has no CPU or eager fallback)")
 
 _lib = ctypes.CDLL(LIB_PATH)
+try:
+    import splat_host as _host      # native host path of the launchers (csrc/host_binding.cpp)
+except ImportError as e:
+    raise ImportError(f"the splat_host extension is missing or does not load ({e}): build it with "
+                      f"`python {os.path.join(_PKG_DIR, 'build.py')}`") from e
 
 _i32, _i64, _f32, _vp = ctypes.c_int32, ctypes.c_int64, ctypes.c_float, ctypes.c_void_p
 
@@ -52,6 +56,7 @@ SIGNATURES = {
     "splat_spmm_tile": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp],
     "splat_selftest_bounded_wait": [_vp, _i64, _vp],
     "splat_debug_check_indices": [_vp],
+    "splat_set_status_mirror": [_vp, _vp],
     "splat_attention_noalloc": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _i64, _i64,
                                 _i64, _i64, _i64, _f32, _i32, _vp],
 }
@@ -185,25 +190,21 @@ _STATUS_MIRRORS: dict = {}
 
 
 def status_word(dev: torch.device) -> torch.Tensor:
-    """Per-device int32 the band kernel sets when one of its bounded waits gives up."""
+    """Per-device int32 the tensor-core kernels set when one of their bounded waits gives up.  Beside it
+    lives a pinned host copy that a kernel started while the word is set writes itself, so that the host
+    can look at it without synchronising or copying anything on the normal path."""
     key = (dev.type, dev.index)
     t = _STATUS_WORDS.get(key)
     if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=dev)
+        with torch.cuda.device(dev):
+            t = torch.zeros(1, dtype=torch.int32, device=dev)
+            torch.cuda.current_stream(dev).synchronize()
+            host = torch.zeros(1, dtype=torch.int32).pin_memory()
+            check(_lib.splat_set_status_mirror(t.data_ptr(), host.data_ptr()), "splat_set_status_mirror")
+        _STATUS_MIRRORS[key] = {"host": host}
         _STATUS_WORDS[key] = t
+        _host.set_status(dev.index, t.data_ptr(), host.data_ptr())
     return t
-
-
-def _mirror(dev: torch.device) -> dict:
-    """Pinned host copy of the status word, refreshed after every tensor-core launch by a copy on
-    a side stream, so that the host can look at it without synchronising the device."""
-    key = (dev.type, dev.index)
-    m = _STATUS_MIRRORS.get(key)
-    if m is None:
-        m = {"host": torch.zeros(1, dtype=torch.int32).pin_memory(), "stream": torch.cuda.Stream(dev),
-             "launched": torch.cuda.Event(), "pending": 0, "stamp": 0.0}
-        _STATUS_MIRRORS[key] = m
-    return m
 
 
 def _raise_if_gave_up(dev: torch.device) -> None:
@@ -223,8 +224,7 @@ def _raise_if_gave_up(dev: torch.device) -> None:
                        "launches are not valid")
 
 
-_MIRROR_EVERY = 32          # launches between two refreshes of the mirror, at most
-_MIRROR_SECONDS = 0.002     # ... or this much time, whichever comes first
+_MIRROR_EVERY = 1           # launches after a kernel that gave up until the host copy of the word is set
 
 
 def _on(dev: torch.device):
@@ -232,24 +232,6 @@ def _on(dev: torch.device):
     if torch.cuda.current_device() == dev.index:
         return contextlib.nullcontext()
     return torch.cuda.device(dev)
-
-
-def _refresh_mirror(dev: torch.device) -> None:
-    """After a tensor-core launch: copy the status word to its pinned mirror behind the launch, on
-    a side stream, so the launching stream is not delayed.  Back-to-back launches share a copy (one
-    per _MIRROR_EVERY launches or _MIRROR_SECONDS): a launch that gave up is reported that many
-    launches later at the latest, and the kernels in between do nothing, as documented."""
-    m = _mirror(dev)
-    m["pending"] += 1
-    now = time.monotonic()
-    if m["pending"] < _MIRROR_EVERY and now - m["stamp"] < _MIRROR_SECONDS:
-        return
-    m["pending"] = 0
-    m["stamp"] = now
-    m["launched"].record(torch.cuda.current_stream(dev))
-    m["stream"].wait_event(m["launched"])
-    with torch.cuda.stream(m["stream"]):
-        m["host"].copy_(status_word(dev), non_blocking=True)
 
 
 _INDEX_CODES = {71: "sddmm", 72: "spmm", 73: "fused"}
@@ -334,6 +316,8 @@ def _band_candidate(x: torch.Tensor, path: int) -> bool:
 
 
 def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = PATH_AUTO) -> None:
+    if _host.sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path):
+        return
     dev = x.device
     _contig(x, "x"); _contig(output, "output")
     B, H, L, d = x.shape
@@ -357,7 +341,6 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
                                        status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE or path == PATH_BAND:
             check(rc, "splat_sddmm_band")
-            _refresh_mirror(dev)
             if os.environ.get("SPLAT_B200_DEBUG"):
                 check_status_word(dev)
             return
@@ -386,6 +369,8 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
 
 
 def softmax(x, output, nnzs, trailing_dim: int, scale: float = 1.0) -> None:
+    if _host.softmax(x, output, nnzs, trailing_dim, scale):
+        return
     dev = x.device
     _contig(x, "x"); _contig(output, "output")
     B, H, L, T = x.shape
@@ -398,6 +383,8 @@ def softmax(x, output, nnzs, trailing_dim: int, scale: float = 1.0) -> None:
 
 
 def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = PATH_AUTO) -> None:
+    if _host.spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path):
+        return
     dev = x.device
     _contig(x, "x"); _contig(y, "y"); _contig(output, "output")
     B, H, L, T = x.shape
@@ -416,7 +403,6 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
                                       status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE or path == PATH_BAND:
             check(rc, "splat_spmm_band")
-            _refresh_mirror(dev)
             if os.environ.get("SPLAT_B200_DEBUG"):
                 check_status_word(dev)
             return
@@ -480,9 +466,18 @@ def attention_fused(q, kt, v, output, sTod_lin, sTod_tr, nnzs, scale: float = 1.
             _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, float(scale), dtype_code(q.dtype),
             int(path), ctypes.cast(plan_arr, _vp) if plan_arr is not None else None,
             sw.data_ptr(), ctypes.byref(ran), _stream(dev)), "splat_attention_fused_lse")
-    if ran.value == PATH_BAND:
-        _refresh_mirror(dev)
-    elif q.dtype != torch.float32 and q.numel() > 0 and path == PATH_AUTO:
+    if ran.value != PATH_BAND and q.dtype != torch.float32 and q.numel() > 0 and path == PATH_AUTO:
         _warn_cuda_core_16bit("attention")
     if os.environ.get("SPLAT_B200_DEBUG"):
         check_status_word(dev)
+
+
+def module_forward(attributes: dict, x):
+    """The fused call of a RegularAttention, from its __dict__ and [q, k^T, v]: the output tensor, or None
+    when attention_fused() has to look at the operands (unusual ones, wrong ones, debug mode)."""
+    return _host.module_forward(attributes, x)
+
+
+_host.bind(*(ctypes.cast(getattr(_lib, name), _vp).value for name in (
+    "splat_attention_fused_lse", "splat_sddmm_band", "splat_spmm_band", "splat_sddmm_tile", "splat_spmm_tile",
+    "splat_softmax")), _warn_cuda_core_16bit)

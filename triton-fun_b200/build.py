@@ -1,12 +1,15 @@
-"""Build libsplat_b200.so (sm_100a only) in-tree with nvcc.
+"""Build libsplat_b200.so (sm_100a only) and SPLAT/splat_host.so in-tree.
 
     python triton-fun_b200/build.py [--force] [--verbose]
 
 The library is a plain C-ABI shared object (see include/splat_b200.h); it does not link torch.
+splat_host is the Python extension module behind the launchers (csrc/host_binding.cpp): it reads torch's
+tensors and calls the library, and is compiled against the installed torch.
 """
 from __future__ import annotations
 
 import os
+import shutil
 import subprocess
 import sys
 
@@ -15,10 +18,12 @@ REPO_ROOT = os.path.dirname(PKG_DIR)
 CSRC = os.path.join(PKG_DIR, "csrc")
 INCLUDE = os.path.join(REPO_ROOT, "include")
 LIB_PATH = os.path.join(PKG_DIR, "libsplat_b200.so")
+HOST_SRC = os.path.join(CSRC, "host_binding.cpp")
+HOST_PATH = os.path.join(PKG_DIR, "SPLAT", "splat_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC", "-shared", "-t", "8",
 ]
 
 
@@ -39,7 +44,29 @@ def up_to_date() -> bool:
     return all(os.path.getmtime(f) <= t for f in sources() + headers() + [__file__])
 
 
+def build_host(force: bool = False) -> str:
+    if not force and os.path.exists(HOST_PATH) and \
+            all(os.path.getmtime(f) <= os.path.getmtime(HOST_PATH) for f in (HOST_SRC, __file__)):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    nvcc = shutil.which(os.environ.get("NVCC", "nvcc")) or "/usr/local/cuda/bin/nvcc"
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc)))
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
+           "-I" + os.path.join(root, "include"),
+           "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_paths()["include"],
+           HOST_SRC, "-o", HOST_PATH, "-L" + os.path.join(root, "lib"),
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    print(" ".join(cmd), file=sys.stderr)
+    subprocess.run(cmd, check=True)
+    return HOST_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_host(force)
     if not force and up_to_date():
         return LIB_PATH
     nvcc = os.environ.get("NVCC", "nvcc")

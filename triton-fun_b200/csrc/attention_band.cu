@@ -81,6 +81,7 @@ struct Params {
     const void* k;     //   them (log-sum-exp output); everything else goes through the tensor maps
     float* lse;        // (BH, L) natural-log log-sum-exp of every row, or null
     int32_t* status;
+    int32_t* mirror;   // host copy of the status word, or null
     int64_t n_rows;    // L
     int rows_v;        // L / stride: rows of one residue class
     int stride;
@@ -210,7 +211,7 @@ attention_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             mbar_init(&ctrl->drain[i], 1);
         }
         mbar_fence_init();
-        ctrl->abort_at_entry = *status;
+        ctrl->abort_at_entry = entry_status(p.status, p.mirror);
     }
 
     // Per-row metadata in class coordinates (softmax threads only).
@@ -670,7 +671,7 @@ attention_band1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         }
         mbar_init(&ctrl->drain, 1);
         mbar_fence_init();
-        ctrl->abort_at_entry = *status;
+        ctrl->abort_at_entry = entry_status(p.status, p.mirror);
     }
     int my_a = 0, my_n = 0, row_nnz = 0, row_start = 0;
     int64_t row_real = -1;
@@ -1198,7 +1199,7 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
         return SPLAT_ERR_DRIVER;
     band::Params prm;
     prm.kt_major = kt_major ? 1 : 0;
-    prm.lin = lin; prm.tr = tr; prm.nnzs = nnzs; prm.v = v; prm.o = o; prm.status = status_word;
+    prm.lin = lin; prm.tr = tr; prm.nnzs = nnzs; prm.v = v; prm.o = o; prm.status = status_word; prm.mirror = status_mirror(status_word);
     prm.q = q; prm.k = k; prm.lse = lse;
     prm.n_rows = n_rows; prm.rows_v = (int)(n_rows / stride); prm.stride = (int)stride;
     prm.scale_log2 = scale * kLog2e;

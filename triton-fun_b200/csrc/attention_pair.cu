@@ -99,6 +99,7 @@ struct Params {
     const void* k;         //   through them (log-sum-exp output)
     float* lse;            // (BH, L) natural-log log-sum-exp of every row, or null
     int32_t* status;
+    int32_t* mirror;   // host copy of the status word, or null
     long long* trace;      // profiling builds only (else null)
     int64_t n_rows;        // L
     int rows_v;            // L / stride: rows of one residue class
@@ -323,7 +324,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         mbar_init(&ctrl->stage_free, 1);
         mbar_init(&ctrl->stage_ready, 4);
         mbar_fence_init();
-        ctrl->abort_at_entry = *status;
+        ctrl->abort_at_entry = entry_status(p.status, p.mirror);
     }
     // Range table: for every (class, row block) the key tiles [n_lo, n_lo + N) that cover every band
     // row of the block's 256 rows.  One warp per entry, lane l looks at rows l, l + 32, ...
@@ -963,7 +964,7 @@ int32_t attention_pair(const void* q, const void* k, int kt_major, const void* v
         !band::make_map(&mo, o, dtype, bh, n_rows, d, stride, pair::kTile))
         return SPLAT_ERR_DRIVER;
     pair::Params prm;
-    prm.lin = lin; prm.tr = tr; prm.nnzs = nnzs; prm.v = v; prm.status = status_word;
+    prm.lin = lin; prm.tr = tr; prm.nnzs = nnzs; prm.v = v; prm.status = status_word; prm.mirror = status_mirror(status_word);
     prm.q = q; prm.k = k; prm.lse = lse;
     prm.trace = pair::g_trace;
     prm.kt_major = kt_major;

@@ -1,5 +1,8 @@
 // Entry points that are not tied to one kernel file: version, status strings and the dispatch of
 // the fused attention call between the tensor-core band kernel and the general CUDA-core kernel.
+#include <atomic>
+#include <mutex>
+
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -39,6 +42,33 @@ extern "C" int32_t splat_selftest_bounded_wait(int32_t* status_word, int64_t lim
     if (!status_word || limit_cycles < 1 || limit_cycles > 2000000000LL) return SPLAT_ERR_BAD_ARG;
     splat::bounded_wait_selftest_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(status_word, limit_cycles);
     return splat::launch_status();
+}
+
+namespace splat {
+static struct { std::atomic<const int32_t*> word; std::atomic<int32_t*> mirror; } g_mirrors[64];
+static std::mutex g_mirrors_mutex;
+
+int32_t* status_mirror(const int32_t* status_word) {   // entries are only ever filled from the front
+    for (auto& e : g_mirrors) {
+        const int32_t* w = e.word.load(std::memory_order_acquire);
+        if (w == nullptr) break;
+        if (w == status_word) return e.mirror.load(std::memory_order_relaxed);
+    }
+    return nullptr;
+}
+}  // namespace splat
+
+extern "C" int32_t splat_set_status_mirror(int32_t* status_word, int32_t* host_copy) {
+    if (!status_word) return SPLAT_ERR_BAD_ARG;
+    std::lock_guard<std::mutex> lock(splat::g_mirrors_mutex);
+    for (auto& e : splat::g_mirrors) {
+        const int32_t* w = e.word.load(std::memory_order_relaxed);
+        if (w != nullptr && w != status_word) continue;
+        e.mirror.store(host_copy, std::memory_order_relaxed);
+        e.word.store(status_word, std::memory_order_release);
+        return SPLAT_OK;
+    }
+    return SPLAT_ERR_UNSUPPORTED_SHAPE;
 }
 
 extern "C" int32_t splat_version(void) { return SPLAT_B200_VERSION; }

@@ -106,6 +106,19 @@ inline int32_t launch_status() {
     return e == cudaSuccess ? SPLAT_OK : SPLAT_ERR_LAUNCH;
 }
 
+// Host copy registered for a status word (splat_set_status_mirror), or null.  Defined in capi.cu.
+int32_t* status_mirror(const int32_t* status_word);
+
+// First thing a tensor-core kernel does (one thread): the status word, passed on to its host copy if set.
+__device__ __forceinline__ int32_t entry_status(const int32_t* status_word, int32_t* mirror) {
+    const int32_t s = *(const volatile int32_t*)status_word;
+    if (s != 0 && mirror != nullptr) {
+        *(volatile int32_t*)mirror = s;
+        __threadfence_system();
+    }
+    return s;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 inline int elem_size(int32_t dtype) { return dtype == SPLAT_F32 ? 4 : 2; }

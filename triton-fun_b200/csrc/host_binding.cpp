@@ -1,0 +1,348 @@
+// Native host path of the Python launchers.
+//
+// One call of RegularAttention.forward used to spend 16 to 18 us on the host: a dozen attribute reads and
+// comparisons on tensors, ctypes conversions of 20 arguments and a periodic copy of the status word --
+// more than the small problems take on the device.  The functions here do the same checks on the tensors'
+// C++ objects and call the C ABI directly.  They only ever take the ordinary case: plain CUDA tensors on
+// the current device, consistent shapes, no debug mode, no reported failure.  For anything else they
+// return None without side effects and the Python code, which also words the errors, carries on.
+//
+// The C ABI entry points are handed over as addresses (bind()), so this module follows whichever build of
+// the library splat_native loaded, and the library itself stays free of torch.
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstdint>
+#include <cstdlib>
+
+namespace {
+
+constexpr int kPathAuto = 0, kPathGeneric = 1, kPathBand = 2;
+constexpr int kMaxDevices = 64;
+
+using FusedFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, const void*, void*, float*,
+                            const float*, const float*, const float*, int64_t, int64_t, int64_t, int64_t, float,
+                            int32_t, int32_t, const int32_t*, int32_t*, int32_t*, void*);
+using SddmmBandFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, void*, const float*, const float*,
+                                const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*,
+                                int32_t*, void*);
+using SpmmBandFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
+                               int64_t, int64_t, int64_t, int32_t, const int32_t*, int32_t*, void*);
+using SddmmTileFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, void*, const float*, const float*,
+                                const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
+using SpmmTileFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
+                               int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
+using SoftmaxFn = int32_t (*)(const void*, void*, const float*, int64_t, int64_t, int64_t, float, int32_t, void*);
+
+struct Api {
+    FusedFn fused;
+    SddmmBandFn sddmm_band;
+    SpmmBandFn spmm_band;
+    SddmmTileFn sddmm_tile;
+    SpmmTileFn spmm_tile;
+    SoftmaxFn softmax;
+} g_api{};
+
+// Per device: the status word (device memory) and its host copy, which the kernels write.
+struct Status {
+    int32_t* word = nullptr;
+    volatile int32_t* mirror = nullptr;
+} g_status[kMaxDevices];
+
+PyObject* g_warn = nullptr;   // splat_native's one-time warning, until it has been given
+PyObject *k_lin, *k_tr, *k_nnzs, *k_out, *k_scale, *k_path, *k_plan, *k_lse, *k_cached_plan;
+
+inline const at::Tensor* tensor(PyObject* o) {
+    return o != nullptr && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
+}
+inline int dtype_code(const at::Tensor& t) {
+    switch (t.scalar_type()) {
+        case at::kFloat: return 0;
+        case at::kHalf: return 1;
+        case at::kBFloat16: return 2;
+        default: return -1;
+    }
+}
+inline const float* meta(const at::Tensor* t, int64_t n, int device) {
+    return t != nullptr && t->scalar_type() == at::kFloat && t->is_cuda() && t->get_device() == device &&
+                   t->is_contiguous() && t->numel() >= n
+               ? static_cast<const float*>(t->const_data_ptr())
+               : nullptr;
+}
+// the 8 plan integers of a tuple
+inline bool read_plan(PyObject* o, int32_t (&plan)[8]) {
+    if (o == nullptr || !PyTuple_Check(o) || PyTuple_GET_SIZE(o) != 8) return false;
+    for (int i = 0; i < 8; ++i) {
+        PyObject* v = PyTuple_GET_ITEM(o, i);
+        if (!PyLong_Check(v)) return false;
+        plan[i] = static_cast<int32_t>(PyLong_AsLong(v));
+    }
+    return !PyErr_Occurred();
+}
+inline bool as_long(PyObject* o, long* v) {
+    if (o == nullptr || !PyLong_Check(o)) return false;
+    *v = PyLong_AsLong(o);
+    return !PyErr_Occurred();
+}
+// The device of an ordinary operand if it is the current one and nothing unusual is going on, else -1.
+inline int ordinary_device(const at::Tensor& t) {
+    if (!t.is_cuda()) return -1;
+    const int dev = t.get_device();
+    if (dev < 0 || dev >= kMaxDevices || g_status[dev].word == nullptr || dev != c10::cuda::current_device()) return -1;
+    if (*g_status[dev].mirror != 0) return -1;             // an earlier launch gave up: Python raises
+    if (const char* e = std::getenv("SPLAT_B200_DEBUG"); e != nullptr && e[0] != 0) return -1;
+    return dev;
+}
+// (B, H, X, Y) with collapsible (B, H)
+inline bool flat_bh(const at::Tensor& t, int64_t* stride_bh) {
+    const auto st = t.strides();
+    const auto sz = t.sizes();
+    if (sz[0] > 1 && sz[1] > 1 && st[0] != sz[1] * st[1]) return false;
+    *stride_bh = sz[1] > 1 ? st[1] : (sz[0] > 1 ? st[0] : sz[2] * sz[3]);
+    return true;
+}
+inline bool same4(const at::Tensor& t, int64_t a, int64_t b, int64_t c, int64_t d) {
+    const auto s = t.sizes();
+    return s.size() == 4 && s[0] == a && s[1] == b && s[2] == c && s[3] == d;
+}
+
+// True if the call was made; false: nothing happened and the Python code decides.
+bool fused(const at::Tensor* q, const at::Tensor* kt, const at::Tensor* v, const at::Tensor* out, const at::Tensor* lin,
+           const at::Tensor* tr, const at::Tensor* nnzs, float scale, long path, PyObject* plan_obj, const at::Tensor* lse) {
+    if (!q || !kt || !v || !out || g_api.fused == nullptr || q->dim() != 4 || kt->dim() != 4) return false;
+    const int dtype = dtype_code(*q);
+    const int dev = ordinary_device(*q);
+    if (dtype < 0 || dev < 0 || q->numel() == 0) return false;
+    if (kt->scalar_type() != q->scalar_type() || v->scalar_type() != q->scalar_type() || out->scalar_type() != q->scalar_type())
+        return false;
+    if (!kt->is_cuda() || !v->is_cuda() || !out->is_cuda() || kt->get_device() != dev || v->get_device() != dev ||
+        out->get_device() != dev)
+        return false;
+    const auto qs = q->sizes();
+    const int64_t B = qs[0], H = qs[1], L = qs[2], d = qs[3], n_cols = kt->size(3);
+    int64_t ksb;
+    if (!same4(*kt, B, H, d, n_cols) || !same4(*v, B, H, n_cols, d) || !same4(*out, B, H, L, d) || !flat_bh(*kt, &ksb))
+        return false;
+    if (!q->is_contiguous() || !v->is_contiguous() || !out->is_contiguous()) return false;
+    const float *pl = meta(lin, L, dev), *pt = meta(tr, L, dev), *pn = meta(nnzs, L, dev);
+    if (!pl || !pt || !pn) return false;
+    float* plse = nullptr;
+    if (lse != nullptr) {
+        const auto s = lse->sizes();
+        if (lse->scalar_type() != at::kFloat || s.size() != 3 || s[0] != B || s[1] != H || s[2] != L ||
+            !lse->is_contiguous() || !lse->is_cuda() || lse->get_device() != dev)
+            return false;
+        plse = static_cast<float*>(lse->data_ptr());
+    }
+    int32_t plan[8];
+    const bool with_plan = path != kPathGeneric;
+    if (with_plan && !read_plan(plan_obj, plan)) return false;
+    int32_t ran = 0;
+    const int32_t rc = g_api.fused(q->const_data_ptr(), kt->const_data_ptr(), ksb, kt->stride(3), kt->stride(2),
+                                   v->const_data_ptr(), out->data_ptr(), plse, pl, pt, pn, B * H, L, n_cols, d, scale, dtype,
+                                   static_cast<int32_t>(path), with_plan ? plan : nullptr, g_status[dev].word, &ran,
+                                   c10::cuda::getCurrentCUDAStream(dev).stream());
+    if (rc != 0) return false;
+    if (ran != kPathBand && dtype != 0 && path == kPathAuto && g_warn != nullptr) {   // 16 bit on the CUDA cores: say so once
+        PyObject* cb = g_warn;
+        g_warn = nullptr;
+        PyObject* r = PyObject_CallFunction(cb, "s", "attention");
+        Py_DECREF(cb);
+        if (r == nullptr) PyErr_Clear();
+        else Py_DECREF(r);
+    }
+    return true;
+}
+
+// plan remembered by splat_native.classify() on the nnzs tensor: ((id, id, version x 3, numel), plan, lin, tr)
+bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, const at::Tensor& lin, PyObject* tr_obj,
+                 const at::Tensor& tr, int32_t (&plan)[8]) {
+    PyObject* hit = PyObject_GetAttr(nnzs_obj, k_cached_plan);
+    if (hit == nullptr) {
+        PyErr_Clear();
+        return false;
+    }
+    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 4 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
+              PyTuple_GET_ITEM(hit, 3) == tr_obj;
+    if (ok) {
+        PyObject* key = PyTuple_GET_ITEM(hit, 0);
+        const int64_t now[4] = {static_cast<int64_t>(lin._version()), static_cast<int64_t>(tr._version()),
+                                static_cast<int64_t>(nnzs._version()), nnzs.numel()};
+        ok = PyTuple_Check(key) && PyTuple_GET_SIZE(key) == 6;
+        for (int i = 0; ok && i < 4; ++i) {
+            long v;
+            ok = as_long(PyTuple_GET_ITEM(key, 2 + i), &v) && v == now[i];
+        }
+        ok = ok && read_plan(PyTuple_GET_ITEM(hit, 1), plan);
+    }
+    Py_DECREF(hit);
+    return ok;
+}
+
+PyObject* yes_or_none(bool yes) {
+    if (PyErr_Occurred()) PyErr_Clear();
+    if (yes) Py_RETURN_TRUE;
+    Py_RETURN_NONE;
+}
+
+// module_forward(module.__dict__, [q, kt, v]) -> the module's output, or None
+PyObject* module_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2 || !PyDict_Check(args[0])) Py_RETURN_NONE;
+    PyObject *dict = args[0], *x = args[1];
+    PyObject* item[3];
+    if (PyList_Check(x) && PyList_GET_SIZE(x) == 3) {
+        for (int i = 0; i < 3; ++i) item[i] = PyList_GET_ITEM(x, i);
+    } else if (PyTuple_Check(x) && PyTuple_GET_SIZE(x) == 3) {
+        for (int i = 0; i < 3; ++i) item[i] = PyTuple_GET_ITEM(x, i);
+    } else {
+        Py_RETURN_NONE;
+    }
+    PyObject* out = PyDict_GetItemWithError(dict, k_out);
+    PyObject* scale = PyDict_GetItemWithError(dict, k_scale);
+    PyObject* lse = PyDict_GetItemWithError(dict, k_lse);
+    long path;
+    if (out == nullptr || scale == nullptr || !PyFloat_Check(scale) || !as_long(PyDict_GetItemWithError(dict, k_path), &path))
+        return yes_or_none(false);
+    const at::Tensor* lse_t = nullptr;
+    if (lse != nullptr && lse != Py_None && (lse_t = tensor(lse)) == nullptr) return yes_or_none(false);
+    if (!fused(tensor(item[0]), tensor(item[1]), tensor(item[2]), tensor(out), tensor(PyDict_GetItemWithError(dict, k_lin)),
+               tensor(PyDict_GetItemWithError(dict, k_tr)), tensor(PyDict_GetItemWithError(dict, k_nnzs)),
+               static_cast<float>(PyFloat_AS_DOUBLE(scale)), path, PyDict_GetItemWithError(dict, k_plan), lse_t))
+        return yes_or_none(false);
+    Py_INCREF(out);
+    return out;
+}
+
+// sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path) -> True, or None
+PyObject* sddmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    long trailing, path;
+    if (n != 8 || !as_long(a[6], &trailing) || !as_long(a[7], &path) || path != kPathAuto) return yes_or_none(false);
+    const at::Tensor *x = tensor(a[0]), *y = tensor(a[1]), *out = tensor(a[2]), *lin = tensor(a[3]), *tr = tensor(a[4]),
+                     *nnzs = tensor(a[5]);
+    if (!x || !y || !out || !lin || !tr || !nnzs || g_api.sddmm_band == nullptr || x->dim() != 4 || y->dim() != 4)
+        return yes_or_none(false);
+    const int dtype = dtype_code(*x), dev = ordinary_device(*x);
+    if (dtype < 0 || dev < 0 || x->numel() == 0 || trailing < 1) return yes_or_none(false);
+    const auto xs = x->sizes();
+    const int64_t B = xs[0], H = xs[1], L = xs[2], d = xs[3], n_cols = y->size(3);
+    int64_t ksb;
+    if (y->scalar_type() != x->scalar_type() || out->scalar_type() != x->scalar_type() || !y->is_cuda() || !out->is_cuda() ||
+        y->get_device() != dev || out->get_device() != dev || !same4(*y, B, H, d, n_cols) || !same4(*out, B, H, L, trailing) ||
+        !flat_bh(*y, &ksb) || !x->is_contiguous() || !out->is_contiguous())
+        return yes_or_none(false);
+    const float *pl = meta(lin, L, dev), *pt = meta(tr, L, dev), *pn = meta(nnzs, L, dev);
+    int32_t plan[8];
+    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan)) return yes_or_none(false);
+    void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
+    const int64_t ksc = y->stride(3), ksk = y->stride(2);
+    const int32_t rc =
+        dtype == 0 ? g_api.sddmm_tile(x->const_data_ptr(), y->const_data_ptr(), ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
+                                      L, n_cols, d, trailing, dtype, plan, st)
+                   : g_api.sddmm_band(x->const_data_ptr(), y->const_data_ptr(), ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
+                                      L, n_cols, d, trailing, dtype, plan, g_status[dev].word, st);
+    return yes_or_none(rc == 0);
+}
+
+// spmm(p, v, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path) -> True, or None
+PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    long trailing, path;
+    if (n != 8 || !as_long(a[6], &trailing) || !as_long(a[7], &path) || path != kPathAuto) return yes_or_none(false);
+    const at::Tensor *x = tensor(a[0]), *y = tensor(a[1]), *out = tensor(a[2]), *lin = tensor(a[3]), *tr = tensor(a[4]),
+                     *nnzs = tensor(a[5]);
+    if (!x || !y || !out || !lin || !tr || !nnzs || g_api.spmm_band == nullptr || x->dim() != 4 || y->dim() != 4)
+        return yes_or_none(false);
+    const int dtype = dtype_code(*x), dev = ordinary_device(*x);
+    if (dtype < 0 || dev < 0 || x->numel() == 0) return yes_or_none(false);
+    const auto xs = x->sizes();
+    const int64_t B = xs[0], H = xs[1], L = xs[2], T = xs[3], n_cols = y->size(2), d = y->size(3);
+    if (T != trailing || y->scalar_type() != x->scalar_type() || out->scalar_type() != x->scalar_type() || !y->is_cuda() ||
+        !out->is_cuda() || y->get_device() != dev || out->get_device() != dev || !same4(*y, B, H, n_cols, d) ||
+        !same4(*out, B, H, L, d) || !x->is_contiguous() || !y->is_contiguous() || !out->is_contiguous())
+        return yes_or_none(false);
+    const float *pl = meta(lin, L, dev), *pt = meta(tr, L, dev), *pn = meta(nnzs, L, dev);
+    int32_t plan[8];
+    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan)) return yes_or_none(false);
+    void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
+    const int32_t rc = dtype == 0 ? g_api.spmm_tile(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
+                                                    n_cols, d, T, dtype, plan, st)
+                                  : g_api.spmm_band(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
+                                                    n_cols, d, T, dtype, plan, g_status[dev].word, st);
+    return yes_or_none(rc == 0);
+}
+
+// softmax(x, output, nnzs, trailing_dim, scale) -> True, or None
+PyObject* softmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    long trailing;
+    if (n != 5 || !as_long(a[3], &trailing) || !PyFloat_Check(a[4])) return yes_or_none(false);
+    const at::Tensor *x = tensor(a[0]), *out = tensor(a[1]), *nnzs = tensor(a[2]);
+    if (!x || !out || !nnzs || g_api.softmax == nullptr || x->dim() != 4) return yes_or_none(false);
+    const int dtype = dtype_code(*x), dev = ordinary_device(*x);
+    if (dtype < 0 || dev < 0) return yes_or_none(false);
+    const auto xs = x->sizes();
+    if (xs[3] != trailing || !same4(*out, xs[0], xs[1], xs[2], xs[3]) || out->scalar_type() != x->scalar_type() ||
+        !out->is_cuda() || out->get_device() != dev || !x->is_contiguous() || !out->is_contiguous())
+        return yes_or_none(false);
+    const float* pn = meta(nnzs, xs[2], dev);
+    if (!pn) return yes_or_none(false);
+    const int32_t rc = g_api.softmax(x->const_data_ptr(), out->data_ptr(), pn, xs[0] * xs[1], xs[2], trailing,
+                                     static_cast<float>(PyFloat_AS_DOUBLE(a[4])), dtype, c10::cuda::getCurrentCUDAStream(dev).stream());
+    return yes_or_none(rc == 0);
+}
+
+// bind(fused, sddmm_band, spmm_band, sddmm_tile, spmm_tile, softmax, warn): addresses of the C ABI entry points
+// and the function that warns of 16-bit operands on the CUDA-core kernels
+PyObject* bind(PyObject*, PyObject* args) {
+    unsigned long long f[6];
+    PyObject* warn;
+    if (!PyArg_ParseTuple(args, "KKKKKKO", f, f + 1, f + 2, f + 3, f + 4, f + 5, &warn)) return nullptr;
+    Py_INCREF(warn);
+    g_warn = warn;
+    g_api.fused = reinterpret_cast<FusedFn>(f[0]);
+    g_api.sddmm_band = reinterpret_cast<SddmmBandFn>(f[1]);
+    g_api.spmm_band = reinterpret_cast<SpmmBandFn>(f[2]);
+    g_api.sddmm_tile = reinterpret_cast<SddmmTileFn>(f[3]);
+    g_api.spmm_tile = reinterpret_cast<SpmmTileFn>(f[4]);
+    g_api.softmax = reinterpret_cast<SoftmaxFn>(f[5]);
+    Py_RETURN_NONE;
+}
+
+// set_status(device index, address of the status word, address of its host copy)
+PyObject* set_status(PyObject*, PyObject* args) {
+    int dev;
+    unsigned long long word, mirror;
+    if (!PyArg_ParseTuple(args, "iKK", &dev, &word, &mirror)) return nullptr;
+    if (dev >= 0 && dev < kMaxDevices) {
+        g_status[dev].mirror = reinterpret_cast<volatile int32_t*>(mirror);
+        g_status[dev].word = reinterpret_cast<int32_t*>(word);
+    }
+    Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"bind", bind, METH_VARARGS, nullptr},
+    {"set_status", set_status, METH_VARARGS, nullptr},
+    {"module_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(module_forward)), METH_FASTCALL, nullptr},
+    {"sddmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sddmm)), METH_FASTCALL, nullptr},
+    {"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(spmm)), METH_FASTCALL, nullptr},
+    {"softmax", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(softmax)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "splat_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_splat_host() {
+    k_lin = PyUnicode_InternFromString("sTod_linear_transformations");
+    k_tr = PyUnicode_InternFromString("sTod_translations");
+    k_nnzs = PyUnicode_InternFromString("nnzs");
+    k_out = PyUnicode_InternFromString("rspmm_output");
+    k_scale = PyUnicode_InternFromString("scale");
+    k_path = PyUnicode_InternFromString("path");
+    k_plan = PyUnicode_InternFromString("plan");
+    k_lse = PyUnicode_InternFromString("lse");
+    k_cached_plan = PyUnicode_InternFromString("_splat_plan");
+    return PyModule_Create(&module_def);
+}

@@ -59,6 +59,7 @@ struct Params {
     const void* kv;      // sddmm: K, spmm: V, (BH, L, d)
     void* sparse;        // sddmm: S out, spmm: P in, (BH, L, trailing_dim)
     int32_t* status;
+    int32_t* mirror;   // host copy of the status word, or null
     int64_t n_rows;      // L
     int rows_v;          // L / stride
     int stride;
@@ -245,7 +246,7 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
         mbar_init(&ctrl->drain, 1);
         mbar_fence_init();
-        ctrl->abort_at_entry = *status;
+        ctrl->abort_at_entry = entry_status(p.status, p.mirror);
     }
     RowInfo me{0, 0, 0, 0};
     if (warp < kRowWarps) {
@@ -515,7 +516,7 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
         }
         mbar_init(&ctrl->drain, 1);
         mbar_fence_init();
-        ctrl->abort_at_entry = *status;
+        ctrl->abort_at_entry = entry_status(p.status, p.mirror);
     }
     RowInfo me{0, 0, 0, 0};
     if (warp < kRowWarps) {
@@ -797,7 +798,7 @@ extern "C" int32_t splat_sddmm_band(const void* q, const void* k, int64_t k_stri
     prm.trace = ops::g_trace;
 #endif
     prm.lin = sTod_lin; prm.tr = sTod_tr; prm.nnzs = nnzs; prm.q = q; prm.kv = k; prm.sparse = s_out;
-    prm.status = status_word; prm.n_rows = n_rows; prm.rows_v = (int)(n_rows / stride);
+    prm.status = status_word; prm.mirror = status_mirror(status_word); prm.n_rows = n_rows; prm.rows_v = (int)(n_rows / stride);
     prm.stride = (int)stride; prm.trailing_dim = (int)trailing_dim;
     prm.direct = ops::aligned16(s_out) ? 1 : 0;
     cudaStream_t st = (cudaStream_t)stream;
@@ -828,7 +829,7 @@ extern "C" int32_t splat_spmm_band(const void* p, const void* v, void* o, const 
 #endif
     prm.lin = sTod_lin; prm.tr = sTod_tr; prm.nnzs = nnzs; prm.q = nullptr; prm.kv = v;
     prm.sparse = const_cast<void*>(p);
-    prm.status = status_word; prm.n_rows = n_rows; prm.rows_v = (int)(n_rows / stride);
+    prm.status = status_word; prm.mirror = status_mirror(status_word); prm.n_rows = n_rows; prm.rows_v = (int)(n_rows / stride);
     prm.stride = (int)stride; prm.trailing_dim = (int)trailing_dim;
     prm.direct = 0;
     prm.kt_major = 0;
