@@ -205,7 +205,7 @@ def torch_dense_masked_baseline(cfgs=(1, 2), budget_s=12.0):
 
 
 # fused band kernel by the library's SPLAT_B200_BAND_TILES switch (default: one Q tile per CTA)
-BAND_KERNELS = {"1": "attention_band1_kernel", "2": "attention_band_kernel", "3": "attention_pair_kernel"}
+BAND_KERNELS = {"1": "attention_wide_kernel", "2": "attention_band_kernel", "3": "attention_pair_kernel"}
 
 
 def ncu_traffic(cfg, heads, path):
@@ -550,7 +550,7 @@ def run_ours(args):
                                                          "ncu capture scaled by heads)",
                      "traffic_source": traffic_source,
                      "kernel": "sddmm + softmax + spmm (three launches)" if unfused else
-                               (BAND_KERNELS.get(os.environ.get("SPLAT_B200_BAND_TILES", "1")[:1], "attention_band1_kernel")
+                               (BAND_KERNELS.get(os.environ.get("SPLAT_B200_BAND_TILES", "1")[:1], "attention_wide_kernel")
                                 if args.path == "band" else "attention_rows_kernel"),
                      "peak_source": peaks["source"],
                      "peak_kind": "burst", "launch_ms": launch_ms, "launch_ms_median": launch_ms_median,

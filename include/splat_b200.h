@@ -238,6 +238,20 @@ int32_t splat_spmm_tile(const void* p, const void* v, void* o, const float* sTod
                         int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
                         const int32_t* plan_i32, void* stream);
 
+/* Band table of metadata whose plan shows bands of one stride: 2 (n_rows + stride ceil(ceil(n_rows / stride) /
+ * 128)) device int32, 8-byte aligned, holding every row's band and every 128-row tile's key range in the
+ * layout the tensor-core kernels want (csrc/acsr_meta.cu).  A caller that keeps its metadata keeps the table
+ * with it and passes it to splat_attention_fused_table (splat_attention_fused_lse with one more argument;
+ * NULL: the kernels work the ranges out themselves).  It has to be rebuilt when the metadata changes. */
+int32_t splat_band_table(const float* sTod_lin, const float* sTod_tr, const float* nnzs, int64_t n_rows,
+                         int64_t stride, int32_t* table, void* stream);
+int32_t splat_attention_fused_table(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
+                                    int64_t k_stride_k, const void* v, void* o, float* lse,
+                                    const float* sTod_lin, const float* sTod_tr, const float* nnzs, int64_t bh,
+                                    int64_t n_rows, int64_t n_cols, int64_t d, float scale, int32_t dtype,
+                                    int32_t path, const int32_t* plan_i32, const int32_t* band_table,
+                                    int32_t* status_word, int32_t* path_ran, void* stream);
+
 /* Host copy of a status word: host_copy is page-locked host memory (device-accessible, one int32, cleared
  * by the caller).  A tensor-core kernel that is started while *status_word is non-zero does nothing but
  * store that value in *host_copy, so a caller sees at a later launch that an earlier one gave up without

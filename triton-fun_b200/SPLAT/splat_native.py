@@ -57,6 +57,9 @@ SIGNATURES = {
     "splat_selftest_bounded_wait": [_vp, _i64, _vp],
     "splat_debug_check_indices": [_vp],
     "splat_set_status_mirror": [_vp, _vp],
+    "splat_band_table": [_vp, _vp, _vp, _i64, _i64, _vp, _vp],
+    "splat_attention_fused_table": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64,
+                                    _i64, _i64, _f32, _i32, _i32, _vp, _vp, _vp, _vp, _vp],
     "splat_attention_noalloc": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _i64, _i64,
                                 _i64, _i64, _i64, _f32, _i32, _vp],
 }
@@ -164,8 +167,8 @@ def acsr_from_row_summary(rows_i32: torch.Tensor, n_cols: int, block_height: int
 
 
 def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) -> tuple:
-    """Host copy of the 8 plan ints of ``splat_acsr_classify``.  The result is remembered ON the
-    ``nnzs`` tensor object (with the identities and versions of all three tensors), so it lives
+    """Host copy of the 8 plan ints of ``splat_acsr_classify``.  The result, with the band table of a band
+    pattern (``splat_band_table``), is remembered ON the ``nnzs`` tensor object (with the identities and versions of all three tensors), so it lives
     exactly as long as that metadata and is recomputed if any of them is modified in place."""
     key = (id(sTod_lin), id(sTod_tr), sTod_lin._version, sTod_tr._version, nnzs._version,
            nnzs.numel())
@@ -180,9 +183,27 @@ def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) 
                                        _f32_vec(nnzs, n, "nnzs"), n, plan.data_ptr(), _stream(dev)),
               "splat_acsr_classify")
     host = tuple(int(v) for v in plan.cpu().tolist())
+    table = None
+    stride = host[1] if host[7] > 0 else 1
+    if 0 < n <= 2**31 - 1 and (host[7] == 0 or host[1] == host[2]) and host[3] == 0 and host[5] <= n and stride <= 65535:
+        tiles = -(-(-(-n // stride)) // 128) * stride
+        table = torch.empty(2 * (n + tiles), dtype=torch.int32, device=dev)
+        with _on(dev):
+            check(_lib.splat_band_table(sTod_lin.data_ptr(), sTod_tr.data_ptr(), nnzs.data_ptr(), n, stride,
+                                        table.data_ptr(), _stream(dev)), "splat_band_table")
+            torch.cuda.current_stream(dev).synchronize()      # any stream may use it
     # keep the two companions alive with the cache entry so their ids cannot be reused
-    nnzs._splat_plan = (key, host, sTod_lin, sTod_tr)
+    nnzs._splat_plan = (key, host, sTod_lin, sTod_tr, table)
     return host
+
+
+def _band_table(sTod_lin, sTod_tr, nnzs):
+    """Address of the band table remembered by classify(), or None if the metadata has changed since."""
+    hit = getattr(nnzs, "_splat_plan", None)
+    if hit is None or hit[4] is None or hit[0] != (id(sTod_lin), id(sTod_tr), sTod_lin._version, sTod_tr._version,
+                                                   nnzs._version, nnzs.numel()):
+        return None
+    return hit[4].data_ptr()
 
 
 _STATUS_WORDS: dict = {}
@@ -459,13 +480,14 @@ def attention_fused(q, kt, v, output, sTod_lin, sTod_tr, nnzs, scale: float = 1.
     ran = ctypes.c_int32(0)
     _debug_before(dev)
     with _on(dev):
-        check(_lib.splat_attention_fused_lse(
+        check(_lib.splat_attention_fused_table(
             q.data_ptr(), kt.data_ptr(), ksb, ksc, ksk, v.data_ptr(), output.data_ptr(),
             lse.data_ptr() if lse is not None and lse.numel() > 0 else None,
             _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
             _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, float(scale), dtype_code(q.dtype),
             int(path), ctypes.cast(plan_arr, _vp) if plan_arr is not None else None,
-            sw.data_ptr(), ctypes.byref(ran), _stream(dev)), "splat_attention_fused_lse")
+            _band_table(sTod_lin, sTod_tr, nnzs), sw.data_ptr(), ctypes.byref(ran), _stream(dev)),
+            "splat_attention_fused_table")
     if ran.value != PATH_BAND and q.dtype != torch.float32 and q.numel() > 0 and path == PATH_AUTO:
         _warn_cuda_core_16bit("attention")
     if os.environ.get("SPLAT_B200_DEBUG"):
@@ -479,5 +501,5 @@ def module_forward(attributes: dict, x):
 
 
 _host.bind(*(ctypes.cast(getattr(_lib, name), _vp).value for name in (
-    "splat_attention_fused_lse", "splat_sddmm_band", "splat_spmm_band", "splat_sddmm_tile", "splat_spmm_tile",
+    "splat_attention_fused_table", "splat_sddmm_band", "splat_spmm_band", "splat_sddmm_tile", "splat_spmm_tile",
     "splat_softmax")), _warn_cuda_core_16bit)

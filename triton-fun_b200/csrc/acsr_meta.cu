@@ -247,9 +247,55 @@ __global__ void classify_kernel(const float* __restrict__ sTod_lin,
     }
 }
 
+// Band table of a pattern whose rows are bands after regrouping by residue class (attention_band.cu): int2 per
+// row, classes one after the other and a class's rows in order, then int2 per class and 128-row tile.
+//   row   (begin, end) of the band in class coordinates; (column, -1) for a single non-zero, (0, INT_MIN / 2)
+//         for none
+//   tile  key range of its rows' bands, (0, 0) if there are none; ceil(ceil(L / stride) / 128) per class
+// One CTA per tile.
+__global__ void __launch_bounds__(128)
+band_table_kernel(const float* __restrict__ lin, const float* __restrict__ tr, const float* __restrict__ nnzs,
+                  int n_rows, int stride, int tile_pitch, int2* __restrict__ table) {
+    const int res = blockIdx.x / tile_pitch, tile = blockIdx.x % tile_pitch;
+    const int rows = (n_rows - res + stride - 1) / stride;
+    const int u = tile * 128 + threadIdx.x;
+    int2 band = make_int2(0, INT_MIN / 2);
+    if (u < rows) {
+        const RowAffine ra = row_affine(lin, tr, nnzs, (int64_t)u * stride + res);
+        if (ra.nnz > 1) {
+            band.x = (ra.start - res) / stride;
+            band.y = band.x + ra.nnz;
+        } else if (ra.nnz == 1) {
+            band = make_int2(ra.start, -1);
+        }
+        const int shorter = n_rows / stride, longer = n_rows % stride;     // classes below `longer` have one row more
+        table[(int64_t)res * shorter + min(res, longer) + u] = band;
+    }
+    __shared__ int s_lo[4], s_hi[4];
+    const int lo = warp_min_i(band.y > 0 ? band.x : INT_MAX), hi = warp_max_i(max(band.y, 0));
+    if ((threadIdx.x & 31) == 0) { s_lo[threadIdx.x >> 5] = lo; s_hi[threadIdx.x >> 5] = hi; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int l = min(min(s_lo[0], s_lo[1]), min(s_lo[2], s_lo[3]));
+        const int h = min(max(max(s_hi[0], s_hi[1]), max(s_hi[2], s_hi[3])), rows);
+        table[(int64_t)n_rows + blockIdx.x] = h > 0 ? make_int2(l, h) : make_int2(0, 0);
+    }
+}
+
 }  // namespace splat
 
 using namespace splat;
+
+extern "C" int32_t splat_band_table(const float* sTod_lin, const float* sTod_tr, const float* nnzs, int64_t n_rows,
+                                    int64_t stride, int32_t* table, void* stream) {
+    if (!sTod_lin || !sTod_tr || !nnzs || !table || n_rows < 1 || stride < 1) return SPLAT_ERR_BAD_ARG;
+    if (n_rows > INT_MAX || stride > 65535) return SPLAT_ERR_UNSUPPORTED_SHAPE;
+    if ((reinterpret_cast<uintptr_t>(table) & 7u) != 0) return SPLAT_ERR_MISALIGNED;
+    const int64_t pitch = ((n_rows + stride - 1) / stride + 127) / 128;
+    band_table_kernel<<<(unsigned)(pitch * stride), 128, 0, (cudaStream_t)stream>>>(
+        sTod_lin, sTod_tr, nnzs, (int)n_rows, (int)stride, (int)pitch, reinterpret_cast<int2*>(table));
+    return launch_status();
+}
 
 extern "C" int32_t splat_mask_row_summary_u8(const uint8_t* mask, int64_t n_rows, int64_t n_cols,
                                              int64_t ld, int32_t* rows_i32, void* stream) {

@@ -57,7 +57,7 @@ namespace band {
 bool make_map(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_rows,
               int64_t d, int64_t stride, int box_rows);
 bool make_map_kt(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_cols,
-                 int64_t d);
+                 int64_t d, int64_t box_d);
 }
 
 namespace pair {
@@ -958,7 +958,7 @@ int32_t attention_pair(const void* q, const void* k, int kt_major, const void* v
         return SPLAT_ERR_UNSUPPORTED_SHAPE;
     CUtensorMap mq, mk, mv, mo;
     if (!band::make_map(&mq, q, dtype, bh, n_rows, d, stride, pair::kTile) ||
-        !(kt_major ? band::make_map_kt(&mk, k, dtype, bh, n_rows, d)
+        !(kt_major ? band::make_map_kt(&mk, k, dtype, bh, n_rows, d, d)
                    : band::make_map(&mk, k, dtype, bh, n_rows, d, stride, 64)) ||
         !band::make_map(&mv, v, dtype, bh, n_rows, d, stride, pair::kTile) ||
         !band::make_map(&mo, o, dtype, bh, n_rows, d, stride, pair::kTile))

@@ -1,0 +1,583 @@
+// Fused band attention, one 128-row Q tile per CTA, two CTAs per SM.  Problem, regrouping by residue class and
+// operand layouts: see attention_band.cu.  The default for every band pattern of 16-bit operands.
+//
+// A step is 128 keys:
+//     S(j)  = Q K(j)^T       tcgen05.mma 128x128x16, operands in shared memory
+//     P(j)  = exp2(S c - m)  thread = row = tensor-memory lane: its 128 scores in registers
+//     O    += P(j) V(j)      tcgen05.mma 128xDx16, A = P from tensor memory, in two halves of 64 keys
+// What this replaced was a kernel with 64-key steps and two score buffers.  Its N = 64 QK MMAs read the whole
+// Q tile from shared memory for every 64 keys and run at 0.64 of the tensor rate, and a softmax step paid its
+// fixed costs (barrier wait, tensor-memory round trip, maximum chain, arrival: more than half of 1 700
+// cycles) per 64 keys.  With 128-key steps a tile has ONE score buffer, so its softmax and its MMAs take
+// turns; the other CTA of the SM, which is in no way synchronised with this one, fills the gaps.
+//   * P of keys 0-63 goes to the tensor core while keys 64-127 are still being exponentiated.
+//   * D = 128: S(128) + O(128) fill the CTA's 256 tensor-memory columns; P(j) (16 bit, two keys per column)
+//     overwrites columns 0-63 of the consumed scores, and S(j+1) follows PV(j).
+//     D = 64: P has columns of its own, and S(j+1) is computed while P(j) is.
+//   * Half steps outside the bands of a warp's rows are not exponentiated, those outside the tile's bands
+//     not multiplied.
+//   * The tile's key range comes from the band table, which the caller's plan keeps (acsr_meta.cu), so that Q,
+//     K and V are on their way some 500 cycles after the start.  Finding it from the row metadata first
+//     (gathers, a division per row, a reduction over the block) cost 1 500 cycles of a CTA's 15 000 to
+//     30 000 at stride 1 and 3 800 at stride 64; it remains for callers without a table.
+//   * Any d that is a multiple of 8 up to 128 runs: the copies fill a tile's columns past d with zeros, and
+//     the store clips them.  Any L: classes of unequal length are two launches.
+// Softmax step of 128 keys by itself (no MMAs, cycles for one / two warps per scheduler): row in registers
+// 1468 / 2262, four chunks with the maximum looked at per chunk 1655 / 2403, a quarter of the exponentials
+// by polynomial on the FMA pipe 1414 / 2002; 64-key steps 2 x 900 / 2 x 1140.  In the kernel the chunked
+// form is 10 to 15 % slower and the polynomial changes nothing: the special function unit is busy 40 % of
+// the time; what a CTA waits for is its own chain softmax -> PV -> QK -> softmax.
+#include <limits.h>
+#include <type_traits>
+
+#include "common.cuh"
+#include "softmax_math.cuh"
+#include "tc_ptx.cuh"
+
+namespace splat {
+namespace band {
+
+using namespace tc;
+
+// defined in attention_band.cu
+bool allow_dynamic_smem(const void* kernel, int bytes);
+bool make_map_view(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_rows, int64_t d, int64_t stride,
+                   int64_t res0, int64_t count, int64_t rows, int box_rows);
+bool make_map_kt(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_cols, int64_t d, int64_t box_d);
+
+namespace wide {
+
+using sm::add2;
+using sm::ex2;
+using sm::fma2;
+using sm::fmax3;
+using sm::pack2;
+
+constexpr int kTile = 128;               // rows of a Q tile, keys of a step
+constexpr int kChunk = 32;               // columns of a tensor-memory load
+constexpr int kChunks = kTile / kChunk;
+constexpr int kSubBytes = kTile * 128;   // one 64-element (128-byte) column chunk of a tile
+constexpr int kTmaWarp = 4;
+constexpr int kMmaWarp = 5;
+constexpr int kThreads = 192;            // warps 0-3 softmax and epilogue, 4 TMA, 5 MMA issuer and tensor-memory owner
+constexpr int kTmemCols = 256;
+constexpr float kRescaleThreshold = 8.0f;   // log2 domain: P stays below 2^8 between rescales
+
+// status-word codes (which wait gave up)
+enum : int { kErrQ = 41, kErrKFull = 42, kErrKFree = 43, kErrVFull = 44, kErrVFree = 45, kErrS = 46, kErrP = 47, kErrO = 48,
+             kErrSFree = 50, kErrPv = 51 };
+
+struct Params {
+    const float* lin;
+    const float* tr;
+    const float* nnzs;
+    const void* q;     // raw operands: rows with one non-zero are handled through them
+    const void* k;
+    const void* v;
+    const int2* rows;  // band table (see acsr_meta.cu): rows in class order, tiles' key ranges; or null
+    const int2* tiles;
+    float* lse;        // (BH, L) or null
+    int32_t* status;
+    int32_t* mirror;   // host copy of the status word, or null
+    int64_t n_rows;    // L
+    int rows_v;        // rows of a class
+    int stride;
+    int res0;          // residue of this launch's first class
+    int row0;          // of which class in the band table
+    int tile0;
+    int tile_pitch;    // tiles of a class in the band table
+    int d;             // real head dimension, <= D and a multiple of 8 (the rest of a tile is zero)
+    int kt_major;
+    float scale_log2;
+};
+
+struct Control {
+    uint64_t q_full, o_full, drain;
+    uint64_t k_full[2], k_free[2], v_full[2], v_free[2];
+    uint64_t s_full;           // MMA -> softmax: scores ready (D = 128: and every earlier PV complete)
+    uint64_t p_full[2];        // softmax -> MMA: probabilities of keys 0-63 / 64-127 stored (4 warp arrivals)
+    uint64_t s_free, pv_done;  // D = 64.  softmax -> MMA: scores read (4 warp arrivals); MMA -> softmax: PV complete
+    uint32_t tmem_base;
+    int32_t abort_at_entry;
+    int32_t lo[4], hi[4];      // key range of the rows' bands: of the tile (table), or per softmax warp
+};
+
+template <int D> struct Layout {
+    static constexpr int kSub = D / 64;
+    static constexpr int kTileBytes = kSub * kSubBytes;
+    static constexpr int kSlots = D == 128 ? 1 : 2;         // K tiles, and V tiles, in shared memory
+    static constexpr int kKOff = kTileBytes;                // behind the Q tile
+    static constexpr int kVOff = kKOff + kSlots * kTileBytes;
+    static constexpr int kCtrlOff = kVOff + kSlots * kTileBytes;
+    static constexpr int kSmemBytes = kCtrlOff + (int)sizeof(Control) + 1024;   // + alignment slack
+};
+
+__device__ __forceinline__ void wait_quiet(uint64_t* bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait(bar, parity))
+        if (clock64() - t0 > 200000000LL) break;
+}
+
+// Bounded wait with nothing but a counter to keep in registers: gives up after 2^22 suspended tries (seconds),
+// or when another CTA has.
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int32_t* status, int code) {
+    if (mbar_test_wait(bar, parity)) return true;
+    uint32_t polls = 0;
+    while (!mbar_try_wait(bar, parity)) {
+        if ((++polls & 0x3ffu) == 0) {
+            if (*(volatile int32_t*)status != 0) return false;
+            if (polls >= (1u << 22)) {
+                atomicCAS(status, 0, code);
+                return false;
+            }
+        }
+    }
+    return true;
+}
+
+// O of the warp's rows (n pieces of 16 columns) times corr.  Rare, and kept out of the main loop.
+__device__ __noinline__ void rescale_o(uint32_t o_addr, int n, float corr) {
+    uint32_t v[16];
+    for (int i = 0; i < n; ++i) {
+        tmem_ld16(o_addr + i * 16, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
+        tmem_st16(o_addr + i * 16, v);
+    }
+    tmem_st_wait();
+}
+
+template <typename T, int D, bool kLse>
+__global__ void __launch_bounds__(kThreads, 2)
+attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Params p) {
+    using L = Layout<D>;
+    constexpr int kSlots = L::kSlots;
+    constexpr bool kOwnP = D == 64;              // P has tensor-memory columns of its own
+    constexpr uint32_t kPCol = kOwnP ? kTile + D : 0;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    Control* ctrl = reinterpret_cast<Control*>(smem + L::kCtrlOff);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int res = blockIdx.y;
+    const int64_t bh = blockIdx.z;
+    const int u0 = blockIdx.x * kTile;
+    const int real_res = res + p.res0;
+
+    // Prologue, one block-wide barrier: tensor-memory allocation, row metadata and the first copies proceed
+    // side by side.
+    int jk = 0, jv = 0;                // TMA warp: K and V tiles requested
+    int klo = 0;                       // first 128-key step
+    auto load_k = [&]() {
+        const int st = jk % kSlots, row = (klo + jk) * kTile;
+        if (jk >= kSlots && !wait_bar(&ctrl->k_free[st], ((uint32_t)(jk / kSlots) & 1u) ^ 1u, p.status, kErrKFree)) return false;
+        mbar_arrive_expect_tx(&ctrl->k_full[st], L::kTileBytes);
+        uint8_t* dst = smem + L::kKOff + st * L::kTileBytes;
+        if (p.kt_major) {
+            for (int ch = 0; ch < kTile / 64; ++ch)       // 64-key chunks of [d][64 keys]
+                tma_load_4d(dst + ch * (D * 128), &tm_k, &ctrl->k_full[st], row + ch * 64, 0, (int)bh, 0);
+        } else {
+            for (int sub = 0; sub < L::kSub; ++sub)
+                tma_load_4d(dst + sub * kSubBytes, &tm_k, &ctrl->k_full[st], sub * 64, res, row, (int)bh);
+        }
+        ++jk;
+        return true;
+    };
+    auto load_v = [&]() {
+        const int st = jv % kSlots;
+        if (jv >= kSlots && !wait_bar(&ctrl->v_free[st], ((uint32_t)(jv / kSlots) & 1u) ^ 1u, p.status, kErrVFree)) return false;
+        mbar_arrive_expect_tx(&ctrl->v_full[st], L::kTileBytes);
+        for (int sub = 0; sub < L::kSub; ++sub)
+            tma_load_4d(smem + L::kVOff + st * L::kTileBytes + sub * kSubBytes, &tm_v, &ctrl->v_full[st], sub * 64, res,
+                        (klo + jv) * kTile, (int)bh);
+        ++jv;
+        return true;
+    };
+    // Band [begin, end) of this thread's row in class coordinates; end = kSingle for a row with one non-zero
+    // (begin = its column), kEmpty for one without and past the end of the class.
+    constexpr int kSingle = -1, kEmpty = INT_MIN / 2;
+    int my_begin = 0, my_end = kEmpty;
+    if (warp == kMmaWarp) {
+        tmem_alloc(&ctrl->tmem_base, kTmemCols);
+        tmem_relinquish();
+    } else if (warp == kTmaWarp) {
+        if (lane == 0) {
+            tma_prefetch_desc(&tm_q);
+            tma_prefetch_desc(&tm_k);
+            tma_prefetch_desc(&tm_v);
+            mbar_init(&ctrl->q_full, 1);
+            mbar_init(&ctrl->o_full, 1);
+            mbar_init(&ctrl->drain, 1);
+            mbar_init(&ctrl->s_full, 1);
+            mbar_init(&ctrl->s_free, 4);
+            mbar_init(&ctrl->pv_done, 1);
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(&ctrl->k_full[i], 1);
+                mbar_init(&ctrl->k_free[i], 1);
+                mbar_init(&ctrl->v_full[i], 1);
+                mbar_init(&ctrl->v_free[i], 1);
+                mbar_init(&ctrl->p_full[i], 4);      // one arrival per softmax warp
+            }
+            mbar_fence_init();
+            int2 range = make_int2(0, 0);
+            if (p.tiles != nullptr) range = __ldg(p.tiles + p.tile0 + res * p.tile_pitch + blockIdx.x);
+            const int32_t stop = entry_status(p.status, p.mirror);
+            ctrl->abort_at_entry = stop;
+            if (stop == 0) {
+                mbar_arrive_expect_tx(&ctrl->q_full, L::kTileBytes);
+                for (int sub = 0; sub < L::kSub; ++sub)
+                    tma_load_4d(smem + sub * kSubBytes, &tm_q, &ctrl->q_full, sub * 64, res, u0, (int)bh);
+                if (range.y > 0) {
+                    klo = range.x / kTile;
+                    load_k();
+                    load_v();
+                }
+            }
+            if (p.tiles != nullptr)
+                for (int w = 0; w < 4; ++w) { ctrl->lo[w] = range.x; ctrl->hi[w] = range.y; }
+        }
+    } else {
+        const int u = u0 + warp * 32 + lane;
+        if (u < p.rows_v) {
+            if (p.rows != nullptr) {
+                const int2 band = __ldg(p.rows + p.row0 + res * p.rows_v + u);
+                my_begin = band.x;
+                my_end = band.y;
+            } else {
+                const RowAffine ra = row_affine(p.lin, p.tr, p.nnzs, (int64_t)u * p.stride + real_res);
+                if (ra.nnz > 1) {
+                    my_begin = p.stride == 1 ? ra.start : (ra.start - real_res) / p.stride;
+                    my_end = my_begin + ra.nnz;
+                } else if (ra.nnz == 1) {
+                    my_begin = ra.start;
+                    my_end = kSingle;
+                }
+            }
+            if (my_end == kSingle) {   // its row of V is copied at the end
+                const char* vrow = reinterpret_cast<const char*>(p.v) + (bh * p.n_rows + my_begin) * p.d * 2;
+                for (int i = 0; i < p.d * 2; i += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(vrow + i));
+            }
+        }
+        if (p.rows == nullptr) {
+            const int lo = warp_min_i(my_end > 0 ? my_begin : INT_MAX), hi = warp_max_i(max(my_end, 0));
+            if (lane == 0) { ctrl->lo[warp] = lo; ctrl->hi[warp] = hi; }
+        }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = ctrl->tmem_base;
+    if (ctrl->abort_at_entry != 0) {   // an earlier launch gave up
+        if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
+        return;
+    }
+    int lo64 = INT_MAX, hi64 = 0;
+    for (int w = 0; w < 4; ++w) { lo64 = min(lo64, ctrl->lo[w]); hi64 = max(hi64, ctrl->hi[w]); }
+    hi64 = min(hi64, p.rows_v);
+    if (hi64 <= 0) lo64 = 0;
+    lo64 = lo64 / 64;          // in 64-key units from here
+    hi64 = (hi64 + 63) / 64;
+    klo = lo64 >> 1;
+    const int steps = ((hi64 + 1) >> 1) - klo;   // 128-key steps
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, int code) {
+        const bool r = wait_bar(bar, parity, p.status, code);
+        return __all_sync(0xffffffffu, r) != 0;
+    };
+
+    if (warp == kTmaWarp) {
+        // ------------------------------------------------------------------ TMA producer
+        if (lane == 0) {
+            bool ok = true;
+            while (ok && jv < steps) {     // K(0) V(0) K(1) V(1) ...: the order in which the slots come free
+                if (jk <= jv) ok = load_k();
+                if (ok) ok = load_v();
+            }
+            if (!ok) {                     // leave only after the copies already issued have landed
+                wait_quiet(&ctrl->q_full, 0);
+                for (int i = max(0, jk - kSlots); i < jk; ++i) wait_quiet(&ctrl->k_full[i % kSlots], (uint32_t)(i / kSlots) & 1u);
+                for (int i = max(0, jv - kSlots); i < jv; ++i) wait_quiet(&ctrl->v_full[i % kSlots], (uint32_t)(i / kSlots) & 1u);
+            }
+        }
+    } else if (warp == kMmaWarp) {
+        // ------------------------------------------------------------------ MMA issuer
+        // (whole warp on warp-uniform values, one elected lane issues)
+        if (steps > 0) {
+            const bool lead = elect_one();
+            constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+            const uint32_t idesc_qk = instr_desc_f16(fmt, kTile, kTile, p.kt_major ? 1u : 0u);
+            const uint32_t idesc_qk_half = instr_desc_f16(fmt, kTile, 64, p.kt_major ? 1u : 0u);
+            constexpr uint32_t idesc_pv = instr_desc_f16(fmt, kTile, D, 1);
+            const uint32_t q_base = smem_u32(smem), k_base = smem_u32(smem + L::kKOff), v_base = smem_u32(smem + L::kVOff);
+            const uint32_t o_tmem = tmem_base + kTile;
+            auto commit = [&](uint64_t* bar) { if (lead) mma_commit(bar); };
+            auto in_range = [&](int j, int half) { const int i = 2 * (klo + j) + half; return i >= lo64 && i < hi64; };
+            bool ok = wait_all(&ctrl->q_full, 0, kErrQ);
+            bool first_pv = true;
+            auto issue_s = [&](int j) {                // S(j); half steps outside the range are left out
+                const int st = j % kSlots;
+                ok = wait_all(&ctrl->k_full[st], (uint32_t)(j / kSlots) & 1u, kErrKFull);
+                if (!ok) return;
+                tc_fence_after_sync();
+                const bool h0 = in_range(j, 0), both = h0 && in_range(j, 1);
+                const uint32_t idesc = both ? idesc_qk : idesc_qk_half;
+                const uint32_t skip = h0 ? 0u : 1u;
+                const uint32_t b_base = k_base + st * L::kTileBytes + skip * (p.kt_major ? D * 128 : 64 * 128);
+#pragma unroll
+                for (int kk = 0; kk < D / 16; ++kk) {
+                    const uint32_t off = (kk >> 2) * kSubBytes + (kk & 3) * 32;
+                    const uint64_t da = smem_desc_sw128(q_base + off, 16, 1024);
+                    const uint64_t db = p.kt_major ? smem_desc_sw128(b_base + kk * 2048, D * 128, 1024)
+                                                   : smem_desc_sw128(b_base + off, 16, 1024);
+                    if (lead) mma_ss(tmem_base + skip * 64, da, db, idesc, kk > 0);
+                }
+                commit(&ctrl->s_full);
+                commit(&ctrl->k_free[st]);
+            };
+            if (ok) issue_s(0);
+            for (int j = 0; j < steps && ok; ++j) {
+                if (kOwnP && j + 1 < steps) {          // the next scores as soon as these have been read
+                    ok = wait_all(&ctrl->s_free, (uint32_t)j & 1u, kErrSFree);
+                    if (ok) issue_s(j + 1);
+                    if (!ok) break;
+                }
+                const int st = j % kSlots;
+                ok = wait_all(&ctrl->v_full[st], (uint32_t)(j / kSlots) & 1u, kErrVFull);
+                if (!ok) break;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    ok = wait_all(&ctrl->p_full[half], (uint32_t)j & 1u, kErrP);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    if (in_range(j, half)) {
+#pragma unroll
+                        for (int kk = half * 4; kk < half * 4 + 4; ++kk) {
+                            const uint64_t db = smem_desc_sw128(v_base + st * L::kTileBytes + kk * 2048, kSubBytes, 1024);
+                            if (lead) mma_ts(o_tmem, tmem_base + kPCol + kk * 8, db, idesc_pv, (!first_pv || (kk & 3) > 0) ? 1u : 0u);
+                        }
+                        first_pv = false;
+                    }
+                }
+                if (!ok) break;
+                commit(j + 1 < steps ? &ctrl->v_free[st] : &ctrl->o_full);
+                if (kOwnP) commit(&ctrl->pv_done);
+                else if (j + 1 < steps) issue_s(j + 1);
+            }
+            // tensor memory is released only after every MMA has completed
+            commit(&ctrl->drain);
+            wait_quiet(&ctrl->drain, 0);
+            __syncwarp();
+        }
+    } else {
+        // ------------------------------------------------------------------ softmax + epilogue
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
+        const uint32_t s_addr = lane_addr, o_addr = lane_addr + kTile, p_addr = lane_addr + kPCol;
+        const float sc = p.scale_log2;
+        const float2 sc2 = make_float2(sc, sc);
+        float m_used = -INFINITY, l_sum = 0.f;
+        bool ok = true;
+        for (int k = 0; k < steps; ++k) {
+            ok = wait_all(&ctrl->s_full, (uint32_t)k & 1u, kErrS);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const int c0 = (klo + k) * kTile;
+            const int v_lo = my_begin - c0, v_hi = my_end - c0;  // valid keys of this step: [v_lo, v_hi)
+            // D = 64: before the first store of P or a rescale of O, PV(k-1) has to be complete (it usually is)
+            auto pv_wait = [&]() {
+                if (!kOwnP || k == 0) return true;
+                const bool r = wait_all(&ctrl->pv_done, (uint32_t)(k - 1) & 1u, kErrPv);
+                tc_fence_after_sync();
+                return r;
+            };
+            auto scores_read = [&]() {
+                if (!kOwnP) return;
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ctrl->s_free);
+            };
+            uint32_t r[kTile];
+#pragma unroll
+            for (int ch = 0; ch < kChunks; ++ch) tmem_ld32(s_addr + ch * kChunk, r + ch * kChunk);
+            tmem_ld_wait();
+            scores_read();
+            if (!__all_sync(0xffffffffu, v_lo <= 0 && v_hi >= kTile)) {
+                // band edge: keys outside [v_lo, v_hi) become -inf (exp2 -> 0)
+#pragma unroll
+                for (int ch = 0; ch < kChunks; ++ch) {
+                    const int lo = min(max(v_lo - ch * kChunk, 0), kChunk), hi = min(max(v_hi - ch * kChunk, 0), kChunk);
+                    const uint32_t valid = (hi >= 32 ? ~0u : (1u << hi) - 1) & ~(lo >= 32 ? ~0u : (1u << lo) - 1);
+#pragma unroll
+                    for (int j = 0; j < kChunk; ++j) r[ch * kChunk + j] = (valid & (1u << j)) ? r[ch * kChunk + j] : 0xff800000u;
+                }
+            }
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int j = 0; j < kTile; j += 8)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    mx[i] = fmax3(mx[i], __uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
+            const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc);
+            // lazy rescale: only when a row's maximum has grown by more than 2^8 (false when both are -inf)
+            const bool need = (m_new - m_used) > kRescaleThreshold;
+            if (__any_sync(0xffffffffu, need)) {
+                ok = pv_wait();
+                if (!ok) break;
+                const float corr = need ? ex2(m_used - m_new) : 1.f;
+                if (need) m_used = m_new;
+                l_sum *= corr;
+                if (k > 0) rescale_o(o_addr, D / 16, corr);
+            }
+            const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
+            const float2 nm2 = make_float2(-m_eff, -m_eff);
+            float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t* c = r + half * (kTile / 2);
+                uint32_t* pk = r + half * (kTile / 4);
+#pragma unroll
+                for (int j = 0; j < kTile / 2; j += 4) {
+                    float2 a0 = fma2(make_float2(__uint_as_float(c[j]), __uint_as_float(c[j + 1])), sc2, nm2);
+                    float2 a1 = fma2(make_float2(__uint_as_float(c[j + 2]), __uint_as_float(c[j + 3])), sc2, nm2);
+                    a0.x = ex2(a0.x); a0.y = ex2(a0.y); a1.x = ex2(a1.x); a1.y = ex2(a1.y);
+                    acc0 = add2(acc0, a0);
+                    acc1 = add2(acc1, a1);
+                    pk[j >> 1] = pack2<T>(a0.x, a0.y);
+                    pk[(j >> 1) + 1] = pack2<T>(a1.x, a1.y);
+                }
+                if (kOwnP && half == 0) ok = pv_wait();
+                tmem_st32(p_addr + half * 32, pk);
+                tmem_st_wait();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ctrl->p_full[half]);      // half 0: on its way to the tensor core
+            }
+            l_sum += (acc0.x + acc0.y) + (acc1.x + acc1.y);
+            if (!ok) break;
+        }
+        const bool have_o = ok && steps > 0;
+        if (have_o) {
+            ok = wait_all(&ctrl->o_full, 0, kErrO);
+            tc_fence_after_sync();
+        } else if (ok) {
+            ok = wait_all(&ctrl->q_full, 0, kErrQ);   // nothing to multiply; the copy of Q has to have landed all the same
+        }
+        // epilogue: O / l for band rows, V[start] for single-element rows, zero otherwise.  Rows are staged in
+        // the Q tile's memory (every MMA has completed) in the 128-byte-swizzled tile layout and leave
+        // through one tiled TMA store per 64 columns and warp (rows and columns past the end are clipped).
+        const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
+        const int64_t head = bh * p.n_rows;
+        const int u = u0 + warp * 32 + lane;
+        const int64_t row_real = u < p.rows_v ? (int64_t)u * p.stride + real_res : -1;
+        const int row_nnz = my_end > 0 ? 2 : (my_end == kSingle ? 1 : 0), row_start = my_begin;
+        if (kLse && row_real >= 0 && ok) {
+            float e = -INFINITY;
+            if (row_nnz > 1) {
+                e = lse_from_log2(m_used, l_sum);
+            } else if (row_nnz == 1) {
+                const T* qr = reinterpret_cast<const T*>(p.q) + (head + row_real) * p.d;
+                const T* kb = reinterpret_cast<const T*>(p.k);
+                const float s = p.kt_major ? dot_strided<T>(qr, kb + head * p.d + row_start, p.n_rows, p.d)
+                                           : dot_strided<T>(qr, kb + (head + row_start) * p.d, 1, p.d);
+                e = s * p.scale_log2 * kLn2;
+            }
+            p.lse[head + row_real] = e;
+        }
+        const T* vrow = reinterpret_cast<const T*>(p.v) + (head + row_start) * p.d;
+        const int t = warp * 32 + lane;
+        uint32_t o_raw[D];
+        if (have_o && ok) {
+#pragma unroll
+            for (int ch = 0; ch < D / 32; ++ch) tmem_ld32(o_addr + ch * 32, o_raw + ch * 32);
+            tmem_ld_wait();
+        }
+#pragma unroll
+        for (int ch = 0; ch < D / 32; ++ch) {
+            const uint32_t* r = o_raw + ch * 32;
+            uint4 out[4];
+            uint32_t* o32 = reinterpret_cast<uint32_t*>(out);
+            if (row_nnz > 1 && have_o && ok) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 2)
+                    o32[j >> 1] = pack2<T>(__uint_as_float(r[j]) * inv, __uint_as_float(r[j + 1]) * inv);
+            } else if (row_nnz == 1) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    out[i] = ch * 32 + i * 8 < p.d ? *reinterpret_cast<const uint4*>(vrow + ch * 32 + i * 8) : make_uint4(0, 0, 0, 0);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) out[i] = make_uint4(0, 0, 0, 0);
+            }
+            uint8_t* srow = smem + (ch >> 1) * kSubBytes + t * 128;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<uint4*>(srow + ((((ch & 1) * 4 + i) ^ (t & 7)) << 4)) = out[i];
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && u0 + warp * 32 < p.rows_v) {
+            for (int sub = 0; sub < L::kSub; ++sub)
+                tma_store_4d(&tm_o, smem + sub * kSubBytes + warp * 32 * 128, sub * 64, res, u0 + warp * 32, (int)bh);
+            tma_store_commit();
+            tma_store_wait_read();
+        }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        __syncwarp();
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, kTmemCols);
+    }
+}
+
+template <typename T, int D>
+static int32_t launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
+                      const Params& prm, int64_t bh, int64_t classes, cudaStream_t st) {
+    auto kern = prm.lse != nullptr ? attention_wide_kernel<T, D, true> : attention_wide_kernel<T, D, false>;
+    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), Layout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
+    const dim3 grid((unsigned)((prm.rows_v + kTile - 1) / kTile), (unsigned)classes, (unsigned)bh);
+    kern<<<grid, kThreads, Layout<D>::kSmemBytes, st>>>(mq, mk, mv, mo, prm);
+    return launch_status();
+}
+
+}  // namespace wide
+}  // namespace band
+
+// Operands checked by attention_band().  Residue classes of one length share a launch: one when the stride
+// divides L, else one for the L mod stride longer classes and one for the rest.
+int32_t attention_wide(const void* q, const void* k, int kt_major, const void* v, void* o, const float* lin, const float* tr,
+                       const float* nnzs, int64_t bh, int64_t n_rows, int64_t d, int64_t stride, float scale, int32_t dtype,
+                       int32_t* status_word, const int32_t* band_table, float* lse, cudaStream_t st) {
+    using namespace band;
+    wide::Params p;
+    p.lin = lin; p.tr = tr; p.nnzs = nnzs; p.q = q; p.k = k; p.v = v; p.lse = lse;
+    p.status = status_word; p.mirror = status_mirror(status_word);
+    p.n_rows = n_rows; p.stride = (int)stride; p.d = (int)d;
+    p.kt_major = kt_major; p.scale_log2 = scale * kLog2e;
+    const int64_t longer = n_rows % stride;
+    p.tile_pitch = (int)(((n_rows + stride - 1) / stride + wide::kTile - 1) / wide::kTile);
+    p.rows = reinterpret_cast<const int2*>(band_table);
+    p.tiles = band_table != nullptr ? p.rows + n_rows : nullptr;
+    for (int part = 0; part < 2; ++part) {
+        const int64_t res0 = part == 0 ? 0 : longer, count = part == 0 ? longer : stride - longer;
+        const int64_t rows = n_rows / stride + (part == 0 ? 1 : 0);
+        if (count == 0 || rows == 0) continue;
+        CUtensorMap mq, mk, mv, mo;
+        if (!make_map_view(&mq, q, dtype, bh, n_rows, d, stride, res0, count, rows, wide::kTile) ||
+            !(kt_major ? make_map_kt(&mk, k, dtype, bh, n_rows, d, d > 64 ? 128 : 64)
+                       : make_map_view(&mk, k, dtype, bh, n_rows, d, stride, res0, count, rows, wide::kTile)) ||
+            !make_map_view(&mv, v, dtype, bh, n_rows, d, stride, res0, count, rows, wide::kTile) ||
+            !make_map_view(&mo, o, dtype, bh, n_rows, d, stride, res0, count, rows, 32))
+            return SPLAT_ERR_DRIVER;
+        p.rows_v = (int)rows; p.res0 = (int)res0;
+        p.row0 = (int)(part == 0 ? 0 : longer * (rows + 1));
+        p.tile0 = (int)res0 * p.tile_pitch;
+        const int32_t rc = dtype == SPLAT_BF16
+            ? (d > 64 ? wide::launch<__nv_bfloat16, 128>(mq, mk, mv, mo, p, bh, count, st) : wide::launch<__nv_bfloat16, 64>(mq, mk, mv, mo, p, bh, count, st))
+            : (d > 64 ? wide::launch<__half, 128>(mq, mk, mv, mo, p, bh, count, st) : wide::launch<__half, 64>(mq, mk, mv, mo, p, bh, count, st));
+        if (rc != SPLAT_OK) return rc;
+    }
+    return SPLAT_OK;
+}
+
+}  // namespace splat

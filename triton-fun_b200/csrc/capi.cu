@@ -20,7 +20,7 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
                        const void* v, void* o, const float* lin, const float* tr,
                        const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
                        float scale, int32_t dtype, const int32_t* plan, int32_t* status_word,
-                       float* lse, cudaStream_t st);
+                       const int32_t* band_table, float* lse, cudaStream_t st);
 }  // namespace splat
 
 namespace splat {
@@ -90,13 +90,14 @@ extern "C" const char* splat_status_string(int32_t status) {
     }
 }
 
-extern "C" int32_t splat_attention_fused_lse(const void* q, const void* k, int64_t k_stride_bh,
-                                             int64_t k_stride_col, int64_t k_stride_k, const void* v,
-                                             void* o, float* lse, const float* sTod_lin,
-                                             const float* sTod_tr, const float* nnzs, int64_t bh,
-                                             int64_t n_rows, int64_t n_cols, int64_t d, float scale,
-                                             int32_t dtype, int32_t path, const int32_t* plan_i32,
-                                             int32_t* status_word, int32_t* path_ran, void* stream) {
+extern "C" int32_t splat_attention_fused_table(const void* q, const void* k, int64_t k_stride_bh,
+                                               int64_t k_stride_col, int64_t k_stride_k, const void* v,
+                                               void* o, float* lse, const float* sTod_lin,
+                                               const float* sTod_tr, const float* nnzs, int64_t bh,
+                                               int64_t n_rows, int64_t n_cols, int64_t d, float scale,
+                                               int32_t dtype, int32_t path, const int32_t* plan_i32,
+                                               const int32_t* band_table, int32_t* status_word,
+                                               int32_t* path_ran, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if (path_ran) *path_ran = SPLAT_PATH_AUTO;   // nothing launched yet
     if (path != SPLAT_PATH_AUTO && path != SPLAT_PATH_GENERIC && path != SPLAT_PATH_BAND)
@@ -104,7 +105,7 @@ extern "C" int32_t splat_attention_fused_lse(const void* q, const void* k, int64
     if (path != SPLAT_PATH_GENERIC && plan_i32 != nullptr && status_word != nullptr) {
         int32_t rc = splat::attention_band(q, k, k_stride_bh, k_stride_col, k_stride_k, v, o,
                                            sTod_lin, sTod_tr, nnzs, bh, n_rows, n_cols, d, scale,
-                                           dtype, plan_i32, status_word, lse, st);
+                                           dtype, plan_i32, status_word, band_table, lse, st);
         // Under SPLAT_PATH_AUTO a tensor-core path that does not apply -- shape, alignment of the
         // caller's buffers, or a driver without tensor-map support -- hands over to the general
         // kernel, which takes any operands; asked for explicitly, it reports why it cannot run.
@@ -126,6 +127,18 @@ extern "C" int32_t splat_attention_fused_lse(const void* q, const void* k, int64
                                       nnzs, bh, n_rows, n_cols, d, scale, dtype, lse, st);
     if (rc == SPLAT_OK && path_ran && bh > 0 && n_rows > 0) *path_ran = SPLAT_PATH_GENERIC;
     return rc;
+}
+
+extern "C" int32_t splat_attention_fused_lse(const void* q, const void* k, int64_t k_stride_bh,
+                                             int64_t k_stride_col, int64_t k_stride_k, const void* v,
+                                             void* o, float* lse, const float* sTod_lin,
+                                             const float* sTod_tr, const float* nnzs, int64_t bh,
+                                             int64_t n_rows, int64_t n_cols, int64_t d, float scale,
+                                             int32_t dtype, int32_t path, const int32_t* plan_i32,
+                                             int32_t* status_word, int32_t* path_ran, void* stream) {
+    return splat_attention_fused_table(q, k, k_stride_bh, k_stride_col, k_stride_k, v, o, lse, sTod_lin,
+                                       sTod_tr, nnzs, bh, n_rows, n_cols, d, scale, dtype, path, plan_i32,
+                                       nullptr, status_word, path_ran, stream);
 }
 
 extern "C" int32_t splat_attention_fused_ex(const void* q, const void* k, int64_t k_stride_bh,

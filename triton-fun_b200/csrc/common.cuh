@@ -66,7 +66,9 @@ __device__ __forceinline__ RowAffine row_affine(const float* __restrict__ sTod_l
     float tr = __ldg(sTod_tr + row);
     r.stride = (int)rintf(lin);
     if (r.stride < 1) r.stride = 1;
-    r.start = (int)rint((double)tr * (double)r.stride);
+    // rint(tr * stride) without double precision: the product and its rounding error separately
+    const float prod = tr * (float)r.stride, err = fmaf(tr, (float)r.stride, -prod), whole = rintf(prod);
+    r.start = (int)whole + (int)rintf((prod - whole) + err);
     r.nnz = (int)rintf(__ldg(nnzs + row));
     if (r.nnz < 0) r.nnz = 0;
     return r;

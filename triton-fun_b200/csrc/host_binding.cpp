@@ -26,7 +26,7 @@ constexpr int kMaxDevices = 64;
 
 using FusedFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, const void*, void*, float*,
                             const float*, const float*, const float*, int64_t, int64_t, int64_t, int64_t, float,
-                            int32_t, int32_t, const int32_t*, int32_t*, int32_t*, void*);
+                            int32_t, int32_t, const int32_t*, const int32_t*, int32_t*, int32_t*, void*);
 using SddmmBandFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, void*, const float*, const float*,
                                 const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*,
                                 int32_t*, void*);
@@ -110,9 +110,39 @@ inline bool same4(const at::Tensor& t, int64_t a, int64_t b, int64_t c, int64_t 
     return s.size() == 4 && s[0] == a && s[1] == b && s[2] == c && s[3] == d;
 }
 
+// plan remembered by splat_native.classify() on the nnzs tensor: ((id, id, version x 3, numel), plan, lin, tr,
+// band table or None); false if the metadata is not what it was made from
+bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, const at::Tensor& lin, PyObject* tr_obj,
+                 const at::Tensor& tr, int32_t (&plan)[8], const int32_t** table = nullptr) {
+    PyObject* hit = PyObject_GetAttr(nnzs_obj, k_cached_plan);
+    if (hit == nullptr) {
+        PyErr_Clear();
+        return false;
+    }
+    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 5 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
+              PyTuple_GET_ITEM(hit, 3) == tr_obj;
+    if (ok) {
+        PyObject* key = PyTuple_GET_ITEM(hit, 0);
+        const int64_t now[4] = {static_cast<int64_t>(lin._version()), static_cast<int64_t>(tr._version()),
+                                static_cast<int64_t>(nnzs._version()), nnzs.numel()};
+        ok = PyTuple_Check(key) && PyTuple_GET_SIZE(key) == 6;
+        for (int i = 0; ok && i < 4; ++i) {
+            long v;
+            ok = as_long(PyTuple_GET_ITEM(key, 2 + i), &v) && v == now[i];
+        }
+        ok = ok && read_plan(PyTuple_GET_ITEM(hit, 1), plan);
+        if (ok && table != nullptr) {
+            const at::Tensor* t = tensor(PyTuple_GET_ITEM(hit, 4));
+            if (t != nullptr) *table = static_cast<const int32_t*>(t->const_data_ptr());
+        }
+    }
+    Py_DECREF(hit);
+    return ok;
+}
+
 // True if the call was made; false: nothing happened and the Python code decides.
 bool fused(const at::Tensor* q, const at::Tensor* kt, const at::Tensor* v, const at::Tensor* out, const at::Tensor* lin,
-           const at::Tensor* tr, const at::Tensor* nnzs, float scale, long path, PyObject* plan_obj, const at::Tensor* lse) {
+           const at::Tensor* tr, const at::Tensor* nnzs, float scale, long path, PyObject* plan_obj, const int32_t* table, const at::Tensor* lse) {
     if (!q || !kt || !v || !out || g_api.fused == nullptr || q->dim() != 4 || kt->dim() != 4) return false;
     const int dtype = dtype_code(*q);
     const int dev = ordinary_device(*q);
@@ -144,7 +174,7 @@ bool fused(const at::Tensor* q, const at::Tensor* kt, const at::Tensor* v, const
     int32_t ran = 0;
     const int32_t rc = g_api.fused(q->const_data_ptr(), kt->const_data_ptr(), ksb, kt->stride(3), kt->stride(2),
                                    v->const_data_ptr(), out->data_ptr(), plse, pl, pt, pn, B * H, L, n_cols, d, scale, dtype,
-                                   static_cast<int32_t>(path), with_plan ? plan : nullptr, g_status[dev].word, &ran,
+                                   static_cast<int32_t>(path), with_plan ? plan : nullptr, table, g_status[dev].word, &ran,
                                    c10::cuda::getCurrentCUDAStream(dev).stream());
     if (rc != 0) return false;
     if (ran != kPathBand && dtype != 0 && path == kPathAuto && g_warn != nullptr) {   // 16 bit on the CUDA cores: say so once
@@ -156,31 +186,6 @@ bool fused(const at::Tensor* q, const at::Tensor* kt, const at::Tensor* v, const
         else Py_DECREF(r);
     }
     return true;
-}
-
-// plan remembered by splat_native.classify() on the nnzs tensor: ((id, id, version x 3, numel), plan, lin, tr)
-bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, const at::Tensor& lin, PyObject* tr_obj,
-                 const at::Tensor& tr, int32_t (&plan)[8]) {
-    PyObject* hit = PyObject_GetAttr(nnzs_obj, k_cached_plan);
-    if (hit == nullptr) {
-        PyErr_Clear();
-        return false;
-    }
-    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 4 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
-              PyTuple_GET_ITEM(hit, 3) == tr_obj;
-    if (ok) {
-        PyObject* key = PyTuple_GET_ITEM(hit, 0);
-        const int64_t now[4] = {static_cast<int64_t>(lin._version()), static_cast<int64_t>(tr._version()),
-                                static_cast<int64_t>(nnzs._version()), nnzs.numel()};
-        ok = PyTuple_Check(key) && PyTuple_GET_SIZE(key) == 6;
-        for (int i = 0; ok && i < 4; ++i) {
-            long v;
-            ok = as_long(PyTuple_GET_ITEM(key, 2 + i), &v) && v == now[i];
-        }
-        ok = ok && read_plan(PyTuple_GET_ITEM(hit, 1), plan);
-    }
-    Py_DECREF(hit);
-    return ok;
 }
 
 PyObject* yes_or_none(bool yes) {
@@ -209,9 +214,14 @@ PyObject* module_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
         return yes_or_none(false);
     const at::Tensor* lse_t = nullptr;
     if (lse != nullptr && lse != Py_None && (lse_t = tensor(lse)) == nullptr) return yes_or_none(false);
-    if (!fused(tensor(item[0]), tensor(item[1]), tensor(item[2]), tensor(out), tensor(PyDict_GetItemWithError(dict, k_lin)),
-               tensor(PyDict_GetItemWithError(dict, k_tr)), tensor(PyDict_GetItemWithError(dict, k_nnzs)),
-               static_cast<float>(PyFloat_AS_DOUBLE(scale)), path, PyDict_GetItemWithError(dict, k_plan), lse_t))
+    PyObject *lin = PyDict_GetItemWithError(dict, k_lin), *tr = PyDict_GetItemWithError(dict, k_tr),
+             *nnzs = PyDict_GetItemWithError(dict, k_nnzs);
+    const at::Tensor *lin_t = tensor(lin), *tr_t = tensor(tr), *nnzs_t = tensor(nnzs);
+    const int32_t* table = nullptr;
+    int32_t unused[8];
+    if (lin_t && tr_t && nnzs_t && !cached_plan(nnzs, *nnzs_t, lin, *lin_t, tr, *tr_t, unused, &table)) table = nullptr;
+    if (!fused(tensor(item[0]), tensor(item[1]), tensor(item[2]), tensor(out), lin_t, tr_t, nnzs_t,
+               static_cast<float>(PyFloat_AS_DOUBLE(scale)), path, PyDict_GetItemWithError(dict, k_plan), table, lse_t))
         return yes_or_none(false);
     Py_INCREF(out);
     return out;

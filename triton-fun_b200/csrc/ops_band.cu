@@ -32,7 +32,7 @@ bool allow_dynamic_smem(const void* kernel, int bytes);
 bool make_map(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_rows,
               int64_t d, int64_t stride, int box_rows);
 bool make_map_kt(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_cols,
-                 int64_t d);
+                 int64_t d, int64_t box_d);
 
 namespace ops {
 
@@ -790,7 +790,7 @@ extern "C" int32_t splat_sddmm_band(const void* q, const void* k, int64_t k_stri
     CUtensorMap mq, mk;
     if (!make_map(&mq, q, dtype, bh, n_rows, d, stride, ops::kTile) ||
         !(k_major ? make_map(&mk, k, dtype, bh, n_rows, d, stride, ops::kStep)
-                  : make_map_kt(&mk, k, dtype, bh, n_cols, d)))
+                  : make_map_kt(&mk, k, dtype, bh, n_cols, d, d)))
         return SPLAT_ERR_DRIVER;
     ops::Params prm;
     prm.kt_major = k_major ? 0 : 1;
