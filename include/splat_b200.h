@@ -252,6 +252,31 @@ int32_t splat_attention_fused_table(const void* q, const void* k, int64_t k_stri
                                     int32_t path, const int32_t* plan_i32, const int32_t* band_table,
                                     int32_t* status_word, int32_t* path_ran, void* stream);
 
+/* The five row vectors, the two span vectors and the largest row count of an explicit uint8 mask in one pass
+ * (what splat_mask_row_summary_u8 and splat_acsr_from_row_summary compute together, same values bit for
+ * bit), for 4 <= block_height <= 64.  work_i32x2: two device int32, zero before the first call and again
+ * afterwards, used by one call at a time.  trailing_dim_host: page-locked host int32, written when the rest is. */
+int32_t splat_acsr_from_mask_u8(const uint8_t* mask, int64_t n_rows, int64_t n_cols, int64_t ld,
+                                int32_t block_height, float* dTos_lin, float* dTos_tr, float* sTod_lin,
+                                float* sTod_tr, float* nnzs, float* span_start, float* span_end,
+                                int32_t* work_i32x2, int32_t* trailing_dim_host, void* stream);
+
+/* out[bh][l][c] = in[bh][c][l] for 16-bit elements: the reference's contiguous (BH, d, L) K^T as rows of d, for
+ * the tensor-core kernels when they cannot fetch that layout directly (stride > 1, or L not a multiple of
+ * 8).  d a multiple of 4, at most 256. */
+int32_t splat_transpose_16(const void* in, void* out, int64_t bh, int64_t d, int64_t n_cols, void* stream);
+
+/* Attention over host-resident (page-locked) q, k, v, o of (BH, n_rows, d), k not transposed, streamed through
+ * the device in chunks of `chunk` heads.  staging_8: two sets of device buffers q, k, v, o of chunk heads.
+ * events_7: CUDA events that have been recorded at least once, used by one caller at a time.  The copies run on
+ * stream_in and stream_out, the kernels on stream, which at the end waits for the last copy. */
+int32_t splat_attention_host(const void* q, const void* k, const void* v, void* o, void* const* staging_8,
+                             int64_t chunk, const float* sTod_lin, const float* sTod_tr, const float* nnzs,
+                             int64_t bh, int64_t n_rows, int64_t d, float scale, int32_t dtype, int32_t path,
+                             const int32_t* plan_i32, const int32_t* band_table, int32_t* status_word,
+                             int32_t* path_ran, void* stream_in, void* stream, void* stream_out,
+                             void* const* events_7);
+
 /* Host copy of a status word: host_copy is page-locked host memory (device-accessible, one int32, cleared
  * by the caller).  A tensor-core kernel that is started while *status_word is non-zero does nothing but
  * store that value in *host_copy, so a caller sees at a later launch that an earlier one gave up without

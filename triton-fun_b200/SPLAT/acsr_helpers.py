@@ -184,7 +184,9 @@ def row_summary(mask, dev: torch.device) -> torch.Tensor:
         return _n.pattern_row_summary(mask.kind, mask.s, mask.p0, mask.p1, dev)
     if isinstance(mask, torch.Tensor):
         m = mask
-        if m.dtype != torch.uint8:
+        if m.dtype == torch.bool:
+            m = m.view(torch.uint8)
+        elif m.dtype != torch.uint8:
             m = (m != 0).to(torch.uint8)
         m = m.to(dev)
     else:
@@ -195,6 +197,10 @@ def row_summary(mask, dev: torch.device) -> torch.Tensor:
 
 
 def _create_acsr_on(mask, BLOCK_HEIGHT: int, dev: torch.device):
+    if isinstance(mask, torch.Tensor) and mask.device == dev and mask.dtype in (torch.uint8, torch.bool):
+        done = _n.acsr_from_mask(mask, BLOCK_HEIGHT)      # one kernel; None where it does not apply
+        if done is not None:
+            return done
     rows = row_summary(mask, dev)
     return _n.acsr_from_row_summary(rows, mask_shape(mask)[1], BLOCK_HEIGHT)
 

@@ -15,6 +15,7 @@ returns the module-owned output buffer (the same tensor object on every call, as
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Any
 
 import torch
@@ -25,6 +26,16 @@ from acsr_helpers import create_acsr, create_blocked_mask, create_windowed_mask,
 from r_sddmm import rsddmm_launcher, rsddmm_preamble
 from r_softmax import rsoftmax_launcher, rsoftmax_preamble
 from r_spmm import rspmm_launcher, rspmm_preamble
+
+
+def host_chunk(heads: int, head_bytes: int) -> int:
+    """Heads per chunk of forward_host.  The first chunk's way in and the last one's way out overlap with
+    nothing, so there should be several; every copy's start-up and the waits between the streams cost some 10
+    us, so they should not be small: a sixth of the operands, at least 8 MB, in chunks of equal size.  32 heads of
+    2 MB: one chunk 4.99 ms, 2 / 4 / 8 / 16 / 32 chunks 4.49 / 4.29 / 4.29 / 4.60 / 4.93 ms; the copies alone, both
+    directions at once, 3.80 ms."""
+    per_chunk = max(1, max(heads * head_bytes // 2, 8 << 20) // (3 * head_bytes))
+    return -(-heads // -(-heads // per_chunk))
 
 
 class RegularAttention(nn.Module):
@@ -122,43 +133,33 @@ class RegularAttention(nn.Module):
         reference, whose operands are always device tensors."""
         B, H, L, d = q_host.shape
         bh = B * H
-        qh, kh, vh, oh = (t.view(1, bh, L, d) for t in (q_host, k_host, v_host, out_host))
-        chunk = max(1, min(chunk_heads, bh))
+        if bh == 0 or L == 0:
+            return out_host
+        hosts = (q_host, k_host, v_host, out_host)
+        if any(tuple(t.shape) != (B, H, L, d) for t in hosts):
+            raise ValueError("forward_host: operands must have one shape (B, H, L, d)")
+        plain = all(t.dtype == self.out_dtype and t.device.type == "cpu" for t in hosts) and out_host.is_contiguous()
+        if not plain:
+            q_host, k_host, v_host = (t.to("cpu", self.out_dtype) for t in hosts[:3])
+        q_host, k_host, v_host = (t.contiguous() for t in (q_host, k_host, v_host))
+        dst = out_host if plain else torch.empty((B, H, L, d), dtype=self.out_dtype).pin_memory()
+        chunk = max(1, min(chunk_heads, bh, host_chunk(bh, L * d * self.out_dtype.itemsize)))
         st = getattr(self, "_host_stage", None)
         if st is None or st["chunk"] != chunk or st["shape"] != (L, d):
-            mk = lambda: torch.empty((1, chunk, L, d), dtype=self.out_dtype, device=self.device)
-            st = {"chunk": chunk, "shape": (L, d),
-                  "bufs": [{"q": mk(), "k": mk(), "v": mk(), "o": mk(),
-                            "in_ready": torch.cuda.Event(), "done": torch.cuda.Event(),
-                            "out_free": torch.cuda.Event()} for _ in range(2)],
+            bufs = [torch.empty((chunk, L, d), dtype=self.out_dtype, device=self.device) for _ in range(8)]
+            events = [torch.cuda.Event() for _ in range(7)]
+            for e in events:
+                e.record(torch.cuda.current_stream(self.device))
+            st = {"chunk": chunk, "shape": (L, d), "keep": (bufs, events),
+                  "staging": (ctypes.c_void_p * 8)(*(t.data_ptr() for t in bufs)),
+                  "events": (ctypes.c_void_p * 7)(*(e.cuda_event for e in events)),
                   "s_in": torch.cuda.Stream(self.device), "s_out": torch.cuda.Stream(self.device)}
             self._host_stage = st
-        cur = torch.cuda.current_stream(self.device)
-        s_in, s_out = st["s_in"], st["s_out"]
-        s_in.wait_stream(cur)
-        for i, b in enumerate(range(0, bh, chunk)):
-            e = min(bh, b + chunk)
-            n = e - b
-            buf = st["bufs"][i % 2]
-            with torch.cuda.stream(s_in):
-                if i >= 2:
-                    s_in.wait_event(buf["done"])        # kernel of chunk i-2 has read its inputs
-                buf["q"][:, :n].copy_(qh[:, b:e], non_blocking=True)
-                buf["k"][:, :n].copy_(kh[:, b:e], non_blocking=True)
-                buf["v"][:, :n].copy_(vh[:, b:e], non_blocking=True)
-                buf["in_ready"].record(s_in)
-            cur.wait_event(buf["in_ready"])
-            if i >= 2:
-                cur.wait_event(buf["out_free"])         # output of chunk i-2 has left the device
-            _n.attention_fused(buf["q"][:, :n], buf["k"][:, :n].transpose(2, 3), buf["v"][:, :n],
-                               buf["o"][:, :n], self.sTod_linear_transformations,
-                               self.sTod_translations, self.nnzs, self.scale, self.path, self.plan)
-            buf["done"].record(cur)
-            with torch.cuda.stream(s_out):
-                s_out.wait_event(buf["done"])
-                oh[:, b:e].copy_(buf["o"][:, :n], non_blocking=True)
-                buf["out_free"].record(s_out)
-        cur.wait_stream(s_out)
+        _n.attention_host(q_host, k_host, v_host, dst, st, self.sTod_linear_transformations, self.sTod_translations,
+                          self.nnzs, self.scale, self.path, self.plan)
+        if not plain:
+            torch.cuda.current_stream(self.device).synchronize()
+            out_host.copy_(dst)
         return out_host
 
     def check_status(self) -> None:

@@ -57,6 +57,9 @@ SIGNATURES = {
     "splat_selftest_bounded_wait": [_vp, _i64, _vp],
     "splat_debug_check_indices": [_vp],
     "splat_set_status_mirror": [_vp, _vp],
+    "splat_acsr_from_mask_u8": [_vp, _i64, _i64, _i64, _i32] + [_vp] * 9 + [_vp],
+    "splat_transpose_16": [_vp, _vp, _i64, _i64, _i64, _vp],
+    "splat_attention_host": [_vp] * 5 + [_i64] + [_vp] * 3 + [_i64] * 3 + [_f32, _i32, _i32] + [_vp] * 8,
     "splat_band_table": [_vp, _vp, _vp, _i64, _i64, _vp, _vp],
     "splat_attention_fused_table": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64,
                                     _i64, _i64, _f32, _i32, _i32, _vp, _vp, _vp, _vp, _vp],
@@ -164,6 +167,47 @@ def acsr_from_row_summary(rows_i32: torch.Tensor, n_cols: int, block_height: int
             spans[0].data_ptr(), spans[1].data_ptr(), td.data_ptr(), _stream(dev)),
             "splat_acsr_from_row_summary")
     return (*vec, int(td.item()), spans[0], spans[1])
+
+
+_MASK_SLOTS = 16
+_MASK_WORK: dict = {}
+
+
+def acsr_from_mask(mask_u8: torch.Tensor, block_height: int):
+    """acsr_from_row_summary(mask_row_summary(mask)) in one kernel, or None where that does not apply (block
+    heights outside 4 .. 64, no unit column stride, another current device)."""
+    dev = mask_u8.device
+    if dev.index not in _MASK_WORK:        # scratch of the calls in progress: 16 slots, device and page-locked host
+        with torch.cuda.device(dev):
+            work = torch.zeros(2 * _MASK_SLOTS, dtype=torch.int32, device=dev)
+            torch.cuda.current_stream(dev).synchronize()
+            host = torch.zeros(_MASK_SLOTS, dtype=torch.int32).pin_memory()
+        _host.set_mask_work(dev.index, _MASK_SLOTS, work.data_ptr(), host.data_ptr())
+        _MASK_WORK[dev.index] = (work, host)
+    return _host.acsr_from_mask(mask_u8, block_height)
+
+
+def attention_host(q, k, v, out, stage: dict, sTod_lin, sTod_tr, nnzs, scale: float, path: int, plan) -> None:
+    """Host tensors (B,H,L,d) through the device in chunks; stage as RegularAttention.forward_host keeps it."""
+    dev = nnzs.device
+    B, H, L, d = q.shape
+    if _band_candidate(q, path):
+        _raise_if_gave_up(dev)
+    sw = status_word(dev)
+    ran = ctypes.c_int32(0)
+    plan_arr = (ctypes.c_int32 * 8)(*plan)
+    _debug_before(dev)
+    with _on(dev):
+        check(_lib.splat_attention_host(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), stage["staging"], stage["chunk"],
+            _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"), _f32_vec(nnzs, L, "nnzs"), B * H, L, d,
+            float(scale), dtype_code(q.dtype), int(path), ctypes.cast(plan_arr, _vp) if path != PATH_GENERIC else None,
+            _band_table(sTod_lin, sTod_tr, nnzs), sw.data_ptr(), ctypes.byref(ran), stage["s_in"].cuda_stream, _stream(dev),
+            stage["s_out"].cuda_stream, stage["events"]), "splat_attention_host")
+    if ran.value != PATH_BAND and q.dtype != torch.float32 and q.numel() > 0 and path == PATH_AUTO:
+        _warn_cuda_core_16bit("attention")
+    if os.environ.get("SPLAT_B200_DEBUG"):
+        check_status_word(dev)
 
 
 def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) -> tuple:
@@ -502,4 +546,4 @@ def module_forward(attributes: dict, x):
 
 _host.bind(*(ctypes.cast(getattr(_lib, name), _vp).value for name in (
     "splat_attention_fused_table", "splat_sddmm_band", "splat_spmm_band", "splat_sddmm_tile", "splat_spmm_tile",
-    "splat_softmax")), _warn_cuda_core_16bit)
+    "splat_softmax", "splat_acsr_from_mask_u8", "splat_transpose_16")), _warn_cuda_core_16bit)

@@ -12,12 +12,15 @@
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
+#include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <chrono>
 #include <cstdint>
 #include <cstdlib>
+#include <mutex>
 
 namespace {
 
@@ -36,6 +39,9 @@ using SddmmTileFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int6
                                 const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
 using SpmmTileFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
                                int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
+using MaskFn = int32_t (*)(const void*, int64_t, int64_t, int64_t, int32_t, float*, float*, float*, float*, float*, float*, float*,
+                           int32_t*, int32_t*, void*);
+using TransposeFn = int32_t (*)(const void*, void*, int64_t, int64_t, int64_t, void*);
 using SoftmaxFn = int32_t (*)(const void*, void*, const float*, int64_t, int64_t, int64_t, float, int32_t, void*);
 
 struct Api {
@@ -45,6 +51,8 @@ struct Api {
     SddmmTileFn sddmm_tile;
     SpmmTileFn spmm_tile;
     SoftmaxFn softmax;
+    MaskFn mask;
+    TransposeFn transpose;
 } g_api{};
 
 // Per device: the status word (device memory) and its host copy, which the kernels write.
@@ -140,6 +148,22 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
     return ok;
 }
 
+// 16-bit K^T as a contiguous (B, H, d, n) array of a band pattern that the tensor-core kernels cannot fetch in
+// this layout (a tensor map has to start and step on 16 bytes, and strided rows are not contiguous in it): a
+// row-major copy, ordered on the current stream, else an undefined tensor.  One pass over K against kernels on
+// the CUDA cores that take 10 to 30 times as long.
+at::Tensor rows_of_k(const at::Tensor& kt, int64_t ksb, const int32_t (&plan)[8], int64_t L, int64_t d, void* stream) {
+    const int64_t n = kt.size(3), bh = kt.size(0) * kt.size(1);
+    const int64_t stride = plan[7] > 0 ? plan[1] : 1;
+    const bool contiguous = kt.stride(3) == 1 && kt.stride(2) == n && ksb == n * d;
+    const bool band = (plan[7] == 0 || plan[1] == plan[2]) && plan[3] == 0 && plan[5] <= n && n == L && d % 8 == 0 && d <= 128;
+    const bool direct = kt.stride(2) == 1 || (stride == 1 && n % 8 == 0);
+    if (!contiguous || !band || direct || bh > 65535 || g_api.transpose == nullptr) return {};
+    at::Tensor rows = at::empty({bh, n, d}, kt.options());
+    if (g_api.transpose(kt.const_data_ptr(), rows.data_ptr(), bh, d, n, stream) != 0) return {};
+    return rows;
+}
+
 // True if the call was made; false: nothing happened and the Python code decides.
 bool fused(const at::Tensor* q, const at::Tensor* kt, const at::Tensor* v, const at::Tensor* out, const at::Tensor* lin,
            const at::Tensor* tr, const at::Tensor* nnzs, float scale, long path, PyObject* plan_obj, const int32_t* table, const at::Tensor* lse) {
@@ -172,10 +196,14 @@ bool fused(const at::Tensor* q, const at::Tensor* kt, const at::Tensor* v, const
     const bool with_plan = path != kPathGeneric;
     if (with_plan && !read_plan(plan_obj, plan)) return false;
     int32_t ran = 0;
-    const int32_t rc = g_api.fused(q->const_data_ptr(), kt->const_data_ptr(), ksb, kt->stride(3), kt->stride(2),
+    void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+    at::Tensor rows;
+    if (dtype != 0 && path == kPathAuto) rows = rows_of_k(*kt, ksb, plan, L, d, stream);
+    const bool copied = rows.defined();
+    const int32_t rc = g_api.fused(q->const_data_ptr(), copied ? rows.const_data_ptr() : kt->const_data_ptr(), copied ? n_cols * d : ksb,
+                                   copied ? d : kt->stride(3), copied ? 1 : kt->stride(2),
                                    v->const_data_ptr(), out->data_ptr(), plse, pl, pt, pn, B * H, L, n_cols, d, scale, dtype,
-                                   static_cast<int32_t>(path), with_plan ? plan : nullptr, table, g_status[dev].word, &ran,
-                                   c10::cuda::getCurrentCUDAStream(dev).stream());
+                                   static_cast<int32_t>(path), with_plan ? plan : nullptr, table, g_status[dev].word, &ran, stream);
     if (rc != 0) return false;
     if (ran != kPathBand && dtype != 0 && path == kPathAuto && g_warn != nullptr) {   // 16 bit on the CUDA cores: say so once
         PyObject* cb = g_warn;
@@ -248,11 +276,16 @@ PyObject* sddmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     int32_t plan[8];
     if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan)) return yes_or_none(false);
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
-    const int64_t ksc = y->stride(3), ksk = y->stride(2);
+    at::Tensor rows;
+    if (dtype != 0) rows = rows_of_k(*y, ksb, plan, L, d, st);
+    const bool copied = rows.defined();
+    const void* yp = copied ? rows.const_data_ptr() : y->const_data_ptr();
+    const int64_t ksc = copied ? d : y->stride(3), ksk = copied ? 1 : y->stride(2);
+    if (copied) ksb = n_cols * d;
     const int32_t rc =
-        dtype == 0 ? g_api.sddmm_tile(x->const_data_ptr(), y->const_data_ptr(), ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
+        dtype == 0 ? g_api.sddmm_tile(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
                                       L, n_cols, d, trailing, dtype, plan, st)
-                   : g_api.sddmm_band(x->const_data_ptr(), y->const_data_ptr(), ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
+                   : g_api.sddmm_band(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
                                       L, n_cols, d, trailing, dtype, plan, g_status[dev].word, st);
     return yes_or_none(rc == 0);
 }
@@ -303,12 +336,12 @@ PyObject* softmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return yes_or_none(rc == 0);
 }
 
-// bind(fused, sddmm_band, spmm_band, sddmm_tile, spmm_tile, softmax, warn): addresses of the C ABI entry points
+// bind(fused, sddmm_band, spmm_band, sddmm_tile, spmm_tile, softmax, mask, transpose, warn): addresses of the C ABI entry points
 // and the function that warns of 16-bit operands on the CUDA-core kernels
 PyObject* bind(PyObject*, PyObject* args) {
-    unsigned long long f[6];
+    unsigned long long f[8];
     PyObject* warn;
-    if (!PyArg_ParseTuple(args, "KKKKKKO", f, f + 1, f + 2, f + 3, f + 4, f + 5, &warn)) return nullptr;
+    if (!PyArg_ParseTuple(args, "KKKKKKKKO", f, f + 1, f + 2, f + 3, f + 4, f + 5, f + 6, f + 7, &warn)) return nullptr;
     Py_INCREF(warn);
     g_warn = warn;
     g_api.fused = reinterpret_cast<FusedFn>(f[0]);
@@ -317,6 +350,8 @@ PyObject* bind(PyObject*, PyObject* args) {
     g_api.sddmm_tile = reinterpret_cast<SddmmTileFn>(f[3]);
     g_api.spmm_tile = reinterpret_cast<SpmmTileFn>(f[4]);
     g_api.softmax = reinterpret_cast<SoftmaxFn>(f[5]);
+    g_api.mask = reinterpret_cast<MaskFn>(f[6]);
+    g_api.transpose = reinterpret_cast<TransposeFn>(f[7]);
     Py_RETURN_NONE;
 }
 
@@ -332,12 +367,100 @@ PyObject* set_status(PyObject*, PyObject* args) {
     Py_RETURN_NONE;
 }
 
+// Scratch of acsr_from_mask calls in progress, per device: `slots` pairs of device words (zero between calls) and
+// `slots` page-locked host words.  Kept by splat_native; a slot is taken for the length of a call.
+struct MaskWork {
+    int32_t* work = nullptr;
+    volatile int32_t* host = nullptr;
+    uint32_t free = 0;
+} g_mask[kMaxDevices];
+std::mutex g_mask_mutex;
+
+// set_mask_work(device index, slots, address of the device words, address of the host words)
+PyObject* set_mask_work(PyObject*, PyObject* args) {
+    int dev, slots;
+    unsigned long long work, host;
+    if (!PyArg_ParseTuple(args, "iiKK", &dev, &slots, &work, &host)) return nullptr;
+    if (dev >= 0 && dev < kMaxDevices && slots > 0 && slots < 32) {
+        std::lock_guard<std::mutex> lock(g_mask_mutex);
+        g_mask[dev].work = reinterpret_cast<int32_t*>(work);
+        g_mask[dev].host = reinterpret_cast<volatile int32_t*>(host);
+        g_mask[dev].free = (1u << slots) - 1;
+    }
+    Py_RETURN_NONE;
+}
+
+// acsr_from_mask(uint8 or bool CUDA tensor (rows, cols), block height) -> the tuple create_acsr returns, or None
+PyObject* acsr_from_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    long height;
+    const at::Tensor* m = n == 2 ? tensor(a[0]) : nullptr;
+    if (m == nullptr || !as_long(a[1], &height) || g_api.mask == nullptr || m->dim() != 2 || !m->is_cuda() ||
+        m->element_size() != 1 || height < 4 || height > 64)
+        return yes_or_none(false);
+    const int dev = m->get_device();
+    const int64_t rows = m->size(0), cols = m->size(1);
+    if (dev >= kMaxDevices || dev != c10::cuda::current_device() || rows < 1 || cols < 1 || m->stride(1) != 1 || m->stride(0) < cols)
+        return yes_or_none(false);
+    int slot = -1;
+    {
+        std::lock_guard<std::mutex> lock(g_mask_mutex);
+        if (g_mask[dev].free != 0) {
+            slot = __builtin_ctz(g_mask[dev].free);
+            g_mask[dev].free &= g_mask[dev].free - 1;
+        }
+    }
+    if (slot < 0) return yes_or_none(false);
+    volatile int32_t* word = g_mask[dev].host + slot;
+    const auto stream = c10::cuda::getCurrentCUDAStream(dev);
+    at::Tensor t[7];
+    int32_t rc = -1, trailing = -1;
+    try {
+        const auto options = m->options().dtype(at::kFloat);
+        for (int i = 0; i < 7; ++i) t[i] = at::empty({i < 5 ? rows : (rows + height - 1) / height}, options);
+        *word = -1;
+        float* p[7];
+        for (int i = 0; i < 7; ++i) p[i] = static_cast<float*>(t[i].data_ptr());
+        rc = g_api.mask(m->const_data_ptr(), rows, cols, m->stride(0), static_cast<int32_t>(height), p[0], p[1], p[2], p[3], p[4],
+                        p[5], p[6], g_mask[dev].work + 2 * slot, const_cast<int32_t*>(word), stream.stream());
+        if (rc == 0) {
+            // The count reaches the host some microseconds before a stream synchronisation would return; work
+            // queued before this call, or an error, is left to the synchronisation.
+            Py_BEGIN_ALLOW_THREADS
+            const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(2);
+            while ((trailing = *word) < 0)
+                if (std::chrono::steady_clock::now() > until) break;
+            Py_END_ALLOW_THREADS
+            if (trailing < 0) {
+                c10::cuda::stream_synchronize(stream.stream());
+                trailing = *word;
+            }
+        }
+    } catch (const std::exception& e) {
+        if (rc == 0) {                  // launched, and the device reports an error: the slot stays taken
+            PyErr_SetString(PyExc_RuntimeError, e.what());
+            return nullptr;
+        }
+    }
+    {
+        std::lock_guard<std::mutex> lock(g_mask_mutex);
+        g_mask[dev].free |= 1u << slot;
+    }
+    if (rc != 0 || trailing < 0) return yes_or_none(false);
+    PyObject* out = PyTuple_New(8);
+    if (out == nullptr) return nullptr;
+    for (int i = 0; i < 8; ++i)
+        PyTuple_SET_ITEM(out, i, i == 5 ? PyLong_FromLong(trailing) : THPVariable_Wrap(t[i < 5 ? i : i - 1]));
+    return out;
+}
+
 PyMethodDef methods[] = {
     {"bind", bind, METH_VARARGS, nullptr},
     {"set_status", set_status, METH_VARARGS, nullptr},
     {"module_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(module_forward)), METH_FASTCALL, nullptr},
     {"sddmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sddmm)), METH_FASTCALL, nullptr},
     {"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(spmm)), METH_FASTCALL, nullptr},
+    {"set_mask_work", set_mask_work, METH_VARARGS, nullptr},
+    {"acsr_from_mask", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(acsr_from_mask)), METH_FASTCALL, nullptr},
     {"softmax", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(softmax)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "splat_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -395,6 +395,43 @@ attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t 
 }
 
 // ---------------------------------------------------------------------------------------------
+// (BH, d, L) -> (BH, L, d), 16-bit elements: 64 columns x all of d per CTA through shared memory, coalesced
+// 4-byte (2-byte for odd L) reads along L and 4-byte writes along d.  A row of the staging tile is d + 2
+// elements, an odd number of words: neither direction conflicts more than twofold.
+// ---------------------------------------------------------------------------------------------
+constexpr int kTransCols = 64;
+__global__ void __launch_bounds__(256)
+transpose_16_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int d, int n_cols, int wide) {
+    extern __shared__ uint16_t s_t[];
+    const int pitch = d + 2;
+    const int64_t head = (int64_t)blockIdx.y * d * n_cols;
+    const int l0 = blockIdx.x * kTransCols, n = min(kTransCols, n_cols - l0);
+    in += head + l0;
+    if (wide) {       // n_cols even: row starts are 4-byte aligned
+        for (int i = threadIdx.x; i < d * (kTransCols / 2); i += 256) {
+            const int c = i / (kTransCols / 2), l = (i % (kTransCols / 2)) * 2;
+            if (l < n) {
+                const uint32_t v = *reinterpret_cast<const uint32_t*>(in + (int64_t)c * n_cols + l);
+                s_t[l * pitch + c] = (uint16_t)v;
+                s_t[(l + 1) * pitch + c] = (uint16_t)(v >> 16);
+            }
+        }
+    } else {
+        for (int i = threadIdx.x; i < d * kTransCols; i += 256) {
+            const int c = i / kTransCols, l = i % kTransCols;
+            if (l < n) s_t[l * pitch + c] = in[(int64_t)c * n_cols + l];
+        }
+    }
+    __syncthreads();
+    uint32_t* o = reinterpret_cast<uint32_t*>(out + head + (int64_t)l0 * d);
+    const int half = d / 2;
+    for (int i = threadIdx.x; i < n * half; i += 256) {
+        const int l = i / half, c = i % half;
+        o[i] = *reinterpret_cast<const uint32_t*>(s_t + l * pitch + 2 * c);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Host dispatch
 // ---------------------------------------------------------------------------------------------
 static bool grouped_d_ok(int64_t d, int vec) {
@@ -509,6 +546,19 @@ int32_t attention_generic(const void* q, const void* k, int64_t ksb, int64_t ksc
 }  // namespace splat
 
 using namespace splat;
+
+extern "C" int32_t splat_transpose_16(const void* in, void* out, int64_t bh, int64_t d, int64_t n_cols, void* stream) {
+    if (bh < 0 || n_cols < 0 || d < 1) return SPLAT_ERR_BAD_ARG;
+    if (d > 256 || d % 4 != 0 || bh > 65535 || n_cols > INT32_MAX) return SPLAT_ERR_UNSUPPORTED_SHAPE;
+    if (bh == 0 || n_cols == 0) return SPLAT_OK;
+    if (!in || !out) return SPLAT_ERR_BAD_ARG;
+    if ((reinterpret_cast<uintptr_t>(out) & 3u) != 0) return SPLAT_ERR_MISALIGNED;
+    const int wide = n_cols % 2 == 0 && (reinterpret_cast<uintptr_t>(in) & 3u) == 0;
+    const dim3 grid((unsigned)((n_cols + kTransCols - 1) / kTransCols), (unsigned)bh);
+    transpose_16_kernel<<<grid, 256, kTransCols * (d + 2) * 2, (cudaStream_t)stream>>>(
+        (const uint16_t*)in, (uint16_t*)out, (int)d, (int)n_cols, wide);
+    return launch_status();
+}
 
 extern "C" int32_t splat_debug_check_indices(int32_t* status_word) {
     g_index_check = status_word;
