@@ -277,6 +277,19 @@ int32_t splat_attention_host(const void* q, const void* k, const void* v, void* 
                              int32_t* path_ran, void* stream_in, void* stream, void* stream_out,
                              void* const* events_7);
 
+/* splat_sddmm_band / splat_spmm_band with the band table (or NULL). */
+int32_t splat_sddmm_band_table(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
+                               int64_t k_stride_k, void* s_out, const float* sTod_lin,
+                               const float* sTod_tr, const float* nnzs, int64_t bh, int64_t n_rows,
+                               int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
+                               const int32_t* plan_i32, const int32_t* band_table, int32_t* status_word,
+                               void* stream);
+int32_t splat_spmm_band_table(const void* p, const void* v, void* o, const float* sTod_lin,
+                              const float* sTod_tr, const float* nnzs, int64_t bh, int64_t n_rows,
+                              int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
+                              const int32_t* plan_i32, const int32_t* band_table, int32_t* status_word,
+                              void* stream);
+
 /* Host copy of a status word: host_copy is page-locked host memory (device-accessible, one int32, cleared
  * by the caller).  A tensor-core kernel that is started while *status_word is non-zero does nothing but
  * store that value in *host_copy, so a caller sees at a later launch that an earlier one gave up without

@@ -54,6 +54,10 @@ SIGNATURES = {
     "splat_sddmm_tile": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64,
                          _i32, _vp, _vp],
     "splat_spmm_tile": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp],
+    "splat_sddmm_band_table": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64,
+                               _i32, _vp, _vp, _vp, _vp],
+    "splat_spmm_band_table": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp,
+                              _vp, _vp],
     "splat_selftest_bounded_wait": [_vp, _i64, _vp],
     "splat_debug_check_indices": [_vp],
     "splat_set_status_mirror": [_vp, _vp],
@@ -399,11 +403,11 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
         _raise_if_gave_up(dev)
         plan_arr = (ctypes.c_int32 * 8)(*classify(sTod_lin, sTod_tr, nnzs))
         with _on(dev):
-            rc = _lib.splat_sddmm_band(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
+            rc = _lib.splat_sddmm_band_table(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
                                        _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
                                        _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, trailing_dim,
                                        dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p),
-                                       status_word(dev).data_ptr(), _stream(dev))
+                                       _band_table(sTod_lin, sTod_tr, nnzs), status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE or path == PATH_BAND:
             check(rc, "splat_sddmm_band")
             if os.environ.get("SPLAT_B200_DEBUG"):
@@ -461,11 +465,11 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
         _raise_if_gave_up(dev)
         plan_arr = (ctypes.c_int32 * 8)(*classify(sTod_lin, sTod_tr, nnzs))
         with _on(dev):
-            rc = _lib.splat_spmm_band(x.data_ptr(), y.data_ptr(), output.data_ptr(),
+            rc = _lib.splat_spmm_band_table(x.data_ptr(), y.data_ptr(), output.data_ptr(),
                                       _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
                                       _f32_vec(nnzs, L, "nnzs"), B * H, L, n_cols, d, T,
                                       dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p),
-                                      status_word(dev).data_ptr(), _stream(dev))
+                                      _band_table(sTod_lin, sTod_tr, nnzs), status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE or path == PATH_BAND:
             check(rc, "splat_spmm_band")
             if os.environ.get("SPLAT_B200_DEBUG"):
@@ -545,5 +549,5 @@ def module_forward(attributes: dict, x):
 
 
 _host.bind(*(ctypes.cast(getattr(_lib, name), _vp).value for name in (
-    "splat_attention_fused_table", "splat_sddmm_band", "splat_spmm_band", "splat_sddmm_tile", "splat_spmm_tile",
+    "splat_attention_fused_table", "splat_sddmm_band_table", "splat_spmm_band_table", "splat_sddmm_tile", "splat_spmm_tile",
     "splat_softmax", "splat_acsr_from_mask_u8", "splat_transpose_16")), _warn_cuda_core_16bit)

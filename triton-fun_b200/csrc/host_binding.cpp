@@ -32,9 +32,9 @@ using FusedFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t,
                             int32_t, int32_t, const int32_t*, const int32_t*, int32_t*, int32_t*, void*);
 using SddmmBandFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, void*, const float*, const float*,
                                 const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*,
-                                int32_t*, void*);
+                                const int32_t*, int32_t*, void*);
 using SpmmBandFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
-                               int64_t, int64_t, int64_t, int32_t, const int32_t*, int32_t*, void*);
+                               int64_t, int64_t, int64_t, int32_t, const int32_t*, const int32_t*, int32_t*, void*);
 using SddmmTileFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, void*, const float*, const float*,
                                 const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
 using SpmmTileFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
@@ -274,7 +274,8 @@ PyObject* sddmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         return yes_or_none(false);
     const float *pl = meta(lin, L, dev), *pt = meta(tr, L, dev), *pn = meta(nnzs, L, dev);
     int32_t plan[8];
-    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan)) return yes_or_none(false);
+    const int32_t* table = nullptr;
+    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, &table)) return yes_or_none(false);
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
     at::Tensor rows;
     if (dtype != 0) rows = rows_of_k(*y, ksb, plan, L, d, st);
@@ -286,7 +287,7 @@ PyObject* sddmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         dtype == 0 ? g_api.sddmm_tile(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
                                       L, n_cols, d, trailing, dtype, plan, st)
                    : g_api.sddmm_band(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
-                                      L, n_cols, d, trailing, dtype, plan, g_status[dev].word, st);
+                                      L, n_cols, d, trailing, dtype, plan, table, g_status[dev].word, st);
     return yes_or_none(rc == 0);
 }
 
@@ -308,12 +309,13 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         return yes_or_none(false);
     const float *pl = meta(lin, L, dev), *pt = meta(tr, L, dev), *pn = meta(nnzs, L, dev);
     int32_t plan[8];
-    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan)) return yes_or_none(false);
+    const int32_t* table = nullptr;
+    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, &table)) return yes_or_none(false);
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
     const int32_t rc = dtype == 0 ? g_api.spmm_tile(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
                                                     n_cols, d, T, dtype, plan, st)
                                   : g_api.spmm_band(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
-                                                    n_cols, d, T, dtype, plan, g_status[dev].word, st);
+                                                    n_cols, d, T, dtype, plan, table, g_status[dev].word, st);
     return yes_or_none(rc == 0);
 }
 

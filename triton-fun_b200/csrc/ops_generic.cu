@@ -14,6 +14,7 @@
 //            scale folded into the exponent, then the SpMM accumulation with the probabilities
 //            broadcast by shuffle.
 #include "common.cuh"
+#include "softmax_math.cuh"
 
 namespace splat {
 
@@ -94,122 +95,104 @@ sddmm_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t ksb,
 }
 
 // ---------------------------------------------------------------------------------------------
-// Row softmax.  Variant A keeps the row in registers (16-byte loads, up to kMaxVec vectors per
-// lane); variant B re-reads the row (any trailing dimension or alignment).
+// Row softmax.  A warp takes R rows at a time and keeps them in registers, NV 16-byte pieces per lane and row; all
+// loads are issued before the first reduction, so that enough bytes are in flight to keep HBM busy.  The pieces
+// are those of the array, not of the row: a row that begins inside a piece (odd trailing dimensions) masks
+// the neighbours' elements when reading, and stores its first and last piece element by element.  Rows
+// longer than kSoftmaxMaxVec pieces per lane take the loop kernel, which reads a row three times.
+// B4 H16 L4096, T = 256 fp16: @@@; T = 257: @@@.
 // ---------------------------------------------------------------------------------------------
-constexpr int kSoftmaxMaxVec = 4;
+constexpr int kSoftmaxWarps = 8;
+constexpr int kSoftmaxMaxVec = 16;
 
-template <typename T>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-softmax_rows_vec_kernel(const T* s, T* p, const float* __restrict__ nnzs,
-                        int64_t total_rows, int64_t n_rows, int trailing, float scale_log2e) {
+template <typename T, int NV, int R>
+__global__ void __launch_bounds__(kSoftmaxWarps * 32)
+softmax_rows_kernel(const T* s, T* p, const float* __restrict__ nnzs, int64_t total_rows, int64_t n_rows, int trailing,
+                    int lead, float scale_log2e) {
     constexpr int V = DT<T>::kVec;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t grow = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
-    if (grow >= total_rows) return;
-    int nnz = (int)rintf(__ldg(nnzs + grow % n_rows));
-    nnz = nnz < 0 ? 0 : (nnz > trailing ? trailing : nnz);
-    const T* srow = s + grow * trailing;
-    T* prow = p + grow * trailing;
-    float vals[kSoftmaxMaxVec][V];
-    float m = -INFINITY;
-#pragma unroll
-    for (int v = 0; v < kSoftmaxMaxVec; ++v) {
-        const int e0 = (v * 32 + lane) * V;
-        if (e0 < nnz) {
-            load16_as_float(srow + e0, vals[v]);
-#pragma unroll
-            for (int t = 0; t < V; ++t) {
-                vals[v][t] = (e0 + t < nnz) ? vals[v][t] * scale_log2e : -INFINITY;
-                m = fmaxf(m, vals[v][t]);
-            }
-        } else {
-#pragma unroll
-            for (int t = 0; t < V; ++t) vals[v][t] = -INFINITY;
-        }
-    }
-    m = warp_max(m);
-    float sum = 0.f;
-#pragma unroll
-    for (int v = 0; v < kSoftmaxMaxVec; ++v)
-#pragma unroll
-        for (int t = 0; t < V; ++t) {
-            const float e = (vals[v][t] == -INFINITY) ? 0.f : exp2f(vals[v][t] - m);
-            vals[v][t] = e;
-            sum += e;
-        }
-    sum = warp_sum(sum);
-    const float inv = sum > 0.f ? 1.f / sum : 0.f;
-#pragma unroll
-    for (int v = 0; v < kSoftmaxMaxVec; ++v) {
-        const int e0 = (v * 32 + lane) * V;
-        if (e0 < trailing) {
-#pragma unroll
-            for (int t = 0; t < V; ++t) vals[v][t] *= inv;
-            store16_from_float(prow + e0, vals[v]);
-        }
-    }
-}
-
-// Rows of at most one 16-byte vector per lane (trailing_dim <= 32 * V): a warp takes R rows at a
-// time and issues all their loads before the first reduction, so that enough bytes are in flight to
-// keep HBM busy (one row per warp leaves the warp waiting on a single 512-byte request).
-template <typename T, int R>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-softmax_rows_short_kernel(const T* s, T* p, const float* __restrict__ nnzs,
-                          int64_t total_rows, int64_t n_rows, int trailing, float scale_log2e) {
-    constexpr int V = DT<T>::kVec;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t grow0 = ((int64_t)blockIdx.x * kWarpsPerBlock + warp) * R;
+    const int64_t grow0 = ((int64_t)blockIdx.x * kSoftmaxWarps + warp) * R;
     if (grow0 >= total_rows) return;
-    const int e0 = lane * V;
-    float vals[R][V];
-    int nnz[R];
     const int64_t in_head0 = grow0 % n_rows;   // one 64-bit division per warp
+    uint4 raw[R][NV];
+    int first[R], nnz[R];       // slot of this lane's first element
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const int64_t grow = grow0 + r;
         nnz[r] = 0;
-        if (grow < total_rows) {
+        // s and p are rounded down to 16 bytes; `lead` elements were lost by that
+        const int64_t e = lead + (grow0 + r) * trailing;
+        first[r] = lane * V - (int)(e & (V - 1));
+        if (grow0 + r < total_rows) {
             int64_t in_head = in_head0 + r;
             while (in_head >= n_rows) in_head -= n_rows;
-            int n = (int)rintf(__ldg(nnzs + in_head));
+            const int n = (int)rintf(__ldg(nnzs + in_head));
             nnz[r] = n < 0 ? 0 : (n > trailing ? trailing : n);
         }
+        const T* row = s + (e & ~(int64_t)(V - 1)) + lane * V;
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            if (first[r] + v * 32 * V < nnz[r] && first[r] + v * 32 * V > -V)
+                raw[r][v] = *reinterpret_cast<const uint4*>(row + v * 32 * V);
     }
+    constexpr bool kKeep = NV <= 2;            // exponentials kept in registers, else formed again for the output
+    float2 vals[kKeep ? R : 1][kKeep ? NV : 1][V / 2];
+    float m[R], sum[R];
+    const float2 sc2 = make_float2(scale_log2e, scale_log2e);
+    // scaled scores of a piece; elements outside the row's non-zeros -inf (a warp whose pieces are all inside them
+    // skips that)
+    auto scores = [&](int r, int v, float2 (&x)[V / 2]) {
+        const T* e = reinterpret_cast<const T*>(&raw[r][v]);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        if (e0 < nnz[r]) {
-            load16_as_float(s + (grow0 + r) * trailing + e0, vals[r]);
-        } else {
+        for (int t = 0; t < V / 2; ++t) x[t] = sm::mul2(make_float2(DT<T>::to_f(e[2 * t]), DT<T>::to_f(e[2 * t + 1])), sc2);
+        const int j = first[r] + v * 32 * V;
+        if (!__all_sync(0xffffffffu, j >= 0 && j + V <= nnz[r])) {
 #pragma unroll
-            for (int t = 0; t < V; ++t) vals[r][t] = 0.f;
+            for (int t = 0; t < V / 2; ++t) {
+                x[t].x = j + 2 * t >= 0 && j + 2 * t < nnz[r] ? x[t].x : -INFINITY;
+                x[t].y = j + 2 * t + 1 >= 0 && j + 2 * t + 1 < nnz[r] ? x[t].y : -INFINITY;
+            }
         }
-    }
-    float m[R];
+    };
+    auto exponentials = [&](float2 (&x)[V / 2], float mm) {
+        const float2 nm = make_float2(-mm, -mm);
+#pragma unroll
+        for (int t = 0; t < V / 2; ++t) {
+            x[t] = sm::add2(x[t], nm);
+            // (16-bit results: flushing exponentials below 2^-126 to zero changes nothing)
+            x[t].x = sizeof(T) == 2 ? sm::ex2(x[t].x) : exp2f(x[t].x);
+            x[t].y = sizeof(T) == 2 ? sm::ex2(x[t].y) : exp2f(x[t].y);
+        }
+    };
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         m[r] = -INFINITY;
 #pragma unroll
-        for (int t = 0; t < V; ++t) {
-            vals[r][t] = (e0 + t < nnz[r]) ? vals[r][t] * scale_log2e : -INFINITY;
-            m[r] = fmaxf(m[r], vals[r][t]);
+        for (int v = 0; v < NV; ++v) {
+            float2 tmp[V / 2];
+            float2 (&x)[V / 2] = kKeep ? vals[kKeep ? r : 0][kKeep ? v : 0] : tmp;
+            scores(r, v, x);
+#pragma unroll
+            for (int t = 0; t < V / 2; ++t) m[r] = sm::fmax3(m[r], x[t].x, x[t].y);
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
         for (int r = 0; r < R; ++r) m[r] = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], o));
-    float sum[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        sum[r] = 0.f;
+        m[r] = m[r] == -INFINITY ? 0.f : m[r];
+        float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int t = 0; t < V; ++t) {
-            const float e = (vals[r][t] == -INFINITY) ? 0.f : exp2f(vals[r][t] - m[r]);
-            vals[r][t] = e;
-            sum[r] += e;
+        for (int v = 0; v < NV; ++v) {
+            float2 tmp[V / 2];
+            float2 (&x)[V / 2] = kKeep ? vals[kKeep ? r : 0][kKeep ? v : 0] : tmp;
+            if (!kKeep) scores(r, v, x);
+            exponentials(x, m[r]);
+#pragma unroll
+            for (int t = 0; t < V / 2; ++t) acc = sm::add2(acc, x[t]);
         }
+        sum[r] = acc.x + acc.y;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -217,11 +200,30 @@ softmax_rows_short_kernel(const T* s, T* p, const float* __restrict__ nnzs,
         for (int r = 0; r < R; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        if (grow0 + r < total_rows && e0 < trailing) {
-            const float inv = sum[r] > 0.f ? 1.f / sum[r] : 0.f;
+        if (grow0 + r >= total_rows) break;
+        const float inv = sum[r] > 0.f ? 1.f / sum[r] : 0.f;
+        const float2 inv2 = make_float2(inv, inv);
+        const int64_t e = lead + (grow0 + r) * trailing;
+        T* row = p + (e & ~(int64_t)(V - 1)) + lane * V;
 #pragma unroll
-            for (int t = 0; t < V; ++t) vals[r][t] *= inv;
-            store16_from_float(p + (grow0 + r) * trailing + e0, vals[r]);
+        for (int v = 0; v < NV; ++v) {
+            const int j0 = first[r] + v * 32 * V;
+            float2 tmp[V / 2];
+            float2 (&x)[V / 2] = kKeep ? vals[kKeep ? r : 0][kKeep ? v : 0] : tmp;
+            if (!kKeep) {
+                scores(r, v, x);
+                exponentials(x, m[r]);
+            }
+#pragma unroll
+            for (int t = 0; t < V / 2; ++t) x[t] = sm::mul2(x[t], inv2);
+            const float* out = reinterpret_cast<const float*>(&x[0]);
+            if (j0 >= 0 && j0 + V <= trailing) {
+                store16_from_float(row + v * 32 * V, out);
+            } else if (j0 > -V && j0 < trailing) {
+#pragma unroll
+                for (int t = 0; t < V; ++t)
+                    if (j0 + t >= 0 && j0 + t < trailing) row[v * 32 * V + t] = DT<T>::from_f(out[t]);
+            }
         }
     }
 }
@@ -464,21 +466,29 @@ template <typename T>
 static int32_t softmax_t(const void* s, void* p, const float* nnzs, int64_t bh, int64_t n_rows,
                          int64_t trailing, float scale, cudaStream_t st) {
     const int64_t total = bh * n_rows;
-    const unsigned grid = (unsigned)((total + kWarpsPerBlock - 1) / kWarpsPerBlock);
     constexpr int V = DT<T>::kVec;
-    const bool vec = (trailing % V == 0) && trailing <= 32 * V * kSoftmaxMaxVec && aligned16(s) &&
-                     aligned16(p);
-    if (vec && trailing <= 32 * V) {
-        constexpr int R = 2;
-        const unsigned grid_r = (unsigned)((total + (int64_t)kWarpsPerBlock * R - 1) / (kWarpsPerBlock * R));
-        softmax_rows_short_kernel<T, R><<<grid_r, kWarpsPerBlock * 32, 0, st>>>(
+    const uintptr_t sa = reinterpret_cast<uintptr_t>(s), pa = reinterpret_cast<uintptr_t>(p);
+    const int lead = (int)(sa & 15) / (int)sizeof(T);
+    // pieces a row can reach into: its own, and one more where rows do not begin with a piece
+    const int64_t pieces = (trailing + V - 1) / V + (lead != 0 || trailing % V != 0 ? 1 : 0);
+    const bool same = (sa & 15) == (pa & 15) && (sa & 15) % sizeof(T) == 0 && pieces <= 32 * kSoftmaxMaxVec;
+    const T* sb = reinterpret_cast<const T*>(sa & ~(uintptr_t)15);
+    T* pb = reinterpret_cast<T*>(pa & ~(uintptr_t)15);
+    auto go = [&](auto kern, int rows_per_warp) {
+        const int64_t per_block = (int64_t)kSoftmaxWarps * rows_per_warp;
+        kern<<<(unsigned)((total + per_block - 1) / per_block), kSoftmaxWarps * 32, 0, st>>>(
+            sb, pb, nnzs, total, n_rows, (int)trailing, lead, scale * kLog2e);
+    };
+    // (more rows per warp the shorter they are: about 2 KB of loads in flight per warp)
+    if (!same)
+        softmax_rows_loop_kernel<T><<<(unsigned)((total + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
             (const T*)s, (T*)p, nnzs, total, n_rows, (int)trailing, scale * kLog2e);
-    } else if (vec)
-        softmax_rows_vec_kernel<T><<<grid, kWarpsPerBlock * 32, 0, st>>>(
-            (const T*)s, (T*)p, nnzs, total, n_rows, (int)trailing, scale * kLog2e);
-    else
-        softmax_rows_loop_kernel<T><<<grid, kWarpsPerBlock * 32, 0, st>>>(
-            (const T*)s, (T*)p, nnzs, total, n_rows, (int)trailing, scale * kLog2e);
+    else if (pieces <= 32) go(softmax_rows_kernel<T, 1, 4>, 4);
+    else if (pieces <= 64) go(softmax_rows_kernel<T, 2, 2>, 2);
+    else if (pieces <= 96) go(softmax_rows_kernel<T, 3, 2>, 2);
+    else if (pieces <= 128) go(softmax_rows_kernel<T, 4, 1>, 1);
+    else if (pieces <= 256) go(softmax_rows_kernel<T, 8, 1>, 1);
+    else go(softmax_rows_kernel<T, 16, 1>, 1);
     return launch_status();
 }
 
