@@ -388,6 +388,7 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
     if _host.sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path):
         return
     dev = x.device
+    status_word(dev)       # (from here on the native path takes ordinary operands)
     _contig(x, "x"); _contig(output, "output")
     B, H, L, d = x.shape
     bh, ksb, ksk, ksc = _flat_bh(y, "y")          # y is (B, H, d, n): dim 2 = k, dim 3 = column
@@ -441,6 +442,7 @@ def softmax(x, output, nnzs, trailing_dim: int, scale: float = 1.0) -> None:
     if _host.softmax(x, output, nnzs, trailing_dim, scale):
         return
     dev = x.device
+    status_word(dev)
     _contig(x, "x"); _contig(output, "output")
     B, H, L, T = x.shape
     if T != trailing_dim or output.shape != x.shape or output.dtype != x.dtype:
@@ -455,6 +457,7 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
     if _host.spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path):
         return
     dev = x.device
+    status_word(dev)
     _contig(x, "x"); _contig(y, "y"); _contig(output, "output")
     B, H, L, T = x.shape
     n_cols, d = y.shape[2], y.shape[3]

@@ -221,6 +221,8 @@ acsr_from_mask_kernel(const uint8_t* __restrict__ mask, int64_t n_rows, int64_t 
                       float* __restrict__ sTod_lin, float* __restrict__ sTod_tr, float* __restrict__ nnzs,
                       float* __restrict__ span_start, float* __restrict__ span_end, int32_t* __restrict__ work,
                       int32_t* __restrict__ trailing_host) {
+    depend_wait();
+    depend_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int64_t r0 = (int64_t)blockIdx.x * block_height, r1 = min(r0 + block_height, n_rows);
     double lo = (double)n_cols, hi = -1.0;     // initial values as in SPLAT/acsr_helpers.py:103,135-140
@@ -413,10 +415,9 @@ extern "C" int32_t splat_acsr_from_mask_u8(const uint8_t* mask, int64_t n_rows, 
     if (n_rows > INT_MAX || n_cols > INT_MAX || block_height < 4 || block_height > 64) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     const int64_t n_blocks = (n_rows + block_height - 1) / block_height;
     const int warps = block_height < kMaskWarps ? block_height : kMaskWarps;
-    acsr_from_mask_kernel<<<(unsigned)n_blocks, warps * 32, 0, (cudaStream_t)stream>>>(
+    return launch_kernel(acsr_from_mask_kernel, (unsigned)n_blocks, warps * 32, 0, (cudaStream_t)stream,
         mask, n_rows, n_cols, ld, block_height, dTos_lin, dTos_tr, sTod_lin, sTod_tr, nnzs, span_start, span_end,
         work_i32x2, trailing_dim_host);
-    return launch_status();
 }
 
 static bool pattern_args_ok(int32_t kind, int64_t n, int64_t p0, int64_t p1) {

@@ -199,6 +199,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     constexpr int kSingle = -1, kEmpty = INT_MIN / 2;
     int my_begin = 0, my_end = kEmpty;
     if (warp == kMmaWarp) {
+        depend_wait();
         tmem_alloc(&ctrl->tmem_base, kTmemCols);
         tmem_relinquish();
     } else if (warp == kTmaWarp) {
@@ -220,6 +221,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 mbar_init(&ctrl->p_full[i], 4);      // one arrival per softmax warp
             }
             mbar_fence_init();
+            depend_wait();
             int2 range = make_int2(0, 0);
             if (p.tiles != nullptr) range = __ldg(p.tiles + p.tile0 + res * p.tile_pitch + blockIdx.x);
             const int32_t stop = entry_status(p.status, p.mirror);
@@ -238,6 +240,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 for (int w = 0; w < 4; ++w) { ctrl->lo[w] = range.x; ctrl->hi[w] = range.y; }
         }
     } else {
+        depend_wait();
         const int u = u0 + warp * 32 + lane;
         if (u < p.rows_v) {
             if (p.rows != nullptr) {
@@ -267,6 +270,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    depend_release();
     const uint32_t tmem_base = ctrl->tmem_base;
     if (ctrl->abort_at_entry != 0) {   // an earlier launch gave up
         if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
@@ -536,8 +540,7 @@ static int32_t launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtens
     auto kern = prm.lse != nullptr ? attention_wide_kernel<T, D, true> : attention_wide_kernel<T, D, false>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), Layout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
     const dim3 grid((unsigned)((prm.rows_v + kTile - 1) / kTile), (unsigned)classes, (unsigned)bh);
-    kern<<<grid, kThreads, Layout<D>::kSmemBytes, st>>>(mq, mk, mv, mo, prm);
-    return launch_status();
+    return launch_kernel(kern, grid, kThreads, Layout<D>::kSmemBytes, st, mq, mk, mv, mo, prm);
 }
 
 }  // namespace wide

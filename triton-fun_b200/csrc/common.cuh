@@ -103,6 +103,31 @@ __device__ __forceinline__ int warp_sum_i(int v) {
 // ---------------------------------------------------------------------------------------------
 // Host-side helpers.
 // ---------------------------------------------------------------------------------------------
+// Launch that may begin while the kernel before it in the stream is finishing (programmatic dependent launch).  A
+// kernel launched this way calls depend_wait() in every thread before it touches global or tensor memory --
+// which returns when the kernel before it has completed and its writes are visible, so the stream's order is
+// kept -- and depend_release() once it holds its tensor memory, from where on the next kernel's blocks may take
+// the places that its own blocks free.  It hides the launch latency and the barrier set-up of every call
+// after the first: calls that follow one another took multiples of 2.05 us, 8.2 us the smallest.
+template <typename... P, typename... A>
+inline int32_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e == cudaSuccess ? SPLAT_OK : SPLAT_ERR_LAUNCH;
+}
+__device__ __forceinline__ void depend_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void depend_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 inline int32_t launch_status() {
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? SPLAT_OK : SPLAT_ERR_LAUNCH;

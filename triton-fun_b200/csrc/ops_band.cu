@@ -202,6 +202,7 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         return true;
     };
     if (warp == kMmaWarp) {
+        depend_wait();
         tmem_alloc(&ctrl->tmem_base, kTmemCols);
         tmem_relinquish();
     } else if (warp == kTmaWarp) {
@@ -219,6 +220,7 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             }
             mbar_init(&ctrl->drain, 1);
             mbar_fence_init();
+            depend_wait();
             int2 range = make_int2(0, 0);
             if (p.tiles != nullptr) range = __ldg(p.tiles + p.tile0 + res * p.tile_pitch + blockIdx.x);
             const int32_t stop = entry_status(p.status, p.mirror);
@@ -237,11 +239,13 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 for (int w = 0; w < 4; ++w) { ctrl->lo[w] = range.x; ctrl->hi[w] = range.y; }
         }
     } else {
+        depend_wait();
         band = load_band(p, ctrl, res, u0 + warp * 32 + lane, warp, lane);
     }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    depend_release();
     const uint32_t tmem_base = ctrl->tmem_base;
     if (ctrl->abort_at_entry != 0) {
         if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
@@ -448,6 +452,7 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
         return true;
     };
     if (warp == kMmaWarp) {
+        depend_wait();
         tmem_alloc(&ctrl->tmem_base, kTmemCols);
         tmem_relinquish();
     } else if (warp == kTmaWarp) {
@@ -463,6 +468,7 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
             }
             mbar_init(&ctrl->drain, 1);
             mbar_fence_init();
+            depend_wait();
             int2 range = make_int2(0, 0);
             if (p.tiles != nullptr) range = __ldg(p.tiles + p.tile0 + res * p.tile_pitch + blockIdx.x);
             const int32_t stop = entry_status(p.status, p.mirror);
@@ -476,11 +482,13 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
                 for (int w = 0; w < 4; ++w) { ctrl->lo[w] = range.x; ctrl->hi[w] = range.y; }
         }
     } else {
+        depend_wait();
         band = load_band(p, ctrl, res, u0 + warp * 32 + lane, warp, lane);
     }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    depend_release();
     const uint32_t tmem_base = ctrl->tmem_base;
     if (ctrl->abort_at_entry != 0) {
         if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
@@ -674,8 +682,7 @@ static int32_t launch_sddmm(const CUtensorMap& mq, const CUtensorMap& mk, const 
     auto kern = sddmm_band_kernel<T, D>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), SddmmLayout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
     dim3 grid((unsigned)((prm.rows_v + kTile - 1) / kTile), (unsigned)classes, (unsigned)bh);
-    kern<<<grid, kThreads, SddmmLayout<D>::kSmemBytes, st>>>(mq, mk, prm);
-    return launch_status();
+    return launch_kernel(kern, grid, kThreads, SddmmLayout<D>::kSmemBytes, st, mq, mk, prm);
 }
 template <typename T, int D>
 static int32_t launch_spmm(const CUtensorMap& mv, const CUtensorMap& mo, const Params& prm, int64_t bh, int64_t classes,
@@ -683,8 +690,7 @@ static int32_t launch_spmm(const CUtensorMap& mv, const CUtensorMap& mo, const P
     auto kern = spmm_band_kernel<T, D>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), SpmmLayout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
     dim3 grid((unsigned)((prm.rows_v + kTile - 1) / kTile), (unsigned)classes, (unsigned)bh);
-    kern<<<grid, kThreads, SpmmLayout<D>::kSmemBytes, st>>>(mv, mo, prm);
-    return launch_status();
+    return launch_kernel(kern, grid, kThreads, SpmmLayout<D>::kSmemBytes, st, mv, mo, prm);
 }
 
 // Checks shared by both operators; fills stride.  plan as written by splat_acsr_classify:

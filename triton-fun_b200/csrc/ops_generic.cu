@@ -76,6 +76,8 @@ sddmm_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t ksb,
                   int64_t ksk, T* __restrict__ out, const float* __restrict__ lin,
                   const float* __restrict__ tr, const float* __restrict__ nnzs, int64_t total_rows,
                   int64_t n_rows, int64_t n_cols, int d, int trailing, int32_t* check) {
+    depend_wait();
+    depend_release();
     extern __shared__ float smem_q[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t grow = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
@@ -109,6 +111,8 @@ template <typename T, int NV, int R>
 __global__ void __launch_bounds__(kSoftmaxWarps * 32)
 softmax_rows_kernel(const T* s, T* p, const float* __restrict__ nnzs, int64_t total_rows, int64_t n_rows, int trailing,
                     int lead, float scale_log2e) {
+    depend_wait();
+    depend_release();
     constexpr int V = DT<T>::kVec;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t grow0 = ((int64_t)blockIdx.x * kSoftmaxWarps + warp) * R;
@@ -233,6 +237,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 softmax_rows_loop_kernel(const T* s, T* p,
                          const float* __restrict__ nnzs, int64_t total_rows, int64_t n_rows,
                          int trailing, float scale_log2e) {
+    depend_wait();
+    depend_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t grow = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
     if (grow >= total_rows) return;
@@ -281,6 +287,8 @@ spmm_rows_kernel(const T* __restrict__ p, const T* __restrict__ v, T* __restrict
                  const float* __restrict__ lin, const float* __restrict__ tr,
                  const float* __restrict__ nnzs, int64_t total_rows, int64_t n_rows,
                  int64_t n_cols, int d, int trailing, int32_t* check) {
+    depend_wait();
+    depend_release();
     constexpr int V = DT<T>::kVec;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t grow = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
@@ -319,6 +327,8 @@ spmm_rows_scalar_kernel(const T* __restrict__ p, const T* __restrict__ v, T* __r
                         const float* __restrict__ lin, const float* __restrict__ tr,
                         const float* __restrict__ nnzs, int64_t total_rows, int64_t n_rows,
                         int64_t n_cols, int d, int trailing, int32_t* check) {
+    depend_wait();
+    depend_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t grow = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
     if (grow >= total_rows) return;
@@ -347,6 +357,8 @@ attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t 
                       const float* __restrict__ lin, const float* __restrict__ tr,
                       const float* __restrict__ nnzs, int64_t total_rows, int64_t n_rows,
                       int64_t n_cols, int d, float scale_log2e, int32_t* check, float* lse) {
+    depend_wait();
+    depend_release();
     constexpr int V = DT<T>::kVec;
     extern __shared__ float smem_q[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -404,6 +416,8 @@ attention_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t 
 constexpr int kTransCols = 64;
 __global__ void __launch_bounds__(256)
 transpose_16_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int d, int n_cols, int wide) {
+    depend_wait();
+    depend_release();
     extern __shared__ uint16_t s_t[];
     const int pitch = d + 2;
     const int64_t head = (int64_t)blockIdx.y * d * n_cols;
@@ -452,14 +466,12 @@ static int32_t sddmm_t(const void* q, const void* k, int64_t ksb, int64_t ksc, i
     const bool contig = ksk == 1 && (d % DT<T>::kVec == 0) && aligned16(k) &&
                         (ksc % DT<T>::kVec == 0) && (ksb % DT<T>::kVec == 0);
     if (contig)
-        sddmm_rows_kernel<T, true><<<grid, kWarpsPerBlock * 32, smem, st>>>(
+        return launch_kernel(sddmm_rows_kernel<T, true>, grid, kWarpsPerBlock * 32, smem, st,
             (const T*)q, (const T*)k, ksb, ksc, ksk, (T*)out, lin, tr, nnzs, total, n_rows, n_cols, (int)d,
             (int)trailing, g_index_check);
-    else
-        sddmm_rows_kernel<T, false><<<grid, kWarpsPerBlock * 32, smem, st>>>(
+    return launch_kernel(sddmm_rows_kernel<T, false>, grid, kWarpsPerBlock * 32, smem, st,
             (const T*)q, (const T*)k, ksb, ksc, ksk, (T*)out, lin, tr, nnzs, total, n_rows, n_cols, (int)d,
             (int)trailing, g_index_check);
-    return launch_status();
 }
 
 template <typename T>
@@ -476,20 +488,20 @@ static int32_t softmax_t(const void* s, void* p, const float* nnzs, int64_t bh, 
     T* pb = reinterpret_cast<T*>(pa & ~(uintptr_t)15);
     auto go = [&](auto kern, int rows_per_warp) {
         const int64_t per_block = (int64_t)kSoftmaxWarps * rows_per_warp;
-        kern<<<(unsigned)((total + per_block - 1) / per_block), kSoftmaxWarps * 32, 0, st>>>(
+        return launch_kernel(kern, (unsigned)((total + per_block - 1) / per_block), kSoftmaxWarps * 32, 0, st,
             sb, pb, nnzs, total, n_rows, (int)trailing, lead, scale * kLog2e);
     };
     // (more rows per warp the shorter they are: about 2 KB of loads in flight per warp)
     if (!same)
-        softmax_rows_loop_kernel<T><<<(unsigned)((total + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st>>>(
+        return launch_kernel(softmax_rows_loop_kernel<T>, (unsigned)((total + kWarpsPerBlock - 1) / kWarpsPerBlock),
+                             kWarpsPerBlock * 32, 0, st,
             (const T*)s, (T*)p, nnzs, total, n_rows, (int)trailing, scale * kLog2e);
-    else if (pieces <= 32) go(softmax_rows_kernel<T, 1, 4>, 4);
-    else if (pieces <= 64) go(softmax_rows_kernel<T, 2, 2>, 2);
-    else if (pieces <= 96) go(softmax_rows_kernel<T, 3, 2>, 2);
-    else if (pieces <= 128) go(softmax_rows_kernel<T, 4, 1>, 1);
-    else if (pieces <= 256) go(softmax_rows_kernel<T, 8, 1>, 1);
-    else go(softmax_rows_kernel<T, 16, 1>, 1);
-    return launch_status();
+    if (pieces <= 32) return go(softmax_rows_kernel<T, 1, 4>, 4);
+    if (pieces <= 64) return go(softmax_rows_kernel<T, 2, 2>, 2);
+    if (pieces <= 96) return go(softmax_rows_kernel<T, 3, 2>, 2);
+    if (pieces <= 128) return go(softmax_rows_kernel<T, 4, 1>, 1);
+    if (pieces <= 256) return go(softmax_rows_kernel<T, 8, 1>, 1);
+    return go(softmax_rows_kernel<T, 16, 1>, 1);
 }
 
 template <typename T>
@@ -499,14 +511,12 @@ static int32_t spmm_t(const void* p, const void* v, void* o, const float* lin, c
     const int64_t total = bh * n_rows;
     const unsigned grid = (unsigned)((total + kWarpsPerBlock - 1) / kWarpsPerBlock);
     if (grouped_d_ok(d, DT<T>::kVec) && aligned16(v) && aligned16(o))
-        spmm_rows_kernel<T><<<grid, kWarpsPerBlock * 32, 0, st>>>(
+        return launch_kernel(spmm_rows_kernel<T>, grid, kWarpsPerBlock * 32, 0, st,
             (const T*)p, (const T*)v, (T*)o, lin, tr, nnzs, total, n_rows, n_cols, (int)d,
             (int)trailing, g_index_check);
-    else
-        spmm_rows_scalar_kernel<T><<<grid, kWarpsPerBlock * 32, 0, st>>>(
+    return launch_kernel(spmm_rows_scalar_kernel<T>, grid, kWarpsPerBlock * 32, 0, st,
             (const T*)p, (const T*)v, (T*)o, lin, tr, nnzs, total, n_rows, n_cols, (int)d,
             (int)trailing, g_index_check);
-    return launch_status();
 }
 
 template <typename T>
@@ -522,14 +532,12 @@ static int32_t attention_t(const void* q, const void* k, int64_t ksb, int64_t ks
     const bool contig = ksk == 1 && aligned16(k) && (ksc % DT<T>::kVec == 0) &&
                         (ksb % DT<T>::kVec == 0);
     if (contig)
-        attention_rows_kernel<T, true><<<grid, kWarpsPerBlock * 32, smem, st>>>(
+        return launch_kernel(attention_rows_kernel<T, true>, grid, kWarpsPerBlock * 32, smem, st,
             (const T*)q, (const T*)k, ksb, ksc, ksk, (const T*)v, (T*)o, lin, tr, nnzs, total,
             n_rows, n_cols, (int)d, scale * kLog2e, g_index_check, lse);
-    else
-        attention_rows_kernel<T, false><<<grid, kWarpsPerBlock * 32, smem, st>>>(
+    return launch_kernel(attention_rows_kernel<T, false>, grid, kWarpsPerBlock * 32, smem, st,
             (const T*)q, (const T*)k, ksb, ksc, ksk, (const T*)v, (T*)o, lin, tr, nnzs, total,
             n_rows, n_cols, (int)d, scale * kLog2e, g_index_check, lse);
-    return launch_status();
 }
 
 static bool sizes_ok(int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d, int64_t trailing) {
@@ -565,9 +573,8 @@ extern "C" int32_t splat_transpose_16(const void* in, void* out, int64_t bh, int
     if ((reinterpret_cast<uintptr_t>(out) & 3u) != 0) return SPLAT_ERR_MISALIGNED;
     const int wide = n_cols % 2 == 0 && (reinterpret_cast<uintptr_t>(in) & 3u) == 0;
     const dim3 grid((unsigned)((n_cols + kTransCols - 1) / kTransCols), (unsigned)bh);
-    transpose_16_kernel<<<grid, 256, kTransCols * (d + 2) * 2, (cudaStream_t)stream>>>(
+    return launch_kernel(transpose_16_kernel, grid, 256, kTransCols * (d + 2) * 2, (cudaStream_t)stream,
         (const uint16_t*)in, (uint16_t*)out, (int)d, (int)n_cols, wide);
-    return launch_status();
 }
 
 extern "C" int32_t splat_debug_check_indices(int32_t* status_word) {

@@ -10,14 +10,14 @@
 // their keys: 4.5 TFLOP/s.  A warp here owns 32 rows x 32 keys, a lane an 8 x 4 block of the scores and
 // an 8 x D/8 block of the output.
 //
-// One CTA = RW x 32 rows of one (bh, class) and RW x KW = 4 warps: KW groups take the 32-key steps of
+// One CTA = RW x 32 rows of one (bh, class) and RW x KW warps: KW groups take the 32-key steps of
 // the rows' bands in turn, each group with key and value buffers of its own, each warp with a running
 // maximum, sum and output block of its own; the KW partial results of a row are merged through shared
 // memory at the end.  A group of two warps synchronises with a named barrier, a group of one with
 // itself.  Three CTAs (two at D = 128) share an SM: a warp's loads are covered by the other warps of its
 // scheduler and are not double buffered.
 //   RW = 2, KW = 2  the usual split: every K and V tile serves 64 rows.
-//   RW = 1, KW = 4  for problems too small to fill the GPU with 64-row CTAs (see run()).
+//   RW = 1, KW = 4 or 8  for problems too small to fill the GPU with 64-row CTAs (see run()).
 // The packed FMA (two results per instruction, two cycles of the pipe) leaves the issue slots that the
 // shared-memory reads and the operand duplication need; in a loop of nothing but such updates an
 // 8 x 8 block takes 75 to 78 cycles instead of 64 (packed) and 77 to 83 (scalar).
@@ -43,9 +43,7 @@
 namespace splat {
 namespace tile {
 
-constexpr int kWarps = 4;
 constexpr int kKeys = 32;            // keys of a step
-constexpr int kThreads = 32 * kWarps;
 
 enum class Op { kFused, kSddmm, kSpmm };
 
@@ -88,8 +86,9 @@ template <int N> __device__ __forceinline__ void cp_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int D, int RW, Op OP> struct Layout {
-    static constexpr int kGroups = kWarps / RW;
+template <int D, int RW, int KW, Op OP> struct Layout {
+    static constexpr int kWarps = RW * KW;
+    static constexpr int kGroups = KW;
     static constexpr int kRows = 32 * RW;
     static constexpr bool kOneBuffer = D == 128 && RW == 1 && OP == Op::kFused;   // V follows K through one buffer
     static constexpr int kQ = OP == Op::kSpmm ? 0 : D * kRows;
@@ -103,7 +102,7 @@ template <int D, int RW, Op OP> struct Layout {
     static constexpr int kPart = 32 * D + 64;           // a warp's partial result: O[32][D], maxima, sums
     static constexpr int kMain = kQ + kGroups * kGroupFloats;
     static constexpr int kFloats = OP == Op::kSddmm || kMain > kWarps * kPart ? kMain : kWarps * kPart;
-    static constexpr int kPerSm = D == 128 ? 2 : 3;     // CTAs per SM the registers are budgeted for
+    static constexpr int kPerSm = KW == 8 ? 1 : (D == 128 ? 2 : 3);     // CTAs per SM the registers are budgeted for
 };
 
 // acc[8 rows][NP pairs of columns] += a[8] x b[NP]
@@ -173,11 +172,13 @@ __device__ __forceinline__ void load_v(float* smem, const float* base, int64_t p
     }
 }
 
-template <int D, int RW, Op OP>
-__global__ void __launch_bounds__(kThreads, Layout<D, RW, OP>::kPerSm) tile_kernel(const Params p) {
-    using L = Layout<D, RW, OP>;
-    constexpr int kRows = L::kRows, kGroups = L::kGroups;
+template <int D, int RW, int KW, Op OP>
+__global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) tile_kernel(const Params p) {
+    using L = Layout<D, RW, KW, OP>;
+    constexpr int kRows = L::kRows, kGroups = L::kGroups, kWarps = L::kWarps;
     extern __shared__ __align__(16) float smem[];
+    depend_wait();
+    depend_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = lane >> 3, t = lane & 7;
     float* s_q = smem;
@@ -237,6 +238,17 @@ __global__ void __launch_bounds__(kThreads, Layout<D, RW, OP>::kPerSm) tile_kern
             else load_transposed<D, kKeys, RW>(s_k, kbase, pitch, c0, rows_v, rw);
         }
         if (OP != Op::kSddmm && !L::kOneBuffer) load_v<D, RW>(s_v, vbase, pitch, c0, rows_v, rw);
+        if (OP == Op::kSpmm) {     // this warp's rows of P into Pt, one row per round, lanes along the keys
+#pragma unroll 8
+            for (int rr = 0; rr < 32; ++rr) {
+                const int lo = __shfl_sync(0xffffffffu, my_a, rr) - c0;
+                const int n = __shfl_sync(0xffffffffu, my_n, rr);
+                const float* src = p.sparse + (head + (int64_t)(u0 + rr) * p.stride + res) * p.trailing - lo;
+                const bool in = lane >= lo && lane < lo + n;
+                cp4((uint32_t)__cvta_generic_to_shared(s_p + lane * 32 + ((((rr >> 2) ^ (lane >> 2)) << 2) | (rr & 3))),
+                    in ? src + lane : p.sparse, in);
+            }
+        }
         cp_commit();
     };
     if (c_first < c_end) load_keys(c_first);
@@ -335,27 +347,19 @@ __global__ void __launch_bounds__(kThreads, Layout<D, RW, OP>::kPerSm) tile_kern
                 *reinterpret_cast<float4*>(row + ((r ^ t) << 2)) = make_float4(x[0], x[1], x[2], x[3]);
                 *reinterpret_cast<float4*>(row + (((r + 4) ^ t) << 2)) = make_float4(x[4], x[5], x[6], x[7]);
             }
-        } else if (active) {
-            if (OP == Op::kSddmm) {
-                // through the warp's tile [32 rows][32 keys] to row-wise coalesced stores
+        } else if (active && OP == Op::kSddmm) {
+            // through the warp's tile [32 rows][32 keys] to row-wise coalesced stores
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    *reinterpret_cast<float4*>(s_p + row_of(i) * 32 + 4 * t) =
-                        make_float4(s[i][0].x, s[i][0].y, s[i][1].x, s[i][1].y);
-                __syncwarp();
-            }
-            // one row per round, lanes along the keys: S out of the tile, or P into Pt
+            for (int i = 0; i < 8; ++i)
+                *reinterpret_cast<float4*>(s_p + row_of(i) * 32 + 4 * t) =
+                    make_float4(s[i][0].x, s[i][0].y, s[i][1].x, s[i][1].y);
+            __syncwarp();
 #pragma unroll 8
             for (int rr = 0; rr < 32; ++rr) {
                 const int lo = __shfl_sync(0xffffffffu, my_a, rr) - c0;
                 const int n = __shfl_sync(0xffffffffu, my_n, rr);
                 float* mem = p.sparse + (head + (int64_t)(u0 + rr) * p.stride + res) * p.trailing - lo;
-                const bool in = lane >= lo && lane < lo + n;
-                if (OP == Op::kSddmm) {
-                    if (in) mem[lane] = s_p[rr * 32 + lane];
-                } else {
-                    s_p[lane * 32 + ((((rr >> 2) ^ (lane >> 2)) << 2) | (rr & 3))] = in ? mem[lane] : 0.f;
-                }
+                if (lane >= lo && lane < lo + n) mem[lane] = s_p[rr * 32 + lane];
             }
         }
         if (OP != Op::kSddmm) {
@@ -488,25 +492,26 @@ bool index_check_on();                                    // ops_generic.cu
 
 namespace tile {
 
-template <int D, int RW, Op OP>
+template <int D, int RW, int KW, Op OP>
 static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
-    constexpr int bytes = Layout<D, RW, OP>::kFloats * (int)sizeof(float);
-    auto kern = tile_kernel<D, RW, OP>;
+    constexpr int bytes = Layout<D, RW, KW, OP>::kFloats * (int)sizeof(float);
+    auto kern = tile_kernel<D, RW, KW, OP>;
     if (!band::allow_dynamic_smem(reinterpret_cast<const void*>(kern), bytes)) return SPLAT_ERR_LAUNCH;
     p.tiles = ((p.n_rows + p.stride - 1) / p.stride + 32 * RW - 1) / (32 * RW);
     const int64_t blocks = (int64_t)p.tiles * p.stride * bh;
     if (blocks > INT32_MAX) return SPLAT_ERR_UNSUPPORTED_SHAPE;
-    kern<<<(unsigned)blocks, kThreads, bytes, st>>>(p);
-    return launch_status();
+    return launch_kernel(kern, (unsigned)blocks, 32 * RW * KW, bytes, st, p);
 }
 
 // 64-row CTAs unless they leave SMs without their three CTAs: then 32-row CTAs, whose four warps share the
-// keys of one row block, finish sooner (L 1024, 8 heads, d 64, window 129: SDDMM + softmax + SpMM calls
-// 73 -> 41 us with host time), while with the GPU full they load every key twice as often.
+// keys of one row block, finish sooner, while with the GPU full they load every key twice as often; and with
+// less than two such CTAs per SM eight warps share them.
 template <int D, Op OP>
 static int32_t run(const Params& p, int64_t bh, cudaStream_t st) {
-    const int64_t blocks = (((int64_t)p.n_rows + p.stride - 1) / p.stride + 63) / 64 * p.stride * bh;
-    return blocks < 3 * 148 ? launch<D, 1, OP>(p, bh, st) : launch<D, 2, OP>(p, bh, st);
+    const int64_t rows = ((int64_t)p.n_rows + p.stride - 1) / p.stride, classes = p.stride * bh;
+    if ((rows + 63) / 64 * classes >= 3 * 148) return launch<D, 2, 2, OP>(p, bh, st);
+    if ((rows + 31) / 32 * classes >= 2 * 148) return launch<D, 1, 4, OP>(p, bh, st);
+    return launch<D, 1, 8, OP>(p, bh, st);
 }
 
 }  // namespace tile
@@ -514,13 +519,16 @@ static int32_t run(const Params& p, int64_t bh, cudaStream_t st) {
 // Fills p and says whether the tile kernels take the problem (SPLAT_ERR_UNSUPPORTED_SHAPE if not).
 // plan: {max_nnz, stride_min, stride_max, misaligned, n_single, max_col+1, n_empty, n_multi}
 static int32_t tile_setup(tile::Params& p, const int32_t* plan, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
-                          int64_t ksb, int64_t ksc, int64_t ksk, bool has_k) {
+                          int64_t ksb, int64_t ksc, int64_t ksk, bool has_k, int64_t min_rows) {
     if (index_check_on()) return SPLAT_ERR_UNSUPPORTED_SHAPE;   // checked columns: the row kernels
     if (plan == nullptr || bh < 1 || n_rows < 1 || n_rows != n_cols || n_rows > INT32_MAX) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     if (d != 32 && d != 64 && d != 128) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     const int64_t stride = plan[7] > 0 ? plan[1] : 1;
     if ((plan[7] > 0 && plan[1] != plan[2]) || plan[3] != 0 || stride < 1 || plan[5] > n_cols)
         return SPLAT_ERR_UNSUPPORTED_SHAPE;
+    // Short classes leave most of a tile empty: strided patterns, 16 to 32 heads, tile against row kernel at 16 / 22 /
+    // 32 / 43 rows per class 0.7 / 0.9 / 1.5 / 2.1 times as fast (fused, SDDMM), SpMM 0.4 / - / 0.85 / -.
+    if ((n_rows + stride - 1) / stride < min_rows && stride > 1) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     p.kt = p.kt_vec = 0;
     if (has_k) {
         const bool k_major = ksk == 1 && ksc == d && ksb == n_cols * d;
@@ -546,7 +554,7 @@ int32_t attention_tile_f32(const void* q, const void* k, int64_t ksb, int64_t ks
                            int64_t n_cols, int64_t d, float scale, const int32_t* plan, float* lse, cudaStream_t st) {
     tile::Params p{};
     if (!q || !k || !v || !o || !lin || !tr || !nnzs) return SPLAT_ERR_UNSUPPORTED_SHAPE;   // left to the row kernel
-    const int32_t rc = tile_setup(p, plan, bh, n_rows, n_cols, d, ksb, ksc, ksk, true);
+    const int32_t rc = tile_setup(p, plan, bh, n_rows, n_cols, d, ksb, ksc, ksk, true, 24);
     if (rc != SPLAT_OK) return rc;
     if (!aligned16(k) || !aligned16(v) || !aligned16(o)) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     p.q = (const float*)q; p.k = (const float*)k; p.v = (const float*)v; p.o = (float*)o; p.lse = lse;
@@ -565,7 +573,7 @@ extern "C" int32_t splat_sddmm_tile(const void* q, const void* k, int64_t k_stri
     if (bh < 0 || n_rows < 0 || trailing_dim < 0) return SPLAT_ERR_BAD_ARG;
     if (dtype != SPLAT_F32 || trailing_dim < 1 || trailing_dim > INT32_MAX) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     tile::Params p{};
-    const int32_t rc = tile_setup(p, plan_i32, bh, n_rows, n_cols, d, k_stride_bh, k_stride_col, k_stride_k, true);
+    const int32_t rc = tile_setup(p, plan_i32, bh, n_rows, n_cols, d, k_stride_bh, k_stride_col, k_stride_k, true, 24);
     if (rc != SPLAT_OK) return rc;
     if (!q || !k || !s_out || !sTod_lin || !sTod_tr || !nnzs) return SPLAT_ERR_BAD_ARG;
     if (plan_i32[0] > trailing_dim) return SPLAT_ERR_UNSUPPORTED_SHAPE;
@@ -581,7 +589,7 @@ extern "C" int32_t splat_spmm_tile(const void* p_in, const void* v, void* o, con
     if (bh < 0 || n_rows < 0 || trailing_dim < 0) return SPLAT_ERR_BAD_ARG;
     if (dtype != SPLAT_F32 || trailing_dim < 1 || trailing_dim > INT32_MAX) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     tile::Params p{};
-    const int32_t rc = tile_setup(p, plan_i32, bh, n_rows, n_cols, d, 0, 0, 0, false);
+    const int32_t rc = tile_setup(p, plan_i32, bh, n_rows, n_cols, d, 0, 0, 0, false, 40);
     if (rc != SPLAT_OK) return rc;
     if (!p_in || !v || !o || !sTod_lin || !sTod_tr || !nnzs) return SPLAT_ERR_BAD_ARG;
     if (plan_i32[0] > trailing_dim) return SPLAT_ERR_UNSUPPORTED_SHAPE;
