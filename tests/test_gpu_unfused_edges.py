@@ -77,3 +77,21 @@ def test_softmax_row_lengths(dtype, lead):
             xd.copy_(torch.where(valid, x, torch.full_like(x, float("nan"))))     # padding is not read
             n.softmax(xd, xd, nnz.float().cuda(), T, scale)
             assert_close(xd, ref, dtype, f"softmax T={T} scale={scale}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_softmax_lanes_per_row(dtype):
+    """Both sides of every change in how many lanes and warps share a row; fewer rows than a block takes, and more."""
+    import splat_native as n
+    v = 4 if dtype == torch.float32 else 8
+    for pieces in (8, 16, 24, 32, 40, 64, 80, 96, 128, 160, 192, 256, 384, 512, 768, 1024, 2048):
+        for T, L in ((pieces * v, 3), (pieces * v, 131), (pieces * v + 1, 5)):
+            torch.manual_seed(T + L)
+            nnz = torch.randint(0, T + 1, (L,))
+            nnz[0], nnz[1] = T, 0
+            x = torch.randn(1, 1, L, T).to(dtype)
+            valid = torch.arange(T)[None, :] < nnz[:, None]
+            ref = torch.softmax(torch.where(valid, x.float() * 0.7, torch.tensor(-torch.inf)), -1).nan_to_num(0.0)
+            out = torch.full((1, 1, L, T), float("nan"), dtype=dtype, device="cuda")
+            n.softmax(x.cuda(), out, nnz.float().cuda(), T, 0.7)
+            assert_close(out, ref, dtype, f"softmax T={T} L={L}")

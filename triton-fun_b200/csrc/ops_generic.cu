@@ -13,6 +13,8 @@
 //   fused  : 32 slots at a time -- scores as in SDDMM, online max/sum with exp2 and the softmax
 //            scale folded into the exponent, then the SpMM accumulation with the probabilities
 //            broadcast by shuffle.
+#include <limits.h>
+
 #include "common.cuh"
 #include "softmax_math.cuh"
 
@@ -97,37 +99,54 @@ sddmm_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t ksb,
 }
 
 // ---------------------------------------------------------------------------------------------
-// Row softmax.  A warp takes R rows at a time and keeps them in registers, NV 16-byte pieces per lane and row; all
-// loads are issued before the first reduction, so that enough bytes are in flight to keep HBM busy.  The pieces
+// Row softmax.  G lanes hold a row in registers, NV 16-byte pieces each (R rows of short ones); all loads are issued
+// before the first reduction, so that enough bytes are in flight to keep HBM busy.  Few lanes per row: the
+// shuffles of the two reductions and a row's fixed work (its number of non-zeros, addresses, a division) are per
+// lane and row, and with 32 lanes and one piece each they were two thirds of the instructions, at 57 % of the
+// issue slots.  Long rows: several warps, which exchange two numbers through shared memory.  The pieces
 // are those of the array, not of the row: a row that begins inside a piece (odd trailing dimensions) masks
 // the neighbours' elements when reading, and stores its first and last piece element by element.  Rows
-// longer than kSoftmaxMaxVec pieces per lane take the loop kernel, which reads a row three times.
-// B4 H16 L4096, T = 256 fp16: @@@; T = 257: @@@.
+// longer than kSoftmaxMaxPieces take the loop kernel, which reads a row three times.
+// 262 144 rows, us, with a warp per row -> now: T = 35 fp16 71.5 -> 20.8, 64 60.8 -> 14.9, 256 59.7 -> 41.1
+// (6.5 TB/s), 257 99.8 -> 52.2, 1024 184 -> 164; T = 257 fp32 118.5 -> 79.9 (6.7 TB/s); 65 536 rows, T = 4096: fp16
+// 339 -> 186, fp32 855 -> 316.
 // ---------------------------------------------------------------------------------------------
 constexpr int kSoftmaxWarps = 8;
-constexpr int kSoftmaxMaxVec = 16;
+constexpr int kSoftmaxMaxPieces = 8 * 32 * kSoftmaxWarps;
 
-template <typename T, int NV, int R>
+template <typename T, int G, int NV, int R>
 __global__ void __launch_bounds__(kSoftmaxWarps * 32)
 softmax_rows_kernel(const T* s, T* p, const float* __restrict__ nnzs, int64_t total_rows, int64_t n_rows, int trailing,
                     int lead, float scale_log2e) {
     depend_wait();
     depend_release();
     constexpr int V = DT<T>::kVec;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t grow0 = ((int64_t)blockIdx.x * kSoftmaxWarps + warp) * R;
-    if (grow0 >= total_rows) return;
-    const int64_t in_head0 = grow0 % n_rows;   // one 64-bit division per warp
+    constexpr int kRows = kSoftmaxWarps * 32 / G;              // rows side by side in the block
+    __shared__ float part[2][kSoftmaxWarps];
+    const int lane = threadIdx.x & (G - 1);
+    const int64_t grow0 = (int64_t)blockIdx.x * (R * kRows) + threadIdx.x / G;
+    // `m` or `sum` of the row's other warps, if it has more than one
+    auto across_warps = [&](int which, float x, auto op) {
+        if (G <= 32) return x;
+        const int warp = threadIdx.x >> 5, first_warp = warp & ~(G / 32 - 1);
+        if ((threadIdx.x & 31) == 0) part[which][warp] = x;
+        __syncthreads();
+        x = part[which][first_warp];
+#pragma unroll
+        for (int w = 1; w < G / 32; ++w) x = op(x, part[which][first_warp + w]);
+        return x;
+    };
+    const int64_t in_head0 = total_rows <= UINT_MAX ? (uint32_t)grow0 % (uint32_t)n_rows : grow0 % n_rows;
     uint4 raw[R][NV];
     int first[R], nnz[R];       // slot of this lane's first element
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         nnz[r] = 0;
         // s and p are rounded down to 16 bytes; `lead` elements were lost by that
-        const int64_t e = lead + (grow0 + r) * trailing;
+        const int64_t e = lead + (grow0 + r * kRows) * trailing;
         first[r] = lane * V - (int)(e & (V - 1));
-        if (grow0 + r < total_rows) {
-            int64_t in_head = in_head0 + r;
+        if (grow0 + r * kRows < total_rows) {
+            int64_t in_head = in_head0 + r * kRows;
             while (in_head >= n_rows) in_head -= n_rows;
             const int n = (int)rintf(__ldg(nnzs + in_head));
             nnz[r] = n < 0 ? 0 : (n > trailing ? trailing : n);
@@ -135,11 +154,10 @@ softmax_rows_kernel(const T* s, T* p, const float* __restrict__ nnzs, int64_t to
         const T* row = s + (e & ~(int64_t)(V - 1)) + lane * V;
 #pragma unroll
         for (int v = 0; v < NV; ++v)
-            if (first[r] + v * 32 * V < nnz[r] && first[r] + v * 32 * V > -V)
-                raw[r][v] = *reinterpret_cast<const uint4*>(row + v * 32 * V);
+            if (first[r] + v * G * V < nnz[r] && first[r] + v * G * V > -V)
+                raw[r][v] = *reinterpret_cast<const uint4*>(row + v * G * V);
     }
-    constexpr bool kKeep = NV <= 2;            // exponentials kept in registers, else formed again for the output
-    float2 vals[kKeep ? R : 1][kKeep ? NV : 1][V / 2];
+    float2 vals[R][NV][V / 2];
     float m[R], sum[R];
     const float2 sc2 = make_float2(scale_log2e, scale_log2e);
     // scaled scores of a piece; elements outside the row's non-zeros -inf (a warp whose pieces are all inside them
@@ -148,7 +166,7 @@ softmax_rows_kernel(const T* s, T* p, const float* __restrict__ nnzs, int64_t to
         const T* e = reinterpret_cast<const T*>(&raw[r][v]);
 #pragma unroll
         for (int t = 0; t < V / 2; ++t) x[t] = sm::mul2(make_float2(DT<T>::to_f(e[2 * t]), DT<T>::to_f(e[2 * t + 1])), sc2);
-        const int j = first[r] + v * 32 * V;
+        const int j = first[r] + v * G * V;
         if (!__all_sync(0xffffffffu, j >= 0 && j + V <= nnz[r])) {
 #pragma unroll
             for (int t = 0; t < V / 2; ++t) {
@@ -172,26 +190,24 @@ softmax_rows_kernel(const T* s, T* p, const float* __restrict__ nnzs, int64_t to
         m[r] = -INFINITY;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            float2 tmp[V / 2];
-            float2 (&x)[V / 2] = kKeep ? vals[kKeep ? r : 0][kKeep ? v : 0] : tmp;
+            float2 (&x)[V / 2] = vals[r][v];
             scores(r, v, x);
 #pragma unroll
             for (int t = 0; t < V / 2; ++t) m[r] = sm::fmax3(m[r], x[t].x, x[t].y);
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = (G < 32 ? G : 32) / 2; o > 0; o >>= 1)
 #pragma unroll
         for (int r = 0; r < R; ++r) m[r] = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], o));
 #pragma unroll
     for (int r = 0; r < R; ++r) {
+        m[r] = across_warps(0, m[r], [](float a, float b) { return fmaxf(a, b); });
         m[r] = m[r] == -INFINITY ? 0.f : m[r];
         float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            float2 tmp[V / 2];
-            float2 (&x)[V / 2] = kKeep ? vals[kKeep ? r : 0][kKeep ? v : 0] : tmp;
-            if (!kKeep) scores(r, v, x);
+            float2 (&x)[V / 2] = vals[r][v];
             exponentials(x, m[r]);
 #pragma unroll
             for (int t = 0; t < V / 2; ++t) acc = sm::add2(acc, x[t]);
@@ -199,34 +215,29 @@ softmax_rows_kernel(const T* s, T* p, const float* __restrict__ nnzs, int64_t to
         sum[r] = acc.x + acc.y;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = (G < 32 ? G : 32) / 2; o > 0; o >>= 1)
 #pragma unroll
         for (int r = 0; r < R; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        if (grow0 + r >= total_rows) break;
+        sum[r] = across_warps(1, sum[r], [](float a, float b) { return a + b; });
         const float inv = sum[r] > 0.f ? 1.f / sum[r] : 0.f;
         const float2 inv2 = make_float2(inv, inv);
-        const int64_t e = lead + (grow0 + r) * trailing;
+        const int64_t e = lead + (grow0 + r * kRows) * trailing;
         T* row = p + (e & ~(int64_t)(V - 1)) + lane * V;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            const int j0 = first[r] + v * 32 * V;
-            float2 tmp[V / 2];
-            float2 (&x)[V / 2] = kKeep ? vals[kKeep ? r : 0][kKeep ? v : 0] : tmp;
-            if (!kKeep) {
-                scores(r, v, x);
-                exponentials(x, m[r]);
-            }
+            const int j0 = grow0 + r * kRows < total_rows ? first[r] + v * G * V : trailing;
+            float2 (&x)[V / 2] = vals[r][v];
 #pragma unroll
             for (int t = 0; t < V / 2; ++t) x[t] = sm::mul2(x[t], inv2);
             const float* out = reinterpret_cast<const float*>(&x[0]);
             if (j0 >= 0 && j0 + V <= trailing) {
-                store16_from_float(row + v * 32 * V, out);
+                store16_from_float(row + v * G * V, out);
             } else if (j0 > -V && j0 < trailing) {
 #pragma unroll
                 for (int t = 0; t < V; ++t)
-                    if (j0 + t >= 0 && j0 + t < trailing) row[v * 32 * V + t] = DT<T>::from_f(out[t]);
+                    if (j0 + t >= 0 && j0 + t < trailing) row[v * G * V + t] = DT<T>::from_f(out[t]);
             }
         }
     }
@@ -483,25 +494,35 @@ static int32_t softmax_t(const void* s, void* p, const float* nnzs, int64_t bh, 
     const int lead = (int)(sa & 15) / (int)sizeof(T);
     // pieces a row can reach into: its own, and one more where rows do not begin with a piece
     const int64_t pieces = (trailing + V - 1) / V + (lead != 0 || trailing % V != 0 ? 1 : 0);
-    const bool same = (sa & 15) == (pa & 15) && (sa & 15) % sizeof(T) == 0 && pieces <= 32 * kSoftmaxMaxVec;
+    const bool same = (sa & 15) == (pa & 15) && (sa & 15) % sizeof(T) == 0 && pieces <= kSoftmaxMaxPieces;
     const T* sb = reinterpret_cast<const T*>(sa & ~(uintptr_t)15);
     T* pb = reinterpret_cast<T*>(pa & ~(uintptr_t)15);
-    auto go = [&](auto kern, int rows_per_warp) {
-        const int64_t per_block = (int64_t)kSoftmaxWarps * rows_per_warp;
+    auto go = [&](auto kern, int per_block) {
         return launch_kernel(kern, (unsigned)((total + per_block - 1) / per_block), kSoftmaxWarps * 32, 0, st,
             sb, pb, nnzs, total, n_rows, (int)trailing, lead, scale * kLog2e);
     };
-    // (more rows per warp the shorter they are: about 2 KB of loads in flight per warp)
     if (!same)
         return launch_kernel(softmax_rows_loop_kernel<T>, (unsigned)((total + kWarpsPerBlock - 1) / kWarpsPerBlock),
                              kWarpsPerBlock * 32, 0, st,
             (const T*)s, (T*)p, nnzs, total, n_rows, (int)trailing, scale * kLog2e);
-    if (pieces <= 32) return go(softmax_rows_kernel<T, 1, 4>, 4);
-    if (pieces <= 64) return go(softmax_rows_kernel<T, 2, 2>, 2);
-    if (pieces <= 96) return go(softmax_rows_kernel<T, 3, 2>, 2);
-    if (pieces <= 128) return go(softmax_rows_kernel<T, 4, 1>, 1);
-    if (pieces <= 256) return go(softmax_rows_kernel<T, 8, 1>, 1);
-    return go(softmax_rows_kernel<T, 16, 1>, 1);
+    // as few lanes per row as hold it in five pieces each, but eight at least (128 contiguous bytes)
+    if (pieces <= 8) return go(softmax_rows_kernel<T, 8, 1, 4>, 128);
+    if (pieces <= 16) return go(softmax_rows_kernel<T, 8, 2, 2>, 64);
+    if (pieces <= 24) return go(softmax_rows_kernel<T, 8, 3, 1>, 32);
+    if (pieces <= 32) return go(softmax_rows_kernel<T, 8, 4, 1>, 32);
+    if (pieces <= 40) return go(softmax_rows_kernel<T, 8, 5, 1>, 32);
+    if (pieces <= 64) return go(softmax_rows_kernel<T, 16, 4, 1>, 16);
+    if (pieces <= 80) return go(softmax_rows_kernel<T, 16, 5, 1>, 16);
+    if (pieces <= 96) return go(softmax_rows_kernel<T, 32, 3, 1>, 8);
+    if (pieces <= 128) return go(softmax_rows_kernel<T, 32, 4, 1>, 8);
+    if (pieces <= 160) return go(softmax_rows_kernel<T, 32, 5, 1>, 8);
+    if (pieces <= 192) return go(softmax_rows_kernel<T, 64, 3, 1>, 4);
+    if (pieces <= 256) return go(softmax_rows_kernel<T, 64, 4, 1>, 4);
+    if (pieces <= 384) return go(softmax_rows_kernel<T, 128, 3, 1>, 2);
+    if (pieces <= 512) return go(softmax_rows_kernel<T, 128, 4, 1>, 2);
+    if (pieces <= 768) return go(softmax_rows_kernel<T, 256, 3, 1>, 1);
+    if (pieces <= 1024) return go(softmax_rows_kernel<T, 256, 4, 1>, 1);
+    return go(softmax_rows_kernel<T, 256, 8, 1>, 1);
 }
 
 template <typename T>
