@@ -285,6 +285,8 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     klo = lo64 >> 1;
     const int steps = ((hi64 + 1) >> 1) - klo;   // 128-key steps
     auto wait_all = [&](uint64_t* bar, uint32_t parity, int code) {
+        // (a uniform branch around the polling loop: 60 cycles when ready, 130 with a divergent one)
+        if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
         const bool r = wait_bar(bar, parity, p.status, code);
         return __all_sync(0xffffffffu, r) != 0;
     };
