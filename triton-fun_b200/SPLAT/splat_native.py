@@ -553,4 +553,4 @@ def module_forward(attributes: dict, x):
 
 _host.bind(*(ctypes.cast(getattr(_lib, name), _vp).value for name in (
     "splat_attention_fused_table", "splat_sddmm_band_table", "splat_spmm_band_table", "splat_sddmm_tile", "splat_spmm_tile",
-    "splat_softmax", "splat_acsr_from_mask_u8", "splat_transpose_16")), _warn_cuda_core_16bit)
+    "splat_softmax", "splat_acsr_from_mask_u8", "splat_transpose_16", "splat_sddmm", "splat_spmm")), _warn_cuda_core_16bit)

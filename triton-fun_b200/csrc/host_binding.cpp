@@ -39,6 +39,10 @@ using SddmmTileFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int6
                                 const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
 using SpmmTileFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
                                int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
+using SddmmFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, void*, const float*, const float*,
+                            const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, void*);
+using SpmmFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
+                           int64_t, int64_t, int64_t, int32_t, void*);
 using MaskFn = int32_t (*)(const void*, int64_t, int64_t, int64_t, int32_t, float*, float*, float*, float*, float*, float*, float*,
                            int32_t*, int32_t*, void*);
 using TransposeFn = int32_t (*)(const void*, void*, int64_t, int64_t, int64_t, void*);
@@ -53,6 +57,8 @@ struct Api {
     SoftmaxFn softmax;
     MaskFn mask;
     TransposeFn transpose;
+    SddmmFn sddmm;
+    SpmmFn spmm;
 } g_api{};
 
 // Per device: the status word (device memory) and its host copy, which the kernels write.
@@ -62,6 +68,18 @@ struct Status {
 } g_status[kMaxDevices];
 
 PyObject* g_warn = nullptr;   // splat_native's one-time warning, until it has been given
+
+void warn_once(const char* what) {     // 16-bit operands on the CUDA cores
+    if (g_warn == nullptr) return;
+    PyObject* cb = g_warn;
+    g_warn = nullptr;
+    PyObject* r = PyObject_CallFunction(cb, "s", what);
+    Py_DECREF(cb);
+    if (r == nullptr) PyErr_Clear();
+    else Py_DECREF(r);
+}
+// return codes of the tile and band kernels that mean "use the row kernels": misaligned, unsupported shape, no tensor map
+bool not_applicable(int32_t rc) { return rc == -3 || rc == -6 || rc == -7; }
 PyObject *k_lin, *k_tr, *k_nnzs, *k_out, *k_scale, *k_path, *k_plan, *k_lse, *k_cached_plan;
 
 inline const at::Tensor* tensor(PyObject* o) {
@@ -205,14 +223,7 @@ bool fused(const at::Tensor* q, const at::Tensor* kt, const at::Tensor* v, const
                                    v->const_data_ptr(), out->data_ptr(), plse, pl, pt, pn, B * H, L, n_cols, d, scale, dtype,
                                    static_cast<int32_t>(path), with_plan ? plan : nullptr, table, g_status[dev].word, &ran, stream);
     if (rc != 0) return false;
-    if (ran != kPathBand && dtype != 0 && path == kPathAuto && g_warn != nullptr) {   // 16 bit on the CUDA cores: say so once
-        PyObject* cb = g_warn;
-        g_warn = nullptr;
-        PyObject* r = PyObject_CallFunction(cb, "s", "attention");
-        Py_DECREF(cb);
-        if (r == nullptr) PyErr_Clear();
-        else Py_DECREF(r);
-    }
+    if (ran != kPathBand && dtype != 0 && path == kPathAuto) warn_once("attention");
     return true;
 }
 
@@ -283,11 +294,15 @@ PyObject* sddmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const void* yp = copied ? rows.const_data_ptr() : y->const_data_ptr();
     const int64_t ksc = copied ? d : y->stride(3), ksk = copied ? 1 : y->stride(2);
     if (copied) ksb = n_cols * d;
-    const int32_t rc =
+    int32_t rc =
         dtype == 0 ? g_api.sddmm_tile(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
                                       L, n_cols, d, trailing, dtype, plan, st)
                    : g_api.sddmm_band(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
                                       L, n_cols, d, trailing, dtype, plan, table, g_status[dev].word, st);
+    if (not_applicable(rc)) {
+        if (dtype != 0) warn_once("sddmm");
+        rc = g_api.sddmm(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H, L, n_cols, d, trailing, dtype, st);
+    }
     return yes_or_none(rc == 0);
 }
 
@@ -312,10 +327,14 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int32_t* table = nullptr;
     if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, &table)) return yes_or_none(false);
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
-    const int32_t rc = dtype == 0 ? g_api.spmm_tile(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
+    int32_t rc = dtype == 0 ? g_api.spmm_tile(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
                                                     n_cols, d, T, dtype, plan, st)
                                   : g_api.spmm_band(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
                                                     n_cols, d, T, dtype, plan, table, g_status[dev].word, st);
+    if (not_applicable(rc)) {
+        if (dtype != 0) warn_once("spmm");
+        rc = g_api.spmm(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L, n_cols, d, T, dtype, st);
+    }
     return yes_or_none(rc == 0);
 }
 
@@ -338,12 +357,12 @@ PyObject* softmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return yes_or_none(rc == 0);
 }
 
-// bind(fused, sddmm_band, spmm_band, sddmm_tile, spmm_tile, softmax, mask, transpose, warn): addresses of the C ABI entry points
+// bind(fused, sddmm_band, spmm_band, sddmm_tile, spmm_tile, softmax, mask, transpose, sddmm, spmm, warn): addresses of the C ABI entry points
 // and the function that warns of 16-bit operands on the CUDA-core kernels
 PyObject* bind(PyObject*, PyObject* args) {
-    unsigned long long f[8];
+    unsigned long long f[10];
     PyObject* warn;
-    if (!PyArg_ParseTuple(args, "KKKKKKKKO", f, f + 1, f + 2, f + 3, f + 4, f + 5, f + 6, f + 7, &warn)) return nullptr;
+    if (!PyArg_ParseTuple(args, "KKKKKKKKKKO", f, f + 1, f + 2, f + 3, f + 4, f + 5, f + 6, f + 7, f + 8, f + 9, &warn)) return nullptr;
     Py_INCREF(warn);
     g_warn = warn;
     g_api.fused = reinterpret_cast<FusedFn>(f[0]);
@@ -354,6 +373,8 @@ PyObject* bind(PyObject*, PyObject* args) {
     g_api.softmax = reinterpret_cast<SoftmaxFn>(f[5]);
     g_api.mask = reinterpret_cast<MaskFn>(f[6]);
     g_api.transpose = reinterpret_cast<TransposeFn>(f[7]);
+    g_api.sddmm = reinterpret_cast<SddmmFn>(f[8]);
+    g_api.spmm = reinterpret_cast<SpmmFn>(f[9]);
     Py_RETURN_NONE;
 }
 
