@@ -21,7 +21,7 @@
 //     (gathers, a division per row, a reduction over the block) cost 1 500 cycles of a CTA's 15 000 to
 //     30 000 at stride 1 and 3 800 at stride 64; it remains for callers without a table.
 //   * Any d that is a multiple of 8 up to 128 runs: the copies fill a tile's columns past d with zeros, and
-//     the store clips them.  Any L: classes of unequal length are two launches.
+//     the store clips them.  Any L: see band_classes.cuh.
 // Softmax step of 128 keys by itself (no MMAs, cycles for one / two warps per scheduler): row in registers
 // 1468 / 2262, four chunks with the maximum looked at per chunk 1655 / 2403, a quarter of the exponentials
 // by polynomial on the FMA pipe 1414 / 2002; 64-key steps 2 x 900 / 2 x 1140.  In the kernel the chunked
@@ -30,6 +30,7 @@
 #include <limits.h>
 #include <type_traits>
 
+#include "band_classes.cuh"
 #include "common.cuh"
 #include "softmax_math.cuh"
 #include "tc_ptx.cuh"
@@ -38,12 +39,6 @@ namespace splat {
 namespace band {
 
 using namespace tc;
-
-// defined in attention_band.cu
-bool allow_dynamic_smem(const void* kernel, int bytes);
-bool make_map_view(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_rows, int64_t d, int64_t stride,
-                   int64_t res0, int64_t count, int64_t rows, int box_rows);
-bool make_map_kt(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_cols, int64_t d, int64_t box_d);
 
 namespace wide {
 
@@ -80,12 +75,8 @@ struct Params {
     int32_t* status;
     int32_t* mirror;   // host copy of the status word, or null
     int64_t n_rows;    // L
-    int rows_v;        // rows of a class
+    Classes cls;
     int stride;
-    int res0;          // residue of this launch's first class
-    int row0;          // of which class in the band table
-    int tile0;
-    int tile_pitch;    // tiles of a class in the band table
     int d;             // real head dimension, <= D and a multiple of 8 (the rest of a tile is zero)
     int kt_major;
     float scale_log2;
@@ -150,8 +141,7 @@ __device__ __noinline__ void rescale_o(uint32_t o_addr, int n, float corr) {
 
 template <typename T, int D, bool kLse>
 __global__ void __launch_bounds__(kThreads, 2)
-attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Params p) {
+attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     using L = Layout<D>;
     constexpr int kSlots = L::kSlots;
     constexpr bool kOwnP = D == 64;              // P has tensor-memory columns of its own
@@ -160,10 +150,11 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     Control* ctrl = reinterpret_cast<Control*>(smem + L::kCtrlOff);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int res = blockIdx.y;
+    const int real_res = blockIdx.y, res = p.cls.in_part(real_res), rows_v = p.cls.rows_of(real_res);
+    const CUtensorMap* map = maps.part[p.cls.part(real_res)];       // Q, K, V, O
     const int64_t bh = blockIdx.z;
     const int u0 = blockIdx.x * kTile;
-    const int real_res = res + p.res0;
+    if (u0 >= rows_v) return;       // (a class one tile shorter than the longest)
 
     // Prologue, one block-wide barrier: tensor-memory allocation, row metadata and the first copies proceed
     // side by side.
@@ -176,10 +167,10 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         uint8_t* dst = smem + L::kKOff + st * L::kTileBytes;
         if (p.kt_major) {
             for (int ch = 0; ch < kTile / 64; ++ch)       // 64-key chunks of [d][64 keys]
-                tma_load_4d(dst + ch * (D * 128), &tm_k, &ctrl->k_full[st], row + ch * 64, 0, (int)bh, 0);
+                tma_load_4d(dst + ch * (D * 128), map + 1, &ctrl->k_full[st], row + ch * 64, 0, (int)bh, 0);
         } else {
             for (int sub = 0; sub < L::kSub; ++sub)
-                tma_load_4d(dst + sub * kSubBytes, &tm_k, &ctrl->k_full[st], sub * 64, res, row, (int)bh);
+                tma_load_4d(dst + sub * kSubBytes, map + 1, &ctrl->k_full[st], sub * 64, res, row, (int)bh);
         }
         ++jk;
         return true;
@@ -189,7 +180,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if (jv >= kSlots && !wait_bar(&ctrl->v_free[st], ((uint32_t)(jv / kSlots) & 1u) ^ 1u, p.status, kErrVFree)) return false;
         mbar_arrive_expect_tx(&ctrl->v_full[st], L::kTileBytes);
         for (int sub = 0; sub < L::kSub; ++sub)
-            tma_load_4d(smem + L::kVOff + st * L::kTileBytes + sub * kSubBytes, &tm_v, &ctrl->v_full[st], sub * 64, res,
+            tma_load_4d(smem + L::kVOff + st * L::kTileBytes + sub * kSubBytes, map + 2, &ctrl->v_full[st], sub * 64, res,
                         (klo + jv) * kTile, (int)bh);
         ++jv;
         return true;
@@ -204,9 +195,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         tmem_relinquish();
     } else if (warp == kTmaWarp) {
         if (lane == 0) {
-            tma_prefetch_desc(&tm_q);
-            tma_prefetch_desc(&tm_k);
-            tma_prefetch_desc(&tm_v);
+            for (int i = 0; i < 3; ++i) tma_prefetch_desc(map + i);
             mbar_init(&ctrl->q_full, 1);
             mbar_init(&ctrl->o_full, 1);
             mbar_init(&ctrl->drain, 1);
@@ -223,13 +212,13 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             mbar_fence_init();
             depend_wait();
             int2 range = make_int2(0, 0);
-            if (p.tiles != nullptr) range = __ldg(p.tiles + p.tile0 + res * p.tile_pitch + blockIdx.x);
+            if (p.tiles != nullptr) range = __ldg(p.tiles + real_res * p.cls.tile_pitch + blockIdx.x);
             const int32_t stop = entry_status(p.status, p.mirror);
             ctrl->abort_at_entry = stop;
             if (stop == 0) {
                 mbar_arrive_expect_tx(&ctrl->q_full, L::kTileBytes);
                 for (int sub = 0; sub < L::kSub; ++sub)
-                    tma_load_4d(smem + sub * kSubBytes, &tm_q, &ctrl->q_full, sub * 64, res, u0, (int)bh);
+                    tma_load_4d(smem + sub * kSubBytes, map, &ctrl->q_full, sub * 64, res, u0, (int)bh);
                 if (range.y > 0) {
                     klo = range.x / kTile;
                     load_k();
@@ -242,9 +231,9 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     } else {
         depend_wait();
         const int u = u0 + warp * 32 + lane;
-        if (u < p.rows_v) {
+        if (u < rows_v) {
             if (p.rows != nullptr) {
-                const int2 band = __ldg(p.rows + p.row0 + res * p.rows_v + u);
+                const int2 band = __ldg(p.rows + p.cls.first_row(real_res) + u);
                 my_begin = band.x;
                 my_end = band.y;
             } else {
@@ -278,7 +267,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
     int lo64 = INT_MAX, hi64 = 0;
     for (int w = 0; w < 4; ++w) { lo64 = min(lo64, ctrl->lo[w]); hi64 = max(hi64, ctrl->hi[w]); }
-    hi64 = min(hi64, p.rows_v);
+    hi64 = min(hi64, rows_v);
     if (hi64 <= 0) lo64 = 0;
     lo64 = lo64 / 64;          // in 64-key units from here
     hi64 = (hi64 + 63) / 64;
@@ -473,7 +462,7 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
         const int64_t head = bh * p.n_rows;
         const int u = u0 + warp * 32 + lane;
-        const int64_t row_real = u < p.rows_v ? (int64_t)u * p.stride + real_res : -1;
+        const int64_t row_real = u < rows_v ? (int64_t)u * p.stride + real_res : -1;
         const int row_nnz = my_end > 0 ? 2 : (my_end == kSingle ? 1 : 0), row_start = my_begin;
         if (kLse && row_real >= 0 && ok) {
             float e = -INFINITY;
@@ -520,9 +509,9 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && u0 + warp * 32 < p.rows_v) {
+        if (lane == 0 && u0 + warp * 32 < rows_v) {
             for (int sub = 0; sub < L::kSub; ++sub)
-                tma_store_4d(&tm_o, smem + sub * kSubBytes + warp * 32 * 128, sub * 64, res, u0 + warp * 32, (int)bh);
+                tma_store_4d(map + 3, smem + sub * kSubBytes + warp * 32 * 128, sub * 64, res, u0 + warp * 32, (int)bh);
             tma_store_commit();
             tma_store_wait_read();
         }
@@ -537,19 +526,16 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 }
 
 template <typename T, int D>
-static int32_t launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
-                      const Params& prm, int64_t bh, int64_t classes, cudaStream_t st) {
+static int32_t launch(const Maps<4>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
     auto kern = prm.lse != nullptr ? attention_wide_kernel<T, D, true> : attention_wide_kernel<T, D, false>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), Layout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
-    const dim3 grid((unsigned)((prm.rows_v + kTile - 1) / kTile), (unsigned)classes, (unsigned)bh);
-    return launch_kernel(kern, grid, kThreads, Layout<D>::kSmemBytes, st, mq, mk, mv, mo, prm);
+    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, Layout<D>::kSmemBytes, st, maps, prm);
 }
 
 }  // namespace wide
 }  // namespace band
 
-// Operands checked by attention_band().  Residue classes of one length share a launch: one when the stride
-// divides L, else one for the L mod stride longer classes and one for the rest.
+// Operands checked by attention_band().
 int32_t attention_wide(const void* q, const void* k, int kt_major, const void* v, void* o, const float* lin, const float* tr,
                        const float* nnzs, int64_t bh, int64_t n_rows, int64_t d, int64_t stride, float scale, int32_t dtype,
                        int32_t* status_word, const int32_t* band_table, float* lse, cudaStream_t st) {
@@ -559,30 +545,23 @@ int32_t attention_wide(const void* q, const void* k, int kt_major, const void* v
     p.status = status_word; p.mirror = status_mirror(status_word);
     p.n_rows = n_rows; p.stride = (int)stride; p.d = (int)d;
     p.kt_major = kt_major; p.scale_log2 = scale * kLog2e;
-    const int64_t longer = n_rows % stride;
-    p.tile_pitch = (int)(((n_rows + stride - 1) / stride + wide::kTile - 1) / wide::kTile);
+    p.cls = Classes(n_rows, stride, wide::kTile);
     p.rows = reinterpret_cast<const int2*>(band_table);
     p.tiles = band_table != nullptr ? p.rows + n_rows : nullptr;
+    Maps<4> maps;
     for (int part = 0; part < 2; ++part) {
-        const int64_t res0 = part == 0 ? 0 : longer, count = part == 0 ? longer : stride - longer;
-        const int64_t rows = n_rows / stride + (part == 0 ? 1 : 0);
-        if (count == 0 || rows == 0) continue;
-        CUtensorMap mq, mk, mv, mo;
-        if (!make_map_view(&mq, q, dtype, bh, n_rows, d, stride, res0, count, rows, wide::kTile) ||
-            !(kt_major ? make_map_kt(&mk, k, dtype, bh, n_rows, d, d > 64 ? 128 : 64)
-                       : make_map_view(&mk, k, dtype, bh, n_rows, d, stride, res0, count, rows, wide::kTile)) ||
-            !make_map_view(&mv, v, dtype, bh, n_rows, d, stride, res0, count, rows, wide::kTile) ||
-            !make_map_view(&mo, o, dtype, bh, n_rows, d, stride, res0, count, rows, 32))
+        if (!p.cls.has(part)) continue;
+        CUtensorMap* m = maps.part[part];
+        if (!p.cls.view(m, q, dtype, bh, n_rows, d, stride, part, wide::kTile) ||
+            !(kt_major ? make_map_kt(m + 1, k, dtype, bh, n_rows, d, d > 64 ? 128 : 64)
+                       : p.cls.view(m + 1, k, dtype, bh, n_rows, d, stride, part, wide::kTile)) ||
+            !p.cls.view(m + 2, v, dtype, bh, n_rows, d, stride, part, wide::kTile) ||
+            !p.cls.view(m + 3, o, dtype, bh, n_rows, d, stride, part, 32))
             return SPLAT_ERR_DRIVER;
-        p.rows_v = (int)rows; p.res0 = (int)res0;
-        p.row0 = (int)(part == 0 ? 0 : longer * (rows + 1));
-        p.tile0 = (int)res0 * p.tile_pitch;
-        const int32_t rc = dtype == SPLAT_BF16
-            ? (d > 64 ? wide::launch<__nv_bfloat16, 128>(mq, mk, mv, mo, p, bh, count, st) : wide::launch<__nv_bfloat16, 64>(mq, mk, mv, mo, p, bh, count, st))
-            : (d > 64 ? wide::launch<__half, 128>(mq, mk, mv, mo, p, bh, count, st) : wide::launch<__half, 64>(mq, mk, mv, mo, p, bh, count, st));
-        if (rc != SPLAT_OK) return rc;
     }
-    return SPLAT_OK;
+    return dtype == SPLAT_BF16
+        ? (d > 64 ? wide::launch<__nv_bfloat16, 128>(maps, p, bh, st) : wide::launch<__nv_bfloat16, 64>(maps, p, bh, st))
+        : (d > 64 ? wide::launch<__half, 128>(maps, p, bh, st) : wide::launch<__half, 64>(maps, p, bh, st));
 }
 
 }  // namespace splat

@@ -26,6 +26,7 @@
 #include <limits.h>
 #include <type_traits>
 
+#include "band_classes.cuh"
 #include "common.cuh"
 #include "softmax_math.cuh"
 #include "tc_ptx.cuh"
@@ -34,12 +35,6 @@ namespace splat {
 namespace band {
 
 using namespace tc;
-
-// defined in attention_band.cu
-bool allow_dynamic_smem(const void* kernel, int bytes);
-bool make_map_view(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_rows, int64_t d, int64_t stride,
-                   int64_t res0, int64_t count, int64_t rows, int box_rows);
-bool make_map_kt(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_cols, int64_t d, int64_t box_d);
 
 namespace ops {
 
@@ -71,9 +66,8 @@ struct Params {
     int32_t* status;
     int32_t* mirror;     // host copy of the status word, or null
     int64_t n_rows;      // L
-    int rows_v;          // rows of a class
     int stride;
-    int res0, row0, tile0, tile_pitch;    // first class of the launch; its place in the band table
+    Classes cls;
     int d;
     int trailing_dim;
     int kt_major;        // sddmm: K is a contiguous (BH, d, L) array (keys innermost), stride 1 only
@@ -107,12 +101,11 @@ struct Control {
 };
 
 // The row warps' share of the prologue: this thread's band, and without a table the warp's key range.
-__device__ __forceinline__ int2 load_band(const Params& p, Control* ctrl, int res, int u, int warp, int lane) {
+__device__ __forceinline__ int2 load_band(const Params& p, Control* ctrl, int real_res, int u, int warp, int lane) {
     int2 band = make_int2(0, kEmpty);
-    const int real_res = res + p.res0;
-    if (u < p.rows_v) {
+    if (u < p.cls.rows_of(real_res)) {
         if (p.rows != nullptr) {
-            band = __ldg(p.rows + p.row0 + res * p.rows_v + u);
+            band = __ldg(p.rows + p.cls.first_row(real_res) + u);
         } else {
             const RowAffine ra = row_affine(p.lin, p.tr, p.nnzs, (int64_t)u * p.stride + real_res);
             if (ra.nnz > 1) {
@@ -129,10 +122,10 @@ __device__ __forceinline__ int2 load_band(const Params& p, Control* ctrl, int re
     }
     return band;
 }
-__device__ __forceinline__ void key_range(const Params& p, const Control* ctrl, int* klo, int* khi) {
+__device__ __forceinline__ void key_range(int rows_v, const Control* ctrl, int* klo, int* khi) {
     int lo = INT_MAX, hi = 0;
     for (int w = 0; w < 4; ++w) { lo = min(lo, ctrl->lo[w]); hi = max(hi, ctrl->hi[w]); }
-    hi = min(hi, p.rows_v);
+    hi = min(hi, rows_v);
     *klo = hi > 0 ? lo / kStep : 0;
     *khi = (hi + kStep - 1) / kStep;
 }
@@ -173,7 +166,7 @@ template <int D> struct SddmmLayout {
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads, SddmmLayout<D>::kPerSm)
-sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const Params p) {
+sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
     using L = SddmmLayout<D>;
     constexpr int kTmemCols = 128;   // two 64-column score buffers
     extern __shared__ uint8_t smem_raw[];
@@ -182,9 +175,11 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     Control* ctrl = reinterpret_cast<Control*>(smem + L::kCtrlOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int res = blockIdx.y, real_res = res + p.res0;
+    const int real_res = blockIdx.y, res = p.cls.in_part(real_res), rows_v = p.cls.rows_of(real_res);
+    const CUtensorMap* map = maps.part[p.cls.part(real_res)];       // Q, K
     const int64_t bh = blockIdx.z;
     const int u0 = blockIdx.x * kTile;
+    if (u0 >= rows_v) return;       // (a class one tile shorter than the longest)
 
     int2 band = make_int2(0, kEmpty);
     int klo = 0, khi = 0, item = 0;
@@ -193,10 +188,10 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if (item >= kStages && !mbar_wait(&ctrl->empty[stage], ((uint32_t)(item / kStages) & 1u) ^ 1u, p.status, kErrEmpty)) return false;
         mbar_arrive_expect_tx(&ctrl->full[stage], L::kItemBytes);
         if (p.kt_major)      // one [d][64 keys] block (K layouts: see attention_band.cu)
-            tma_load_4d(s_ring + stage * L::kItemBytes, &tm_k, &ctrl->full[stage], k * kStep, 0, (int)bh, 0);
+            tma_load_4d(s_ring + stage * L::kItemBytes, map + 1, &ctrl->full[stage], k * kStep, 0, (int)bh, 0);
         else
             for (int sub = 0; sub < L::kSub; ++sub)
-                tma_load_4d(s_ring + stage * L::kItemBytes + sub * kStepBytesPerSub, &tm_k, &ctrl->full[stage], sub * 64, res,
+                tma_load_4d(s_ring + stage * L::kItemBytes + sub * kStepBytesPerSub, map + 1, &ctrl->full[stage], sub * 64, res,
                             k * kStep, (int)bh);
         ++item;
         return true;
@@ -207,8 +202,8 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         tmem_relinquish();
     } else if (warp == kTmaWarp) {
         if (lane == 0) {
-            tma_prefetch_desc(&tm_q);
-            tma_prefetch_desc(&tm_k);
+            tma_prefetch_desc(map);
+            tma_prefetch_desc(map + 1);
             mbar_init(&ctrl->q_full, 1);
             for (int i = 0; i < kStages; ++i) {
                 mbar_init(&ctrl->full[i], 1);
@@ -222,13 +217,13 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             mbar_fence_init();
             depend_wait();
             int2 range = make_int2(0, 0);
-            if (p.tiles != nullptr) range = __ldg(p.tiles + p.tile0 + res * p.tile_pitch + blockIdx.x);
+            if (p.tiles != nullptr) range = __ldg(p.tiles + real_res * p.cls.tile_pitch + blockIdx.x);
             const int32_t stop = entry_status(p.status, p.mirror);
             ctrl->abort_at_entry = stop;
             if (stop == 0) {
                 mbar_arrive_expect_tx(&ctrl->q_full, L::kQBytes);
                 for (int sub = 0; sub < L::kSub; ++sub)
-                    tma_load_4d(smem + sub * kSubBytes, &tm_q, &ctrl->q_full, sub * 64, res, u0, (int)bh);
+                    tma_load_4d(smem + sub * kSubBytes, map, &ctrl->q_full, sub * 64, res, u0, (int)bh);
                 if (range.y > 0) {
                     klo = range.x / kStep;
                     khi = (range.y + kStep - 1) / kStep;
@@ -240,7 +235,7 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
     } else {
         depend_wait();
-        band = load_band(p, ctrl, res, u0 + warp * 32 + lane, warp, lane);
+        band = load_band(p, ctrl, real_res, u0 + warp * 32 + lane, warp, lane);
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -251,7 +246,7 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
         return;
     }
-    key_range(p, ctrl, &klo, &khi);
+    key_range(rows_v, ctrl, &klo, &khi);
 
     if (warp == kTmaWarp) {
         // ------------------------------------------------------------------ TMA producer
@@ -377,7 +372,7 @@ sddmm_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
         // padding slots, rows with one non-zero (a dot product by hand) and rows with none
         const int nnz = band.y > 0 ? band.y - band.x : (band.y == kSingle ? 1 : 0);
-        unsigned todo = __ballot_sync(0xffffffffu, u0 + warp * 32 + lane < p.rows_v && (nnz < p.trailing_dim || band.y == kSingle));
+        unsigned todo = __ballot_sync(0xffffffffu, u0 + warp * 32 + lane < rows_v && (nnz < p.trailing_dim || band.y == kSingle));
         const T* qg = reinterpret_cast<const T*>(p.q);
         const T* kg = reinterpret_cast<const T*>(p.kv);
         while (todo) {
@@ -426,7 +421,7 @@ template <int D> struct SpmmLayout {
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads, 2)
-spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Params p) {
+spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
     using L = SpmmLayout<D>;
     constexpr int kTmemCols = D == 128 ? 256 : 128;   // the output accumulator, two steps of P (32 columns each)
     extern __shared__ uint8_t smem_raw[];
@@ -435,9 +430,11 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
     Control* ctrl = reinterpret_cast<Control*>(smem + L::kCtrlOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int res = blockIdx.y, real_res = res + p.res0;
+    const int real_res = blockIdx.y, res = p.cls.in_part(real_res), rows_v = p.cls.rows_of(real_res);
+    const CUtensorMap* map = maps.part[p.cls.part(real_res)];       // V, O
     const int64_t bh = blockIdx.z;
     const int u0 = blockIdx.x * kTile;
+    if (u0 >= rows_v) return;       // (a class one tile shorter than the longest)
 
     int2 band = make_int2(0, kEmpty);
     int klo = 0, khi = 0, item = 0;
@@ -446,7 +443,7 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
         if (item >= kStages && !mbar_wait(&ctrl->empty[stage], ((uint32_t)(item / kStages) & 1u) ^ 1u, p.status, kErrEmpty)) return false;
         mbar_arrive_expect_tx(&ctrl->full[stage], L::kItemBytes);
         for (int sub = 0; sub < L::kSub; ++sub)
-            tma_load_4d(s_ring + stage * L::kItemBytes + sub * kStepBytesPerSub, &tm_v, &ctrl->full[stage], sub * 64, res, k * kStep,
+            tma_load_4d(s_ring + stage * L::kItemBytes + sub * kStepBytesPerSub, map, &ctrl->full[stage], sub * 64, res, k * kStep,
                         (int)bh);
         ++item;
         return true;
@@ -457,7 +454,7 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
         tmem_relinquish();
     } else if (warp == kTmaWarp) {
         if (lane == 0) {
-            tma_prefetch_desc(&tm_v);
+            tma_prefetch_desc(map);
             for (int i = 0; i < kStages; ++i) {
                 mbar_init(&ctrl->full[i], 1);
                 mbar_init(&ctrl->empty[i], 1);
@@ -470,7 +467,7 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
             mbar_fence_init();
             depend_wait();
             int2 range = make_int2(0, 0);
-            if (p.tiles != nullptr) range = __ldg(p.tiles + p.tile0 + res * p.tile_pitch + blockIdx.x);
+            if (p.tiles != nullptr) range = __ldg(p.tiles + real_res * p.cls.tile_pitch + blockIdx.x);
             const int32_t stop = entry_status(p.status, p.mirror);
             ctrl->abort_at_entry = stop;
             if (stop == 0 && range.y > 0) {
@@ -483,7 +480,7 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
         }
     } else {
         depend_wait();
-        band = load_band(p, ctrl, res, u0 + warp * 32 + lane, warp, lane);
+        band = load_band(p, ctrl, real_res, u0 + warp * 32 + lane, warp, lane);
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -494,7 +491,7 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
         if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
         return;
     }
-    key_range(p, ctrl, &klo, &khi);
+    key_range(rows_v, ctrl, &klo, &khi);
     const uint32_t p_col = D;        // tensor-memory columns of P behind the accumulator
 
     if (warp == kTmaWarp) {
@@ -657,9 +654,9 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && u0 + warp * 32 < p.rows_v) {
+        if (lane == 0 && u0 + warp * 32 < rows_v) {
             for (int sub = 0; sub < L::kSub; ++sub)
-                tma_store_4d(&tm_o, smem + sub * kSubBytes + warp * 32 * 128, sub * 64, res, u0 + warp * 32, (int)bh);
+                tma_store_4d(map + 1, smem + sub * kSubBytes + warp * 32 * 128, sub * 64, res, u0 + warp * 32, (int)bh);
             tma_store_commit();
             tma_store_wait_read();
         }
@@ -677,20 +674,16 @@ spmm_band_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant
 // host
 // ---------------------------------------------------------------------------------------------
 template <typename T, int D>
-static int32_t launch_sddmm(const CUtensorMap& mq, const CUtensorMap& mk, const Params& prm, int64_t bh, int64_t classes,
-                            cudaStream_t st) {
+static int32_t launch_sddmm(const Maps<2>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
     auto kern = sddmm_band_kernel<T, D>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), SddmmLayout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
-    dim3 grid((unsigned)((prm.rows_v + kTile - 1) / kTile), (unsigned)classes, (unsigned)bh);
-    return launch_kernel(kern, grid, kThreads, SddmmLayout<D>::kSmemBytes, st, mq, mk, prm);
+    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, SddmmLayout<D>::kSmemBytes, st, maps, prm);
 }
 template <typename T, int D>
-static int32_t launch_spmm(const CUtensorMap& mv, const CUtensorMap& mo, const Params& prm, int64_t bh, int64_t classes,
-                           cudaStream_t st) {
+static int32_t launch_spmm(const Maps<2>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
     auto kern = spmm_band_kernel<T, D>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), SpmmLayout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
-    dim3 grid((unsigned)((prm.rows_v + kTile - 1) / kTile), (unsigned)classes, (unsigned)bh);
-    return launch_kernel(kern, grid, kThreads, SpmmLayout<D>::kSmemBytes, st, mv, mo, prm);
+    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, SpmmLayout<D>::kSmemBytes, st, maps, prm);
 }
 
 // Checks shared by both operators; fills stride.  plan as written by splat_acsr_classify:
@@ -723,21 +716,10 @@ static Params params(const void* sparse, const float* lin, const float* tr, cons
     p.lead = (int)(a & 15) / 2;
     p.status = status_word; p.mirror = status_mirror(status_word);
     p.n_rows = n_rows; p.stride = (int)stride; p.d = (int)d; p.trailing_dim = (int)trailing_dim;
-    p.tile_pitch = (int)(((n_rows + stride - 1) / stride + kTile - 1) / kTile);
+    p.cls = Classes(n_rows, stride, kTile);
     p.rows = reinterpret_cast<const int2*>(band_table);
     p.tiles = band_table != nullptr ? p.rows + n_rows : nullptr;
     return p;
-}
-
-// Residue classes of one length share a launch: part 0 the L mod stride longer ones, part 1 the rest.
-struct Part { int64_t res0, count, rows; };
-static Part part_of(Params& p, int part) {
-    const int64_t longer = p.n_rows % p.stride;
-    const Part x{part == 0 ? 0 : longer, part == 0 ? longer : p.stride - longer, p.n_rows / p.stride + (part == 0 ? 1 : 0)};
-    p.rows_v = (int)x.rows; p.res0 = (int)x.res0;
-    p.row0 = (int)(part == 0 ? 0 : longer * (x.rows + 1));
-    p.tile0 = (int)x.res0 * p.tile_pitch;
-    return x;
 }
 
 }  // namespace ops
@@ -765,23 +747,18 @@ extern "C" int32_t splat_sddmm_band_table(const void* q, const void* k, int64_t 
     ops::Params p = ops::params(s_out, sTod_lin, sTod_tr, nnzs, n_rows, d, trailing_dim, stride, band_table, status_word);
     p.q = q; p.kv = k; p.kt_major = k_major ? 0 : 1;
     cudaStream_t st = (cudaStream_t)stream;
+    Maps<2> maps;
     for (int part = 0; part < 2; ++part) {
-        const ops::Part x = ops::part_of(p, part);
-        if (x.count == 0 || x.rows == 0) continue;
-        CUtensorMap mq, mk;
-        if (!make_map_view(&mq, q, dtype, bh, n_rows, d, stride, x.res0, x.count, x.rows, ops::kTile) ||
-            !(k_major ? make_map_view(&mk, k, dtype, bh, n_rows, d, stride, x.res0, x.count, x.rows, ops::kStep)
-                      : make_map_kt(&mk, k, dtype, bh, n_cols, d, d > 64 ? 128 : 64)))
+        CUtensorMap* m = maps.part[part];
+        if (p.cls.has(part) &&
+            (!p.cls.view(m, q, dtype, bh, n_rows, d, stride, part, ops::kTile) ||
+             !(k_major ? p.cls.view(m + 1, k, dtype, bh, n_rows, d, stride, part, ops::kStep)
+                       : make_map_kt(m + 1, k, dtype, bh, n_cols, d, d > 64 ? 128 : 64))))
             return SPLAT_ERR_DRIVER;
-        if (dtype == SPLAT_BF16)
-            rc = d > 64 ? ops::launch_sddmm<__nv_bfloat16, 128>(mq, mk, p, bh, x.count, st)
-                        : ops::launch_sddmm<__nv_bfloat16, 64>(mq, mk, p, bh, x.count, st);
-        else
-            rc = d > 64 ? ops::launch_sddmm<__half, 128>(mq, mk, p, bh, x.count, st)
-                        : ops::launch_sddmm<__half, 64>(mq, mk, p, bh, x.count, st);
-        if (rc != SPLAT_OK) return rc;
     }
-    return SPLAT_OK;
+    if (dtype == SPLAT_BF16)
+        return d > 64 ? ops::launch_sddmm<__nv_bfloat16, 128>(maps, p, bh, st) : ops::launch_sddmm<__nv_bfloat16, 64>(maps, p, bh, st);
+    return d > 64 ? ops::launch_sddmm<__half, 128>(maps, p, bh, st) : ops::launch_sddmm<__half, 64>(maps, p, bh, st);
 }
 
 extern "C" int32_t splat_spmm_band_table(const void* p_in, const void* v, void* o, const float* sTod_lin,
@@ -798,22 +775,16 @@ extern "C" int32_t splat_spmm_band_table(const void* p_in, const void* v, void* 
     ops::Params p = ops::params(p_in, sTod_lin, sTod_tr, nnzs, n_rows, d, trailing_dim, stride, band_table, status_word);
     p.kv = v;
     cudaStream_t st = (cudaStream_t)stream;
+    Maps<2> maps;
     for (int part = 0; part < 2; ++part) {
-        const ops::Part x = ops::part_of(p, part);
-        if (x.count == 0 || x.rows == 0) continue;
-        CUtensorMap mv, mo;
-        if (!make_map_view(&mv, v, dtype, bh, n_rows, d, stride, x.res0, x.count, x.rows, ops::kStep) ||
-            !make_map_view(&mo, o, dtype, bh, n_rows, d, stride, x.res0, x.count, x.rows, 32))
+        CUtensorMap* m = maps.part[part];
+        if (p.cls.has(part) && (!p.cls.view(m, v, dtype, bh, n_rows, d, stride, part, ops::kStep) ||
+                                !p.cls.view(m + 1, o, dtype, bh, n_rows, d, stride, part, 32)))
             return SPLAT_ERR_DRIVER;
-        if (dtype == SPLAT_BF16)
-            rc = d > 64 ? ops::launch_spmm<__nv_bfloat16, 128>(mv, mo, p, bh, x.count, st)
-                        : ops::launch_spmm<__nv_bfloat16, 64>(mv, mo, p, bh, x.count, st);
-        else
-            rc = d > 64 ? ops::launch_spmm<__half, 128>(mv, mo, p, bh, x.count, st)
-                        : ops::launch_spmm<__half, 64>(mv, mo, p, bh, x.count, st);
-        if (rc != SPLAT_OK) return rc;
     }
-    return SPLAT_OK;
+    if (dtype == SPLAT_BF16)
+        return d > 64 ? ops::launch_spmm<__nv_bfloat16, 128>(maps, p, bh, st) : ops::launch_spmm<__nv_bfloat16, 64>(maps, p, bh, st);
+    return d > 64 ? ops::launch_spmm<__half, 128>(maps, p, bh, st) : ops::launch_spmm<__half, 64>(maps, p, bh, st);
 }
 
 extern "C" int32_t splat_sddmm_band(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
