@@ -14,11 +14,11 @@
 // The sparse layout shifts every row by its own number of elements against the dense columns, so a row's 64
 // columns of a step begin anywhere in a 16-byte piece of the sparse array.  They begin at the SAME place in
 // every step (64 elements are eight pieces): with e the element index of the step's first column and
-// sft = e mod 8, a step of a row is eight whole pieces made of the last sft elements of the step before and the
-// first 64 - sft of this one.  The thread forms them in registers (barrel()), and a warp moves them through a
+// sft = e mod 8, a step of a row is eight whole pieces made of the last sft elements of the step before and
+// the first 64 - sft of this one.  The thread forms them in registers (barrel()), and a warp moves them through a
 // swizzled staging tile so that global memory sees 128 contiguous bytes per row.  The kernels before did this
 // with 2-byte accesses, or 16-byte ones of 32 different rows per instruction: 70 % of the L1 wavefronts, a
-// third of the memory bandwidth.  B4 H16 L4096 d64 fp16 window 256: @@@
+// third of the memory bandwidth.  B4 H16 L4096 d64 fp16 window 256: SDDMM 102 -> 59 us, SpMM 114 -> 65.
 // Pieces that a row's band only partly covers (its ends, if trailing_dim is no multiple of 8) are stored element
 // by element.  Rows with one non-zero (described by the metadata as column `start`, outside the band) and rows
 // with none are fixed up by plain loads, padding slots of S are written as zero like the CUDA-core kernels do.
@@ -130,10 +130,11 @@ __device__ __forceinline__ void key_range(int rows_v, const Control* ctrl, int* 
     *khi = (hi + kStep - 1) / kStep;
 }
 
-// out[0..31] = 64 elements (two per word) of the 72 in x[0..35] from element t on, 0 <= t <= 8.
+// out[0..31] = 64 elements (two per word) of the 72 in x[0..35] from element t on, 0 <= t <= kMax.
+template <int kMax>
 __device__ __forceinline__ void barrel(uint32_t (&x)[36], int t, uint32_t (&out)[32]) {
     const int s = t >> 1;
-    if (s & 4) {
+    if (kMax == 8 && (s & 4)) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i] = x[i + 4];
     }
@@ -298,7 +299,7 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         const int64_t head = bh * p.n_rows;
         // element index (in p.sparse) of class column 0 of this row, were its band to reach that far
         const int64_t e_row = p.lead + (head + (int64_t)(u0 + warp * 32 + lane) * p.stride + real_res) * p.trailing_dim - band.x;
-        const int sft = (int)((e_row + (int64_t)klo * kStep) & 7);
+        const int sft = (int)(e_row & 7);
         // The rows whose pieces this lane stores: row 4 i + lane / 8, piece lane mod 8.  Byte offset of the piece of
         // class column 0's step, and the column range in which the piece's first column is inside the band.
         uint8_t* base = reinterpret_cast<uint8_t*>(p.sparse) +
@@ -348,7 +349,7 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             for (int i = 0; i < 4; ++i) x[i] = tail[i];
 #pragma unroll
             for (int i = 0; i < 4; ++i) tail[i] = x[32 + i];
-            barrel(x, 8 - sft, out);
+            barrel<8>(x, 8 - sft, out);
 #pragma unroll
             for (int q4 = 0; q4 < 8; ++q4)
                 *reinterpret_cast<uint4*>(stage + lane * 128 + ((q4 ^ (lane & 7)) << 4)) =
@@ -372,27 +373,42 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         }
         // padding slots, rows with one non-zero (a dot product by hand) and rows with none
         const int nnz = band.y > 0 ? band.y - band.x : (band.y == kSingle ? 1 : 0);
-        unsigned todo = __ballot_sync(0xffffffffu, u0 + warp * 32 + lane < rows_v && (nnz < p.trailing_dim || band.y == kSingle));
+        const bool real = u0 + warp * 32 + lane < rows_v;
+        if (__any_sync(0xffffffffu, real && nnz < p.trailing_dim)) {
+            const int pad = real ? nnz : p.trailing_dim;
+            // eight lanes per row, as above (a warp per row took 2 to 3 us of a small call)
+            for (int i = 0; i < 8; ++i) {
+                const int row = 4 * i + (lane >> 3);
+                const int64_t e0 = __shfl_sync(0xffffffffu, e_row + band.x, row), end = e0 + p.trailing_dim;
+                const int64_t from = e0 + __shfl_sync(0xffffffffu, pad, row);
+                for (int64_t e = (from & ~(int64_t)7) + (lane & 7) * 8; e < end; e += 64) {
+                    if (e >= from && e + 8 <= end) {
+                        *reinterpret_cast<uint4*>(p.sparse + e) = make_uint4(0, 0, 0, 0);
+                    } else {
+#pragma unroll
+                        for (int t = 0; t < 8; ++t)
+                            if (e + t >= from && e + t < end) p.sparse[e + t] = 0;
+                    }
+                }
+            }
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, real && band.y == kSingle);
         const T* qg = reinterpret_cast<const T*>(p.q);
         const T* kg = reinterpret_cast<const T*>(p.kv);
         while (todo) {
             const int rr = __ffs(todo) - 1;
             todo &= todo - 1;
-            const int n = __shfl_sync(0xffffffffu, nnz, rr);
             const int start = __shfl_sync(0xffffffffu, band.x, rr);
-            const int64_t real = head + (int64_t)(u0 + warp * 32 + rr) * p.stride + real_res;
-            uint16_t* row = p.sparse + p.lead + real * p.trailing_dim;
-            for (int j = n + lane; j < p.trailing_dim; j += 32) row[j] = 0;
-            if (n == 1) {
-                float acc = 0.f;
-                const T* qr = qg + real * p.d;
-                // K[bh][start][c]: rows of d elements, or column `start` of the (d, L) array
-                const int64_t k0 = p.kt_major ? head * p.d + start : (head + start) * p.d;
-                const int64_t kc = p.kt_major ? p.n_rows : 1;
-                for (int c = lane; c < p.d; c += 32) acc += to_f<T>(qr[c]) * to_f<T>(kg[k0 + c * kc]);
-                acc = warp_sum(acc);
-                if (lane == 0) *reinterpret_cast<T*>(row) = DT<T>::from_f(acc);
-            }
+            const int64_t row_real = head + (int64_t)(u0 + warp * 32 + rr) * p.stride + real_res;
+            uint16_t* row = p.sparse + p.lead + row_real * p.trailing_dim;
+            float acc = 0.f;
+            const T* qr = qg + row_real * p.d;
+            // K[bh][start][c]: rows of d elements, or column `start` of the (d, L) array
+            const int64_t k0 = p.kt_major ? head * p.d + start : (head + start) * p.d;
+            const int64_t kc = p.kt_major ? p.n_rows : 1;
+            for (int c = lane; c < p.d; c += 32) acc += to_f<T>(qr[c]) * to_f<T>(kg[k0 + c * kc]);
+            acc = warp_sum(acc);
+            if (lane == 0) *reinterpret_cast<T*>(row) = DT<T>::from_f(acc);
         }
     }
     tc_fence_before_sync();
@@ -583,7 +599,7 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
                     const uint4 v = *reinterpret_cast<const uint4*>(mine + i * 16);
                     x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
                 }
-                barrel(x, sft, out);          // the step's columns begin sft elements into the pieces
+                barrel<7>(x, sft, out);          // the step's columns begin sft elements into the pieces
                 if (!__all_sync(0xffffffffu, lo <= 0 && hi >= kStep)) {
                     // pairs of columns: 64 mask bits, two per word
                     const int l = min(max(lo, 0), 64), h = min(max(hi, 0), 64);
