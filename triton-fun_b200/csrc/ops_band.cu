@@ -98,6 +98,7 @@ struct Control {
     int32_t abort_at_entry;
     int32_t lo[4];
     int32_t hi[4];
+    int4 about[kTile];   // sddmm: what a lane knows of its row, for the lanes that store it
 };
 
 // The row warps' share of the prologue: this thread's band, and without a table the warp's key range.
@@ -302,18 +303,22 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         const int sft = (int)(e_row & 7);
         // The rows whose pieces this lane stores: row 4 i + lane / 8, piece lane mod 8.  Byte offset of the piece of
         // class column 0's step, and the column range in which the piece's first column is inside the band.
-        uint8_t* base = reinterpret_cast<uint8_t*>(p.sparse) +
-                        (__shfl_sync(0xffffffffu, e_row + band.x, 0) & ~(int64_t)7) * 2;
+        // (what a lane knows of its row reaches the others through shared memory: five shuffles per row took 1 300 cycles)
+        const int64_t e_base = __shfl_sync(0xffffffffu, e_row + band.x, 0) & ~(int64_t)7;
+        uint8_t* base = reinterpret_cast<uint8_t*>(p.sparse + e_base);
+        const int e_rel = (int)(e_row - e_base);
+        int4* about = ctrl->about + warp * 32;
+        about[lane] = make_int4(e_rel, u0 + warp * 32 + lane < rows_v ? 1 : 0, band.x, max(band.y, -64));     // (-64, below every step: no band)
+        __syncwarp();
         int32_t off[8];
         int lo8[8], hi8[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int row = 4 * i + (lane >> 3);
-            const int64_t e = __shfl_sync(0xffffffffu, e_row, row);
-            const int behind = (lane & 7) * 8 - __shfl_sync(0xffffffffu, sft, row);       // first column - step's
-            off[i] = (int32_t)(reinterpret_cast<uint8_t*>(p.sparse) + ((e & ~(int64_t)7) + (lane & 7) * 8) * 2 - base);
-            lo8[i] = __shfl_sync(0xffffffffu, band.x, row) - behind;
-            hi8[i] = max(__shfl_sync(0xffffffffu, band.y, row), -64) - behind;            // (below every step: no band)
+            const int4 r = about[4 * i + (lane >> 3)];
+            const int behind = (lane & 7) * 8 - (r.x & 7);       // first column - step's
+            off[i] = (r.x + behind) * 2;
+            lo8[i] = r.z - behind;
+            hi8[i] = r.w - behind;
         }
         // this warp's first and last step with columns of its rows' bands
         const int w_lo = warp_min_i(band.y > 0 ? band.x : INT_MAX), w_hi = warp_max_i(band.y > 0 ? band.y + sft : 0);
@@ -372,33 +377,30 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             __syncwarp();   // the staging tile is rewritten in the next step
         }
         // padding slots, rows with one non-zero (a dot product by hand) and rows with none
-        const int nnz = band.y > 0 ? band.y - band.x : (band.y == kSingle ? 1 : 0);
-        const bool real = u0 + warp * 32 + lane < rows_v;
-        if (__any_sync(0xffffffffu, real && nnz < p.trailing_dim)) {
-            const int pad = real ? nnz : p.trailing_dim;
-            // eight lanes per row, as above (a warp per row took 2 to 3 us of a small call)
+        // (eight lanes per row: one element each of the pieces at either end, 16-byte stores between; a warp per row,
+        // element by element, took 2 to 3 us of a small call)
+        const int4 mine = about[lane];
+        const int nnz = mine.w > 0 ? mine.w - mine.z : (mine.w == kSingle ? 1 : 0);
+        if (__any_sync(0xffffffffu, mine.y != 0 && nnz < p.trailing_dim)) {
+            uint16_t* to = reinterpret_cast<uint16_t*>(base);
+#pragma unroll 1
             for (int i = 0; i < 8; ++i) {
-                const int row = 4 * i + (lane >> 3);
-                const int64_t e0 = __shfl_sync(0xffffffffu, e_row + band.x, row), end = e0 + p.trailing_dim;
-                const int64_t from = e0 + __shfl_sync(0xffffffffu, pad, row);
-                for (int64_t e = (from & ~(int64_t)7) + (lane & 7) * 8; e < end; e += 64) {
-                    if (e >= from && e + 8 <= end) {
-                        *reinterpret_cast<uint4*>(p.sparse + e) = make_uint4(0, 0, 0, 0);
-                    } else {
-#pragma unroll
-                        for (int t = 0; t < 8; ++t)
-                            if (e + t >= from && e + t < end) p.sparse[e + t] = 0;
-                    }
-                }
+                const int4 r = about[4 * i + (lane >> 3)];
+                const int l = lane & 7, slot0 = r.x + r.z, end = slot0 + p.trailing_dim;
+                const int from = r.y == 0 ? end : slot0 + (r.w > 0 ? r.w - r.z : (r.w == kSingle ? 1 : 0));
+                const int first = (from + 7) & ~7, last = end & ~7;      // whole pieces
+                if (from + l < min(first, end)) to[from + l] = 0;
+                for (int e = first + l * 8; e < last; e += 64) *reinterpret_cast<uint4*>(to + e) = make_uint4(0, 0, 0, 0);
+                if (last >= first && last + l < end) to[last + l] = 0;
             }
         }
-        unsigned todo = __ballot_sync(0xffffffffu, real && band.y == kSingle);
+        unsigned todo = __ballot_sync(0xffffffffu, mine.y != 0 && mine.w == kSingle);
         const T* qg = reinterpret_cast<const T*>(p.q);
         const T* kg = reinterpret_cast<const T*>(p.kv);
         while (todo) {
             const int rr = __ffs(todo) - 1;
             todo &= todo - 1;
-            const int start = __shfl_sync(0xffffffffu, band.x, rr);
+            const int start = about[rr].z;
             const int64_t row_real = head + (int64_t)(u0 + warp * 32 + rr) * p.stride + real_res;
             uint16_t* row = p.sparse + p.lead + row_real * p.trailing_dim;
             float acc = 0.f;
@@ -555,20 +557,23 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         const int sft = (int)((e_row + (int64_t)klo * kStep) & 7);
         // Pieces of a step: nine per row, 288 per warp, piece idx = lane + 32 i of row idx / 9: byte offset of the
         // piece in class column 0's step, and the range of a step's first column in which it holds some of the band.
-        const uint8_t* base = reinterpret_cast<const uint8_t*>(p.sparse) +
-                              (__shfl_sync(0xffffffffu, e_row + band.x, 0) & ~(int64_t)7) * 2;
+        const int64_t e_base = __shfl_sync(0xffffffffu, e_row + band.x, 0) & ~(int64_t)7;
+        const uint8_t* base = reinterpret_cast<const uint8_t*>(p.sparse + e_base);
+        int4* about = reinterpret_cast<int4*>(smem + L::kPOff + warp * 32 * kPPitch);      // (as in SDDMM)
+        about[lane] = make_int4((int)(e_row - e_base), sft, band.x, band.y);
+        __syncwarp();
         int32_t off[9];
         int first[9], last[9];
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
             const int idx = lane + 32 * i, row = idx / 9, piece = idx - row * 9;
-            const int64_t e = __shfl_sync(0xffffffffu, e_row, row);
-            const int behind = piece * 8 - __shfl_sync(0xffffffffu, sft, row);
-            const int hi = __shfl_sync(0xffffffffu, band.y, row);
-            off[i] = (int32_t)(reinterpret_cast<const uint8_t*>(p.sparse) + ((e & ~(int64_t)7) + piece * 8) * 2 - base);
-            first[i] = __shfl_sync(0xffffffffu, band.x, row) - behind - 7;
-            last[i] = hi > 0 ? hi - behind : INT_MIN;
+            const int4 r = about[row];
+            const int behind = piece * 8 - r.y;
+            off[i] = ((r.x & ~7) + piece * 8) * 2;
+            first[i] = r.z - behind - 7;
+            last[i] = r.w > 0 ? r.w - behind : INT_MIN;
         }
+        __syncwarp();
         auto fetch = [&](int it) {
             if (klo + it < khi) {
                 const uint32_t dst = smem_u32(smem + L::kPOff) + (it % kPStages) * L::kPBytes + warp * 32 * kPPitch + lane * 16;
@@ -657,8 +662,15 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
                 for (int j = 0; j < 32; j += 2) o32[j >> 1] = pack2<T>(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
             } else if (single) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 2)
-                    o32[j >> 1] = ch * 32 + j < p.d ? pack2<T>(p0 * to_f<T>(vrow[ch * 32 + j]), p0 * to_f<T>(vrow[ch * 32 + j + 1])) : 0u;
+                for (int q4 = 0; q4 < 4; ++q4) {
+                    const int c = ch * 32 + q4 * 8;
+                    outv[q4] = c < p.d ? *reinterpret_cast<const uint4*>(vrow + c) : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const T* e = reinterpret_cast<const T*>(o32 + j);
+                    o32[j] = pack2<T>(p0 * to_f<T>(e[0]), p0 * to_f<T>(e[1]));
+                }
             } else {
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) outv[q4] = make_uint4(0, 0, 0, 0);
