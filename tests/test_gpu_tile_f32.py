@@ -10,13 +10,15 @@ from oracle import attention_oracle as at
 
 pytestmark = pytest.mark.gpu
 
-#        kind, L, p0, p1, heads (32-row CTAs below 444 64-row tiles over all heads, 64-row CTAs from there)
+#        kind, L, p0, p1, heads (64-row CTAs from 444 of them over all heads, below that 32-row ones of four warps from 296,
+#        else of eight)
 PATTERNS = [
     (ao.PATTERN_CAUSAL_WINDOWED, 65, 63, 0, 3),      # one row in the second tile
     (ao.PATTERN_CAUSAL_WINDOWED, 127, 126, 0, 3),    # dense causal, one row short of two tiles
     (ao.PATTERN_CAUSAL_WINDOWED, 389, 64, 0, 64),    # L not a multiple of 4; 448 tiles
     (ao.PATTERN_WINDOWED, 256, 37, 0, 111),          # 444 tiles
     (ao.PATTERN_BLOCKED, 200, 48, 0, 3),
+    (ao.PATTERN_BLOCKED, 200, 48, 0, 50),            # 350 32-row tiles, 200 64-row ones
     (ao.PATTERN_STRIDED, 203, 8, 0, 56),             # classes of 26 and 25 rows, single-element rows; 448 tiles
     (ao.PATTERN_DILATED, 301, 40, 3, 3),             # classes of 101 and 100 rows
     (ao.PATTERN_CAUSAL_WINDOWED, 3, 1, 0, 3),        # smallest
