@@ -477,12 +477,12 @@ def run_ours(args):
             st["s_in"].wait_stream(cur)
             st["s_out"].wait_stream(cur)
             for i in range(-(-heads // c)):
-                buf = st["bufs"][i % 2]
+                buf = st["keep"][0][4 * (i % 2):4 * (i % 2) + 4]          # q, k, v, o of one staging set
                 with torch.cuda.stream(st["s_in"]):
-                    for key, src in (("q", host[0]), ("k", host[1]), ("v", host[2])):
-                        buf[key][:, :c].copy_(src[:, :c], non_blocking=True)
+                    for t, src in zip(buf[:3], host[:3]):
+                        t.copy_(src[0, :c], non_blocking=True)
                 with torch.cuda.stream(st["s_out"]):
-                    host[3][:, :c].copy_(buf["o"][:, :c], non_blocking=True)
+                    host[3][0, :c].copy_(buf[3], non_blocking=True)
             cur.wait_stream(st["s_in"])
             cur.wait_stream(st["s_out"])
         barrier()
