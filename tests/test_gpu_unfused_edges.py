@@ -95,3 +95,26 @@ def test_softmax_lanes_per_row(dtype):
             out = torch.full((1, 1, L, T), float("nan"), dtype=dtype, device="cuda")
             n.softmax(x.cuda(), out, nnz.float().cuda(), T, 0.7)
             assert_close(out, ref, dtype, f"softmax T={T} L={L}")
+
+
+@pytest.mark.parametrize("d", [64, 32])
+@pytest.mark.parametrize("lead", [0, 3])
+def test_spmm_more_tiles_than_fit_twice(d, lead):
+    """SpMM with more than two 128-row tiles per SM (296 on 148), which run three to an SM with a shorter pipeline."""
+    import acsr_helpers as ah
+    import splat_native as n
+    for kind, L, p0, p1, H in ((ao.PATTERN_CAUSAL_WINDOWED, 300, 256, 0, 99), (ao.PATTERN_WINDOWED, 700, 130, 0, 50),
+                               (ao.PATTERN_STRIDED, 1003, 7, 0, 22)):
+        torch.manual_seed(L + d)
+        acsr = ah.create_acsr(ah.PatternMask(kind, L, p0, p1), 16, 0)
+        meta = ao.metadata_from_pattern(kind, L, p0, p1, 16)
+        T = acsr[5]
+        v = torch.randn(1, H, L, d).half()
+        _cols, valid = at._cols(meta, T)
+        p = torch.rand(1, H, L, T)
+        p_dev = _shifted((1, H, L, T), torch.float16, lead)
+        p_dev.copy_(torch.where(valid, p, torch.full_like(p, float("nan"))))     # padding is not read
+        o = torch.full((1, H, L, d), float("nan"), dtype=torch.float16, device="cuda")
+        n.spmm(p_dev, v.cuda(), o, acsr[2], acsr[3], acsr[4], T, n.PATH_BAND)
+        n.check_status_word(0)
+        assert_close(o, at.spmm_acsr(p.half(), v, meta), torch.float16, f"spmm {(kind, L, p0, p1, H)} d={d} lead={lead}")

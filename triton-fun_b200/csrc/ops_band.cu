@@ -48,7 +48,6 @@ constexpr int kThreads = 192;
 constexpr int kTmaWarp = 4;
 constexpr int kMmaWarp = 5;
 constexpr int kStages = 3;                      // K / V ring
-constexpr int kPStages = 3;                     // steps of P on their way
 constexpr int kPPitch = 144;                    // bytes of a row's nine pieces: conflict-free 16-byte reads
 constexpr int kSingle = -1, kEmpty = INT_MIN / 2;   // row kinds, as in the band table (acsr_meta.cu)
 enum : int { kErrQ = 11, kErrFull = 12, kErrEmpty = 13, kErrReady = 14, kErrFree = 15 };
@@ -425,10 +424,14 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
 // ---------------------------------------------------------------------------------------------
 // SpMM
 // ---------------------------------------------------------------------------------------------
-template <int D> struct SpmmLayout {
+// kPerSm CTAs share an SM: two with three steps of P on their way, or, at D = 64 and with more than two CTAs per SM to
+// run, three with two steps each (96 registers and some spills): B3 H44 L7680 window 224 216 -> 200 us, B2 H116 L4032
+// +-17 146 -> 124 us; a single wave (H8 L1024) is faster with two, 7.5 against 8.3 us.
+template <int D, int kPerSm> struct SpmmLayout {
     static constexpr int kSub = D / 64;
     static constexpr int kItemBytes = kSub * kStepBytesPerSub;    // 64 keys of V
     static constexpr int kPBytes = kTile * kPPitch;               // a step's pieces of P
+    static constexpr int kPStages = kPerSm == 2 ? 3 : 2;          // steps of P on their way
     static constexpr int kPOff = 0;                               // later reused as the output's staging
     static constexpr int kFront = (kPStages * kPBytes + 1023) / 1024 * 1024;
     static constexpr int kRingOff = kFront;
@@ -437,10 +440,11 @@ template <int D> struct SpmmLayout {
     static_assert(kFront >= kSub * kSubBytes, "output staging");
 };
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kThreads, 2)
+template <typename T, int D, int kPerSm>
+__global__ void __launch_bounds__(kThreads, kPerSm)
 spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
-    using L = SpmmLayout<D>;
+    using L = SpmmLayout<D, kPerSm>;
+    constexpr int kPStages = L::kPStages;
     constexpr int kTmemCols = D == 128 ? 256 : 128;   // the output accumulator, two steps of P (32 columns each)
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -707,11 +711,18 @@ static int32_t launch_sddmm(const Maps<2>& maps, const Params& prm, int64_t bh, 
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), SddmmLayout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
     return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, SddmmLayout<D>::kSmemBytes, st, maps, prm);
 }
-template <typename T, int D>
+template <typename T, int D, int kPerSm>
 static int32_t launch_spmm(const Maps<2>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
-    auto kern = spmm_band_kernel<T, D>;
-    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), SpmmLayout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
-    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, SpmmLayout<D>::kSmemBytes, st, maps, prm);
+    auto kern = spmm_band_kernel<T, D, kPerSm>;
+    constexpr int bytes = SpmmLayout<D, kPerSm>::kSmemBytes;
+    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), bytes)) return SPLAT_ERR_LAUNCH;
+    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, bytes, st, maps, prm);
+}
+template <typename T>
+static int32_t launch_spmm(const Maps<2>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
+    if (prm.d > 64) return launch_spmm<T, 128, 2>(maps, prm, bh, st);
+    const dim3 grid = prm.cls.grid(prm.stride, bh);
+    return (int64_t)grid.x * grid.y * grid.z > 2 * 148 ? launch_spmm<T, 64, 3>(maps, prm, bh, st) : launch_spmm<T, 64, 2>(maps, prm, bh, st);
 }
 
 // Checks shared by both operators; fills stride.  plan as written by splat_acsr_classify:
@@ -810,9 +821,7 @@ extern "C" int32_t splat_spmm_band_table(const void* p_in, const void* v, void* 
                                 !p.cls.view(m + 1, o, dtype, bh, n_rows, d, stride, part, 32)))
             return SPLAT_ERR_DRIVER;
     }
-    if (dtype == SPLAT_BF16)
-        return d > 64 ? ops::launch_spmm<__nv_bfloat16, 128>(maps, p, bh, st) : ops::launch_spmm<__nv_bfloat16, 64>(maps, p, bh, st);
-    return d > 64 ? ops::launch_spmm<__half, 128>(maps, p, bh, st) : ops::launch_spmm<__half, 64>(maps, p, bh, st);
+    return dtype == SPLAT_BF16 ? ops::launch_spmm<__nv_bfloat16>(maps, p, bh, st) : ops::launch_spmm<__half>(maps, p, bh, st);
 }
 
 extern "C" int32_t splat_sddmm_band(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
