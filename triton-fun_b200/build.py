@@ -59,7 +59,7 @@ def build_host(force: bool = False) -> str:
            "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
            "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_paths()["include"],
            HOST_SRC, "-o", HOST_PATH, "-L" + os.path.join(root, "lib"),
-           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
     print(" ".join(cmd), file=sys.stderr)
     subprocess.run(cmd, check=True)
     return HOST_PATH
