@@ -269,7 +269,8 @@ int32_t splat_transpose_16(const void* in, void* out, int64_t bh, int64_t d, int
 /* Attention over host-resident (page-locked) q, k, v, o of (BH, n_rows, d), k not transposed, streamed through
  * the device in chunks of `chunk` heads.  staging_8: two sets of device buffers q, k, v, o of chunk heads.
  * events_7: CUDA events that have been recorded at least once, used by one caller at a time.  The copies run on
- * stream_in and stream_out, the kernels on stream, which at the end waits for the last copy. */
+ * stream_in and stream_out, the kernels on stream, which at the end waits for the last copy.  The host arrays
+ * have to stay until then. */
 int32_t splat_attention_host(const void* q, const void* k, const void* v, void* o, void* const* staging_8,
                              int64_t chunk, const float* sTod_lin, const float* sTod_tr, const float* nnzs,
                              int64_t bh, int64_t n_rows, int64_t d, float scale, int32_t dtype, int32_t path,

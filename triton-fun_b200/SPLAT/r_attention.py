@@ -129,8 +129,8 @@ class RegularAttention(nn.Module):
         ``chunk_heads``: the host->device copy of chunk i+1 and the device->host copy of chunk
         i-1 overlap the fused kernel of chunk i (three streams, two staging buffers, allocated on
         first use).  Work is enqueued asynchronously; the caller's current stream waits for the last
-        device->host copy, so synchronising that stream makes ``out_host`` valid.  Not in the
-        reference, whose operands are always device tensors."""
+        device->host copy, so synchronising that stream makes ``out_host`` valid.  Page-locked operands may
+        be dropped right away (torch's allocator keeps their blocks until they have been copied).  Not in the reference, whose operands are always device tensors."""
         B, H, L, d = q_host.shape
         bh = B * H
         if bh == 0 or L == 0:

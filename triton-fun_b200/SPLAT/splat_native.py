@@ -202,12 +202,16 @@ def attention_host(q, k, v, out, stage: dict, sTod_lin, sTod_tr, nnzs, scale: fl
     plan_arr = (ctypes.c_int32 * 8)(*plan)
     _debug_before(dev)
     with _on(dev):
-        check(_lib.splat_attention_host(
+        rc = _lib.splat_attention_host(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), stage["staging"], stage["chunk"],
             _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"), _f32_vec(nnzs, L, "nnzs"), B * H, L, d,
             float(scale), dtype_code(q.dtype), int(path), ctypes.cast(plan_arr, _vp) if path != PATH_GENERIC else None,
             _band_table(sTod_lin, sTod_tr, nnzs), sw.data_ptr(), ctypes.byref(ran), stage["s_in"].cuda_stream, _stream(dev),
-            stage["s_out"].cuda_stream, stage["events"]), "splat_attention_host")
+            stage["s_out"].cuda_stream, stage["events"])
+        # the caller may drop its tensors now: their page-locked blocks are reused only when the copies are done
+        for t, s in ((q, stage["s_in"]), (k, stage["s_in"]), (v, stage["s_in"]), (out, stage["s_out"])):
+            _host.record_pinned(t, s.stream_id, s.device_index, s.device_type)
+    check(rc, "splat_attention_host")
     if ran.value != PATH_BAND and q.dtype != torch.float32 and q.numel() > 0 and path == PATH_AUTO:
         _warn_cuda_core_16bit("attention")
     if os.environ.get("SPLAT_B200_DEBUG"):

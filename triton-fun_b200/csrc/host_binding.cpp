@@ -11,6 +11,7 @@
 // the library splat_native loaded, and the library itself stays free of torch.
 #include <Python.h>
 
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
@@ -478,6 +479,28 @@ PyObject* acsr_from_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return out;
 }
 
+// record_pinned(host tensor, stream id, device index, device type): a copy from or to the tensor has been queued on the
+// stream by other means than torch's copy_().  The page-locked allocator then keeps the block, once it is
+// freed, until what the stream holds at that time is done; memory that is not the allocator's is left alone.
+PyObject* record_pinned(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    const at::Tensor* t = n == 4 ? tensor(a[0]) : nullptr;
+    long id, device, type;
+    if (t == nullptr || !as_long(a[1], &id) || !as_long(a[2], &device) || !as_long(a[3], &type)) {
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "record_pinned(tensor, stream id, device index, device type)");
+        return nullptr;
+    }
+    try {
+        const auto stream = c10::Stream::unpack3(id, static_cast<c10::DeviceIndex>(device), static_cast<c10::DeviceType>(type));
+        if (t->device().is_cpu())
+            at::getHostAllocator(at::kCUDA)->record_event(const_cast<void*>(t->const_data_ptr()),
+                                                          t->storage().data_ptr().get_context(), stream);
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+    Py_RETURN_NONE;
+}
+
 PyMethodDef methods[] = {
     {"bind", bind, METH_VARARGS, nullptr},
     {"set_status", set_status, METH_VARARGS, nullptr},
@@ -486,6 +509,7 @@ PyMethodDef methods[] = {
     {"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(spmm)), METH_FASTCALL, nullptr},
     {"set_mask_work", set_mask_work, METH_VARARGS, nullptr},
     {"acsr_from_mask", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(acsr_from_mask)), METH_FASTCALL, nullptr},
+    {"record_pinned", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(record_pinned)), METH_FASTCALL, nullptr},
     {"softmax", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(softmax)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "splat_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
