@@ -158,6 +158,10 @@ int32_t splat_spmm(const void* p, const void* v, void* o, const float* sTod_lin,
  *                 enqueue time).  Read the word wherever the stream is synchronised anyway; a
  *                 non-zero value means the outputs of that launch and of every later one are not
  *                 valid until the word is cleared.
+ * A row's result depends on its own keys alone, whatever Q, K and V hold elsewhere (splat_spmm* likewise) -- with
+ * one exception: 16-bit operands of d = 64 or 128 whose stride divides n_rows, on the tensor-core kernels.
+ * There V has to be finite at every key that some row of the same 128-row tile attends to, and a row with one
+ * non-zero returns V[start] whatever its score.
  * Under SPLAT_PATH_AUTO a band path that does not apply (shape, pattern, operand alignment, no
  * tensor-map support in the driver) falls through to the generic kernel. */
 int32_t splat_attention_fused(const void* q, const void* k, int64_t k_stride_bh,

@@ -661,7 +661,7 @@ static void map_cache_put(const MapKey& key, const CUtensorMap& map) {
 bool allow_dynamic_smem(const void* kernel, int bytes) {
     struct Seen { const void* kernel; int device; };
     static std::mutex mutex;
-    static Seen seen[64];
+    static Seen seen[128];
     static int n_seen = 0;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
@@ -670,7 +670,7 @@ bool allow_dynamic_smem(const void* kernel, int bytes) {
         if (seen[i].kernel == kernel && seen[i].device == dev) return true;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
         return false;
-    if (n_seen < 64) seen[n_seen++] = Seen{kernel, dev};
+    if (n_seen < 128) seen[n_seen++] = Seen{kernel, dev};
     return true;
 }
 

@@ -32,6 +32,7 @@
 
 #include "band_classes.cuh"
 #include "common.cuh"
+#include "row_exact.cuh"
 #include "softmax_math.cuh"
 #include "tc_ptx.cuh"
 
@@ -69,6 +70,7 @@ struct Params {
     const void* q;     // raw operands: rows with one non-zero are handled through them
     const void* k;
     const void* v;
+    void* o;
     const int2* rows;  // band table (see acsr_meta.cu): rows in class order, tiles' key ranges; or null
     const int2* tiles;
     float* lse;        // (BH, L) or null
@@ -91,6 +93,8 @@ struct Control {
     uint32_t tmem_base;
     int32_t abort_at_entry;
     int32_t lo[4], hi[4];      // key range of the rows' bands: of the tile (table), or per softmax warp
+    alignas(16) uint32_t again[4];   // rows whose result is not finite
+    alignas(16) uint32_t single[4];  // rows with one non-zero; later those of them whose score is not finite
 };
 
 template <int D> struct Layout {
@@ -139,7 +143,77 @@ __device__ __noinline__ void rescale_o(uint32_t o_addr, int n, float corr) {
     tmem_st_wait();
 }
 
-template <typename T, int D, bool kLse>
+// Band [begin, end) of a row in class coordinates; end = kSingle for a row with one non-zero (begin = its column),
+// kEmpty for one without and past the end of the class.
+constexpr int kSingle = -1, kEmpty = INT_MIN / 2;
+__device__ __forceinline__ int2 band_of(const Params& p, int res, int u) {
+    if (p.rows != nullptr) return __ldg(p.rows + p.cls.first_row(res) + u);
+    const RowAffine ra = row_affine(p.lin, p.tr, p.nnzs, (int64_t)u * p.stride + res);
+    if (ra.nnz > 1) {
+        const int begin = p.stride == 1 ? ra.start : (ra.start - res) / p.stride;
+        return make_int2(begin, begin + ra.nnz);
+    }
+    return ra.nnz == 1 ? make_int2(ra.start, kSingle) : make_int2(0, kEmpty);
+}
+
+// Rows of a tile that came out not finite, perhaps by keys outside their bands: from their own keys (row_exact.cuh),
+// after the tile has been stored.
+template <typename T>
+__device__ __noinline__ void rows_again(const Params p, uint4 again, int64_t bh, int res, int u0) {
+    const uint32_t mask[4] = {again.x, again.y, again.z, again.w};
+    const int64_t head = bh * p.n_rows;
+    const T* k = reinterpret_cast<const T*>(p.k) + head * p.d;
+    const T* v = reinterpret_cast<const T*>(p.v) + head * p.d;
+    for (int t = threadIdx.x >> 5; t < kTile; t += kThreads / 32) {
+        if (((mask[t >> 5] >> (t & 31)) & 1u) == 0) continue;
+        const int2 band = band_of(p, res, u0 + t);
+        const int64_t row = head + (int64_t)(u0 + t) * p.stride + res;
+        const bool one = band.y == kSingle;
+        const float4 x = attention_row<T>(reinterpret_cast<const T*>(p.q) + row * p.d, k, p.kt_major ? 1 : p.d,
+                                          p.kt_major ? p.n_rows : 1, v, one ? band.x : (int64_t)band.x * p.stride + res,
+                                          p.stride, one ? 1 : min(band.y, p.cls.rows_of(res)) - band.x, p.d, p.scale_log2);
+        store_row<T>(reinterpret_cast<T*>(p.o) + row * p.d, p.d, x);
+    }
+}
+
+// Rows of a tile with one non-zero whose score is not finite, of those in `single` (a bit per row).  Such a row takes
+// V[start] without its score having been formed (the metadata gives column 0 as its place, outside its band as a
+// rule).  By the TMA warp, which has requested all it can for now, a row per lane: in the softmax warps it cost 40 us
+// of a strided call's 103.
+template <typename T>
+__device__ __forceinline__ uint4 odd_singles(const Params& p, uint4 single, int64_t bh, int res, int u0) {
+    const int lane = threadIdx.x & 31;
+    uint32_t rows[4] = {single.x, single.y, single.z, single.w};
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        float s = 0.f;
+        if ((rows[w] >> lane) & 1u) {
+            const int u = u0 + w * 32 + lane;
+            const int64_t col = band_of(p, res, u).x;
+            const T* q = reinterpret_cast<const T*>(p.q) + (bh * p.n_rows + (int64_t)u * p.stride + res) * p.d;
+            const T* k = reinterpret_cast<const T*>(p.k) + bh * p.n_rows * p.d + (p.kt_major ? col : col * p.d);
+#pragma unroll 4
+            for (int c = 0; c < p.d; c += 8) {
+                const uint4 a = *reinterpret_cast<const uint4*>(q + c);
+                uint4 b;
+                T* kc = reinterpret_cast<T*>(&b);
+                if (p.kt_major) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) kc[i] = k[(int64_t)(c + i) * p.n_rows];
+                } else {
+                    b = *reinterpret_cast<const uint4*>(k + c);
+                }
+                const T* qc = reinterpret_cast<const T*>(&a);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) s = fmaf(DT<T>::to_f(qc[i]), DT<T>::to_f(kc[i]), s);
+            }
+        }
+        rows[w] = __ballot_sync(0xffffffffu, !isfinite(s * p.scale_log2));
+    }
+    return make_uint4(rows[0], rows[1], rows[2], rows[3]);
+}
+
+template <typename T, int D, bool kLse, bool kOwn>
 __global__ void __launch_bounds__(kThreads, 2)
 attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     using L = Layout<D>;
@@ -185,10 +259,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
         ++jv;
         return true;
     };
-    // Band [begin, end) of this thread's row in class coordinates; end = kSingle for a row with one non-zero
-    // (begin = its column), kEmpty for one without and past the end of the class.
-    constexpr int kSingle = -1, kEmpty = INT_MIN / 2;
-    int my_begin = 0, my_end = kEmpty;
+    int my_begin = 0, my_end = kEmpty;      // band of this thread's row
     if (warp == kMmaWarp) {
         depend_wait();
         tmem_alloc(&ctrl->tmem_base, kTmemCols);
@@ -232,24 +303,17 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
         depend_wait();
         const int u = u0 + warp * 32 + lane;
         if (u < rows_v) {
-            if (p.rows != nullptr) {
-                const int2 band = __ldg(p.rows + p.cls.first_row(real_res) + u);
-                my_begin = band.x;
-                my_end = band.y;
-            } else {
-                const RowAffine ra = row_affine(p.lin, p.tr, p.nnzs, (int64_t)u * p.stride + real_res);
-                if (ra.nnz > 1) {
-                    my_begin = p.stride == 1 ? ra.start : (ra.start - real_res) / p.stride;
-                    my_end = my_begin + ra.nnz;
-                } else if (ra.nnz == 1) {
-                    my_begin = ra.start;
-                    my_end = kSingle;
-                }
-            }
+            const int2 band = band_of(p, real_res, u);
+            my_begin = band.x;
+            my_end = band.y;
             if (my_end == kSingle) {   // its row of V is copied at the end
                 const char* vrow = reinterpret_cast<const char*>(p.v) + (bh * p.n_rows + my_begin) * p.d * 2;
                 for (int i = 0; i < p.d * 2; i += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(vrow + i));
             }
+        }
+        if constexpr (kOwn) {
+            const unsigned single = __ballot_sync(0xffffffffu, my_end == kSingle);
+            if (lane == 0) ctrl->single[warp] = single;
         }
         if (p.rows == nullptr) {
             const int lo = warp_min_i(my_end > 0 ? my_begin : INT_MAX), hi = warp_max_i(max(my_end, 0));
@@ -282,6 +346,14 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
 
     if (warp == kTmaWarp) {
         // ------------------------------------------------------------------ TMA producer
+        if constexpr (kOwn) {
+            const uint4 single = *reinterpret_cast<const uint4*>(ctrl->single);
+            if ((single.x | single.y | single.z | single.w) != 0) {
+                const uint4 odd = odd_singles<T>(p, single, bh, real_res, u0);
+                __syncwarp();
+                if (lane == 0) *reinterpret_cast<uint4*>(ctrl->single) = odd;
+            }
+        }
         if (lane == 0) {
             bool ok = true;
             while (ok && jv < steps) {     // K(0) V(0) K(1) V(1) ...: the order in which the slots come free
@@ -459,7 +531,8 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
         // epilogue: O / l for band rows, V[start] for single-element rows, zero otherwise.  Rows are staged in
         // the Q tile's memory (every MMA has completed) in the 128-byte-swizzled tile layout and leave
         // through one tiled TMA store per 64 columns and warp (rows and columns past the end are clipped).
-        const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
+        // (all scores of a row -inf: zeros, or NaN like the row kernels)
+        const float inv = kOwn || l_sum > 0.f ? 1.f / l_sum : 0.f;
         const int64_t head = bh * p.n_rows;
         const int u = u0 + warp * 32 + lane;
         const int64_t row_real = u < rows_v ? (int64_t)u * p.stride + real_res : -1;
@@ -480,10 +553,18 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
         const T* vrow = reinterpret_cast<const T*>(p.v) + (head + row_start) * p.d;
         const int t = warp * 32 + lane;
         uint32_t o_raw[D];
+        float2 odd0 = make_float2(0.f, 0.f), odd1 = odd0;       // not finite: nor is the row
         if (have_o && ok) {
 #pragma unroll
             for (int ch = 0; ch < D / 32; ++ch) tmem_ld32(o_addr + ch * 32, o_raw + ch * 32);
             tmem_ld_wait();
+            if constexpr (kOwn) {
+#pragma unroll
+                for (int j = 0; j < D; j += 8) {
+                    odd0 = note_nonfinite(odd0, o_raw + j);
+                    odd1 = note_nonfinite(odd1, o_raw + j + 4);
+                }
+            }
         }
 #pragma unroll
         for (int ch = 0; ch < D / 32; ++ch) {
@@ -507,6 +588,10 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
             for (int i = 0; i < 4; ++i)
                 *reinterpret_cast<uint4*>(srow + ((((ch & 1) * 4 + i) ^ (t & 7)) << 4)) = out[i];
         }
+        if constexpr (kOwn) {
+            const unsigned again = __ballot_sync(0xffffffffu, row_nnz > 1 && !isfinite(odd0.x + odd0.y + (odd1.x + odd1.y)));
+            if (lane == 0) ctrl->again[warp] = again;
+        }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && u0 + warp * 32 < rows_v) {
@@ -523,11 +608,26 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kTmemCols);
     }
+    if constexpr (kOwn) {
+        const uint4 again = *reinterpret_cast<const uint4*>(ctrl->again), odd = *reinterpret_cast<const uint4*>(ctrl->single);
+        if ((again.x | again.y | again.z | again.w | odd.x | odd.y | odd.z | odd.w) != 0) {
+            if (warp < 4 && lane == 0) tma_store_wait_all();      // the tile is in memory before its rows are written again
+            __syncthreads();
+            rows_again<T>(p, make_uint4(again.x | odd.x, again.y | odd.y, again.z | odd.z, again.w | odd.w), bh, real_res, u0);
+        }
+    }
 }
 
+// `own`: a row's result depends on its own keys alone, also where Q, K or V is not finite at other ones.  It takes a look at
+// every result and code for the rows that need it; that costs 3 % (fp16 B4 H16 L4096 d64 window 256 64.1 -> 66.0 us, bf16
+// B8 H64 L32768 d128 window 1024 11.71 -> 12.12 ms).  Problems with d = 64 or 128 and classes of one length do without:
+// they have only ever run on tensor cores, with finite V as a condition (splat_b200.h); the others came from the row
+// kernels, which read nothing but a row's own keys.
 template <typename T, int D>
 static int32_t launch(const Maps<4>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
-    auto kern = prm.lse != nullptr ? attention_wide_kernel<T, D, true> : attention_wide_kernel<T, D, false>;
+    const bool own = (prm.d != 64 && prm.d != 128) || prm.cls.longer != 0;
+    auto kern = own ? (prm.lse != nullptr ? attention_wide_kernel<T, D, true, true> : attention_wide_kernel<T, D, false, true>)
+                    : (prm.lse != nullptr ? attention_wide_kernel<T, D, true, false> : attention_wide_kernel<T, D, false, false>);
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), Layout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
     return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, Layout<D>::kSmemBytes, st, maps, prm);
 }
@@ -541,7 +641,7 @@ int32_t attention_wide(const void* q, const void* k, int kt_major, const void* v
                        int32_t* status_word, const int32_t* band_table, float* lse, cudaStream_t st) {
     using namespace band;
     wide::Params p;
-    p.lin = lin; p.tr = tr; p.nnzs = nnzs; p.q = q; p.k = k; p.v = v; p.lse = lse;
+    p.lin = lin; p.tr = tr; p.nnzs = nnzs; p.q = q; p.k = k; p.v = v; p.o = o; p.lse = lse;
     p.status = status_word; p.mirror = status_mirror(status_word);
     p.n_rows = n_rows; p.stride = (int)stride; p.d = (int)d;
     p.kt_major = kt_major; p.scale_log2 = scale * kLog2e;

@@ -28,6 +28,7 @@
 
 #include "band_classes.cuh"
 #include "common.cuh"
+#include "row_exact.cuh"
 #include "softmax_math.cuh"
 #include "tc_ptx.cuh"
 
@@ -60,6 +61,7 @@ struct Params {
     const int2* tiles;
     const void* q;       // sddmm: (BH, L, d), for rows with one non-zero
     const void* kv;      // sddmm: K, spmm: V
+    void* o;             // spmm: (BH, L, d)
     uint16_t* sparse;    // sddmm: S out, spmm: P in, (BH, L, trailing_dim), rounded down to 16 bytes ...
     int lead;            // ... and the elements lost by that
     int32_t* status;
@@ -652,12 +654,15 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         const bool single = band.y == kSingle;
         const T* vrow = reinterpret_cast<const T*>(p.kv) + (head + band.x) * p.d;
         const float p0 = single ? to_f<T>(*reinterpret_cast<const T*>(p.sparse + e_row + band.x)) : 0.f;
+        float2 odd = make_float2(0.f, 0.f);       // not finite: nor is the row
 #pragma unroll
         for (int ch = 0; ch < D / 32; ++ch) {
             uint32_t r[32];
             if (have_o && ok) {
                 tmem_ld32(lane_addr + ch * 32, r);
                 tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) odd = note_nonfinite(odd, r + j);
             }
             uint4 outv[4];
             uint32_t* o32 = reinterpret_cast<uint32_t*>(outv);
@@ -684,13 +689,26 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             for (int q4 = 0; q4 < 4; ++q4)
                 *reinterpret_cast<uint4*>(srow + ((((ch & 1) * 4 + q4) ^ (t & 7)) << 4)) = outv[q4];
         }
+        unsigned again = __ballot_sync(0xffffffffu, band.y > 0 && !isfinite(odd.x + odd.y));
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && u0 + warp * 32 < rows_v) {
             for (int sub = 0; sub < L::kSub; ++sub)
                 tma_store_4d(map + 1, smem + sub * kSubBytes + warp * 32 * 128, sub * 64, res, u0 + warp * 32, (int)bh);
             tma_store_commit();
-            tma_store_wait_read();
+            if (again == 0) tma_store_wait_read();
+            else tma_store_wait_all();
+        }
+        while (again) {        // rows that are not finite, perhaps by keys outside their bands
+            __syncwarp();
+            const int rr = __ffs(again) - 1;
+            again &= again - 1;
+            const int begin = __shfl_sync(0xffffffffu, band.x, rr), end = min(__shfl_sync(0xffffffffu, band.y, rr), rows_v);
+            const int64_t row = head + (int64_t)(u0 + warp * 32 + rr) * p.stride + real_res;
+            const float4 x = spmm_row<T>(reinterpret_cast<const T*>(p.sparse + p.lead + row * p.trailing_dim),
+                                         reinterpret_cast<const T*>(p.kv) + head * p.d, (int64_t)begin * p.stride + real_res,
+                                         p.stride, end - begin, p.d);
+            store_row<T>(reinterpret_cast<T*>(p.o) + row * p.d, p.d, x);
         }
     }
     tc_fence_before_sync();
@@ -812,7 +830,7 @@ extern "C" int32_t splat_spmm_band_table(const void* p_in, const void* v, void* 
     if (!p_in || !v || !o || !sTod_lin || !sTod_tr || !nnzs || !status_word) return SPLAT_ERR_BAD_ARG;
     if (!aligned16(v) || !aligned16(o)) return SPLAT_ERR_MISALIGNED;
     ops::Params p = ops::params(p_in, sTod_lin, sTod_tr, nnzs, n_rows, d, trailing_dim, stride, band_table, status_word);
-    p.kv = v;
+    p.kv = v; p.o = o;
     cudaStream_t st = (cudaStream_t)stream;
     Maps<2> maps;
     for (int part = 0; part < 2; ++part) {

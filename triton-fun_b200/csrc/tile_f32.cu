@@ -39,6 +39,7 @@
 #include <limits.h>
 
 #include "common.cuh"
+#include "row_exact.cuh"
 
 namespace splat {
 namespace tile {
@@ -172,8 +173,45 @@ __device__ __forceinline__ void load_v(float* smem, const float* base, int64_t p
     }
 }
 
+// One row of the fused operator that may have come out not finite by keys outside its band: from its own n keys
+// (row_exact.cuh).
+template <int D>
+__device__ __noinline__ void fused_row_again(const Params& p, int64_t head, int64_t row, int start, int n) {
+    float* o = p.o + row * D;
+    bool odd = false;
+#pragma unroll
+    for (int c = threadIdx.x & 31; c < D; c += 32) odd = odd || !isfinite(o[c]);
+    if (__any_sync(0xffffffffu, odd))
+        store_row(o, D, attention_row<float>(p.q + row * D, p.k + head * D, p.kt ? 1 : D, p.kt ? p.n_rows : 1, p.v + head * D,
+                                             start, p.stride, n, D, p.scale_log2));
+}
+// Rows with one non-zero elsewhere, a row per lane that has one: V[start] so far, NaN if the score is not finite.
+template <int D>
+__device__ __noinline__ void fused_singles_again(const Params& p, int64_t head, int64_t row, int start, bool mine) {
+    float s = 0.f;
+    if (mine) {
+        const float* q = p.q + row * D;
+        const float* k = p.k + head * D + (p.kt ? start : (int64_t)start * D);
+        const int64_t ksk = p.kt ? p.n_rows : 1;
+#pragma unroll 16
+        for (int c = 0; c < D; ++c) s = fmaf(q[c], k[c * ksk], s);
+    }
+    for (unsigned odd = __ballot_sync(0xffffffffu, !isfinite(s * p.scale_log2)); odd != 0; odd &= odd - 1) {
+        const int64_t r = __shfl_sync(0xffffffffu, row, __ffs(odd) - 1);
+        for (int c = threadIdx.x & 31; c < D; c += 32) p.o[r * D + c] = NAN;
+    }
+}
+// ... of SpMM (parameters by value: see tile_kernel)
+template <int D>
+__device__ __noinline__ void spmm_row_again(const float* prow, const float* v, float* o, int start, int stride, int n) {
+    bool odd = false;
+#pragma unroll
+    for (int c = threadIdx.x & 31; c < D; c += 32) odd = odd || !isfinite(o[c]);
+    if (__any_sync(0xffffffffu, odd)) store_row(o, D, spmm_row<float>(prow, v, start, stride, n, D));
+}
+
 template <int D, int RW, int KW, Op OP>
-__global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) tile_kernel(const Params p) {
+__device__ __forceinline__ void tile_body(const Params& p) {
     using L = Layout<D, RW, KW, OP>;
     constexpr int kRows = L::kRows, kGroups = L::kGroups, kWarps = L::kWarps;
     extern __shared__ __align__(16) float smem[];
@@ -225,6 +263,11 @@ __global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) t
 #pragma unroll
         for (int x = 0; x < RW; ++x) { k_lo = min(k_lo, ranges[x].x); k_hi = max(k_hi, ranges[x].y); }
         __syncthreads();           // the ranges have been read: the key buffers may be filled
+    }
+    // A row with one non-zero among the warp's keys is a band like any other (its probability comes out as 1).
+    if (OP == Op::kFused && my_nnz == 1) {
+        const int b = (my_start - res) / p.stride;
+        if (b * p.stride == my_start - res && b >= min_a && b < max_end) { my_a = b; my_n = 1; my_nnz = 2; }
     }
     k_lo = k_hi > 0 ? k_lo / kKeys : 0;
     k_hi = (k_hi + kKeys - 1) / kKeys;
@@ -431,6 +474,7 @@ __global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) t
     }
     __syncthreads();
     // a group's warp merges and writes 32 / kGroups of its rows, lanes along D
+    float odd = 0.f;               // NaN: a row is not finite, or has its only non-zero elsewhere
     const float* parts = smem + rw * L::kPart;          // of these rows by group 0; the next group RW parts on
 #pragma unroll 2
     for (int i = 0; i < 32 / kGroups; ++i) {
@@ -454,7 +498,7 @@ __global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) t
             }
         }
         if (OP == Op::kFused) {
-            const float inv = lt > 0.f ? 1.f / lt : 0.f;
+            const float inv = 1.f / lt;        // (rows whose scores are all -inf: NaN; empty ones are zeroed below)
 #pragma unroll
             for (int x = 0; x < kGroups; ++x) w[x] *= inv;
         }
@@ -471,7 +515,9 @@ __global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) t
                 y = w1 * p.v[(head + start) * D + c];
             }
             p.o[real * D + c] = y;
+            odd = fmaf(y, 0.f, odd);
         }
+        if (OP == Op::kFused && nnz == 1) odd = NAN;
         if (OP == Op::kFused && p.lse != nullptr && lane == 0) {
             float e = nnz > 1 ? lse_from_log2(mt, lt) : -INFINITY;
             if (nnz == 1) {
@@ -481,6 +527,34 @@ __global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) t
             p.lse[real] = e;
         }
     }
+    if (__any_sync(0xffffffffu, odd != 0.f)) {
+        if (OP == Op::kFused)
+            fused_singles_again<D>(p, head, head + (int64_t)(u0 + lane) * p.stride + res, my_start,
+                                   my_nnz == 1 && lane / (32 / kGroups) == group);
+#pragma unroll 1
+        for (int i = 0; i < 32 / kGroups; ++i) {
+            const int row = group * (32 / kGroups) + i;
+            const int start = __shfl_sync(0xffffffffu, my_start, row);
+            const int n = __shfl_sync(0xffffffffu, my_n, row);
+            if (n == 0) continue;
+            const int64_t real = head + (int64_t)(u0 + row) * p.stride + res;
+            const int own = min(n, (p.n_rows - 1 - start) / p.stride + 1);
+            if (OP == Op::kFused) fused_row_again<D>(p, head, real, start, own);
+            else spmm_row_again<D>(p.sparse + real * p.trailing, p.v + head * D, p.o + real * D, start, p.stride, own);
+        }
+    }
+}
+
+// (Parameters by value, or by reference to where they are: the repair at the end of tile_body changes how the rest is
+// compiled.  Fused B2 H16 L4096 d64 270 against 262 us, the three launchers of H8 L1024 32.3 against 33.7 us.)
+template <int D, int RW, int KW, Op OP>
+__global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) tile_kernel(const Params p) {
+    tile_body<D, RW, KW, OP>(p);
+}
+template <int D, int RW, int KW>
+__global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, Op::kFused>::kPerSm)
+tile_kernel_fused(const __grid_constant__ Params p) {
+    tile_body<D, RW, KW, Op::kFused>(p);
 }
 
 }  // namespace tile
@@ -495,7 +569,9 @@ namespace tile {
 template <int D, int RW, int KW, Op OP>
 static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
     constexpr int bytes = Layout<D, RW, KW, OP>::kFloats * (int)sizeof(float);
-    auto kern = tile_kernel<D, RW, KW, OP>;
+    void (*kern)(const Params);
+    if constexpr (OP == Op::kFused) kern = tile_kernel_fused<D, RW, KW>;
+    else kern = tile_kernel<D, RW, KW, OP>;
     if (!band::allow_dynamic_smem(reinterpret_cast<const void*>(kern), bytes)) return SPLAT_ERR_LAUNCH;
     p.tiles = ((p.n_rows + p.stride - 1) / p.stride + 32 * RW - 1) / (32 * RW);
     const int64_t blocks = (int64_t)p.tiles * p.stride * bh;
