@@ -246,7 +246,8 @@ int32_t splat_spmm_tile(const void* p, const void* v, void* o, const float* sTod
  * 128)) device int32, 8-byte aligned, holding every row's band and every 128-row tile's key range in the
  * layout the tensor-core kernels want (csrc/acsr_meta.cu).  A caller that keeps its metadata keeps the table
  * with it and passes it to splat_attention_fused_table (splat_attention_fused_lse with one more argument;
- * NULL: the kernels work the ranges out themselves).  It has to be rebuilt when the metadata changes. */
+ * NULL: the kernels work the ranges out themselves).  It has to be rebuilt when the metadata changes; a launch that
+ * is captured into a graph keeps its address. */
 int32_t splat_band_table(const float* sTod_lin, const float* sTod_tr, const float* nnzs, int64_t n_rows,
                          int64_t stride, int32_t* table, void* stream);
 int32_t splat_attention_fused_table(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,

@@ -3,6 +3,10 @@ when the caller drops or changes it right after the (asynchronous) call."""
 import pytest
 import torch
 
+from conftest import assert_close
+from oracle import acsr_oracle as ao
+from oracle import attention_oracle as at
+
 pytestmark = pytest.mark.gpu
 
 SLEEP = 400_000_000      # SM clocks, some 0.2 s: what is queued behind it has not begun when the host goes on
@@ -32,3 +36,41 @@ def test_forward_host_operands_may_be_dropped():
     others = [torch.full((B, H, L, d), 7.0, dtype=torch.bfloat16).pin_memory() for _ in range(6)]
     torch.cuda.synchronize()
     assert all((t == 7).all() for t in others)
+
+
+def test_captured_calls_follow_their_metadata():
+    """A replayed graph works with the metadata that the tensors hold at the replay, like any other operand."""
+    import acsr_helpers as ah
+    import r_attention
+    import splat_native as n
+    L, H, d, dtype = 640, 2, 64, torch.bfloat16
+    attn = r_attention.RegularAttention(1, L, H, d, ah.create_causal_windowed_mask(L, 200), 16, 16, 0, dtype, scale=0.125)
+    acsr = ah.create_acsr(ah.create_causal_windowed_mask(L, 200), 16, 0)
+    torch.manual_seed(4)
+    q, k, v = (torch.randn(1, H, L, d).to(dtype) for _ in range(3))
+    qd, vd, kt = q.cuda(), v.cuda(), k.cuda().transpose(2, 3)
+    s = torch.empty(1, H, L, acsr[5], dtype=dtype, device="cuda")
+    p = torch.rand(1, H, L, acsr[5]).to(dtype)
+    pd, o = p.cuda(), torch.empty_like(qd)
+
+    def calls():
+        fused = attn([qd, kt, vd])
+        n.sddmm(qd, kt, s, acsr[2], acsr[3], acsr[4], acsr[5])
+        n.spmm(pd, vd, o, acsr[2], acsr[3], acsr[4], acsr[5])
+        return fused
+
+    calls()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        fused = calls()
+    narrow = ah.create_acsr(ah.create_causal_windowed_mask(L, 70), 16, 0)
+    for i, name in ((2, "sTod_linear_transformations"), (3, "sTod_translations"), (4, "nnzs")):
+        getattr(attn, name).copy_(narrow[i])
+        acsr[i].copy_(narrow[i])
+    graph.replay()
+    torch.cuda.synchronize()
+    meta = ao.metadata_from_pattern(ao.PATTERN_CAUSAL_WINDOWED, L, 70, 0, 16)
+    assert_close(fused, at.attention_acsr(q, k.transpose(2, 3), v, meta, meta["trailing_dim"], 0.125), dtype, "fused")
+    assert_close(s, at.sddmm_acsr(q, k.transpose(2, 3), meta, acsr[5]), dtype, "sddmm")
+    assert_close(o, at.spmm_acsr(p, v, meta), dtype, "spmm")

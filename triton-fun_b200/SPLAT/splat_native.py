@@ -250,9 +250,10 @@ def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) 
 
 
 def _band_table(sTod_lin, sTod_tr, nnzs):
-    """Address of the band table remembered by classify(), or None if the metadata has changed since."""
+    """Address of the band table remembered by classify(), or None if the metadata has changed since -- or for
+    a captured launch, which has to work with the metadata as they are at the replay."""
     hit = getattr(nnzs, "_splat_plan", None)
-    if hit is None or hit[4] is None or hit[0] != (id(sTod_lin), id(sTod_tr), sTod_lin._version, sTod_tr._version,
+    if hit is None or hit[4] is None or _capturing(nnzs.device) or hit[0] != (id(sTod_lin), id(sTod_tr), sTod_lin._version, sTod_tr._version,
                                                    nnzs._version, nnzs.numel()):
         return None
     return hit[4].data_ptr()
@@ -305,6 +306,12 @@ def _on(dev: torch.device):
     if torch.cuda.current_device() == dev.index:
         return contextlib.nullcontext()
     return torch.cuda.device(dev)
+
+
+def _capturing(dev: torch.device) -> bool:
+    """Whether dev's current stream records a graph instead of running."""
+    with _on(dev):
+        return torch.cuda.is_current_stream_capturing()
 
 
 _INDEX_CODES = {71: "sddmm", 72: "spmm", 73: "fused"}

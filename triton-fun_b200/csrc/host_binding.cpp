@@ -16,6 +16,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -139,7 +140,8 @@ inline bool same4(const at::Tensor& t, int64_t a, int64_t b, int64_t c, int64_t 
 }
 
 // plan remembered by splat_native.classify() on the nnzs tensor: ((id, id, version x 3, numel), plan, lin, tr,
-// band table or None); false if the metadata is not what it was made from
+// band table or None); false if the metadata is not what it was made from.  A captured launch gets no table: a replay has to
+// follow the metadata as they are then, and the table's memory goes with the Python objects.
 bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, const at::Tensor& lin, PyObject* tr_obj,
                  const at::Tensor& tr, int32_t (&plan)[8], const int32_t** table = nullptr) {
     PyObject* hit = PyObject_GetAttr(nnzs_obj, k_cached_plan);
@@ -159,7 +161,8 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
             ok = as_long(PyTuple_GET_ITEM(key, 2 + i), &v) && v == now[i];
         }
         ok = ok && read_plan(PyTuple_GET_ITEM(hit, 1), plan);
-        if (ok && table != nullptr) {
+        if (ok && table != nullptr &&
+            c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
             const at::Tensor* t = tensor(PyTuple_GET_ITEM(hit, 4));
             if (t != nullptr) *table = static_cast<const int32_t*>(t->const_data_ptr());
         }
