@@ -74,3 +74,36 @@ def test_captured_calls_follow_their_metadata():
     assert_close(fused, at.attention_acsr(q, k.transpose(2, 3), v, meta, meta["trailing_dim"], 0.125), dtype, "fused")
     assert_close(s, at.sddmm_acsr(q, k.transpose(2, 3), meta, acsr[5]), dtype, "sddmm")
     assert_close(o, at.spmm_acsr(p, v, meta), dtype, "spmm")
+
+
+@pytest.mark.parametrize("call", ["module", "sddmm"])
+def test_band_table_of_a_call_on_another_stream(call):
+    """Metadata dropped while a call on a side stream waits: the caller records the tensors it knows of, the table
+    behind them has to last as long."""
+    import acsr_helpers as ah
+    import r_attention
+    import splat_native as n
+    L, H, d, dtype = 640, 2, 64, torch.bfloat16
+    attn = r_attention.RegularAttention(1, L, H, d, ah.create_causal_windowed_mask(L, 200), 16, 16, 0, dtype, scale=0.125)
+    T, side = attn.acsr_trailing_dim, torch.cuda.Stream()
+    q, k, v = (torch.randn(1, H, L, d, device="cuda").to(dtype) for _ in range(3))
+    s = torch.empty(1, H, L, T, dtype=dtype, device="cuda")
+
+    def run():
+        if call == "module":
+            return attn([q, k.transpose(2, 3), v])
+        n.sddmm(q, k.transpose(2, 3), s, attn.sTod_linear_transformations, attn.sTod_translations, attn.nnzs, T)
+        return s
+
+    expected = run().clone()
+    torch.cuda.synchronize()
+    size = attn.nnzs._splat_plan[4].numel()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(SLEEP)
+        out = run()
+    for t in (attn.sTod_linear_transformations, attn.sTod_translations, attn.nnzs):
+        t.record_stream(side)
+    del attn, t
+    others = [torch.zeros(size, dtype=torch.int32, device="cuda") for _ in range(8)]
+    torch.cuda.synchronize()
+    assert torch.equal(out, expected) and all((t == 0).all() for t in others)

@@ -245,7 +245,7 @@ def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) 
                                         table.data_ptr(), _stream(dev)), "splat_band_table")
             torch.cuda.current_stream(dev).synchronize()      # any stream may use it
     # keep the two companions alive with the cache entry so their ids cannot be reused
-    nnzs._splat_plan = (key, host, sTod_lin, sTod_tr, table)
+    nnzs._splat_plan = (key, host, sTod_lin, sTod_tr, table, _stream(dev))
     return host
 
 
@@ -256,6 +256,8 @@ def _band_table(sTod_lin, sTod_tr, nnzs):
     if hit is None or hit[4] is None or _capturing(nnzs.device) or hit[0] != (id(sTod_lin), id(sTod_tr), sTod_lin._version, sTod_tr._version,
                                                    nnzs._version, nnzs.numel()):
         return None
+    if hit[5] != _stream(nnzs.device):      # the table is nobody's tensor but ours: its use elsewhere is ours to record
+        hit[4].record_stream(torch.cuda.current_stream(nnzs.device))
     return hit[4].data_ptr()
 
 

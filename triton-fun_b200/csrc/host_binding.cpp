@@ -15,6 +15,7 @@
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
@@ -140,8 +141,9 @@ inline bool same4(const at::Tensor& t, int64_t a, int64_t b, int64_t c, int64_t 
 }
 
 // plan remembered by splat_native.classify() on the nnzs tensor: ((id, id, version x 3, numel), plan, lin, tr,
-// band table or None); false if the metadata is not what it was made from.  A captured launch gets no table: a replay has to
-// follow the metadata as they are then, and the table's memory goes with the Python objects.
+// band table or None, stream it was made on); false if the metadata is not what it was made from.  A captured launch gets
+// no table: a replay has to follow the metadata as they are then, and the table's memory goes with the Python objects.
+// The caller knows nothing of the table, so its use on another stream is recorded here.
 bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, const at::Tensor& lin, PyObject* tr_obj,
                  const at::Tensor& tr, int32_t (&plan)[8], const int32_t** table = nullptr) {
     PyObject* hit = PyObject_GetAttr(nnzs_obj, k_cached_plan);
@@ -149,7 +151,7 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
         PyErr_Clear();
         return false;
     }
-    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 5 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
+    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 6 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
               PyTuple_GET_ITEM(hit, 3) == tr_obj;
     if (ok) {
         PyObject* key = PyTuple_GET_ITEM(hit, 0);
@@ -164,7 +166,12 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
         if (ok && table != nullptr &&
             c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
             const at::Tensor* t = tensor(PyTuple_GET_ITEM(hit, 4));
-            if (t != nullptr) *table = static_cast<const int32_t*>(t->const_data_ptr());
+            if (t != nullptr) {
+                const auto stream = c10::cuda::getCurrentCUDAStream(t->get_device());
+                if (PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 5)) != stream.stream())
+                    c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
+                *table = static_cast<const int32_t*>(t->const_data_ptr());
+            }
         }
     }
     Py_DECREF(hit);
