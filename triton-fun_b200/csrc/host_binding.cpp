@@ -189,7 +189,12 @@ at::Tensor rows_of_k(const at::Tensor& kt, int64_t ksb, const int32_t (&plan)[8]
     const bool band = (plan[7] == 0 || plan[1] == plan[2]) && plan[3] == 0 && plan[5] <= n && n == L && d % 8 == 0 && d <= 128;
     const bool direct = kt.stride(2) == 1 || (stride == 1 && n % 8 == 0);
     if (!contiguous || !band || direct || bh > 65535 || g_api.transpose == nullptr) return {};
-    at::Tensor rows = at::empty({bh, n, d}, kt.options());
+    at::Tensor rows;
+    try {
+        rows = at::empty({bh, n, d}, kt.options());
+    } catch (const std::exception&) {      // no memory for it: the kernels that need none
+        return {};
+    }
     if (g_api.transpose(kt.const_data_ptr(), rows.data_ptr(), bh, d, n, stream) != 0) return {};
     return rows;
 }
@@ -245,8 +250,19 @@ PyObject* yes_or_none(bool yes) {
     Py_RETURN_NONE;
 }
 
+// Torch throws for tensors it has no data, strides or version of (fake, functional, sparse ones); nothing of that may
+// leave through CPython's frames.  Everything that throws comes before a call's launch, so Python can start over.
+template <PyObject* (*F)(PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    try {
+        return F(args, n);
+    } catch (...) {
+        return yes_or_none(false);
+    }
+}
+
 // module_forward(module.__dict__, [q, kt, v]) -> the module's output, or None
-PyObject* module_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* module_forward(PyObject* const* args, Py_ssize_t n) {
     if (n != 2 || !PyDict_Check(args[0])) Py_RETURN_NONE;
     PyObject *dict = args[0], *x = args[1];
     PyObject* item[3];
@@ -279,7 +295,7 @@ PyObject* module_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path) -> True, or None
-PyObject* sddmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+PyObject* sddmm(PyObject* const* a, Py_ssize_t n) {
     long trailing, path;
     if (n != 8 || !as_long(a[6], &trailing) || !as_long(a[7], &path) || path != kPathAuto) return yes_or_none(false);
     const at::Tensor *x = tensor(a[0]), *y = tensor(a[1]), *out = tensor(a[2]), *lin = tensor(a[3]), *tr = tensor(a[4]),
@@ -319,7 +335,7 @@ PyObject* sddmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // spmm(p, v, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path) -> True, or None
-PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+PyObject* spmm(PyObject* const* a, Py_ssize_t n) {
     long trailing, path;
     if (n != 8 || !as_long(a[6], &trailing) || !as_long(a[7], &path) || path != kPathAuto) return yes_or_none(false);
     const at::Tensor *x = tensor(a[0]), *y = tensor(a[1]), *out = tensor(a[2]), *lin = tensor(a[3]), *tr = tensor(a[4]),
@@ -351,7 +367,7 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // softmax(x, output, nnzs, trailing_dim, scale) -> True, or None
-PyObject* softmax(PyObject*, PyObject* const* a, Py_ssize_t n) {
+PyObject* softmax(PyObject* const* a, Py_ssize_t n) {
     long trailing;
     if (n != 5 || !as_long(a[3], &trailing) || !PyFloat_Check(a[4])) return yes_or_none(false);
     const at::Tensor *x = tensor(a[0]), *out = tensor(a[1]), *nnzs = tensor(a[2]);
@@ -514,13 +530,13 @@ PyObject* record_pinned(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef methods[] = {
     {"bind", bind, METH_VARARGS, nullptr},
     {"set_status", set_status, METH_VARARGS, nullptr},
-    {"module_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(module_forward)), METH_FASTCALL, nullptr},
-    {"sddmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sddmm)), METH_FASTCALL, nullptr},
-    {"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(spmm)), METH_FASTCALL, nullptr},
+    {"module_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<module_forward>)), METH_FASTCALL, nullptr},
+    {"sddmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<sddmm>)), METH_FASTCALL, nullptr},
+    {"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<spmm>)), METH_FASTCALL, nullptr},
     {"set_mask_work", set_mask_work, METH_VARARGS, nullptr},
     {"acsr_from_mask", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(acsr_from_mask)), METH_FASTCALL, nullptr},
     {"record_pinned", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(record_pinned)), METH_FASTCALL, nullptr},
-    {"softmax", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(softmax)), METH_FASTCALL, nullptr},
+    {"softmax", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<softmax>)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "splat_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
