@@ -163,11 +163,12 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
             ok = as_long(PyTuple_GET_ITEM(key, 2 + i), &v) && v == now[i];
         }
         ok = ok && read_plan(PyTuple_GET_ITEM(hit, 1), plan);
-        if (ok && table != nullptr &&
-            c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
+        if (ok && table != nullptr) {
             const at::Tensor* t = tensor(PyTuple_GET_ITEM(hit, 4));
-            if (t != nullptr) {
-                const auto stream = c10::cuda::getCurrentCUDAStream(t->get_device());
+            const auto stream = c10::cuda::getCurrentCUDAStream(t != nullptr ? t->get_device() : -1);
+            // (the legacy stream is never captured: asking costs 0.3 us of a small call)
+            if (t != nullptr && (stream.stream() == nullptr || c10::cuda::currentStreamCaptureStatusMayInitCtx() ==
+                                                                   c10::cuda::CaptureStatus::None)) {
                 if (PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 5)) != stream.stream())
                     c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
                 *table = static_cast<const int32_t*>(t->const_data_ptr());
