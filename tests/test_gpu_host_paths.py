@@ -82,3 +82,29 @@ def test_forward_host_in_chunks(dtype):
         torch.cuda.current_stream().synchronize()
         assert_close(out, at.attention_acsr(q, k.transpose(2, 3), v, meta, meta["trailing_dim"], 0.125), dtype, f"call {seed}")
     assert [r_attention.host_chunk(h, b) for h, b in ((32, 2 << 20), (6, 400 << 10), (1, 64 << 20), (7, 1 << 20))] == [5, 6, 1, 2]
+
+
+def test_other_threads_run_while_metadata_wait():
+    """create_acsr behind queued work waits without the interpreter lock."""
+    import threading
+    import time
+
+    import acsr_helpers as ah
+    mask = torch.ones(64, 64, dtype=torch.uint8, device="cuda").tril()
+    ah.create_acsr(mask, 16, 0)
+    took = []
+
+    def metadata():
+        t0 = time.monotonic()
+        ah.create_acsr(mask, 16, 0)
+        took.append(time.monotonic() - t0)
+    torch.cuda._sleep(600_000_000)              # SM clocks, some 0.3 s
+    thread = threading.Thread(target=metadata)
+    thread.start()
+    longest, last = 0.0, time.monotonic()
+    while thread.is_alive():
+        time.sleep(0.001)
+        now = time.monotonic()
+        longest, last = max(longest, now - last), now
+    thread.join()
+    assert took[0] > 0.15 and longest < 0.1, (took, longest)

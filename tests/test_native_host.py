@@ -2,8 +2,11 @@
 import subprocess
 import sys
 import textwrap
+import threading
+import time
 
 import pytest
+import torch
 
 from conftest import ROOT, SPLAT_DIR
 
@@ -36,3 +39,73 @@ def test_operands_without_data_end_no_process(call):
         print("alive")
         """)
     assert r.returncode == 0 and "alive" in r.stdout, (r.returncode, r.stderr[-2000:])
+
+
+class _Stream:
+    cuda_stream = 0
+
+    def synchronize(self):
+        time.sleep(0.05)
+
+
+def _on_a_machine_without_gpu(monkeypatch):
+    """torch's device calls replaced by ones that work here; synchronising gives the other threads a turn."""
+    import contextlib
+    zeros = torch.zeros
+    monkeypatch.setattr(torch, "zeros", lambda *a, device=None, **k: zeros(*a, **k))
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: _Stream())
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda t: t.clone())
+
+
+def _from_threads(f, count=4):
+    results, failures = [], []
+
+    def go():
+        try:
+            results.append(f())
+        except BaseException as e:
+            failures.append(e)
+    threads = [threading.Thread(target=go) for _ in range(count)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
+    return results
+
+
+def test_mask_scratch_is_set_up_once(monkeypatch):
+    """First calls from several threads: one registers the scratch, the others wait for it."""
+    import splat_native as n
+    _on_a_machine_without_gpu(monkeypatch)
+    registered = []
+
+    class Host:
+        set_mask_work = staticmethod(lambda *a: registered.append(a))
+        acsr_from_mask = staticmethod(lambda m, h: registered[0])
+    monkeypatch.setattr(n, "_host", Host)
+    monkeypatch.setattr(n, "_MASK_WORK", {})
+
+    class Mask:
+        device = torch.device("cuda", 0)
+    got = _from_threads(lambda: n.acsr_from_mask(Mask, 16))
+    assert len(registered) == 1 and got == [registered[0]] * 4
+
+
+def test_status_word_is_set_up_once(monkeypatch):
+    import splat_native as n
+    _on_a_machine_without_gpu(monkeypatch)
+    mirrors = []
+
+    class Host:
+        set_status = staticmethod(lambda *a: None)
+
+    class Lib:
+        splat_set_status_mirror = staticmethod(lambda *a: mirrors.append(a) or 0)
+    monkeypatch.setattr(n, "_host", Host)
+    monkeypatch.setattr(n, "_lib", Lib)
+    monkeypatch.setattr(n, "_STATUS_WORDS", {})
+    monkeypatch.setattr(n, "_STATUS_MIRRORS", {})
+    words = _from_threads(lambda: n.status_word(torch.device("cuda", 0)))
+    assert len(mirrors) == 1 and all(w is words[0] for w in words)

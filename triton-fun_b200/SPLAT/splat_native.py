@@ -9,6 +9,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import os
+import threading
 
 import torch
 
@@ -173,6 +174,7 @@ def acsr_from_row_summary(rows_i32: torch.Tensor, n_cols: int, block_height: int
     return (*vec, int(td.item()), spans[0], spans[1])
 
 
+_SET_UP = threading.Lock()      # what a device gets once: kernels and the native path keep the addresses
 _MASK_SLOTS = 16
 _MASK_WORK: dict = {}
 
@@ -181,13 +183,15 @@ def acsr_from_mask(mask_u8: torch.Tensor, block_height: int):
     """acsr_from_row_summary(mask_row_summary(mask)) in one kernel, or None where that does not apply (block
     heights outside 4 .. 64, no unit column stride, another current device)."""
     dev = mask_u8.device
-    if dev.index not in _MASK_WORK:        # scratch of the calls in progress: 16 slots, device and page-locked host
-        with torch.cuda.device(dev):
-            work = torch.zeros(2 * _MASK_SLOTS, dtype=torch.int32, device=dev)
-            torch.cuda.current_stream(dev).synchronize()
-            host = torch.zeros(_MASK_SLOTS, dtype=torch.int32).pin_memory()
-        _host.set_mask_work(dev.index, _MASK_SLOTS, work.data_ptr(), host.data_ptr())
-        _MASK_WORK[dev.index] = (work, host)
+    if dev.index not in _MASK_WORK:
+        with _SET_UP:
+            if dev.index not in _MASK_WORK:        # scratch of the calls in progress: 16 slots, device and page-locked host
+                with torch.cuda.device(dev):
+                    work = torch.zeros(2 * _MASK_SLOTS, dtype=torch.int32, device=dev)
+                    torch.cuda.current_stream(dev).synchronize()
+                    host = torch.zeros(_MASK_SLOTS, dtype=torch.int32).pin_memory()
+                _host.set_mask_work(dev.index, _MASK_SLOTS, work.data_ptr(), host.data_ptr())
+                _MASK_WORK[dev.index] = (work, host)
     return _host.acsr_from_mask(mask_u8, block_height)
 
 
@@ -271,7 +275,12 @@ def status_word(dev: torch.device) -> torch.Tensor:
     can look at it without synchronising or copying anything on the normal path."""
     key = (dev.type, dev.index)
     t = _STATUS_WORDS.get(key)
-    if t is None:
+    if t is not None:
+        return t
+    with _SET_UP:
+        t = _STATUS_WORDS.get(key)
+        if t is not None:
+            return t
         with torch.cuda.device(dev):
             t = torch.zeros(1, dtype=torch.int32, device=dev)
             torch.cuda.current_stream(dev).synchronize()

@@ -24,6 +24,7 @@
 #include <chrono>
 #include <cstdint>
 #include <cstdlib>
+#include <exception>
 #include <mutex>
 
 namespace {
@@ -477,16 +478,22 @@ PyObject* acsr_from_mask(PyObject*, PyObject* const* a, Py_ssize_t n) {
                         p[5], p[6], g_mask[dev].work + 2 * slot, const_cast<int32_t*>(word), stream.stream());
         if (rc == 0) {
             // The count reaches the host some microseconds before a stream synchronisation would return; work
-            // queued before this call, or an error, is left to the synchronisation.
+            // queued before this call, or an error, is left to the synchronisation.  Other threads run meanwhile.
+            std::exception_ptr failed;
             Py_BEGIN_ALLOW_THREADS
             const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(2);
             while ((trailing = *word) < 0)
                 if (std::chrono::steady_clock::now() > until) break;
-            Py_END_ALLOW_THREADS
             if (trailing < 0) {
-                c10::cuda::stream_synchronize(stream.stream());
-                trailing = *word;
+                try {
+                    c10::cuda::stream_synchronize(stream.stream());
+                    trailing = *word;
+                } catch (...) {
+                    failed = std::current_exception();
+                }
             }
+            Py_END_ALLOW_THREADS
+            if (failed) std::rethrow_exception(failed);
         }
     } catch (const std::exception& e) {
         if (rc == 0) {                  // launched, and the device reports an error: the slot stays taken
