@@ -56,13 +56,36 @@ def test_contiguous_kt_that_is_copied(d, L):
         kt = k.cuda().transpose(2, 3).contiguous()
         attn = r_attention.RegularAttention(2, L, 3, d, ah.PatternMask(kind, L, p0, p1), 16, 16, 0, torch.bfloat16,
                                             scale=d ** -0.5)
-        out = attn([q.cuda(), kt, v.cuda()])
-        n.classify(acsr[2], acsr[3], acsr[4])
+        out = attn([q.cuda(), kt, v.cuda()]).clone()
+        # (the kernels on the CUDA cores sum in another order: the same bits mean the same kernel)
+        assert torch.equal(out, attn([q.cuda(), k.cuda().transpose(2, 3), v.cuda()])), "not the tensor-core kernel"
         assert_close(out, at.attention_acsr(q, k.transpose(2, 3), v, meta, meta["trailing_dim"], d ** -0.5), torch.bfloat16,
                      f"fused {(kind, L, p0, p1)} d={d}")
         s = torch.full((2, 3, L, acsr[5]), float("nan"), dtype=torch.bfloat16, device="cuda")
-        n.sddmm(q.cuda(), kt, s, acsr[2], acsr[3], acsr[4], acsr[5])
+        n.sddmm(q.cuda(), kt, s, acsr[2], acsr[3], acsr[4], acsr[5])        # the first call on these metadata
+        for other in (kt, k.cuda().transpose(2, 3)):
+            again = torch.full_like(s, float("nan"))
+            n.sddmm(q.cuda(), other, again, acsr[2], acsr[3], acsr[4], acsr[5])
+            assert torch.equal(s, again), f"the first call takes another kernel {(kind, L, p0, p1)} d={d}"
         assert_close(s, at.sddmm_acsr(q, k.transpose(2, 3), meta, acsr[5]), torch.bfloat16, f"sddmm {(kind, L, p0, p1)} d={d}")
+
+
+def test_contiguous_kt_in_the_python_path(monkeypatch):
+    """Calls that the native path leaves to Python (debug mode here) take the kernels that they take without it."""
+    import acsr_helpers as ah
+    import r_attention
+    import splat_native as n
+    L, H, d = 301, 2, 64
+    attn = r_attention.RegularAttention(1, L, H, d, ah.create_strided_mask(L, 7), 16, 16, 0, torch.float16, scale=0.125)
+    q, k, v = (torch.randn(1, H, L, d, device="cuda").half() for _ in range(3))
+    x = [q, k.transpose(2, 3).contiguous(), v]
+    expected = attn(x).clone()
+    monkeypatch.setenv("SPLAT_B200_DEBUG", "1")
+    try:
+        out = attn(x).clone()
+    finally:
+        n.check_indices(0, False)
+    assert torch.equal(out, expected)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

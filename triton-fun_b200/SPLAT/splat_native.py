@@ -406,6 +406,13 @@ def _band_candidate(x: torch.Tensor, path: int) -> bool:
     return path != PATH_GENERIC and x.dtype in (torch.float16, torch.bfloat16) and x.numel() > 0
 
 
+def _rows_of_k(kt, plan, n_rows: int):
+    """What the native path does with a 16-bit K^T that the tensor-core kernels cannot fetch: the row-major copy to
+    work with, or None (not needed, no band pattern, no memory)."""
+    with _on(kt.device):
+        return _host.rows_of_k(kt, tuple(plan), n_rows)
+
+
 def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = PATH_AUTO) -> None:
     if _host.sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path):
         return
@@ -424,7 +431,11 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
     k_layout_ok = ksb == n_cols * d and ((ksk == 1 and ksc == d) or (ksc == 1 and ksk == n_cols))
     if _band_candidate(x, path) and k_layout_ok:
         _raise_if_gave_up(dev)
-        plan_arr = (ctypes.c_int32 * 8)(*classify(sTod_lin, sTod_tr, nnzs))
+        plan = classify(sTod_lin, sTod_tr, nnzs)
+        plan_arr = (ctypes.c_int32 * 8)(*plan)
+        rows = _rows_of_k(y, plan, L) if path == PATH_AUTO else None
+        if rows is not None:
+            y, ksb, ksk, ksc = rows, n_cols * d, 1, d
         with _on(dev):
             rc = _lib.splat_sddmm_band_table(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
                                        _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
@@ -549,6 +560,9 @@ def attention_fused(q, kt, v, output, sTod_lin, sTod_tr, nnzs, scale: float = 1.
         plan_arr = (ctypes.c_int32 * 8)(*plan)
     if tensor_core:
         _raise_if_gave_up(dev)
+        rows = _rows_of_k(kt, plan, L) if path == PATH_AUTO else None
+        if rows is not None:
+            kt, ksb, ksk, ksc = rows, n_cols * d, 1, d
     sw = status_word(dev)
     ran = ctypes.c_int32(0)
     _debug_before(dev)

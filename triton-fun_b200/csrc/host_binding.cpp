@@ -387,6 +387,20 @@ PyObject* softmax(PyObject* const* a, Py_ssize_t n) {
     return yes_or_none(rc == 0);
 }
 
+// rows_of_k(K^T (B, H, d, n), plan, query rows) -> the row-major copy (B H, n, d) that the calls above work with where they
+// need one, or None: for the launchers' Python path.  K^T's device is the current one.
+PyObject* rows_of_k(PyObject* const* a, Py_ssize_t n) {
+    long L;
+    int32_t plan[8];
+    int64_t ksb;
+    const at::Tensor* kt = n == 3 ? tensor(a[0]) : nullptr;
+    if (!kt || kt->dim() != 4 || !kt->is_cuda() || kt->element_size() != 2 || !read_plan(a[1], plan) || !as_long(a[2], &L) ||
+        !flat_bh(*kt, &ksb))
+        return yes_or_none(false);
+    at::Tensor rows = rows_of_k(*kt, ksb, plan, L, kt->size(2), c10::cuda::getCurrentCUDAStream(kt->get_device()).stream());
+    return rows.defined() ? THPVariable_Wrap(rows) : yes_or_none(false);
+}
+
 // bind(fused, sddmm_band, spmm_band, sddmm_tile, spmm_tile, softmax, mask, transpose, sddmm, spmm, warn): addresses of the C ABI entry points
 // and the function that warns of 16-bit operands on the CUDA-core kernels
 PyObject* bind(PyObject*, PyObject* args) {
@@ -543,6 +557,7 @@ PyMethodDef methods[] = {
     {"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<spmm>)), METH_FASTCALL, nullptr},
     {"set_mask_work", set_mask_work, METH_VARARGS, nullptr},
     {"acsr_from_mask", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(acsr_from_mask)), METH_FASTCALL, nullptr},
+    {"rows_of_k", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<rows_of_k>)), METH_FASTCALL, nullptr},
     {"record_pinned", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(record_pinned)), METH_FASTCALL, nullptr},
     {"softmax", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<softmax>)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
