@@ -68,3 +68,41 @@ def test_operands_without_data():
             attn([f, f.transpose(2, 3), f])
     with pytest.raises(Exception):
         attn([x.to_sparse(), x.transpose(2, 3), x])
+
+
+def test_first_fp32_launchers_under_capture():
+    """The fp32 launchers and the softmax of any type need nothing from the device but their operands: a process may
+    capture its very first calls."""
+    r = run_python("""
+        import acsr_helpers as ah, splat_native as n
+        from conftest import assert_close
+        from oracle import acsr_oracle as ao, attention_oracle as at
+        L, H, d = 300, 2, 64
+        acsr = ah.create_acsr(ah.create_causal_windowed_mask(L, 40), 16, 0)
+        torch.manual_seed(1)
+        q, k, v = (torch.randn(1, H, L, d) for _ in range(3))
+        qd, kt, vd = q.cuda(), k.cuda().transpose(2, 3), v.cuda()
+        s = torch.empty(1, H, L, acsr[5], device="cuda")
+        p, o = torch.empty_like(s), torch.empty_like(qd)
+        x16 = torch.randn(1, H, L, acsr[5], dtype=torch.bfloat16, device="cuda")
+        y16 = torch.empty_like(x16)
+        torch.cuda.synchronize()
+        def calls():
+            n.softmax(x16, y16, acsr[4], acsr[5])
+            n.sddmm(qd, kt, s, acsr[2], acsr[3], acsr[4], acsr[5])
+            n.softmax(s, p, acsr[4], acsr[5], 0.125)
+            n.spmm(p, vd, o, acsr[2], acsr[3], acsr[4], acsr[5])
+        meta = ao.metadata_from_pattern(ao.PATTERN_CAUSAL_WINDOWED, L, 40, 0, 16)
+        for attempt in ("first calls", "known metadata"):
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                calls()
+            o.fill_(float("nan")); y16.fill_(float("nan"))
+            g.replay()
+            torch.cuda.synchronize()
+            assert_close(o, at.attention_acsr(q, k.transpose(2, 3), v, meta, acsr[5], 0.125), torch.float32, attempt)
+            assert_close(y16, at.softmax_acsr(x16.cpu(), meta), torch.bfloat16, attempt)
+            calls()
+            torch.cuda.synchronize()
+        """)
+    assert r.returncode == 0, r.stderr[-2000:]

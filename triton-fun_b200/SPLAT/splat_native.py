@@ -222,16 +222,26 @@ def attention_host(q, k, v, out, stage: dict, sTod_lin, sTod_tr, nnzs, scale: fl
         check_status_word(dev)
 
 
+def _plan_key(sTod_lin, sTod_tr, nnzs) -> tuple:
+    return (id(sTod_lin), id(sTod_tr), sTod_lin._version, sTod_tr._version, nnzs._version, nnzs.numel())
+
+
+def _known_plan(sTod_lin, sTod_tr, nnzs):
+    """What classify() remembers of these metadata, or None if it has not seen them as they are."""
+    hit = getattr(nnzs, "_splat_plan", None)
+    return hit if hit is not None and hit[0] == _plan_key(sTod_lin, sTod_tr, nnzs) else None
+
+
 def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) -> tuple:
     """Host copy of the 8 plan ints of ``splat_acsr_classify``.  The result, with the band table of a band
     pattern (``splat_band_table``), is remembered ON the ``nnzs`` tensor object (with the identities and versions of all three tensors), so it lives
     exactly as long as that metadata and is recomputed if any of them is modified in place."""
-    key = (id(sTod_lin), id(sTod_tr), sTod_lin._version, sTod_tr._version, nnzs._version,
-           nnzs.numel())
-    hit = getattr(nnzs, "_splat_plan", None)
-    if hit is not None and hit[0] == key:
+    hit = _known_plan(sTod_lin, sTod_tr, nnzs)
+    if hit is not None:
         return hit[1]
+    key = _plan_key(sTod_lin, sTod_tr, nnzs)
     dev = nnzs.device
+    status_word(dev)        # (the launches that follow may be captured, and setting it up synchronises)
     n = nnzs.numel()
     plan = torch.empty(8, dtype=torch.int32, device=dev)
     with _on(dev):
@@ -256,9 +266,8 @@ def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) 
 def _band_table(sTod_lin, sTod_tr, nnzs):
     """Address of the band table remembered by classify(), or None if the metadata has changed since -- or for
     a captured launch, which has to work with the metadata as they are at the replay."""
-    hit = getattr(nnzs, "_splat_plan", None)
-    if hit is None or hit[4] is None or _capturing(nnzs.device) or hit[0] != (id(sTod_lin), id(sTod_tr), sTod_lin._version, sTod_tr._version,
-                                                   nnzs._version, nnzs.numel()):
+    hit = _known_plan(sTod_lin, sTod_tr, nnzs)
+    if hit is None or hit[4] is None or _capturing(nnzs.device):
         return None
     if hit[5] != _stream(nnzs.device):      # the table is nobody's tensor but ours: its use elsewhere is ours to record
         hit[4].record_stream(torch.cuda.current_stream(nnzs.device))
@@ -406,6 +415,20 @@ def _band_candidate(x: torch.Tensor, path: int) -> bool:
     return path != PATH_GENERIC and x.dtype in (torch.float16, torch.bfloat16) and x.numel() > 0
 
 
+def _native_from_now_on(dev: torch.device) -> None:
+    """The native path takes ordinary operands once the status word exists.  Setting it up synchronises, which a
+    capture does not allow; the kernels without bounded waits need none."""
+    if not _capturing(dev):
+        status_word(dev)
+
+
+def _plan_unless_captured(sTod_lin, sTod_tr, nnzs):
+    """classify(), or None where a capture forbids to look at metadata that are new."""
+    if _known_plan(sTod_lin, sTod_tr, nnzs) is None and _capturing(nnzs.device):
+        return None
+    return classify(sTod_lin, sTod_tr, nnzs)
+
+
 def _rows_of_k(kt, plan, n_rows: int):
     """What the native path does with a 16-bit K^T that the tensor-core kernels cannot fetch: the row-major copy to
     work with, or None (not needed, no band pattern, no memory)."""
@@ -417,7 +440,7 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
     if _host.sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path):
         return
     dev = x.device
-    status_word(dev)       # (from here on the native path takes ordinary operands)
+    _native_from_now_on(dev)
     _contig(x, "x"); _contig(output, "output")
     B, H, L, d = x.shape
     bh, ksb, ksk, ksc = _flat_bh(y, "y")          # y is (B, H, d, n): dim 2 = k, dim 3 = column
@@ -452,8 +475,11 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
     if x.dtype != torch.float32 and x.numel() > 0:
         _warn_cuda_core_16bit("sddmm")
     debug = _debug_before(dev)
+    plan = None
     if x.dtype == torch.float32 and path == PATH_AUTO and x.numel() > 0:
-        plan_arr = (ctypes.c_int32 * 8)(*classify(sTod_lin, sTod_tr, nnzs))
+        plan = _plan_unless_captured(sTod_lin, sTod_tr, nnzs)
+    if plan is not None:
+        plan_arr = (ctypes.c_int32 * 8)(*plan)
         with _on(dev):
             rc = _lib.splat_sddmm_tile(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
                                        _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
@@ -475,7 +501,7 @@ def softmax(x, output, nnzs, trailing_dim: int, scale: float = 1.0) -> None:
     if _host.softmax(x, output, nnzs, trailing_dim, scale):
         return
     dev = x.device
-    status_word(dev)
+    _native_from_now_on(dev)
     _contig(x, "x"); _contig(output, "output")
     B, H, L, T = x.shape
     if T != trailing_dim or output.shape != x.shape or output.dtype != x.dtype:
@@ -490,7 +516,7 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
     if _host.spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim, path):
         return
     dev = x.device
-    status_word(dev)
+    _native_from_now_on(dev)
     _contig(x, "x"); _contig(y, "y"); _contig(output, "output")
     B, H, L, T = x.shape
     n_cols, d = y.shape[2], y.shape[3]
@@ -516,8 +542,11 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
     if x.dtype != torch.float32 and x.numel() > 0:
         _warn_cuda_core_16bit("spmm")
     debug = _debug_before(dev)
+    plan = None
     if x.dtype == torch.float32 and path == PATH_AUTO and x.numel() > 0:
-        plan_arr = (ctypes.c_int32 * 8)(*classify(sTod_lin, sTod_tr, nnzs))
+        plan = _plan_unless_captured(sTod_lin, sTod_tr, nnzs)
+    if plan is not None:
+        plan_arr = (ctypes.c_int32 * 8)(*plan)
         with _on(dev):
             rc = _lib.splat_spmm_tile(x.data_ptr(), y.data_ptr(), output.data_ptr(),
                                       _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
