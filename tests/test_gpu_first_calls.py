@@ -106,3 +106,33 @@ def test_first_fp32_launchers_under_capture():
             torch.cuda.synchronize()
         """)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("shape", ["flat", "one batch", "slices"])
+def test_forward_host_takes_any_split_of_batch_and_heads(shape):
+    """Operands that view as (1, batch * heads, L, d), whatever their own leading dimensions; others are refused."""
+    import acsr_helpers as ah
+    import r_attention
+    B, H, L, d = 2, 3, 256, 64
+    attn = r_attention.RegularAttention(B, L, H, d, ah.create_causal_windowed_mask(L, 30), 16, 16, 0, torch.bfloat16)
+    torch.manual_seed(5)
+    q, k, v = (torch.randn(B, H, L, d).to(torch.bfloat16) for _ in range(3))
+    out = torch.empty_like(q).pin_memory()
+    attn.forward_host(q.pin_memory(), k.pin_memory(), v.pin_memory(), out)
+    torch.cuda.synchronize()
+    if shape == "slices":           # rows of a wider array, also for the result
+        wide = [torch.zeros(B, H, L, 2 * d, dtype=torch.bfloat16).pin_memory() for _ in range(4)]
+        operands = [t[..., :d] for t in wide]
+        for t, x in zip(operands, (q, k, v)):
+            t.copy_(x)
+        other = operands[3]
+    else:
+        other = torch.empty((B * H, L, d) if shape == "flat" else (1, B * H, L, d), dtype=torch.bfloat16).pin_memory()
+        operands = [q.pin_memory(), k.view(other.shape).pin_memory(), v.view(other.shape).pin_memory(), other]
+    result = attn.forward_host(*operands)
+    torch.cuda.synchronize()
+    assert result is other and torch.equal(other.reshape(out.shape), out)
+    with pytest.raises(RuntimeError):
+        attn.forward_host(q, k.transpose(1, 2), v, out)
+    with pytest.raises(RuntimeError):
+        attn.forward_host(q, k[:, :, 1:], v, out)

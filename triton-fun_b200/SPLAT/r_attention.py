@@ -124,25 +124,23 @@ class RegularAttention(nn.Module):
 
     def forward_host(self, q_host: torch.Tensor, k_host: torch.Tensor, v_host: torch.Tensor,
                      out_host: torch.Tensor, chunk_heads: int = 32) -> torch.Tensor:
-        """Attention over HOST-resident operands (pinned (B,H,L,d) tensors; k is row-major, not
-        transposed).  The flat batch*head axis is streamed through the device in chunks of
-        ``chunk_heads``: the host->device copy of chunk i+1 and the device->host copy of chunk
+        """Attention over HOST-resident operands (pinned (B,H,L,d) tensors, k, v and out_host of any shape that
+        views as (B*H,L,d); k is row-major, not transposed).  The flat batch*head axis is streamed through the
+        device in chunks of host_chunk() heads, ``chunk_heads`` at most: the host->device copy of chunk i+1 and the device->host copy of chunk
         i-1 overlap the fused kernel of chunk i (three streams, two staging buffers, allocated on
         first use).  Work is enqueued asynchronously; the caller's current stream waits for the last
         device->host copy, so synchronising that stream makes ``out_host`` valid.  Page-locked operands may
         be dropped right away (torch's allocator keeps their blocks until they have been copied).  Not in the reference, whose operands are always device tensors."""
         B, H, L, d = q_host.shape
         bh = B * H
+        q, k, v, out = hosts = [t.view(1, bh, L, d) for t in (q_host, k_host, v_host, out_host)]
         if bh == 0 or L == 0:
             return out_host
-        hosts = (q_host, k_host, v_host, out_host)
-        if any(tuple(t.shape) != (B, H, L, d) for t in hosts):
-            raise ValueError("forward_host: operands must have one shape (B, H, L, d)")
-        plain = all(t.dtype == self.out_dtype and t.device.type == "cpu" for t in hosts) and out_host.is_contiguous()
+        plain = all(t.dtype == self.out_dtype and t.device.type == "cpu" for t in hosts) and out.is_contiguous()
         if not plain:
-            q_host, k_host, v_host = (t.to("cpu", self.out_dtype) for t in hosts[:3])
-        q_host, k_host, v_host = (t.contiguous() for t in (q_host, k_host, v_host))
-        dst = out_host if plain else torch.empty((B, H, L, d), dtype=self.out_dtype).pin_memory()
+            q, k, v = (t.to("cpu", self.out_dtype) for t in (q, k, v))
+        q, k, v = (t.contiguous() for t in (q, k, v))
+        dst = out if plain else torch.empty((1, bh, L, d), dtype=self.out_dtype).pin_memory()
         chunk = max(1, min(chunk_heads, bh, host_chunk(bh, L * d * self.out_dtype.itemsize)))
         st = getattr(self, "_host_stage", None)
         if st is None or st["chunk"] != chunk or st["shape"] != (L, d):
@@ -155,11 +153,11 @@ class RegularAttention(nn.Module):
                   "events": (ctypes.c_void_p * 7)(*(e.cuda_event for e in events)),
                   "s_in": torch.cuda.Stream(self.device), "s_out": torch.cuda.Stream(self.device)}
             self._host_stage = st
-        _n.attention_host(q_host, k_host, v_host, dst, st, self.sTod_linear_transformations, self.sTod_translations,
+        _n.attention_host(q, k, v, dst, st, self.sTod_linear_transformations, self.sTod_translations,
                           self.nnzs, self.scale, self.path, self.plan)
         if not plain:
             torch.cuda.current_stream(self.device).synchronize()
-            out_host.copy_(dst)
+            out.copy_(dst)
         return out_host
 
     def check_status(self) -> None:
