@@ -136,3 +136,24 @@ def test_forward_host_takes_any_split_of_batch_and_heads(shape):
         attn.forward_host(q, k.transpose(1, 2), v, out)
     with pytest.raises(RuntimeError):
         attn.forward_host(q, k[:, :, 1:], v, out)
+
+
+@pytest.mark.parametrize("call", ["attn([x, x.transpose(2, 3), x])", "n.spmm(s, x, o, *meta, T); n.spmm(s, x, o, *meta, T)",
+                                  "n.sddmm(x, x.transpose(2, 3), s, *meta, T); n.sddmm(x, x.transpose(2, 3), s, *meta, T)"])
+def test_cuda_core_warning_as_an_error(call):
+    """A caller who turns warnings into errors gets one for 16-bit operands on the CUDA cores."""
+    r = run_python(f"""
+        import acsr_helpers as ah, r_attention, splat_native as n, warnings
+        mask = torch.zeros(64, 64, dtype=torch.uint8, device="cuda")
+        mask[::2, ::2] = 1; mask[1::2, ::3] = 1                # rows of two strides
+        attn = r_attention.RegularAttention(1, 64, 1, 64, mask, 16, 16, 0, torch.float16)
+        T, meta = attn.acsr_trailing_dim, (attn.sTod_linear_transformations, attn.sTod_translations, attn.nnzs)
+        x = torch.randn(1, 1, 64, 64, dtype=torch.float16, device="cuda")
+        s, o = torch.zeros(1, 1, 64, T, dtype=torch.float16, device="cuda"), torch.empty_like(x)
+        warnings.simplefilter("error")
+        try:
+            {call}
+        except RuntimeWarning:
+            print("raised")
+        """)
+    assert r.returncode == 0 and "raised" in r.stdout, (r.stdout, r.stderr[-2000:])

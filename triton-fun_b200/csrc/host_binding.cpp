@@ -74,14 +74,16 @@ struct Status {
 
 PyObject* g_warn = nullptr;   // splat_native's one-time warning, until it has been given
 
-void warn_once(const char* what) {     // 16-bit operands on the CUDA cores
+struct PythonError {};        // thrown while a Python exception is set
+
+void warn_once(const char* what) {     // 16-bit operands on the CUDA cores; a warning may be an error to the caller
     if (g_warn == nullptr) return;
     PyObject* cb = g_warn;
     g_warn = nullptr;
     PyObject* r = PyObject_CallFunction(cb, "s", what);
     Py_DECREF(cb);
-    if (r == nullptr) PyErr_Clear();
-    else Py_DECREF(r);
+    if (r == nullptr) throw PythonError{};
+    Py_DECREF(r);
 }
 // return codes of the tile and band kernels that mean "use the row kernels": misaligned, unsupported shape, no tensor map
 bool not_applicable(int32_t rc) { return rc == -3 || rc == -6 || rc == -7; }
@@ -253,11 +255,13 @@ PyObject* yes_or_none(bool yes) {
 }
 
 // Torch throws for tensors it has no data, strides or version of (fake, functional, sparse ones); nothing of that may
-// leave through CPython's frames.  Everything that throws comes before a call's launch, so Python can start over.
+// leave through CPython's frames.  Everything of torch that throws comes before a call's launch, so Python can start over.
 template <PyObject* (*F)(PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject*, PyObject* const* args, Py_ssize_t n) {
     try {
         return F(args, n);
+    } catch (const PythonError&) {
+        return nullptr;
     } catch (...) {
         return yes_or_none(false);
     }
