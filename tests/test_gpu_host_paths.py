@@ -131,3 +131,29 @@ def test_other_threads_run_while_metadata_wait():
         longest, last = max(longest, now - last), now
     thread.join()
     assert took[0] > 0.15 and longest < 0.1, (took, longest)
+
+
+@pytest.mark.parametrize("L", [300, 512])
+def test_metadata_of_more_rows_than_the_operands(L):
+    """Metadata vectors padded with empty rows: the launchers take vectors of at least L elements."""
+    import acsr_helpers as ah
+    import splat_native as n
+    H, d, dtype = 2, 64, torch.bfloat16
+    acsr = ah.create_acsr(ah.create_causal_windowed_mask(L, 40), 16, 0)
+    pad = torch.zeros(200, device="cuda")
+    lin, tr, nnzs = torch.cat([acsr[2], pad + 1]), torch.cat([acsr[3], pad]), torch.cat([acsr[4], pad])
+    meta = ao.metadata_from_pattern(ao.PATTERN_CAUSAL_WINDOWED, L, 40, 0, 16)
+    torch.manual_seed(8)
+    q, k, v = (torch.randn(1, H, L, d).to(dtype) for _ in range(3))
+    qd, kt, vd = q.cuda(), k.cuda().transpose(2, 3), v.cuda()
+    p = torch.rand(1, H, L, acsr[5]).to(dtype)
+    s, o, fused = torch.empty_like(p, device="cuda"), torch.empty_like(qd), torch.empty_like(qd)
+    for _ in range(2):                  # through Python, through the native path
+        for t in (s, o, fused):
+            t.fill_(float("nan"))
+        n.attention_fused(qd, kt, vd, fused, lin, tr, nnzs, 0.125)
+        n.sddmm(qd, kt, s, lin, tr, nnzs, acsr[5])
+        n.spmm(p.cuda(), vd, o, lin, tr, nnzs, acsr[5])
+        assert_close(fused, at.attention_acsr(q, k.transpose(2, 3), v, meta, acsr[5], 0.125), dtype, "fused")
+        assert_close(s, at.sddmm_acsr(q, k.transpose(2, 3), meta, acsr[5]), dtype, "sddmm")
+        assert_close(o, at.spmm_acsr(p, v, meta), dtype, "spmm")

@@ -210,7 +210,7 @@ def attention_host(q, k, v, out, stage: dict, sTod_lin, sTod_tr, nnzs, scale: fl
             q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), stage["staging"], stage["chunk"],
             _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"), _f32_vec(nnzs, L, "nnzs"), B * H, L, d,
             float(scale), dtype_code(q.dtype), int(path), ctypes.cast(plan_arr, _vp) if path != PATH_GENERIC else None,
-            _band_table(sTod_lin, sTod_tr, nnzs), sw.data_ptr(), ctypes.byref(ran), stage["s_in"].cuda_stream, _stream(dev),
+            _band_table(sTod_lin, sTod_tr, nnzs, L), sw.data_ptr(), ctypes.byref(ran), stage["s_in"].cuda_stream, _stream(dev),
             stage["s_out"].cuda_stream, stage["events"])
         # the caller may drop its tensors now: their page-locked blocks are reused only when the copies are done
         for t, s in ((q, stage["s_in"]), (k, stage["s_in"]), (v, stage["s_in"]), (out, stage["s_out"])):
@@ -263,11 +263,11 @@ def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) 
     return host
 
 
-def _band_table(sTod_lin, sTod_tr, nnzs):
-    """Address of the band table remembered by classify(), or None if the metadata has changed since -- or for
-    a captured launch, which has to work with the metadata as they are at the replay."""
+def _band_table(sTod_lin, sTod_tr, nnzs, n_rows: int):
+    """Address of the band table remembered by classify(), or None if the metadata has changed since, has more rows
+    than the operands -- or for a captured launch, which has to work with the metadata as they are at the replay."""
     hit = _known_plan(sTod_lin, sTod_tr, nnzs)
-    if hit is None or hit[4] is None or _capturing(nnzs.device):
+    if hit is None or hit[4] is None or nnzs.numel() != n_rows or _capturing(nnzs.device):
         return None
     if hit[5] != _stream(nnzs.device):      # the table is nobody's tensor but ours: its use elsewhere is ours to record
         hit[4].record_stream(torch.cuda.current_stream(nnzs.device))
@@ -464,7 +464,7 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
                                        _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
                                        _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, trailing_dim,
                                        dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p),
-                                       _band_table(sTod_lin, sTod_tr, nnzs), status_word(dev).data_ptr(), _stream(dev))
+                                       _band_table(sTod_lin, sTod_tr, nnzs, L), status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE or path == PATH_BAND:
             check(rc, "splat_sddmm_band")
             if os.environ.get("SPLAT_B200_DEBUG"):
@@ -531,7 +531,7 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
                                       _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
                                       _f32_vec(nnzs, L, "nnzs"), B * H, L, n_cols, d, T,
                                       dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p),
-                                      _band_table(sTod_lin, sTod_tr, nnzs), status_word(dev).data_ptr(), _stream(dev))
+                                      _band_table(sTod_lin, sTod_tr, nnzs, L), status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE or path == PATH_BAND:
             check(rc, "splat_spmm_band")
             if os.environ.get("SPLAT_B200_DEBUG"):
@@ -602,7 +602,7 @@ def attention_fused(q, kt, v, output, sTod_lin, sTod_tr, nnzs, scale: float = 1.
             _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
             _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, float(scale), dtype_code(q.dtype),
             int(path), ctypes.cast(plan_arr, _vp) if plan_arr is not None else None,
-            _band_table(sTod_lin, sTod_tr, nnzs), sw.data_ptr(), ctypes.byref(ran), _stream(dev)),
+            _band_table(sTod_lin, sTod_tr, nnzs, L), sw.data_ptr(), ctypes.byref(ran), _stream(dev)),
             "splat_attention_fused_table")
     if ran.value != PATH_BAND and q.dtype != torch.float32 and q.numel() > 0 and path == PATH_AUTO:
         _warn_cuda_core_16bit("attention")

@@ -234,6 +234,7 @@ bool fused(const at::Tensor* q, const at::Tensor* kt, const at::Tensor* v, const
     int32_t plan[8];
     const bool with_plan = path != kPathGeneric;
     if (with_plan && !read_plan(plan_obj, plan)) return false;
+    if (nnzs->numel() != L) table = nullptr;       // (made for as many rows as the metadata have)
     int32_t ran = 0;
     void* stream = c10::cuda::getCurrentCUDAStream(dev).stream();
     at::Tensor rows;
@@ -321,6 +322,7 @@ PyObject* sddmm(PyObject* const* a, Py_ssize_t n) {
     int32_t plan[8];
     const int32_t* table = nullptr;
     if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, &table)) return yes_or_none(false);
+    if (nnzs->numel() != L) table = nullptr;
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
     at::Tensor rows;
     if (dtype != 0) rows = rows_of_k(*y, ksb, plan, L, d, st);
@@ -360,6 +362,7 @@ PyObject* spmm(PyObject* const* a, Py_ssize_t n) {
     int32_t plan[8];
     const int32_t* table = nullptr;
     if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, &table)) return yes_or_none(false);
+    if (nnzs->numel() != L) table = nullptr;
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
     int32_t rc = dtype == 0 ? g_api.spmm_tile(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
                                                     n_cols, d, T, dtype, plan, st)
