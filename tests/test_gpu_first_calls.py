@@ -157,3 +157,60 @@ def test_cuda_core_warning_as_an_error(call):
             print("raised")
         """)
     assert r.returncode == 0 and "raised" in r.stdout, (r.stdout, r.stderr[-2000:])
+
+
+def test_only_calls_that_read_it_make_the_band_table():
+    import acsr_helpers as ah
+    import splat_native as n
+    L, d = 256, 64
+    for dtype in (torch.float32, torch.bfloat16):
+        acsr = ah.create_acsr(ah.create_causal_windowed_mask(L, 40), 16, 0)
+        q = torch.randn(1, 2, L, d, device="cuda").to(dtype)
+        s, o = torch.empty(1, 2, L, acsr[5], dtype=dtype, device="cuda"), torch.empty_like(q)
+        for _ in range(2):
+            n.sddmm(q, q.transpose(2, 3), s, acsr[2], acsr[3], acsr[4], acsr[5])
+            n.spmm(s, q, o, acsr[2], acsr[3], acsr[4], acsr[5])
+            n.attention_fused(q, q.transpose(2, 3), q, o, acsr[2], acsr[3], acsr[4])
+        table = acsr[4]._splat_plan[4]
+        assert (table is None) if dtype == torch.float32 else table.numel() == 2 * (L + 2)
+
+
+@pytest.mark.parametrize("call", ["module", "sddmm", "host"])
+def test_first_calls_on_two_streams(call):
+    """The band table is made on one stream, behind work that is queued there; a call on another one waits for it."""
+    import acsr_helpers as ah
+    import r_attention
+    import splat_native as n
+    L, H, d, dtype = 640, 2, 64, torch.bfloat16
+    one, other = torch.cuda.Stream(), torch.cuda.Stream()
+    q, k, v = (torch.randn(1, H, L, d, device="cuda").to(dtype) for _ in range(3))
+    hosts = [t.cpu().pin_memory() for t in (q, k, v)]
+
+    def make():
+        return r_attention.RegularAttention(1, L, H, d, ah.create_causal_windowed_mask(L, 200), 16, 16, 0, dtype, scale=0.125)
+
+    def run(attn):
+        if call == "module":
+            return attn([q, k.transpose(2, 3), v])
+        if call == "host":
+            return attn.forward_host(*hosts, torch.empty(1, H, L, d, dtype=dtype).pin_memory())
+        s = torch.full((1, H, L, attn.acsr_trailing_dim), float("nan"), dtype=dtype, device="cuda")
+        n.sddmm(q, k.transpose(2, 3), s, attn.sTod_linear_transformations, attn.sTod_translations, attn.nnzs, attn.acsr_trailing_dim)
+        return s
+
+    expected = run(make()).clone()
+    torch.cuda.synchronize()
+    attn = make()
+    meta = attn.sTod_linear_transformations, attn.sTod_translations, attn.nnzs
+    attn.nnzs._splat_plan = attn.nnzs._splat_plan[:4] + (None, 0, 0, None)         # as classify() leaves it
+    torch.cuda.synchronize()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(400_000_000)         # SM clocks, some 0.2 s
+        n.band_table(*meta, L)
+    with torch.cuda.stream(other):
+        first, second = run(attn).clone(), run(attn)
+    other.synchronize()
+    torch.cuda.synchronize()
+    if call != "host":                         # (the copy of a host result does not wait for it)
+        assert torch.equal(first, expected)
+    assert torch.equal(second, expected)

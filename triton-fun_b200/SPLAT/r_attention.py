@@ -60,6 +60,8 @@ class RegularAttention(nn.Module):
          self.span_loop_start, self.span_loop_end) = create_acsr(mask, BLOCK_SIZE_Y, self.device)
         self.plan = _n.classify(self.sTod_linear_transformations, self.sTod_translations, self.nnzs)
         _n.status_word(self.device)
+        if self.path != _n.PATH_GENERIC and out_dtype != torch.float32:
+            _n.band_table(self.sTod_linear_transformations, self.sTod_translations, self.nnzs, seq_length)
 
         self.BLOCK_SIZE_Y = BLOCK_SIZE_Y
         self.BLOCK_SIZE_X = BLOCK_SIZE_X

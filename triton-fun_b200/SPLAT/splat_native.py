@@ -202,6 +202,7 @@ def attention_host(q, k, v, out, stage: dict, sTod_lin, sTod_tr, nnzs, scale: fl
     if _band_candidate(q, path):
         _raise_if_gave_up(dev)
     sw = status_word(dev)
+    table = band_table(sTod_lin, sTod_tr, nnzs, L) if _band_candidate(q, path) else None
     ran = ctypes.c_int32(0)
     plan_arr = (ctypes.c_int32 * 8)(*plan)
     _debug_before(dev)
@@ -210,7 +211,7 @@ def attention_host(q, k, v, out, stage: dict, sTod_lin, sTod_tr, nnzs, scale: fl
             q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), stage["staging"], stage["chunk"],
             _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"), _f32_vec(nnzs, L, "nnzs"), B * H, L, d,
             float(scale), dtype_code(q.dtype), int(path), ctypes.cast(plan_arr, _vp) if path != PATH_GENERIC else None,
-            _band_table(sTod_lin, sTod_tr, nnzs, L), sw.data_ptr(), ctypes.byref(ran), stage["s_in"].cuda_stream, _stream(dev),
+            table, sw.data_ptr(), ctypes.byref(ran), stage["s_in"].cuda_stream, _stream(dev),
             stage["s_out"].cuda_stream, stage["events"])
         # the caller may drop its tensors now: their page-locked blocks are reused only when the copies are done
         for t, s in ((q, stage["s_in"]), (k, stage["s_in"]), (v, stage["s_in"]), (out, stage["s_out"])):
@@ -233,9 +234,9 @@ def _known_plan(sTod_lin, sTod_tr, nnzs):
 
 
 def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) -> tuple:
-    """Host copy of the 8 plan ints of ``splat_acsr_classify``.  The result, with the band table of a band
-    pattern (``splat_band_table``), is remembered ON the ``nnzs`` tensor object (with the identities and versions of all three tensors), so it lives
-    exactly as long as that metadata and is recomputed if any of them is modified in place."""
+    """Host copy of the 8 plan ints of ``splat_acsr_classify``.  The result is remembered ON the ``nnzs`` tensor
+    object (with the identities and versions of all three tensors), so it lives exactly as long as that
+    metadata and is recomputed if any of them is modified in place."""
     hit = _known_plan(sTod_lin, sTod_tr, nnzs)
     if hit is not None:
         return hit[1]
@@ -249,28 +250,37 @@ def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) 
                                        _f32_vec(nnzs, n, "nnzs"), n, plan.data_ptr(), _stream(dev)),
               "splat_acsr_classify")
     host = tuple(int(v) for v in plan.cpu().tolist())
-    table = None
-    stride = host[1] if host[7] > 0 else 1
-    if 0 < n <= 2**31 - 1 and (host[7] == 0 or host[1] == host[2]) and host[3] == 0 and host[5] <= n and stride <= 65535:
+    # keep the two companions alive with the cache entry so their ids cannot be reused
+    nnzs._splat_plan = (key, host, sTod_lin, sTod_tr, None, 0, 0, None)
+    return host
+
+
+def band_table(sTod_lin, sTod_tr, nnzs, n_rows: int):
+    """Address of the band table (``splat_band_table``) of classified metadata, which lives with their plan; made by
+    the first call that reads it, in the order of that call's stream.  None if the pattern has none, if the
+    metadata have changed since classify() or have more rows than the operands -- or for a captured launch,
+    which has to work with the metadata as they are at the replay."""
+    hit = _known_plan(sTod_lin, sTod_tr, nnzs)
+    dev = nnzs.device
+    if hit is None or hit[4] is False or nnzs.numel() != n_rows or _capturing(dev):
+        return None
+    stream = torch.cuda.current_stream(dev)
+    if hit[4] is None:
+        plan, n = hit[1], n_rows
+        stride = plan[1] if plan[7] > 0 else 1
+        if not (0 < n <= 2**31 - 1 and (plan[7] == 0 or plan[1] == plan[2]) and plan[3] == 0 and plan[5] <= n and stride <= 65535):
+            nnzs._splat_plan = hit[:4] + (False, 0, 0, None)
+            return None
         tiles = -(-(-(-n // stride)) // 128) * stride
         table = torch.empty(2 * (n + tiles), dtype=torch.int32, device=dev)
         with _on(dev):
             check(_lib.splat_band_table(sTod_lin.data_ptr(), sTod_tr.data_ptr(), nnzs.data_ptr(), n, stride,
-                                        table.data_ptr(), _stream(dev)), "splat_band_table")
-            torch.cuda.current_stream(dev).synchronize()      # any stream may use it
-    # keep the two companions alive with the cache entry so their ids cannot be reused
-    nnzs._splat_plan = (key, host, sTod_lin, sTod_tr, table, _stream(dev))
-    return host
-
-
-def _band_table(sTod_lin, sTod_tr, nnzs, n_rows: int):
-    """Address of the band table remembered by classify(), or None if the metadata has changed since, has more rows
-    than the operands -- or for a captured launch, which has to work with the metadata as they are at the replay."""
-    hit = _known_plan(sTod_lin, sTod_tr, nnzs)
-    if hit is None or hit[4] is None or nnzs.numel() != n_rows or _capturing(nnzs.device):
-        return None
-    if hit[5] != _stream(nnzs.device):      # the table is nobody's tensor but ours: its use elsewhere is ours to record
-        hit[4].record_stream(torch.cuda.current_stream(nnzs.device))
+                                        table.data_ptr(), stream.cuda_stream), "splat_band_table")
+            made = stream.record_event()
+        hit = nnzs._splat_plan = hit[:4] + (table, stream.cuda_stream, made.cuda_event, made)
+    if hit[5] != stream.cuda_stream:      # the table is nobody's tensor but ours: its order and its use elsewhere are ours to see to
+        stream.wait_event(hit[7])
+        hit[4].record_stream(stream)
     return hit[4].data_ptr()
 
 
@@ -464,7 +474,7 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
                                        _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
                                        _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, trailing_dim,
                                        dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p),
-                                       _band_table(sTod_lin, sTod_tr, nnzs, L), status_word(dev).data_ptr(), _stream(dev))
+                                       band_table(sTod_lin, sTod_tr, nnzs, L), status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE or path == PATH_BAND:
             check(rc, "splat_sddmm_band")
             if os.environ.get("SPLAT_B200_DEBUG"):
@@ -531,7 +541,7 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
                                       _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
                                       _f32_vec(nnzs, L, "nnzs"), B * H, L, n_cols, d, T,
                                       dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p),
-                                      _band_table(sTod_lin, sTod_tr, nnzs, L), status_word(dev).data_ptr(), _stream(dev))
+                                      band_table(sTod_lin, sTod_tr, nnzs, L), status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE or path == PATH_BAND:
             check(rc, "splat_spmm_band")
             if os.environ.get("SPLAT_B200_DEBUG"):
@@ -593,6 +603,7 @@ def attention_fused(q, kt, v, output, sTod_lin, sTod_tr, nnzs, scale: float = 1.
         if rows is not None:
             kt, ksb, ksk, ksc = rows, n_cols * d, 1, d
     sw = status_word(dev)
+    table = band_table(sTod_lin, sTod_tr, nnzs, L) if tensor_core else None
     ran = ctypes.c_int32(0)
     _debug_before(dev)
     with _on(dev):
@@ -602,7 +613,7 @@ def attention_fused(q, kt, v, output, sTod_lin, sTod_tr, nnzs, scale: float = 1.
             _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
             _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, float(scale), dtype_code(q.dtype),
             int(path), ctypes.cast(plan_arr, _vp) if plan_arr is not None else None,
-            _band_table(sTod_lin, sTod_tr, nnzs, L), sw.data_ptr(), ctypes.byref(ran), _stream(dev)),
+            table, sw.data_ptr(), ctypes.byref(ran), _stream(dev)),
             "splat_attention_fused_table")
     if ran.value != PATH_BAND and q.dtype != torch.float32 and q.numel() > 0 and path == PATH_AUTO:
         _warn_cuda_core_16bit("attention")

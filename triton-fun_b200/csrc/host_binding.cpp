@@ -144,9 +144,11 @@ inline bool same4(const at::Tensor& t, int64_t a, int64_t b, int64_t c, int64_t 
 }
 
 // plan remembered by splat_native.classify() on the nnzs tensor: ((id, id, version x 3, numel), plan, lin, tr,
-// band table or None, stream it was made on); false if the metadata is not what it was made from.  A captured launch gets
-// no table: a replay has to follow the metadata as they are then, and the table's memory goes with the Python objects.
-// The caller knows nothing of the table, so its use on another stream is recorded here.
+// band table, stream it was made on, event behind its making, owner of the event); false if the metadata is not what it
+// was made from.  With `table`, also its address -- null for a pattern without one -- and false if Python has yet to
+// make it.  A captured launch gets no table: a replay has to follow the metadata as they are then, and the table's
+// memory goes with the Python objects.  The caller knows nothing of the table, so on another stream than its own it
+// is waited for, and its use recorded, here.
 bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, const at::Tensor& lin, PyObject* tr_obj,
                  const at::Tensor& tr, int32_t (&plan)[8], const int32_t** table = nullptr) {
     PyObject* hit = PyObject_GetAttr(nnzs_obj, k_cached_plan);
@@ -154,7 +156,7 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
         PyErr_Clear();
         return false;
     }
-    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 6 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
+    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 8 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
               PyTuple_GET_ITEM(hit, 3) == tr_obj;
     if (ok) {
         PyObject* key = PyTuple_GET_ITEM(hit, 0);
@@ -166,17 +168,23 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
             ok = as_long(PyTuple_GET_ITEM(key, 2 + i), &v) && v == now[i];
         }
         ok = ok && read_plan(PyTuple_GET_ITEM(hit, 1), plan);
-        if (ok && table != nullptr) {
-            const at::Tensor* t = tensor(PyTuple_GET_ITEM(hit, 4));
-            const auto stream = c10::cuda::getCurrentCUDAStream(t != nullptr ? t->get_device() : -1);
-            // (the legacy stream is never captured: asking costs 0.3 us of a small call)
-            if (t != nullptr && (stream.stream() == nullptr || c10::cuda::currentStreamCaptureStatusMayInitCtx() ==
-                                                                   c10::cuda::CaptureStatus::None)) {
-                if (PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 5)) != stream.stream())
-                    c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
-                *table = static_cast<const int32_t*>(t->const_data_ptr());
+    }
+    if (ok && table != nullptr) {
+        *table = nullptr;
+        PyObject* made = PyTuple_GET_ITEM(hit, 4);          // a tensor, False (no such table) or None (not made)
+        const at::Tensor* t = tensor(made);
+        const auto stream = c10::cuda::getCurrentCUDAStream(t != nullptr ? t->get_device() : -1);
+        // (the legacy stream is never captured: asking costs 0.3 us of a small call)
+        if (t != nullptr && (stream.stream() == nullptr ||
+                             c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)) {
+            if (PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 5)) != stream.stream()) {
+                ok = cudaStreamWaitEvent(stream.stream(), static_cast<cudaEvent_t>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 6))), 0) ==
+                     cudaSuccess;
+                c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
             }
+            *table = static_cast<const int32_t*>(t->const_data_ptr());
         }
+        ok = ok && made != Py_None;
     }
     Py_DECREF(hit);
     return ok;
@@ -321,8 +329,8 @@ PyObject* sddmm(PyObject* const* a, Py_ssize_t n) {
     const float *pl = meta(lin, L, dev), *pt = meta(tr, L, dev), *pn = meta(nnzs, L, dev);
     int32_t plan[8];
     const int32_t* table = nullptr;
-    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, &table)) return yes_or_none(false);
-    if (nnzs->numel() != L) table = nullptr;
+    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, dtype != 0 && nnzs->numel() == L ? &table : nullptr))
+        return yes_or_none(false);
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
     at::Tensor rows;
     if (dtype != 0) rows = rows_of_k(*y, ksb, plan, L, d, st);
@@ -361,8 +369,8 @@ PyObject* spmm(PyObject* const* a, Py_ssize_t n) {
     const float *pl = meta(lin, L, dev), *pt = meta(tr, L, dev), *pn = meta(nnzs, L, dev);
     int32_t plan[8];
     const int32_t* table = nullptr;
-    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, &table)) return yes_or_none(false);
-    if (nnzs->numel() != L) table = nullptr;
+    if (!pl || !pt || !pn || !cached_plan(a[5], *nnzs, a[3], *lin, a[4], *tr, plan, dtype != 0 && nnzs->numel() == L ? &table : nullptr))
+        return yes_or_none(false);
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
     int32_t rc = dtype == 0 ? g_api.spmm_tile(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
                                                     n_cols, d, T, dtype, plan, st)
