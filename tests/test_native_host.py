@@ -1,4 +1,7 @@
 """CPU: the native host path of the launchers (the splat_host extension) and the state behind it, without a device."""
+import importlib.util
+import os
+import shutil
 import subprocess
 import sys
 import textwrap
@@ -109,3 +112,22 @@ def test_status_word_is_set_up_once(monkeypatch):
     monkeypatch.setattr(n, "_STATUS_MIRRORS", {})
     words = _from_threads(lambda: n.status_word(torch.device("cuda", 0)))
     assert len(mirrors) == 1 and all(w is words[0] for w in words)
+
+
+def test_extension_of_another_torch_is_rebuilt(monkeypatch, tmp_path):
+    """An installed torch that changes makes the extension stale, whatever the ages of the files."""
+    spec = importlib.util.spec_from_file_location("splat_build", os.path.join(ROOT, "triton-fun_b200", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    note = tmp_path / "built-for"
+    shutil.copyfile(build.HOST_BUILT_FOR, note)
+    monkeypatch.setattr(build, "HOST_BUILT_FOR", str(note))
+    commands = []
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **k: commands.append(cmd))
+    build.build_host()
+    assert not commands
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    build.build_host()
+    assert len(commands) == 1
+    build.build_host()
+    assert len(commands) == 1

@@ -20,6 +20,7 @@ INCLUDE = os.path.join(REPO_ROOT, "include")
 LIB_PATH = os.path.join(PKG_DIR, "libsplat_b200.so")
 HOST_SRC = os.path.join(CSRC, "host_binding.cpp")
 HOST_PATH = os.path.join(PKG_DIR, "SPLAT", "splat_host.so")
+HOST_BUILT_FOR = HOST_PATH + ".built-for"      # the torch and Python that it was compiled against
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -45,12 +46,15 @@ def up_to_date() -> bool:
 
 
 def build_host(force: bool = False) -> str:
-    if not force and os.path.exists(HOST_PATH) and \
-            all(os.path.getmtime(f) <= os.path.getmtime(HOST_PATH) for f in (HOST_SRC, __file__)):
-        return HOST_PATH
     import sysconfig
 
     import torch
+    built_for = f"torch {torch.__version__}, Python {sys.version}"
+    if not force and os.path.exists(HOST_PATH) and os.path.exists(HOST_BUILT_FOR) and \
+            all(os.path.getmtime(f) <= os.path.getmtime(HOST_PATH) for f in (HOST_SRC, __file__)):
+        with open(HOST_BUILT_FOR) as f:
+            if f.read() == built_for:
+                return HOST_PATH
     root = os.path.dirname(torch.__file__)
     nvcc = shutil.which(os.environ.get("NVCC", "nvcc")) or "/usr/local/cuda/bin/nvcc"
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc)))
@@ -62,6 +66,8 @@ def build_host(force: bool = False) -> str:
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
     print(" ".join(cmd), file=sys.stderr)
     subprocess.run(cmd, check=True)
+    with open(HOST_BUILT_FOR, "w") as f:
+        f.write(built_for)
     return HOST_PATH
 
 
