@@ -69,8 +69,8 @@ def measured_peaks():
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons of one GPU.  The sampler is started early (nvidia-smi
-    takes a while to produce its first row); ``mark()`` brackets the timed region and only rows
+    """nvidia-smi clocks / throttle reasons of one GPU.  start() waits for the first row (nvidia-smi
+    takes longer to produce it than a short timed region lasts); ``mark()`` brackets the timed region and only rows
     whose host timestamp falls inside it are summarised."""
     FIELDS = ("clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.hw_slowdown,"
               "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
@@ -90,6 +90,9 @@ class ClockSampler:
             self.thread.start()
         except OSError:
             self.proc = None
+        until = time.perf_counter() + 5
+        while self.proc is not None and not self.rows and time.perf_counter() < until:
+            time.sleep(0.01)
         return self
 
     def _read(self):
