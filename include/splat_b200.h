@@ -133,7 +133,8 @@ int32_t splat_sddmm(const void* q, const void* k, int64_t k_stride_bh, int64_t k
                     int64_t trailing_dim, int32_t dtype, void* stream);
 
 /* P[bh,i,j] = softmax_j(scale * S[bh,i,j]) over j < nnz_i, for ALL rows.  s_in == p_out (in place)
- * is allowed.
+ * is allowed.  s_in is read in whole aligned 16-byte pieces: up to 14 bytes before its first and behind its last element
+ * are read too (never written), which matters to nobody but a caller whose other streams write them meanwhile.
  * Stands in for rsoftmax_launcher -> r_softmax_1d_kernel (SPLAT/r_softmax.py:17-59,126-150);
  * the reference applies no scale (scale = 1). */
 int32_t splat_softmax(const void* s_in, void* p_out, const float* nnzs, int64_t bh, int64_t n_rows,
@@ -283,7 +284,8 @@ int32_t splat_attention_host(const void* q, const void* k, const void* v, void* 
                              int32_t* path_ran, void* stream_in, void* stream, void* stream_out,
                              void* const* events_7);
 
-/* splat_sddmm_band / splat_spmm_band with the band table (or NULL). */
+/* splat_sddmm_band / splat_spmm_band with the band table (or NULL).  P is read in whole aligned 16-byte pieces, up to 14
+ * bytes before its first and behind its last element included (see splat_softmax). */
 int32_t splat_sddmm_band_table(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
                                int64_t k_stride_k, void* s_out, const float* sTod_lin,
                                const float* sTod_tr, const float* nnzs, int64_t bh, int64_t n_rows,

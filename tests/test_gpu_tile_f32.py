@@ -1,6 +1,8 @@
 """GPU: the fp32 register-tile kernels (fused, SDDMM, SpMM) against the CPU oracle at the edges of their
 tiles: lengths around multiples of 64, classes with a missing last row, both K layouts, rows with one or
 no non-zero."""
+import ctypes
+
 import pytest
 import torch
 
@@ -40,7 +42,9 @@ def test_tile_kernels_against_oracle(d, contiguous):
         kt = kt.contiguous() if contiguous else kt
         scale = d ** -0.5
         plan = n.classify(acsr[2], acsr[3], acsr[4])
-        assert plan[3] == 0 and (plan[7] == 0 or plan[1] == plan[2])     # a band pattern: the tile kernels run
+        assert plan[3] == 0 and (plan[7] == 0 or plan[1] == plan[2])     # a band pattern
+        plan_arr = ctypes.cast((ctypes.c_int32 * 8)(*plan), ctypes.c_void_p)
+        vectors = [t.data_ptr() for t in acsr[2:5]]
         o = torch.full((1, H, L, d), float("nan"), device="cuda")
         lse = torch.full((1, H, L), float("nan"), device="cuda")
         n.attention_fused(q.cuda(), kt, v.cuda(), o, acsr[2], acsr[3], acsr[4], scale, n.PATH_AUTO, lse=lse)
@@ -50,6 +54,15 @@ def test_tile_kernels_against_oracle(d, contiguous):
         s = torch.full((1, H, L, T), float("nan"), device="cuda")
         n.sddmm(q.cuda(), kt, s, acsr[2], acsr[3], acsr[4], T)
         assert_close(s, s_ref, torch.float32, f"sddmm {what}")
+        # the tile kernels ran: asked for by name they take the call and give the same bits
+        qd, tile = q.cuda(), torch.full_like(s, float("nan"))
+        _bh, ksb, ksk, ksc = n._flat_bh(kt, "kt")
+        assert n._lib.splat_sddmm_tile(qd.data_ptr(), kt.data_ptr(), ksb, ksc, ksk, tile.data_ptr(), *vectors, H, L, L, d, T,
+                                       n.dtype_code(s.dtype), plan_arr, n._stream(s.device)) == 0 and torch.equal(s, tile), what
+        if L > 32:      # (row kernels sum in another order)
+            rows = torch.empty_like(o)
+            n.attention_fused(qd, kt, v.cuda(), rows, acsr[2], acsr[3], acsr[4], scale, n.PATH_GENERIC)
+            assert not torch.equal(o, rows), f"fused {what}: the row kernel"
         _cols, valid = at._cols(meta, T)
         assert torch.count_nonzero(s.cpu() * (~valid)) == 0, "padding slots must be zero"
         p = torch.rand(1, H, L, T)
@@ -57,3 +70,10 @@ def test_tile_kernels_against_oracle(d, contiguous):
         o2 = torch.full((1, H, L, d), float("nan"), device="cuda")
         n.spmm(p_dev, v.cuda(), o2, acsr[2], acsr[3], acsr[4], T)
         assert_close(o2, at.spmm_acsr(p, v, meta), torch.float32, f"spmm {what}")
+        vd, tile = v.cuda(), torch.full_like(o2, float("nan"))
+        rc = n._lib.splat_spmm_tile(p_dev.data_ptr(), vd.data_ptr(), tile.data_ptr(), *vectors, H, L, L, d, T,
+                                    n.dtype_code(p.dtype), plan_arr, n._stream(s.device))
+        if kind == ao.PATTERN_STRIDED:      # classes of 26 rows: too short for SpMM, which the row kernel does
+            assert rc == n.ERR_UNSUPPORTED_SHAPE
+        else:
+            assert rc == 0 and torch.equal(o2, tile), what

@@ -421,7 +421,8 @@ def _warn_cuda_core_16bit(what: str) -> None:
 
 
 def _band_candidate(x: torch.Tensor, path: int) -> bool:
-    """The tensor-core kernels take 16-bit operands with d = 64 or 128 (the library checks the rest)."""
+    """The tensor-core kernels take 16-bit operands (of any d that is a multiple of 8 up to 128; the library checks
+    that and the rest)."""
     return path != PATH_GENERIC and x.dtype in (torch.float16, torch.bfloat16) and x.numel() > 0
 
 

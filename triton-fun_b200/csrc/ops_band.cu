@@ -427,8 +427,8 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
 // SpMM
 // ---------------------------------------------------------------------------------------------
 // kPerSm CTAs share an SM: two with three steps of P on their way, or, at D = 64 and with more than two CTAs per SM to
-// run, three with two steps each (96 registers and some spills): B3 H44 L7680 window 224 216 -> 200 us, B2 H116 L4032
-// +-17 146 -> 124 us; a single wave (H8 L1024) is faster with two, 7.5 against 8.3 us.
+// run, three with two steps each (96 registers and some spills): B3 H44 L7680 +-224 294 -> 270 us, B2 H116 L4032
+// +-17 165 -> 144 us; a single wave (H8 L1024) is faster with two, 7.5 against 8.3 us.
 template <int D, int kPerSm> struct SpmmLayout {
     static constexpr int kSub = D / 64;
     static constexpr int kItemBytes = kSub * kStepBytesPerSub;    // 64 keys of V

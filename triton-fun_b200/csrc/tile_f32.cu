@@ -581,7 +581,10 @@ static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
 
 // 64-row CTAs unless they leave SMs without their three CTAs: then 32-row CTAs, whose four warps share the
 // keys of one row block, finish sooner, while with the GPU full they load every key twice as often; and with
-// less than two such CTAs per SM eight warps share them.
+// less than two such CTAs per SM eight warps share them.  Four / eight warps, us, at 256 CTAs (L1024, +-64, where five or
+// six steps leave some of the eight groups without any): d64 fused 33.9 / 24.7, SDDMM 16.5 / 16.3, SpMM 16.9 / 14.1;
+// d128 42.1 / 43.7, 29.1 / 28.9, 19.8 / 21.5; d32 16.8 / 16.9, 12.0 / 10.9, 8.2 / 8.8; +-400, d64: 98 / 67, 55 / 53, 50 / 35.
+// At 192 CTAs +-64 fused d64 30.3 / 24.5, SpMM 11.0 / 13.9.
 template <int D, Op OP>
 static int32_t run(const Params& p, int64_t bh, cudaStream_t st) {
     const int64_t rows = ((int64_t)p.n_rows + p.stride - 1) / p.stride, classes = p.stride * bh;
