@@ -177,7 +177,7 @@ def test_only_calls_that_read_it_make_the_band_table():
 
 @pytest.mark.parametrize("call", ["module", "sddmm", "host"])
 def test_first_calls_on_two_streams(call):
-    """The band table is made on one stream, behind work that is queued there; a call on another one waits for it."""
+    """The band table is made on one stream, behind work that is queued there; a call on another one reads it whole."""
     import acsr_helpers as ah
     import r_attention
     import splat_native as n
@@ -202,7 +202,7 @@ def test_first_calls_on_two_streams(call):
     torch.cuda.synchronize()
     attn = make()
     meta = attn.sTod_linear_transformations, attn.sTod_translations, attn.nnzs
-    attn.nnzs._splat_plan = attn.nnzs._splat_plan[:4] + (None, 0, 0, None)         # as classify() leaves it
+    attn.nnzs._splat_plan = attn.nnzs._splat_plan[:4] + (None, 0)         # as classify() leaves it
     torch.cuda.synchronize()
     with torch.cuda.stream(one):
         torch.cuda._sleep(400_000_000)         # SM clocks, some 0.2 s

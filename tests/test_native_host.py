@@ -35,7 +35,7 @@ def test_operands_without_data_end_no_process(call):
         with FakeTensorMode(allow_non_fake_inputs=True):
             x, vec = torch.empty(1, 1, 8, 8, device="cuda:0"), torch.empty(8, device="cuda:0")
             plan = (8, 1, 1, 0, 0, 8, 0, 8)
-            vec._splat_plan = ((0, 0, vec._version, vec._version, vec._version, 8), plan, vec, vec, False, 0, 0, None)
+            vec._splat_plan = ((0, 0, vec._version, vec._version, vec._version, 8), plan, vec, vec, False, 0)
             module = dict(rspmm_output=x, scale=1.0, path=0, lse=None, plan=plan, nnzs=vec,
                           sTod_linear_transformations=vec, sTod_translations=vec)
             assert {call} is None

@@ -251,13 +251,13 @@ def classify(sTod_lin: torch.Tensor, sTod_tr: torch.Tensor, nnzs: torch.Tensor) 
               "splat_acsr_classify")
     host = tuple(int(v) for v in plan.cpu().tolist())
     # keep the two companions alive with the cache entry so their ids cannot be reused
-    nnzs._splat_plan = (key, host, sTod_lin, sTod_tr, None, 0, 0, None)
+    nnzs._splat_plan = (key, host, sTod_lin, sTod_tr, None, 0)
     return host
 
 
 def band_table(sTod_lin, sTod_tr, nnzs, n_rows: int):
     """Address of the band table (``splat_band_table``) of classified metadata, which lives with their plan; made by
-    the first call that reads it, in the order of that call's stream.  None if the pattern has none, if the
+    the first call that reads it.  None if the pattern has none, if the
     metadata have changed since classify() or have more rows than the operands -- or for a captured launch,
     which has to work with the metadata as they are at the replay."""
     hit = _known_plan(sTod_lin, sTod_tr, nnzs)
@@ -269,17 +269,17 @@ def band_table(sTod_lin, sTod_tr, nnzs, n_rows: int):
         plan, n = hit[1], n_rows
         stride = plan[1] if plan[7] > 0 else 1
         if not (0 < n <= 2**31 - 1 and (plan[7] == 0 or plan[1] == plan[2]) and plan[3] == 0 and plan[5] <= n and stride <= 65535):
-            nnzs._splat_plan = hit[:4] + (False, 0, 0, None)
+            nnzs._splat_plan = hit[:4] + (False, 0)
             return None
         tiles = -(-(-(-n // stride)) // 128) * stride
         table = torch.empty(2 * (n + tiles), dtype=torch.int32, device=dev)
         with _on(dev):
             check(_lib.splat_band_table(sTod_lin.data_ptr(), sTod_tr.data_ptr(), nnzs.data_ptr(), n, stride,
                                         table.data_ptr(), stream.cuda_stream), "splat_band_table")
-            made = stream.record_event()
-        hit = nnzs._splat_plan = hit[:4] + (table, stream.cuda_stream, made.cuda_event, made)
-    if hit[5] != stream.cuda_stream:      # the table is nobody's tensor but ours: its order and its use elsewhere are ours to see to
-        stream.wait_event(hit[7])
+            # any stream may use it.  (An event for the others to wait for instead: 30 us where metadata are kept, for its creation)
+            stream.synchronize()
+        hit = nnzs._splat_plan = hit[:4] + (table, stream.cuda_stream)
+    if hit[5] != stream.cuda_stream:      # the table is nobody's tensor but ours: its use elsewhere is ours to record
         hit[4].record_stream(stream)
     return hit[4].data_ptr()
 

@@ -144,11 +144,10 @@ inline bool same4(const at::Tensor& t, int64_t a, int64_t b, int64_t c, int64_t 
 }
 
 // plan remembered by splat_native.classify() on the nnzs tensor: ((id, id, version x 3, numel), plan, lin, tr,
-// band table, stream it was made on, event behind its making, owner of the event); false if the metadata is not what it
-// was made from.  With `table`, also its address -- null for a pattern without one -- and false if Python has yet to
+// band table, stream it was made on); false if the metadata is not what it was made from.  With `table`, also its address -- null for a pattern without one -- and false if Python has yet to
 // make it.  A captured launch gets no table: a replay has to follow the metadata as they are then, and the table's
-// memory goes with the Python objects.  The caller knows nothing of the table, so on another stream than its own it
-// is waited for, and its use recorded, here.
+// memory goes with the Python objects.  The caller knows nothing of the table, so its use on another stream than its own
+// is recorded here.
 bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, const at::Tensor& lin, PyObject* tr_obj,
                  const at::Tensor& tr, int32_t (&plan)[8], const int32_t** table = nullptr) {
     PyObject* hit = PyObject_GetAttr(nnzs_obj, k_cached_plan);
@@ -156,7 +155,7 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
         PyErr_Clear();
         return false;
     }
-    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 8 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
+    bool ok = PyTuple_Check(hit) && PyTuple_GET_SIZE(hit) == 6 && PyTuple_GET_ITEM(hit, 2) == lin_obj &&
               PyTuple_GET_ITEM(hit, 3) == tr_obj;
     if (ok) {
         PyObject* key = PyTuple_GET_ITEM(hit, 0);
@@ -177,11 +176,8 @@ bool cached_plan(PyObject* nnzs_obj, const at::Tensor& nnzs, PyObject* lin_obj, 
         // (the legacy stream is never captured: asking costs 0.3 us of a small call)
         if (t != nullptr && (stream.stream() == nullptr ||
                              c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)) {
-            if (PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 5)) != stream.stream()) {
-                ok = cudaStreamWaitEvent(stream.stream(), static_cast<cudaEvent_t>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 6))), 0) ==
-                     cudaSuccess;
+            if (PyLong_AsVoidPtr(PyTuple_GET_ITEM(hit, 5)) != stream.stream())
                 c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
-            }
             *table = static_cast<const int32_t*>(t->const_data_ptr());
         }
         ok = ok && made != Py_None;
