@@ -135,13 +135,16 @@ class RegularAttention(nn.Module):
         be dropped right away (torch's allocator keeps their blocks until they have been copied).  Not in the reference, whose operands are always device tensors."""
         B, H, L, d = q_host.shape
         bh = B * H
-        q, k, v, out = hosts = [t.view(1, bh, L, d) for t in (q_host, k_host, v_host, out_host)]
+        q, k, v, out = hosts = (q_host, k_host, v_host, out_host)
+        plain = all(t.shape == q_host.shape and t.is_contiguous() and t.dtype == self.out_dtype and t.is_cpu for t in hosts)
+        if not plain:
+            q, k, v, out = hosts = [t.view(1, bh, L, d) for t in hosts]
+            plain = all(t.dtype == self.out_dtype and t.is_cpu for t in hosts) and out.is_contiguous()
+            if not plain:
+                q, k, v = (t.to("cpu", self.out_dtype) for t in (q, k, v))
+            q, k, v = (t.contiguous() for t in (q, k, v))
         if bh == 0 or L == 0:
             return out_host
-        plain = all(t.dtype == self.out_dtype and t.device.type == "cpu" for t in hosts) and out.is_contiguous()
-        if not plain:
-            q, k, v = (t.to("cpu", self.out_dtype) for t in (q, k, v))
-        q, k, v = (t.contiguous() for t in (q, k, v))
         dst = out if plain else torch.empty((1, bh, L, d), dtype=self.out_dtype).pin_memory()
         chunk = max(1, min(chunk_heads, bh, host_chunk(bh, L * d * self.out_dtype.itemsize)))
         st = getattr(self, "_host_stage", None)
@@ -154,6 +157,9 @@ class RegularAttention(nn.Module):
                   "staging": (ctypes.c_void_p * 8)(*(t.data_ptr() for t in bufs)),
                   "events": (ctypes.c_void_p * 7)(*(e.cuda_event for e in events)),
                   "s_in": torch.cuda.Stream(self.device), "s_out": torch.cuda.Stream(self.device)}
+            for name in ("s_in", "s_out"):
+                s = st[name]
+                st[name + "_key"] = s.stream_id, s.device_index, s.device_type
             self._host_stage = st
         _n.attention_host(q, k, v, dst, st, self.sTod_linear_transformations, self.sTod_translations,
                           self.nnzs, self.scale, self.path, self.plan)

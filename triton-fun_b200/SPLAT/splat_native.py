@@ -214,8 +214,9 @@ def attention_host(q, k, v, out, stage: dict, sTod_lin, sTod_tr, nnzs, scale: fl
             table, sw.data_ptr(), ctypes.byref(ran), stage["s_in"].cuda_stream, _stream(dev),
             stage["s_out"].cuda_stream, stage["events"])
         # the caller may drop its tensors now: their page-locked blocks are reused only when the copies are done
-        for t, s in ((q, stage["s_in"]), (k, stage["s_in"]), (v, stage["s_in"]), (out, stage["s_out"])):
-            _host.record_pinned(t, s.stream_id, s.device_index, s.device_type)
+        for t in (q, k, v):
+            _host.record_pinned(t, *stage["s_in_key"])
+        _host.record_pinned(out, *stage["s_out_key"])
     check(rc, "splat_attention_host")
     if ran.value != PATH_BAND and q.dtype != torch.float32 and q.numel() > 0 and path == PATH_AUTO:
         _warn_cuda_core_16bit("attention")
@@ -262,9 +263,11 @@ def band_table(sTod_lin, sTod_tr, nnzs, n_rows: int):
     which has to work with the metadata as they are at the replay."""
     hit = _known_plan(sTod_lin, sTod_tr, nnzs)
     dev = nnzs.device
-    if hit is None or hit[4] is False or nnzs.numel() != n_rows or _capturing(dev):
+    if hit is None or hit[4] is False or nnzs.numel() != n_rows:
         return None
     stream = torch.cuda.current_stream(dev)
+    if stream.cuda_stream != 0 and _capturing(dev):        # (the legacy stream is never captured)
+        return None
     if hit[4] is None:
         plan, n = hit[1], n_rows
         stride = plan[1] if plan[7] > 0 else 1
