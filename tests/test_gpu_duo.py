@@ -1,0 +1,80 @@
+"""GPU: the persistent two-tile kernel of d = 128, which takes over at 592 tiles of 128 rows.  It multiplies and sums in the
+order of the kernel with a tile per CTA, so the two agree bit for bit (and so do shards of a problem on either side of the
+line); the first and last head are also compared with the CPU oracle."""
+import pytest
+import torch
+
+from conftest import assert_close
+from oracle import acsr_oracle as ao
+from oracle import attention_oracle as at
+
+pytestmark = pytest.mark.gpu
+
+#        kind, L, p0, p1, batch * heads
+PATTERNS = [
+    (ao.PATTERN_CAUSAL_WINDOWED, 128, 40, 0, 592),     # one tile per head: neighbours never share keys; the fewest tiles
+    (ao.PATTERN_CAUSAL_WINDOWED, 384, 200, 0, 199),    # odd number of tiles per head and in all: items across heads, half an item
+    (ao.PATTERN_CAUSAL_WINDOWED, 1000, 255, 0, 80),    # a short last tile
+    (ao.PATTERN_CAUSAL_WINDOWED, 2048, 0, 0, 38),      # single-element rows only: nothing to multiply
+    (ao.PATTERN_CAUSAL_WINDOWED, 2048, 1500, 0, 40),   # ranges that grow with the row
+    (ao.PATTERN_WINDOWED, 1536, 300, 0, 50),
+    (ao.PATTERN_BLOCKED, 2560, 777, 0, 30),            # neighbours whose ranges jump by more than the ring holds
+    (ao.PATTERN_BLOCKED, 2048, 64, 0, 37),             # half steps at both ends
+    (ao.PATTERN_STRIDED, 1024, 64, 0, 10),             # classes of 16 rows
+    (ao.PATTERN_STRIDED, 4096, 4, 0, 20),              # triangular classes of eight tiles
+    (ao.PATTERN_DILATED, 3072, 300, 2, 26),
+]
+
+
+@pytest.mark.parametrize("contiguous,dtype", [(False, torch.bfloat16), (True, torch.bfloat16), (False, torch.float16)])
+@pytest.mark.parametrize("kind,L,p0,p1,H", PATTERNS)
+def test_duo_patterns(kind, L, p0, p1, H, contiguous, dtype, monkeypatch):
+    import acsr_helpers as ah
+    import splat_native as n
+    if contiguous and kind in (ao.PATTERN_STRIDED, ao.PATTERN_DILATED):
+        pytest.skip("a contiguous K^T of a strided pattern is copied to rows first")
+    d, scale = 128, 128 ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(L + p0)
+    acsr = ah.create_acsr(ah.PatternMask(kind, L, p0, p1), 16, 0)
+    q, k, v = (torch.randn(1, H, L, d, device="cuda", generator=g).to(dtype) for _ in range(3))
+    kt = k.transpose(2, 3)
+    kt = kt.contiguous() if contiguous else kt
+
+    def run(lse):
+        out = torch.full((1, H, L, d), float("nan"), dtype=dtype, device="cuda")
+        n.attention_fused(q, kt, v, out, acsr[2], acsr[3], acsr[4], scale, n.PATH_BAND, lse=lse)
+        n.check_status_word(0)
+        return out
+
+    monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
+    lse, lse_one = (torch.full((1, H, L), float("nan"), device="cuda") for _ in range(2))
+    out, plain = run(lse), run(None)
+    monkeypatch.setenv("SPLAT_B200_BAND_TILES", "1")
+    one = run(lse_one)
+    assert torch.equal(out, plain), "the log-sum-exp output changes the result"
+    assert torch.equal(out, one)
+    assert (lse - lse_one).abs().max().item() < 1e-5      # (a single row's score: sums in another order)
+    meta = ao.metadata_from_pattern(kind, L, p0, p1, 16)
+    ends = [0, H - 1]
+    qc, kc, vc = (t[:, ends].cpu() for t in (q, k, v))
+    assert_close(out[:, ends], at.attention_acsr(qc, kc.transpose(2, 3), vc, meta, meta["trailing_dim"], scale), dtype)
+
+
+def test_duo_unscaled_scores_need_the_running_max(monkeypatch):
+    """scale = 1 gives scores of sigma ~ 11: the rescale of O, also while the other tile is in mid-step."""
+    import acsr_helpers as ah
+    import splat_native as n
+    B, H, L, d = 1, 40, 2048, 128
+    acsr = ah.create_acsr(ah.create_causal_windowed_mask(L, 511), 16, 0)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(B, H, L, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    outs = []
+    for variant in (None, "1"):
+        if variant:
+            monkeypatch.setenv("SPLAT_B200_BAND_TILES", variant)
+        else:
+            monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
+        outs.append(torch.full_like(q, float("nan")))
+        n.attention_fused(q, k.transpose(2, 3), v, outs[-1], acsr[2], acsr[3], acsr[4], 1.0, n.PATH_BAND)
+        n.check_status_word(0)
+    assert torch.isfinite(outs[0].float()).all() and torch.equal(*outs)

@@ -756,6 +756,9 @@ int32_t attention_pair(const void* q, const void* k, int kt_major, const void* v
 int32_t attention_wide(const void* q, const void* k, int kt_major, const void* v, void* o, const float* lin, const float* tr,
                        const float* nnzs, int64_t bh, int64_t n_rows, int64_t d, int64_t stride, float scale, int32_t dtype,
                        int32_t* status_word, const int32_t* band_table, float* lse, cudaStream_t st);
+int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v, void* o, int64_t bh, int64_t n_rows, int64_t d,
+                      int64_t stride, float scale, int32_t dtype, int32_t* status_word, const int32_t* band_table, float* lse,
+                      cudaStream_t st);
 
 int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, int64_t ksk,
                        const void* v, void* o, const float* lin, const float* tr,
@@ -785,15 +788,22 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
     if (!k_major && (stride != 1 || n_cols % 8 != 0)) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return SPLAT_ERR_MISALIGNED;
 
-    // Kernel choice.  1 (default): one Q tile per CTA, two CTAs per SM (attention_wide.cu), the fastest on every
+    // Kernel choice.  1: one Q tile per CTA, two CTAs per SM (attention_wide.cu), the fastest on every
     // shape tried and the only one that takes any d and classes of unequal length.  2: two Q tiles per CTA
     // sharing every K/V tile (half the L2 -> SM traffic).  3: persistent CTA pairs (attention_pair.cu),
     // d = 128 only.  SPLAT_B200_BAND_TILES=1|2|3 selects; SPLAT_B200_PAIR_MAX limits the resident pairs of 3.
-    int variant = 1;
+    // Unset: two tiles per persistent CTA (attention_duo.cu) where there are enough tiles, else 1.  Below two waves of two
+    // tiles per SM the persistent kernel's longer start is not made up for (d 128, us, a CTA per tile / persistent: +-200
+    // at 320 / 384 / 512 / 592 tiles 26.2 / 27.8, 29.0 / 28.0, 33.8 / 30.7, 35.5 / 31.3; strided 16 12.3 / 14.0, 13.1 /
+    // 14.4, 16.8 / 16.7, 18.0 / 17.4); at d = 64 it is no faster (+-200, 1024 tiles 47 / 51).
+    int variant = 0;
     if (const char* e = getenv("SPLAT_B200_BAND_TILES"))
         if (e[0] >= '1' && e[0] <= '3') variant = e[0] - '0';
     if ((d != 64 && d != 128) || n_rows % stride != 0) variant = 1;
-    if (variant == 1)
+    const int64_t tiles = bh * stride * ((n_rows / stride + 127) / 128);
+    if (variant == 0 && d == 128 && band_table != nullptr && tiles >= 4 * 148 && tiles <= INT32_MAX)
+        return attention_duo(q, k, kt_major ? 1 : 0, v, o, bh, n_rows, d, stride, scale, dtype, status_word, band_table, lse, st);
+    if (variant <= 1)
         return attention_wide(q, k, kt_major ? 1 : 0, v, o, lin, tr, nnzs, bh, n_rows, d, stride, scale, dtype, status_word,
                               band_table, lse, st);
     if (variant == 3 && d == 128) {

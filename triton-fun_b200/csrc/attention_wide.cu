@@ -1,5 +1,6 @@
 // Fused band attention, one 128-row Q tile per CTA, two CTAs per SM.  Problem, regrouping by residue class and
-// operand layouts: see attention_band.cu.  The default for every band pattern of 16-bit operands.
+// operand layouts: see attention_band.cu.  The default for band patterns of 16-bit operands, but for large problems with
+// d = 128 (attention_duo.cu).
 //
 // A step is 128 keys:
 //     S(j)  = Q K(j)^T       tcgen05.mma 128x128x16, operands in shared memory
