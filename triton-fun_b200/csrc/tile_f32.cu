@@ -103,7 +103,8 @@ template <int D, int RW, int KW, Op OP> struct Layout {
     static constexpr int kPart = 32 * D + 64;           // a warp's partial result: O[32][D], maxima, sums
     static constexpr int kMain = kQ + kGroups * kGroupFloats;
     static constexpr int kFloats = OP == Op::kSddmm || kMain > kWarps * kPart ? kMain : kWarps * kPart;
-    static constexpr int kPerSm = KW == 8 ? 1 : (D == 128 ? 2 : 3);     // CTAs per SM the registers are budgeted for
+    static constexpr int kPerSm = KW == 8 ? (D == 128 || OP == Op::kFused ? 1 : 2) : (D == 128 ? 2 : 3);     // CTAs per SM the registers are budgeted for ...
+    static constexpr int kPerSmFull = D != 128 ? 4 : OP == Op::kSddmm ? 3 : 2;    // ... where there are more to run than kPerSm (SDDMM, SpMM)
 };
 
 // acc[8 rows][NP pairs of columns] += a[8] x b[NP]
@@ -241,13 +242,17 @@ __device__ __forceinline__ void tile_body(const Params& p) {
     const float* kbase = p.kt ? p.k + head * D : p.k + (head + res) * D;
     const float* vbase = p.v + (head + res) * D;
 
+    // metadata of the rows, one row per lane, in class coordinates: band columns [a, a + n).  Asked for before the copies of
+    // Q, which take a thousand cycles to issue; the fused kernel of one row block is faster the other way round (a tiny problem
+    // 6.56 against 6.70 us; with two row blocks 254 against 249).
+    int my_a = 0, my_n = 0, my_nnz = 0, my_start = 0;   // handed out by shuffles
+    RowAffine ra = {0, 1, 0};
+    constexpr bool kQFirst = OP == Op::kFused && RW == 1;
+    if (!kQFirst && u0 + lane < rows_v) ra = row_affine(p.lin, p.tr, p.nnzs, (int64_t)(u0 + lane) * p.stride + res);
     if (OP != Op::kSpmm) load_transposed<D, kRows, kWarps>(s_q, qbase, pitch, cta_u0, rows_v, warp);
     cp_commit();
-
-    // metadata of the rows, one row per lane, in class coordinates: band columns [a, a + n)
-    int my_a = 0, my_n = 0, my_nnz = 0, my_start = 0;   // handed out by shuffles
+    if (kQFirst && u0 + lane < rows_v) ra = row_affine(p.lin, p.tr, p.nnzs, (int64_t)(u0 + lane) * p.stride + res);
     if (u0 + lane < rows_v) {
-        const RowAffine ra = row_affine(p.lin, p.tr, p.nnzs, (int64_t)(u0 + lane) * p.stride + res);
         my_nnz = ra.nnz;
         my_start = ra.start;
         if (my_nnz > 1) { my_a = (my_start - res) / p.stride; my_n = my_nnz; }
@@ -275,6 +280,9 @@ __device__ __forceinline__ void tile_body(const Params& p) {
     // of every CTA
     const int c_first = (k_lo + ((group + (int)blockIdx.x) & (kGroups - 1))) * kKeys, c_end = k_hi * kKeys;
 
+    // this warp's first row of the sparse operand, and from one row to the next
+    float* const sparse_row = OP == Op::kFused ? nullptr : p.sparse + (head + (int64_t)u0 * p.stride + res) * p.trailing;
+    const int64_t sparse_pitch = (int64_t)p.stride * p.trailing;
     auto load_keys = [&](int c0) {
         if (OP != Op::kSpmm) {
             if (p.kt) load_kt<D, RW>(s_k, kbase, p, res, c0, rows_v, rw);
@@ -282,14 +290,14 @@ __device__ __forceinline__ void tile_body(const Params& p) {
         }
         if (OP != Op::kSddmm && !L::kOneBuffer) load_v<D, RW>(s_v, vbase, pitch, c0, rows_v, rw);
         if (OP == Op::kSpmm) {     // this warp's rows of P into Pt, one row per round, lanes along the keys
+            const float* src = sparse_row;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_p + lane * 32);
+            const int behind = c0 + lane - my_a;       // row `lane`'s slot of column c0 + lane; row rr's: behind(rr) - rr + lane
 #pragma unroll 8
-            for (int rr = 0; rr < 32; ++rr) {
-                const int lo = __shfl_sync(0xffffffffu, my_a, rr) - c0;
-                const int n = __shfl_sync(0xffffffffu, my_n, rr);
-                const float* src = p.sparse + (head + (int64_t)(u0 + rr) * p.stride + res) * p.trailing - lo;
-                const bool in = lane >= lo && lane < lo + n;
-                cp4((uint32_t)__cvta_generic_to_shared(s_p + lane * 32 + ((((rr >> 2) ^ (lane >> 2)) << 2) | (rr & 3))),
-                    in ? src + lane : p.sparse, in);
+            for (int rr = 0; rr < 32; ++rr, src += sparse_pitch) {
+                const int slot = __shfl_sync(0xffffffffu, behind, rr) - rr + lane;
+                const bool in = (unsigned)slot < (unsigned)__shfl_sync(0xffffffffu, my_n, rr);
+                cp4(dst + (((((rr >> 2) ^ (lane >> 2)) << 2) | (rr & 3)) << 2), in ? src + slot : p.sparse, in);
             }
         }
         cp_commit();
@@ -397,12 +405,13 @@ __device__ __forceinline__ void tile_body(const Params& p) {
                 *reinterpret_cast<float4*>(s_p + row_of(i) * 32 + 4 * t) =
                     make_float4(s[i][0].x, s[i][0].y, s[i][1].x, s[i][1].y);
             __syncwarp();
+            // (a row costs eight instructions: with 64-bit addresses formed for each this was half of a small call)
+            float* mem = sparse_row;
+            const int behind = c0 + lane - my_a;       // (as in load_keys)
 #pragma unroll 8
-            for (int rr = 0; rr < 32; ++rr) {
-                const int lo = __shfl_sync(0xffffffffu, my_a, rr) - c0;
-                const int n = __shfl_sync(0xffffffffu, my_n, rr);
-                float* mem = p.sparse + (head + (int64_t)(u0 + rr) * p.stride + res) * p.trailing - lo;
-                if (lane >= lo && lane < lo + n) mem[lane] = s_p[rr * 32 + lane];
+            for (int rr = 0; rr < 32; ++rr, mem += sparse_pitch) {
+                const int slot = __shfl_sync(0xffffffffu, behind, rr) - rr + lane;
+                if ((unsigned)slot < (unsigned)__shfl_sync(0xffffffffu, my_n, rr)) mem[slot] = s_p[rr * 32 + lane];
             }
         }
         if (OP != Op::kSddmm) {
@@ -476,32 +485,30 @@ __device__ __forceinline__ void tile_body(const Params& p) {
     // a group's warp merges and writes 32 / kGroups of its rows, lanes along D
     float odd = 0.f;               // NaN: a row is not finite, or has its only non-zero elsewhere
     const float* parts = smem + rw * L::kPart;          // of these rows by group 0; the next group RW parts on
-#pragma unroll 2
+    // Weights of the partial results: 32 / kGroups rows with kGroups parts each, one per lane.  (With every lane forming the
+    // weights of every row the merge was a quarter of a small call.)
+    float w_mine = 1.f, mt = 0.f, lt = 0.f;
+    if (OP == Op::kFused) {
+        const float* about = parts + (lane % kGroups) * RW * L::kPart + 32 * D + group * (32 / kGroups) + lane / kGroups;
+        const float mp = about[0];
+        mt = mp;
+#pragma unroll
+        for (int o = 1; o < kGroups; o <<= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o));
+        w_mine = mp == -INFINITY ? 0.f : exp2f(mp - mt);
+        lt = w_mine * about[32];
+#pragma unroll
+        for (int o = 1; o < kGroups; o <<= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o);
+        w_mine *= 1.f / lt;            // (rows whose scores are all -inf: NaN; empty ones are zeroed below)
+    }
+#pragma unroll 4
     for (int i = 0; i < 32 / kGroups; ++i) {
         const int row = group * (32 / kGroups) + i;
         const int nnz = __shfl_sync(0xffffffffu, my_nnz, row), start = __shfl_sync(0xffffffffu, my_start, row);
         if (u0 + row >= rows_v) break;
         const int64_t real = head + (int64_t)(u0 + row) * p.stride + res;
-        float w[kGroups], mt = -INFINITY, lt = 0.f;
+        float w[kGroups];
 #pragma unroll
-        for (int x = 0; x < kGroups; ++x) {
-            w[x] = OP == Op::kFused ? parts[x * RW * L::kPart + 32 * D + row] : 0.f;
-            mt = fmaxf(mt, w[x]);
-        }
-#pragma unroll
-        for (int x = 0; x < kGroups; ++x) {
-            if (OP == Op::kFused) {
-                w[x] = w[x] == -INFINITY ? 0.f : exp2f(w[x] - mt);
-                lt += w[x] * parts[x * RW * L::kPart + 32 * D + 32 + row];
-            } else {
-                w[x] = 1.f;
-            }
-        }
-        if (OP == Op::kFused) {
-            const float inv = 1.f / lt;        // (rows whose scores are all -inf: NaN; empty ones are zeroed below)
-#pragma unroll
-            for (int x = 0; x < kGroups; ++x) w[x] *= inv;
-        }
+        for (int x = 0; x < kGroups; ++x) w[x] = OP == Op::kFused ? __shfl_sync(0xffffffffu, w_mine, i * kGroups + x) : 1.f;
         // a row with one non-zero is described by the metadata as column `start`, outside the band
         const float w1 = OP == Op::kSpmm && nnz == 1 ? p.sparse[real * p.trailing] : 1.f;
 #pragma unroll
@@ -518,7 +525,7 @@ __device__ __forceinline__ void tile_body(const Params& p) {
             odd = fmaf(y, 0.f, odd);
         }
         if (OP == Op::kFused && nnz == 1) odd = NAN;
-        if (OP == Op::kFused && p.lse != nullptr && lane == 0) {
+        if (OP == Op::kFused && p.lse != nullptr && lane == i * kGroups) {
             float e = nnz > 1 ? lse_from_log2(mt, lt) : -INFINITY;
             if (nnz == 1) {
                 const float* kr = p.kt ? p.k + head * D + start : p.k + (head + start) * D;
@@ -547,8 +554,8 @@ __device__ __forceinline__ void tile_body(const Params& p) {
 
 // (Parameters by value, or by reference to where they are: the repair at the end of tile_body changes how the rest is
 // compiled.  Fused B2 H16 L4096 d64 270 against 262 us, the three launchers of H8 L1024 32.3 against 33.7 us.)
-template <int D, int RW, int KW, Op OP>
-__global__ void __launch_bounds__(32 * RW * KW, Layout<D, RW, KW, OP>::kPerSm) tile_kernel(const Params p) {
+template <int D, int RW, int KW, Op OP, int kPerSm>
+__global__ void __launch_bounds__(32 * RW * KW, kPerSm) tile_kernel(const Params p) {
     tile_body<D, RW, KW, OP>(p);
 }
 template <int D, int RW, int KW>
@@ -566,12 +573,12 @@ bool index_check_on();                                    // ops_generic.cu
 
 namespace tile {
 
-template <int D, int RW, int KW, Op OP>
+template <int D, int RW, int KW, Op OP, int kPerSm = Layout<D, RW, KW, OP>::kPerSm>
 static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
     constexpr int bytes = Layout<D, RW, KW, OP>::kFloats * (int)sizeof(float);
     void (*kern)(const Params);
     if constexpr (OP == Op::kFused) kern = tile_kernel_fused<D, RW, KW>;
-    else kern = tile_kernel<D, RW, KW, OP>;
+    else kern = tile_kernel<D, RW, KW, OP, kPerSm>;
     if (!band::allow_dynamic_smem(reinterpret_cast<const void*>(kern), bytes)) return SPLAT_ERR_LAUNCH;
     p.tiles = ((p.n_rows + p.stride - 1) / p.stride + 32 * RW - 1) / (32 * RW);
     const int64_t blocks = (int64_t)p.tiles * p.stride * bh;
@@ -585,11 +592,23 @@ static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
 // six steps leave some of the eight groups without any): d64 fused 33.9 / 24.7, SDDMM 16.5 / 16.3, SpMM 16.9 / 14.1;
 // d128 42.1 / 43.7, 29.1 / 28.9, 19.8 / 21.5; d32 16.8 / 16.9, 12.0 / 10.9, 8.2 / 8.8; +-400, d64: 98 / 67, 55 / 53, 50 / 35.
 // At 192 CTAs +-64 fused d64 30.3 / 24.5, SpMM 11.0 / 13.9.
+// SDDMM and SpMM at d <= 64: four CTAs per SM instead of three where there are more than three to run, with 128 registers: H16
+// L1024 d64 +-64 (512 CTAs of 32 rows) 22.9 / 22.4 -> 20.0 / 20.4, B2 H16 L4096 window 256 161 / 155 -> 149 / 146; 384 CTAs
+// are one wave either way and slower with fewer registers, 16.7 / 16.4 against 19.5 / 19.7.  Eight warps: two CTAs per
+// SM, SpMM at 256 CTAs 14.2 -> 12.5.
 template <int D, Op OP>
 static int32_t run(const Params& p, int64_t bh, cudaStream_t st) {
     const int64_t rows = ((int64_t)p.n_rows + p.stride - 1) / p.stride, classes = p.stride * bh;
-    if ((rows + 63) / 64 * classes >= 3 * 148) return launch<D, 2, 2, OP>(p, bh, st);
-    if ((rows + 31) / 32 * classes >= 2 * 148) return launch<D, 1, 4, OP>(p, bh, st);
+    if ((rows + 63) / 64 * classes >= 3 * 148) {
+        if constexpr (OP == Op::kFused) return launch<D, 2, 2, OP>(p, bh, st);
+        else return launch<D, 2, 2, OP, Layout<D, 2, 2, OP>::kPerSmFull>(p, bh, st);
+    }
+    if ((rows + 31) / 32 * classes >= 2 * 148) {
+        using L = Layout<D, 1, 4, OP>;
+        if constexpr (OP != Op::kFused && L::kPerSmFull != L::kPerSm)
+            if ((rows + 31) / 32 * classes > L::kPerSm * 148) return launch<D, 1, 4, OP, L::kPerSmFull>(p, bh, st);
+        return launch<D, 1, 4, OP>(p, bh, st);
+    }
     return launch<D, 1, 8, OP>(p, bh, st);
 }
 
