@@ -792,16 +792,19 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
     // shape tried and the only one that takes any d and classes of unequal length.  2: two Q tiles per CTA
     // sharing every K/V tile (half the L2 -> SM traffic).  3: persistent CTA pairs (attention_pair.cu),
     // d = 128 only.  SPLAT_B200_BAND_TILES=1|2|3 selects; SPLAT_B200_PAIR_MAX limits the resident pairs of 3.
-    // Unset: two tiles per persistent CTA (attention_duo.cu) where there are enough tiles, else 1.  Below two waves of two
-    // tiles per SM the persistent kernel's longer start is not made up for (d 128, us, a CTA per tile / persistent: +-200
-    // at 320 / 384 / 512 / 592 tiles 26.2 / 27.8, 29.0 / 28.0, 33.8 / 30.7, 35.5 / 31.3; strided 16 12.3 / 14.0, 13.1 /
-    // 14.4, 16.8 / 16.7, 18.0 / 17.4); at d = 64 it is no faster (+-200, 1024 tiles 47 / 51).
+    // Unset: two tiles per persistent CTA (attention_duo.cu) for d = 128 and enough tiles, else 1.  The persistent kernel takes
+    // 0.83 to 0.95 of the time where the waves of two tiles per SM are many or the last one is half full at least; a few
+    // tiles beyond two or three whole waves cost it a wave of its own (us, a CTA per tile / persistent: +-566 at 500 / 600 /
+    // 700 / 800 / 900 / 1200 tiles 58.1 / 58.2, 63.7 / 69.3, 81.0 / 71.9, 85.2 / 75.1, 89.6 / 94.2, 116 / 110; +-60 at 640 / 720 /
+    // 800 / 1040 / 1184 31.5 / 30.3, 34.2 / 36.0, 35.8 / 33.1, 45.2 / 41.2, 48.9 / 41.1).  At d = 64 it is no faster
+    // (+-200, 1024 tiles 47 / 51).
     int variant = 0;
     if (const char* e = getenv("SPLAT_B200_BAND_TILES"))
         if (e[0] >= '1' && e[0] <= '3') variant = e[0] - '0';
     if ((d != 64 && d != 128) || n_rows % stride != 0) variant = 1;
     const int64_t tiles = bh * stride * ((n_rows / stride + 127) / 128);
-    if (variant == 0 && d == 128 && band_table != nullptr && tiles >= 4 * 148 && tiles <= INT32_MAX)
+    if (variant == 0 && d == 128 && band_table != nullptr && (tiles >= 8 * 148 || (tiles >= 4 * 148 && tiles % (2 * 148) >= 148)) &&
+        tiles <= INT32_MAX)
         return attention_duo(q, k, kt_major ? 1 : 0, v, o, bh, n_rows, d, stride, scale, dtype, status_word, band_table, lse, st);
     if (variant <= 1)
         return attention_wide(q, k, kt_major ? 1 : 0, v, o, lin, tr, nnzs, bh, n_rows, d, stride, scale, dtype, status_word,

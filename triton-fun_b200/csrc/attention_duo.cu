@@ -12,7 +12,7 @@
 //     tile in turn.  It is read into registers within some 200 cycles of its completion.
 // Tensor memory: P of pipe 0 (64 columns), S (128), P of pipe 1 (64), O of pipe 0 and of pipe 1 (128 each).
 //
-// Work: an item is two neighbouring tiles (of the list head by head, class by class).  A CTA begins with the item of its
+// Work: an item is two neighbouring tiles (of the list head by head, class by class), or one in a short last wave.  A CTA begins with the item of its
 // index and then takes over CTAs that have not started (clusterlaunchcontrol), two items ahead.  The K / V blocks of an
 // item travel as a stream of entries through a ring of two slots each; every role derives the same numbering of the
 // entries from the items.
@@ -95,6 +95,7 @@ struct Params {
     Classes cls;
     uint32_t classes;  // ... their number
     uint32_t total;    // tiles of all heads and classes
+    uint32_t pairs;    // items of two tiles; the rest have one
     int stride;
     int d;             // head dimension, <= kD and a multiple of 8
     int kt_major;
@@ -311,7 +312,8 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                 if (next >= 0) {
 #pragma unroll 1
                     for (int x = 0; x < 2; ++x) {
-                        const Tile t = tile_of(p, 2 * (uint32_t)next + x);
+                        const uint32_t i = (uint32_t)next;
+                        const Tile t = tile_of(p, i < p.pairs ? 2 * i + x : x == 0 ? i + p.pairs : p.total);
                         if (lane == 0) ctrl->item[slot].t[x] = t;
                     }
                 }
@@ -748,7 +750,7 @@ template <typename T>
 static int32_t launch(const Maps<3>& maps, const Params& prm, cudaStream_t st) {
     auto kern = prm.lse != nullptr ? attention_duo_kernel<T, true> : attention_duo_kernel<T, false>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes)) return SPLAT_ERR_LAUNCH;
-    return launch_kernel(kern, (prm.total + 1) / 2, kThreads, kSmemBytes, st, maps, prm);
+    return launch_kernel(kern, prm.pairs + (prm.total > 2 * prm.pairs ? prm.total - 2 * prm.pairs : 0), kThreads, kSmemBytes, st, maps, prm);
 }
 
 }  // namespace duo
@@ -769,6 +771,9 @@ int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v,
     p.rows = reinterpret_cast<const int2*>(band_table);
     p.tiles = p.rows + n_rows;
     p.total = (uint32_t)(bh * p.classes * p.cls.tile_pitch);     // (the caller has seen that it fits)
+    // A last wave of no more tiles than SMs goes one tile to an SM: alone a tile takes two thirds of the time of two.
+    const uint32_t rest = p.total % (2 * 148);
+    p.pairs = rest <= 148 ? (p.total - rest) / 2 : (p.total + 1) / 2;
     Maps<3> maps;
     for (int part = 0; part < 2; ++part) {
         if (!p.cls.has(part)) continue;
