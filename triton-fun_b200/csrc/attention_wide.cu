@@ -23,6 +23,10 @@
 //     30 000 at stride 1 and 3 800 at stride 64; it remains for callers without a table.
 //   * Any d that is a multiple of 8 up to 128 runs: the copies fill a tile's columns past d with zeros, and
 //     the store clips them.  Any L: see band_classes.cuh.
+//   * Few instructions where they are not the point: waits are a try and a counter (looking at the status word, a clock and an
+//     atomic in each of 15 of them were a quarter of the code), the control block has constant addresses, an MMA's
+//     descriptor is an addition.  us, before -> after: fp16 B4 H16 L4096 d64 window 256 64.1 -> 60.7; bf16 B4 H16 L4096
+//     d32 window 256 65.1 -> 60.7, B2 H16 L8000 d64 strided 13 73.7 -> 67.1, H2 L256 d64 window 32 6.04 -> 5.78.
 // Softmax step of 128 keys by itself (no MMAs, cycles for one / two warps per scheduler): row in registers
 // 1468 / 2262, four chunks with the maximum looked at per chunk 1655 / 2403, a quarter of the exponentials
 // by polynomial on the FMA pipe 1414 / 2002; 64-key steps 2 x 900 / 2 x 1140.  In the kernel the chunked
@@ -93,6 +97,7 @@ struct Control {
     uint64_t s_free, pv_done;  // D = 64.  softmax -> MMA: scores read (4 warp arrivals); MMA -> softmax: PV complete
     uint32_t tmem_base;
     int32_t abort_at_entry;
+    int32_t gave_up;           // code of a wait that ran out
     int32_t lo[4], hi[4];      // key range of the rows' bands: of the tile (table), or per softmax warp
     alignas(16) uint32_t again[4];   // rows whose result is not finite
     alignas(16) uint32_t single[4];  // rows with one non-zero; later those of them whose score is not finite
@@ -104,36 +109,31 @@ template <int D> struct Layout {
     static constexpr int kSlots = D == 128 ? 1 : 2;         // K tiles, and V tiles, in shared memory
     static constexpr int kKOff = kTileBytes;                // behind the Q tile
     static constexpr int kVOff = kKOff + kSlots * kTileBytes;
-    static constexpr int kCtrlOff = kVOff + kSlots * kTileBytes;
-    static constexpr int kSmemBytes = kCtrlOff + (int)sizeof(Control) + 1024;   // + alignment slack
+    static constexpr int kSmemBytes = kVOff + kSlots * kTileBytes + 1024;   // + alignment slack
 };
 
 __device__ __forceinline__ void wait_quiet(uint64_t* bar, uint32_t parity) {
     const long long t0 = clock64();
+#pragma unroll 1
     while (!mbar_try_wait(bar, parity))
         if (clock64() - t0 > 200000000LL) break;
 }
-
-// Bounded wait with nothing but a counter to keep in registers: gives up after 2^22 suspended tries (seconds),
-// or when another CTA has.
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int32_t* status, int code) {
-    if (mbar_test_wait(bar, parity)) return true;
+// Bounded wait of few instructions: gives up after 2^22 suspended tries (seconds).
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int32_t* gave_up, int code) {
     uint32_t polls = 0;
-    while (!mbar_try_wait(bar, parity)) {
-        if ((++polls & 0x3ffu) == 0) {
-            if (*(volatile int32_t*)status != 0) return false;
-            if (polls >= (1u << 22)) {
-                atomicCAS(status, 0, code);
-                return false;
-            }
+#pragma unroll 1
+    while (!mbar_try_wait(bar, parity))
+        if (++polls == (1u << 22)) {
+            *gave_up = code;
+            return false;
         }
-    }
     return true;
 }
 
 // O of the warp's rows (n pieces of 16 columns) times corr.  Rare, and kept out of the main loop.
-__device__ __noinline__ void rescale_o(uint32_t o_addr, int n, float corr) {
+__device__ __forceinline__ void rescale_o(uint32_t o_addr, int n, float corr) {
     uint32_t v[16];
+#pragma unroll 1
     for (int i = 0; i < n; ++i) {
         tmem_ld16(o_addr + i * 16, v);
         tmem_ld_wait();
@@ -222,8 +222,9 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     constexpr bool kOwnP = D == 64;              // P has tensor-memory columns of its own
     constexpr uint32_t kPCol = kOwnP ? kTile + D : 0;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    Control* ctrl = reinterpret_cast<Control*>(smem + L::kCtrlOff);
+    uint8_t* smem = smem_raw + (((smem_u32(smem_raw) + 1023) & ~1023u) - smem_u32(smem_raw));
+    __shared__ Control ctrl_mem;             // (static: constant addresses)
+    Control* const ctrl = &ctrl_mem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int real_res = blockIdx.y, res = p.cls.in_part(real_res), rows_v = p.cls.rows_of(real_res);
     const CUtensorMap* map = maps.part[p.cls.part(real_res)];       // Q, K, V, O
@@ -237,7 +238,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     int klo = 0;                       // first 128-key step
     auto load_k = [&]() {
         const int st = jk % kSlots, row = (klo + jk) * kTile;
-        if (jk >= kSlots && !wait_bar(&ctrl->k_free[st], ((uint32_t)(jk / kSlots) & 1u) ^ 1u, p.status, kErrKFree)) return false;
+        if (jk >= kSlots && !wait_bar(&ctrl->k_free[st], ((uint32_t)(jk / kSlots) & 1u) ^ 1u, &ctrl->gave_up, kErrKFree)) return false;
         mbar_arrive_expect_tx(&ctrl->k_full[st], L::kTileBytes);
         uint8_t* dst = smem + L::kKOff + st * L::kTileBytes;
         if (p.kt_major) {
@@ -252,7 +253,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     };
     auto load_v = [&]() {
         const int st = jv % kSlots;
-        if (jv >= kSlots && !wait_bar(&ctrl->v_free[st], ((uint32_t)(jv / kSlots) & 1u) ^ 1u, p.status, kErrVFree)) return false;
+        if (jv >= kSlots && !wait_bar(&ctrl->v_free[st], ((uint32_t)(jv / kSlots) & 1u) ^ 1u, &ctrl->gave_up, kErrVFree)) return false;
         mbar_arrive_expect_tx(&ctrl->v_full[st], L::kTileBytes);
         for (int sub = 0; sub < L::kSub; ++sub)
             tma_load_4d(smem + L::kVOff + st * L::kTileBytes + sub * kSubBytes, map + 2, &ctrl->v_full[st], sub * 64, res,
@@ -287,6 +288,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
             if (p.tiles != nullptr) range = __ldg(p.tiles + real_res * p.cls.tile_pitch + blockIdx.x);
             const int32_t stop = entry_status(p.status, p.mirror);
             ctrl->abort_at_entry = stop;
+            ctrl->gave_up = 0;
             if (stop == 0) {
                 mbar_arrive_expect_tx(&ctrl->q_full, L::kTileBytes);
                 for (int sub = 0; sub < L::kSub; ++sub)
@@ -339,10 +341,14 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     klo = lo64 >> 1;
     const int steps = ((hi64 + 1) >> 1) - klo;   // 128-key steps
     auto wait_all = [&](uint64_t* bar, uint32_t parity, int code) {
-        // (a uniform branch around the polling loop: 60 cycles when ready, 130 with a divergent one)
-        if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
-        const bool r = wait_bar(bar, parity, p.status, code);
-        return __all_sync(0xffffffffu, r) != 0;
+        uint32_t polls = 0;
+#pragma unroll 1
+        while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
+            if (++polls == (1u << 22)) {
+                ctrl->gave_up = code;
+                return false;
+            }
+        return true;
     };
 
     if (warp == kTmaWarp) {
@@ -376,7 +382,10 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
             const uint32_t idesc_qk = instr_desc_f16(fmt, kTile, kTile, p.kt_major ? 1u : 0u);
             const uint32_t idesc_qk_half = instr_desc_f16(fmt, kTile, 64, p.kt_major ? 1u : 0u);
             constexpr uint32_t idesc_pv = instr_desc_f16(fmt, kTile, D, 1);
-            const uint32_t q_base = smem_u32(smem), k_base = smem_u32(smem + L::kKOff), v_base = smem_u32(smem + L::kVOff);
+            const uint64_t q_desc = smem_desc_sw128(smem_u32(smem), 16, 1024);
+            const uint64_t k_desc = smem_desc_sw128(smem_u32(smem + L::kKOff), p.kt_major ? D * 128 : 16, 1024);
+            const uint64_t v_desc = smem_desc_sw128(smem_u32(smem + L::kVOff), kSubBytes, 1024);
+            const uint32_t k_step = (p.kt_major ? 2048 : 32) >> 4, k_sub = (p.kt_major ? 4 * 2048 : kSubBytes) >> 4;
             const uint32_t o_tmem = tmem_base + kTile;
             auto commit = [&](uint64_t* bar) { if (lead) mma_commit(bar); };
             auto in_range = [&](int j, int half) { const int i = 2 * (klo + j) + half; return i >= lo64 && i < hi64; };
@@ -390,17 +399,17 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
                 const bool h0 = in_range(j, 0), both = h0 && in_range(j, 1);
                 const uint32_t idesc = both ? idesc_qk : idesc_qk_half;
                 const uint32_t skip = h0 ? 0u : 1u;
-                const uint32_t b_base = k_base + st * L::kTileBytes + skip * (p.kt_major ? D * 128 : 64 * 128);
+                const uint32_t b_base = st * L::kTileBytes + skip * (p.kt_major ? D * 128 : 64 * 128);
+                if (lead) {
+                    uint64_t da = q_desc, db = k_desc + (b_base >> 4);
+#pragma unroll 1
+                    for (int sub = 0; sub < L::kSub; ++sub, da += kSubBytes >> 4, db += k_sub)
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t off = (kk >> 2) * kSubBytes + (kk & 3) * 32;
-                    const uint64_t da = smem_desc_sw128(q_base + off, 16, 1024);
-                    const uint64_t db = p.kt_major ? smem_desc_sw128(b_base + kk * 2048, D * 128, 1024)
-                                                   : smem_desc_sw128(b_base + off, 16, 1024);
-                    if (lead) mma_ss(tmem_base + skip * 64, da, db, idesc, kk > 0);
+                        for (int kk = 0; kk < 4; ++kk) mma_ss(tmem_base + skip * 64, da + kk * 2, db + kk * k_step, idesc, sub + kk > 0);
+                    mma_commit(&ctrl->s_full);
+                    mma_commit(&ctrl->k_free[st]);
                 }
-                commit(&ctrl->s_full);
-                commit(&ctrl->k_free[st]);
+                __syncwarp();
             };
             if (ok) issue_s(0);
             for (int j = 0; j < steps && ok; ++j) {
@@ -412,17 +421,19 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
                 const int st = j % kSlots;
                 ok = wait_all(&ctrl->v_full[st], (uint32_t)(j / kSlots) & 1u, kErrVFull);
                 if (!ok) break;
-#pragma unroll
+#pragma unroll 1
                 for (int half = 0; half < 2; ++half) {
                     ok = wait_all(&ctrl->p_full[half], (uint32_t)j & 1u, kErrP);
                     if (!ok) break;
                     tc_fence_after_sync();
                     if (in_range(j, half)) {
+                        if (lead) {
+                            const uint64_t db = v_desc + (uint32_t)((st * L::kTileBytes >> 4) + half * 512);
 #pragma unroll
-                        for (int kk = half * 4; kk < half * 4 + 4; ++kk) {
-                            const uint64_t db = smem_desc_sw128(v_base + st * L::kTileBytes + kk * 2048, kSubBytes, 1024);
-                            if (lead) mma_ts(o_tmem, tmem_base + kPCol + kk * 8, db, idesc_pv, (!first_pv || (kk & 3) > 0) ? 1u : 0u);
+                            for (int kk = 0; kk < 4; ++kk)
+                                mma_ts(o_tmem, tmem_base + kPCol + half * 32 + kk * 8, db + kk * 128, idesc_pv, (!first_pv || kk > 0) ? 1u : 0u);
                         }
+                        __syncwarp();
                         first_pv = false;
                     }
                 }
@@ -604,6 +615,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     }
     tc_fence_before_sync();
     __syncthreads();
+    if (threadIdx.x == 0 && ctrl->gave_up != 0) atomicCAS(p.status, 0, ctrl->gave_up);
     if (warp == kMmaWarp) {
         __syncwarp();
         tc_fence_after_sync();
