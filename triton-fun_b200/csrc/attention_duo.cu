@@ -59,7 +59,7 @@ constexpr int kSubBytes = kTile * 128;   // one 64-element (128-byte) column chu
 constexpr int kTileBytes = kSub * kSubBytes;
 constexpr int kTmaWarp = 8;
 constexpr int kQkWarp = 9;
-constexpr int kPvWarp = 10;
+// (warp 10: PV)
 constexpr int kPlanWarp = 11;
 constexpr int kThreads = 384;
 constexpr int kSoftmaxRegs = 208, kOtherRegs = 88;   // 2 x 208 + 88 = 3 x 168, the registers of the launch
