@@ -304,10 +304,11 @@ int32_t splat_spmm_band_table(const void* p, const void* v, void* o, const float
  * copying or synchronising anything on the normal path.  NULL host_copy removes the pair; at most 64. */
 int32_t splat_set_status_mirror(int32_t* status_word, int32_t* host_copy);
 
-/* Self-test of the bounded device-side wait used by the tensor-core kernels: one CTA waits on an
- * mbarrier that nothing arrives on, gives up after limit_cycles SM clocks (1 .. 2e9), stores code
- * 99 in *status_word (device int32, cleared by the caller) and ends normally; the context stays
- * usable.  No counterpart in the reference. */
+/* Self-test of the bounded device-side waits used by the tensor-core kernels: one warp waits on an
+ * mbarrier that nothing arrives on, with each of the three forms in turn; each gives up after about
+ * limit_cycles SM clocks (1 .. 2e9).  It stores code 99 in *status_word (device int32, cleared by the
+ * caller; a value that is there stays) and ends normally; the context stays usable.  No counterpart in the
+ * reference. */
 int32_t splat_selftest_bounded_wait(int32_t* status_word, int64_t limit_cycles, void* stream);
 
 /* Checked-index mode of the CUDA-core kernels (splat_sddmm, splat_spmm and the CUDA-core path of

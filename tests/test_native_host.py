@@ -131,3 +131,13 @@ def test_extension_of_another_torch_is_rebuilt(monkeypatch, tmp_path):
     assert len(commands) == 1
     build.build_host()
     assert len(commands) == 1
+
+
+def test_kernels_wait_through_the_tested_functions_only():
+    """The bounded waits that splat_selftest_bounded_wait makes run out are the ones in tc_ptx.cuh: no kernel polls a barrier
+    in a loop of its own."""
+    csrc = os.path.join(ROOT, "triton-fun_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        if name != "tc_ptx.cuh":
+            with open(os.path.join(csrc, name)) as f:
+                assert "mbar_try_wait" not in f.read(), name

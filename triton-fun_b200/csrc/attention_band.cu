@@ -144,13 +144,6 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Wait that ignores the status word (used only while leaving after an error).
-__device__ __forceinline__ void mbar_wait_quiet(uint64_t* bar, uint32_t parity) {
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > 200000000LL) break;
-}
-
 // Natural-log log-sum-exp of a row: from the running maximum and sum of a band row (log2 domain), the
 // one score scale * q_i . k_start of a row with a single non-zero (computed here from the raw
 // operands; such rows are outside the band), -inf for a row without non-zeros.
@@ -306,9 +299,9 @@ attention_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             }
             if (!ok) {
                 // leave only after the copies already issued have landed
-                mbar_wait_quiet(&ctrl->q_full, 0);
+                wait_quiet(&ctrl->q_full, 0);
                 for (int i = max(0, item - kStages); i < item; ++i)
-                    mbar_wait_quiet(&ctrl->kv_full[i % kStages], (uint32_t)(i / kStages) & 1u);
+                    wait_quiet(&ctrl->kv_full[i % kStages], (uint32_t)(i / kStages) & 1u);
             }
         }
     } else if (warp == kMmaWarp || warp == kMmaWarp + 1) {
@@ -428,7 +421,7 @@ attention_band_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             if (!ok) {
                 // let the tensor pipe drain before tensor memory is released
                 commit(&ctrl->drain[x]);
-                mbar_wait_quiet(&ctrl->drain[x], 0);
+                wait_quiet(&ctrl->drain[x], 0);
             }
             __syncwarp();
         }

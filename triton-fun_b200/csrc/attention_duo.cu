@@ -70,6 +70,7 @@ constexpr int kItems = 2;                // items known ahead
 constexpr int kItemReaders = 8 + 2 + 1;  // softmax warps, the QK warp once per pipe, the TMA thread
 constexpr int kOrders = 8;               // S issued whose PV has not been: never more than three per pipe, and the end
 constexpr float kRescaleThreshold = 8.0f;   // log2 domain: P stays below 2^8 between rescales
+constexpr uint32_t kIdlePolls = 1u << 22;   // of the QK warp without an S to issue: less than a second
 
 // shared memory
 constexpr int kKOff = 2 * kTileBytes;            // behind the Q tiles
@@ -145,37 +146,9 @@ struct Control {
 };
 static_assert(kSmemBytes + sizeof(Control) <= 232448, "shared memory of a CTA");
 
-__device__ __forceinline__ void wait_quiet(uint64_t* bar, uint32_t parity) {
-    const long long t0 = clock64();
-#pragma unroll 1
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > 200000000LL) break;
-}
-// Bounded waits of few instructions: they give up after 2^22 suspended tries (seconds).
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int32_t* gave_up, int code) {
-    uint32_t polls = 0;
-#pragma unroll 1
-    while (!mbar_try_wait(bar, parity))
-        if (++polls == (1u << 22)) {
-            *gave_up = code;
-            return false;
-        }
-    return true;
-}
 __device__ __forceinline__ bool test_all(uint64_t* bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) != 0;
 }
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int32_t* gave_up, int code) {
-    uint32_t polls = 0;
-#pragma unroll 1
-    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
-        if (++polls == (1u << 22)) {
-            *gave_up = code;
-            return false;
-        }
-    return true;
-}
-
 // O of the warp's rows times corr.
 __device__ __forceinline__ void rescale_o(uint32_t o_addr, float corr) {
     uint32_t v[16];
@@ -500,7 +473,7 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                     polls = 0;
                 } else if (me.done && other.done) {
                     break;
-                } else if (++polls == (1u << 24)) {
+                } else if (++polls == kIdlePolls) {
                     ctrl->gave_up = kErrIdle;
                     break;
                 } else {
@@ -738,7 +711,7 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (threadIdx.x == 0 && ctrl->gave_up != 0) atomicCAS(p.status, 0, ctrl->gave_up);
+    if (threadIdx.x == 0) publish_gave_up(p.status, &ctrl->gave_up);
     if (warp == kQkWarp) {
         __syncwarp();
         tc_fence_after_sync();

@@ -549,9 +549,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             if (!ok && lead) {
                 // let the tensor pipe drain before tensor memory is released
                 mma_commit_pair(smem_u32(&ctrl->drain));
-                const long long t0 = clock64();
-                while (!mbar_try_wait(&ctrl->drain, 0))
-                    if (clock64() - t0 > 200000000LL) break;
+                wait_quiet(&ctrl->drain, 0);
             }
             __syncwarp();
         }

@@ -112,24 +112,6 @@ template <int D> struct Layout {
     static constexpr int kSmemBytes = kVOff + kSlots * kTileBytes + 1024;   // + alignment slack
 };
 
-__device__ __forceinline__ void wait_quiet(uint64_t* bar, uint32_t parity) {
-    const long long t0 = clock64();
-#pragma unroll 1
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > 200000000LL) break;
-}
-// Bounded wait of few instructions: gives up after 2^22 suspended tries (seconds).
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int32_t* gave_up, int code) {
-    uint32_t polls = 0;
-#pragma unroll 1
-    while (!mbar_try_wait(bar, parity))
-        if (++polls == (1u << 22)) {
-            *gave_up = code;
-            return false;
-        }
-    return true;
-}
-
 // O of the warp's rows (n pieces of 16 columns) times corr.  Rare, and kept out of the main loop.
 __device__ __forceinline__ void rescale_o(uint32_t o_addr, int n, float corr) {
     uint32_t v[16];
@@ -340,16 +322,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     hi64 = (hi64 + 63) / 64;
     klo = lo64 >> 1;
     const int steps = ((hi64 + 1) >> 1) - klo;   // 128-key steps
-    auto wait_all = [&](uint64_t* bar, uint32_t parity, int code) {
-        uint32_t polls = 0;
-#pragma unroll 1
-        while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
-            if (++polls == (1u << 22)) {
-                ctrl->gave_up = code;
-                return false;
-            }
-        return true;
-    };
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, int code) { return tc::wait_all(bar, parity, &ctrl->gave_up, code); };
 
     if (warp == kTmaWarp) {
         // ------------------------------------------------------------------ TMA producer
@@ -615,7 +588,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (threadIdx.x == 0 && ctrl->gave_up != 0) atomicCAS(p.status, 0, ctrl->gave_up);
+    if (threadIdx.x == 0) publish_gave_up(p.status, &ctrl->gave_up);
     if (warp == kMmaWarp) {
         __syncwarp();
         tc_fence_after_sync();

@@ -24,23 +24,34 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
 }  // namespace splat
 
 namespace splat {
-// One CTA waits, with the same bounded wait the band kernels use, on an mbarrier that nothing ever
-// arrives on.  The wait must give up after limit_cycles, record the code and let the kernel end.
-__global__ void bounded_wait_selftest_kernel(int32_t* status_word, long long limit_cycles) {
+// One warp waits on an mbarrier that nothing ever arrives on, with each of the bounded waits of the tensor-core kernels
+// in turn: each must give up, leave its code, and the code must arrive in the status word the way the kernels pass it on.
+constexpr int kSelftestCode = 99;
+__global__ void bounded_wait_selftest_kernel(int32_t* status_word, uint32_t tries, long long limit_cycles) {
     __shared__ uint64_t bar;
+    __shared__ int32_t gave_up, word;
     if (threadIdx.x == 0) {
         tc::mbar_init(&bar, 1);
         tc::mbar_fence_init();
+        gave_up = word = 0;
     }
     __syncthreads();
-    const bool ok = tc::mbar_wait(&bar, 0, status_word, 99, limit_cycles);
-    if (ok) atomicExch(status_word, -1);   // cannot happen: nobody arrives
+    bool ok = tc::wait_all(&bar, 0, &gave_up, kSelftestCode + 1, tries);       // cannot pass: nobody arrives
+    __syncwarp();
+    if (threadIdx.x == 0) {
+        ok = gave_up != kSelftestCode + 1 || ok;
+        ok = tc::wait_bar(&bar, 0, &gave_up, kSelftestCode, tries) || ok;
+        ok = tc::mbar_wait(&bar, 0, &word, kSelftestCode, limit_cycles) || word != kSelftestCode || ok;
+        if (ok) gave_up = -1;
+        tc::publish_gave_up(status_word, &gave_up);
+    }
 }
 }  // namespace splat
 
 extern "C" int32_t splat_selftest_bounded_wait(int32_t* status_word, int64_t limit_cycles, void* stream) {
-    if (!status_word || limit_cycles < 1 || limit_cycles > 2000000000LL) return SPLAT_ERR_BAD_ARG;
-    splat::bounded_wait_selftest_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(status_word, limit_cycles);
+    if (!status_word || limit_cycles < 1 || limit_cycles > splat::tc::kTimeoutCycles) return SPLAT_ERR_BAD_ARG;
+    const int64_t tries = (limit_cycles * splat::tc::kWaitTries + splat::tc::kTimeoutCycles - 1) / splat::tc::kTimeoutCycles;
+    splat::bounded_wait_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(status_word, (uint32_t)tries, limit_cycles);
     return splat::launch_status();
 }
 

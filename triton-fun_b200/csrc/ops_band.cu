@@ -74,36 +74,6 @@ struct Params {
     int kt_major;        // sddmm: K is a contiguous (BH, d, L) array (keys innermost), stride 1 only
 };
 
-// (Waits of few instructions: what these kernels are bound by is instructions: SDDMM at d = 128 70.1 -> 66.2 us,
-// SpMM 70.1 -> 68.7, B4 H16 L4096 window 256, with these and the control block at constant addresses.)
-__device__ __forceinline__ void wait_quiet(uint64_t* bar, uint32_t parity) {
-    const long long t0 = clock64();
-#pragma unroll 1
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > 200000000LL) break;
-}
-// They give up after 2^22 suspended tries (seconds).
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int32_t* gave_up, int code) {
-    uint32_t polls = 0;
-#pragma unroll 1
-    while (!mbar_try_wait(bar, parity))
-        if (++polls == (1u << 22)) {
-            *gave_up = code;
-            return false;
-        }
-    return true;
-}
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int32_t* gave_up, int code) {
-    uint32_t polls = 0;
-#pragma unroll 1
-    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
-        if (++polls == (1u << 22)) {
-            *gave_up = code;
-            return false;
-        }
-    return true;
-}
-
 template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<__half>(__half v) { return __half2float(v); }
 template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
@@ -438,7 +408,7 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (threadIdx.x == 0 && ctrl->gave_up != 0) atomicCAS(p.status, 0, ctrl->gave_up);
+    if (threadIdx.x == 0) publish_gave_up(p.status, &ctrl->gave_up);
     if (warp == kMmaWarp) {
         __syncwarp();
         tc_fence_after_sync();
@@ -737,7 +707,7 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (threadIdx.x == 0 && ctrl->gave_up != 0) atomicCAS(p.status, 0, ctrl->gave_up);
+    if (threadIdx.x == 0) publish_gave_up(p.status, &ctrl->gave_up);
     if (warp == kMmaWarp) {
         __syncwarp();
         tc_fence_after_sync();

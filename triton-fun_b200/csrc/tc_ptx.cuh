@@ -2,8 +2,8 @@
 // loads, tcgen05 (tensor memory allocation, MMA, commit, ld/st, fences) and the shared-memory /
 // instruction descriptors that tcgen05.mma consumes.
 //
-// All waits are bounded (see BoundedWait): a kernel that gives up records a code in a status word
-// and leaves through its normal exit path, so the context stays usable.
+// All waits are bounded (wait_bar, wait_all, mbar_wait): a kernel that gives up records a code in a status
+// word and leaves through its normal exit path, so the context stays usable.
 #pragma once
 
 #include <cuda.h>
@@ -66,10 +66,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Bounded wait on an mbarrier phase.  Gives up after ~kTimeoutCycles SM clocks, or as soon as the
-// global status word is seen non-zero (another CTA already gave up), and then reports false.
-constexpr long long kTimeoutCycles = 2000000000LL;  // about one second
-
 // non-blocking test of a phase (no suspend window: cheapest when the phase has usually completed)
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
@@ -85,6 +81,48 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+// Bounded waits on an mbarrier phase, by one thread (wait_bar) or by a whole warp on uniform values (wait_all).  They give up
+// after `tries` suspended tries, leave their code in the CTA's `gave_up` and report false; the kernel passes the code on
+// when its warps have met again (publish_gave_up).  A try and a counter, because these loops are in every role of the
+// kernels and a problem of their code cache: with a look at the status word every 1024 tries, so that a CTA stops within
+// 2 ms of another's giving up instead of by its own limit, window 1024 of B8 H64 L32768 d128 took 10.40 ms (10.04),
+// dilated 207 us (203), with an atomic for the first code instead of the last 10.22 ms and 206 us.
+constexpr uint32_t kWaitTries = 1u << 18;           // about one second (a try of 2 us takes 4, measured)
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int32_t* gave_up, int code, uint32_t tries = kWaitTries) {
+    uint32_t polls = 0;
+#pragma unroll 1
+    while (!mbar_try_wait(bar, parity))
+        if (++polls >= tries) {
+            *gave_up = code;
+            return false;
+        }
+    return true;
+}
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int32_t* gave_up, int code, uint32_t tries = kWaitTries) {
+    uint32_t polls = 0;
+#pragma unroll 1
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
+        if (++polls >= tries) {
+            *gave_up = code;
+            return false;
+        }
+    return true;
+}
+// After the block's last barrier, one thread.
+__device__ __forceinline__ void publish_gave_up(int32_t* status, const int32_t* gave_up) {
+    if (*gave_up != 0) atomicCAS(status, 0, *gave_up);
+}
+// A wait without a report: for copies and MMAs in flight when a kernel leaves.
+__device__ __forceinline__ void wait_quiet(uint64_t* bar, uint32_t parity) {
+    const long long t0 = clock64();
+#pragma unroll 1
+    while (!mbar_try_wait(bar, parity))
+        if (clock64() - t0 > 200000000LL) break;
+}
+
+// The wait of the opt-in kernels (attention_band.cu, attention_pair.cu): gives up after ~kTimeoutCycles SM clocks or when
+// the status word is seen non-zero, and writes the status word itself.
+constexpr long long kTimeoutCycles = 2000000000LL;  // about one second
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
                                           volatile int32_t* status_word, int code,
                                           long long limit_cycles = kTimeoutCycles) {
