@@ -1,5 +1,5 @@
-"""GPU: the bounded waits of the tensor-core kernels and what a set status word does to a launch.
-Nothing here hangs or faults: the one wait that runs out has a short limit."""
+"""GPU: the bounded waits of the tensor-core kernels and what a set status word does -- to a launch, and to a persistent
+kernel that is already running.  Nothing here hangs or faults: the one wait that runs out has a short limit."""
 import time
 
 import pytest
@@ -63,3 +63,42 @@ def test_launches_do_nothing_while_the_status_word_is_set():
         launch(out)
         n.check_status_word(0)
         assert torch.isfinite(out.float()).all(), name
+
+
+def test_running_kernel_stops_when_the_status_word_is_set():
+    """A CTA that has not begun when another gives up does no work; a persistent CTA that is running takes no more tiles."""
+    import acsr_helpers as ah
+    import splat_native as n
+    H, L, d = 256, 32768, 128                            # some 5 ms
+    acsr = ah.create_acsr(ah.create_causal_windowed_mask(L, 1023), 16, 0)
+    q = torch.randn(1, 1, L, d, device="cuda").to(torch.bfloat16).expand(1, H, L, d).contiguous()
+    out = torch.empty_like(q)
+    word, five, side = n.status_word(torch.device("cuda", 0)), torch.full((1,), 5, dtype=torch.int32).pin_memory(), torch.cuda.Stream()
+
+    def launch():
+        n.attention_fused(q, q.transpose(2, 3), q, out, acsr[2], acsr[3], acsr[4], d ** -0.5, n.PATH_BAND)
+
+    launch()
+    n.check_status_word(0)
+    for _ in range(5):
+        out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        launch()
+        done = torch.cuda.Event()
+        done.record()
+        until = time.perf_counter() + 1e-3
+        while time.perf_counter() < until:
+            pass
+        with torch.cuda.stream(side):                    # (by a copy engine: the SMs are full)
+            word.copy_(five, non_blocking=True)
+        side.synchronize()
+        in_time = not done.query()
+        torch.cuda.synchronize()
+        first, last = torch.isfinite(out[0, 0].float()).all().item(), torch.isfinite(out[0, -1].float()).all().item()
+        with pytest.raises(RuntimeError):
+            n.check_status_word(0)
+        if in_time:
+            break
+    else:
+        pytest.skip("the word was never set while the kernel ran")
+    assert first and not last

@@ -282,6 +282,8 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
             for (int n = 0;; ++n) {
                 const int slot = n % kItems;
                 if (n >= kItems && !wait_all(&ctrl->item_free[slot], ((uint32_t)(n / kItems) & 1u) ^ 1u, &ctrl->gave_up, kErrItemFree)) break;
+                // (once a CTA has given up no other is taken over, as none that starts then does anything)
+                if (n > 0 && __any_sync(0xffffffffu, *(const volatile int32_t*)p.status != 0)) next = -1;
                 if (next >= 0) {
 #pragma unroll 1
                     for (int x = 0; x < 2; ++x) {
