@@ -302,7 +302,10 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                     clc_request(&ctrl->clc, &ctrl->clc_full);
                 }
                 __syncwarp();
-                if (!wait_all(&ctrl->clc_full, (uint32_t)n & 1u, &ctrl->gave_up, kErrClc)) break;
+                if (!wait_all(&ctrl->clc_full, (uint32_t)n & 1u, &ctrl->gave_up, kErrClc)) {
+                    wait_quiet(&ctrl->clc_full, (uint32_t)n & 1u);     // leave only after the answer has been written
+                    break;
+                }
                 next = clc_answer(&ctrl->clc);
                 fence_proxy_async_smem();      // read before the next answer is written
                 __syncwarp();
