@@ -440,7 +440,10 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                     // (entry e - kSlots has been issued in both pipes: its phase of the slot's barrier is not mistaken for e's)
                     go = e - kSlots < other.next && (k > 0 || test_all(&ctrl->q_full[x], (uint32_t)me.tiles & 1u)) &&
                          test_all(&ctrl->k_full[st], (uint32_t)(e / kSlots) & 1u);
-                    if (go && last_x == x) go = test_all(&ctrl->p_full[x][0], (uint32_t)(me.scores - 1) & 1u);
+                    // (s_free first: once the last S, this pipe's, has been read, p_full can be no more than one phase behind, and its
+                    // parity tells which)
+                    if (go && last_x == x)
+                        go = test_all(&ctrl->s_free, (uint32_t)(issued - 1) & 1u) && test_all(&ctrl->p_full[x][0], (uint32_t)(me.scores - 1) & 1u);
                 }
                 if (go) {
                     const int block = (me.lo >> 1) + me.k;
