@@ -1,6 +1,7 @@
 """GPU: the persistent two-tile kernel of d = 128, which takes over at 592 to 1184 tiles of 128 rows.  It multiplies and sums in the
-order of the kernel with a tile per CTA, so the two agree bit for bit (and so do shards of a problem on either side of the
-line); the first and last head are also compared with the CPU oracle."""
+order of the kernel with a tile per CTA, so the results of the two agree bit for bit (and so do shards of a problem on either
+side of the line; the log-sum-exp of a row with one non-zero is summed in another order); the first and last head are
+also compared with the CPU oracle."""
 import pytest
 import torch
 
@@ -26,8 +27,37 @@ PATTERNS = [
 ]
 
 
+# Too small for the kernel to be chosen: forced.
+SMALL = [
+    (ao.PATTERN_CAUSAL_WINDOWED, 128, 127, 0, 1),      # one tile
+    (ao.PATTERN_CAUSAL_WINDOWED, 64, 9, 0, 1),         # half a tile
+    (ao.PATTERN_CAUSAL_WINDOWED, 256, 255, 0, 1),      # two, an item each
+    (ao.PATTERN_CAUSAL_WINDOWED, 120, 30, 0, 3),       # three, short
+    (ao.PATTERN_CAUSAL_WINDOWED, 384, 0, 0, 1),        # nothing to multiply
+    (ao.PATTERN_BLOCKED, 384, 128, 0, 1),
+    (ao.PATTERN_STRIDED, 384, 3, 0, 1),                # three classes of one tile
+    (ao.PATTERN_DILATED, 512, 100, 2, 1),
+    (ao.PATTERN_WINDOWED, 128, 50, 0, 149),            # the fewest tiles that go in pairs, of two heads; the last item has one
+    (ao.PATTERN_WINDOWED, 2048, 300, 0, 18),           # 288 tiles, 144 pairs: a wave, nothing to take over
+    (ao.PATTERN_WINDOWED, 2048, 300, 0, 19),           # 304: 148 pairs and 8 single tiles that are taken over
+]
+
+
+def test_where_it_does_not_apply_it_refuses(monkeypatch):
+    import acsr_helpers as ah
+    import splat_native as n
+    monkeypatch.setenv("SPLAT_B200_BAND_TILES", "4")
+    for d, kind, L, p0, p1 in ((64, ao.PATTERN_CAUSAL_WINDOWED, 256, 31, 0), (128, ao.PATTERN_DILATED, 257, 30, 2)):
+        acsr = ah.create_acsr(ah.PatternMask(kind, L, p0, p1), 16, 0)
+        q = torch.randn(1, 1, L, d, device="cuda").to(torch.bfloat16)
+        out = torch.full_like(q, 5.0)
+        with pytest.raises(RuntimeError):
+            n.attention_fused(q, q.transpose(2, 3), q, out, acsr[2], acsr[3], acsr[4], 0.125, n.PATH_BAND)
+        assert (out == 5.0).all()
+
+
 @pytest.mark.parametrize("contiguous,dtype", [(False, torch.bfloat16), (True, torch.bfloat16), (False, torch.float16)])
-@pytest.mark.parametrize("kind,L,p0,p1,H", PATTERNS)
+@pytest.mark.parametrize("kind,L,p0,p1,H", PATTERNS + SMALL)
 def test_duo_patterns(kind, L, p0, p1, H, contiguous, dtype, monkeypatch):
     import acsr_helpers as ah
     import splat_native as n
@@ -46,7 +76,14 @@ def test_duo_patterns(kind, L, p0, p1, H, contiguous, dtype, monkeypatch):
         n.check_status_word(0)
         return out
 
-    monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
+    stride = {ao.PATTERN_STRIDED: p0, ao.PATTERN_DILATED: p1}.get(kind, 1)
+    if (kind, L, p0, p1, H) in SMALL:
+        monkeypatch.setenv("SPLAT_B200_BAND_TILES", "4")
+    else:
+        monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
+        n.classify(acsr[2], acsr[3], acsr[4])
+        assert n.band_table(acsr[2], acsr[3], acsr[4], L) is not None
+        assert n._lib.splat_band_kernel_choice(H, L, d, stride, 1) == 4, "this kernel is not the one that runs"
     lse, lse_one = (torch.full((1, H, L), float("nan"), device="cuda") for _ in range(2))
     out, plain = run(lse), run(None)
     monkeypatch.setenv("SPLAT_B200_BAND_TILES", "1")
@@ -55,7 +92,7 @@ def test_duo_patterns(kind, L, p0, p1, H, contiguous, dtype, monkeypatch):
     assert torch.equal(out, one)
     assert (lse - lse_one).abs().max().item() < 1e-5      # (a single row's score: sums in another order)
     meta = ao.metadata_from_pattern(kind, L, p0, p1, 16)
-    ends = [0, H - 1]
+    ends = sorted({0, H - 1})
     qc, kc, vc = (t[:, ends].cpu() for t in (q, k, v))
     assert_close(out[:, ends], at.attention_acsr(qc, kc.transpose(2, 3), vc, meta, meta["trailing_dim"], scale), dtype)
 
@@ -74,6 +111,7 @@ def test_duo_unscaled_scores_need_the_running_max(monkeypatch):
             monkeypatch.setenv("SPLAT_B200_BAND_TILES", variant)
         else:
             monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
+            assert n._lib.splat_band_kernel_choice(B * H, L, d, 1, 1) == 4
         outs.append(torch.full_like(q, float("nan")))
         n.attention_fused(q, k.transpose(2, 3), v, outs[-1], acsr[2], acsr[3], acsr[4], 1.0, n.PATH_BAND)
         n.check_status_word(0)

@@ -141,3 +141,24 @@ def test_kernels_wait_through_the_tested_functions_only():
         if name != "tc_ptx.cuh":
             with open(os.path.join(csrc, name)) as f:
                 assert "mbar_try_wait" not in f.read(), name
+
+
+def test_choice_of_the_fused_band_kernel(monkeypatch):
+    import splat_native as n
+    choice = n._lib.splat_band_kernel_choice
+    monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
+    assert choice(64, 2048, 128, 1, 1) == 1                       # 1024 tiles: the last wave of 296 is less than half full
+    assert choice(70, 2048, 128, 1, 1) == 4                       # 1120
+    assert choice(512, 32768, 128, 1, 1) == 4
+    assert choice(512, 32768, 128, 1, 0) == 1                     # without a band table
+    assert choice(512, 32768, 64, 1, 1) == 1
+    assert choice(512, 32767, 128, 2, 1) == 1                     # classes of unequal length
+    assert choice(65535, 2147483647, 128, 1, 1) == 1              # more tiles than a grid has
+    assert choice(1, 128, 128, 1, 1) == 1
+    assert choice(0, 128, 128, 1, 1) < 0
+    for forced, d, stride, expected in (("4", 128, 1, 4), ("4", 64, 1, -6), ("4", 128, 3, -6), ("1", 128, 1, 1), ("2", 128, 1, 2),
+                                        ("3", 128, 1, 3), ("3", 64, 1, 2), ("2", 32, 1, 1), ("2", 128, 3, 1), ("7", 128, 1, 1)):
+        monkeypatch.setenv("SPLAT_B200_BAND_TILES", forced)
+        assert choice(1, 256, d, stride, 1) == expected, (forced, d, stride)
+    monkeypatch.setenv("SPLAT_B200_BAND_TILES", "4")
+    assert choice(1, 256, 128, 1, 0) == -6

@@ -65,6 +65,7 @@ SIGNATURES = {
     "splat_acsr_from_mask_u8": [_vp, _i64, _i64, _i64, _i32] + [_vp] * 9 + [_vp],
     "splat_transpose_16": [_vp, _vp, _i64, _i64, _i64, _vp],
     "splat_attention_host": [_vp] * 5 + [_i64] + [_vp] * 3 + [_i64] * 3 + [_f32, _i32, _i32] + [_vp] * 8,
+    "splat_band_kernel_choice": [_i64, _i64, _i64, _i64, _i32],
     "splat_band_table": [_vp, _vp, _vp, _i64, _i64, _vp, _vp],
     "splat_attention_fused_table": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64,
                                     _i64, _i64, _f32, _i32, _i32, _vp, _vp, _vp, _vp, _vp],

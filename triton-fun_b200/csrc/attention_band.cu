@@ -753,6 +753,29 @@ int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v,
                       int64_t stride, float scale, int32_t dtype, int32_t* status_word, const int32_t* band_table, float* lse,
                       cudaStream_t st);
 
+// Kernel of a band problem (see attention_band() for what one is).  1: one Q tile per CTA, two CTAs per SM (attention_wide.cu),
+// the only one that takes any d and classes of unequal length.  2: two Q tiles per CTA sharing every K/V tile (half the
+// L2 -> SM traffic), below.  3: persistent CTA pairs (attention_pair.cu), d = 128 only.  4: two tiles per persistent CTA
+// (attention_duo.cu), d = 128 and a band table only.  SPLAT_B200_BAND_TILES=1|2|3|4 selects; where 2 or 3 does not apply,
+// another runs, and where 4 does not, none.
+// Unset: 4 for enough tiles, else 1.  The persistent kernel takes
+// 0.83 to 0.95 of the time where the waves of two tiles per SM are many or the last one is half full at least; a few
+// tiles beyond two or three whole waves cost it a wave of its own (us, a CTA per tile / persistent: +-566 at 500 / 600 /
+// 700 / 800 / 900 / 1200 tiles 58.1 / 58.2, 63.7 / 69.3, 81.0 / 71.9, 85.2 / 75.1, 89.6 / 94.2, 116 / 110; +-60 at 640 / 720 /
+// 800 / 1040 / 1184 31.5 / 30.3, 34.2 / 36.0, 35.8 / 33.1, 45.2 / 41.2, 48.9 / 41.1).  At d = 64 it is no faster
+// (+-200, 1024 tiles 47 / 51).
+static int band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, int64_t stride, bool has_table) {
+    int forced = 0;
+    if (const char* e = getenv("SPLAT_B200_BAND_TILES"))
+        if (e[0] >= '1' && e[0] <= '4') forced = e[0] - '0';
+    const int64_t tiles = bh * stride * ((n_rows / stride + 127) / 128);
+    const bool duo_takes = d == 128 && n_rows % stride == 0 && has_table && tiles <= INT32_MAX;
+    if (forced == 4) return duo_takes ? 4 : SPLAT_ERR_UNSUPPORTED_SHAPE;
+    if ((d != 64 && d != 128) || n_rows % stride != 0) return 1;
+    if (forced == 0) return duo_takes && (tiles >= 8 * 148 || (tiles >= 4 * 148 && tiles % (2 * 148) >= 148)) ? 4 : 1;
+    return forced == 3 && d != 128 ? 2 : forced;
+}
+
 int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, int64_t ksk,
                        const void* v, void* o, const float* lin, const float* tr,
                        const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
@@ -781,28 +804,14 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
     if (!k_major && (stride != 1 || n_cols % 8 != 0)) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return SPLAT_ERR_MISALIGNED;
 
-    // Kernel choice.  1: one Q tile per CTA, two CTAs per SM (attention_wide.cu), the fastest on every
-    // shape tried and the only one that takes any d and classes of unequal length.  2: two Q tiles per CTA
-    // sharing every K/V tile (half the L2 -> SM traffic).  3: persistent CTA pairs (attention_pair.cu),
-    // d = 128 only.  SPLAT_B200_BAND_TILES=1|2|3 selects; SPLAT_B200_PAIR_MAX limits the resident pairs of 3.
-    // Unset: two tiles per persistent CTA (attention_duo.cu) for d = 128 and enough tiles, else 1.  The persistent kernel takes
-    // 0.83 to 0.95 of the time where the waves of two tiles per SM are many or the last one is half full at least; a few
-    // tiles beyond two or three whole waves cost it a wave of its own (us, a CTA per tile / persistent: +-566 at 500 / 600 /
-    // 700 / 800 / 900 / 1200 tiles 58.1 / 58.2, 63.7 / 69.3, 81.0 / 71.9, 85.2 / 75.1, 89.6 / 94.2, 116 / 110; +-60 at 640 / 720 /
-    // 800 / 1040 / 1184 31.5 / 30.3, 34.2 / 36.0, 35.8 / 33.1, 45.2 / 41.2, 48.9 / 41.1).  At d = 64 it is no faster
-    // (+-200, 1024 tiles 47 / 51).
-    int variant = 0;
-    if (const char* e = getenv("SPLAT_B200_BAND_TILES"))
-        if (e[0] >= '1' && e[0] <= '3') variant = e[0] - '0';
-    if ((d != 64 && d != 128) || n_rows % stride != 0) variant = 1;
-    const int64_t tiles = bh * stride * ((n_rows / stride + 127) / 128);
-    if (variant == 0 && d == 128 && band_table != nullptr && (tiles >= 8 * 148 || (tiles >= 4 * 148 && tiles % (2 * 148) >= 148)) &&
-        tiles <= INT32_MAX)
+    const int variant = band_kernel_choice(bh, n_rows, d, stride, band_table != nullptr);
+    if (variant < 0) return variant;
+    if (variant == 4)
         return attention_duo(q, k, kt_major ? 1 : 0, v, o, bh, n_rows, d, stride, scale, dtype, status_word, band_table, lse, st);
-    if (variant <= 1)
+    if (variant == 1)
         return attention_wide(q, k, kt_major ? 1 : 0, v, o, lin, tr, nnzs, bh, n_rows, d, stride, scale, dtype, status_word,
                               band_table, lse, st);
-    if (variant == 3 && d == 128) {
+    if (variant == 3) {
         int max_pairs = 0;
         if (const char* e = getenv("SPLAT_B200_PAIR_MAX")) max_pairs = atoi(e);
         const int32_t rc = attention_pair(q, k, kt_major ? 1 : 0, v, o, lin, tr, nnzs, bh, n_rows, stride,
@@ -830,6 +839,11 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
 }
 
 }  // namespace splat
+
+extern "C" int32_t splat_band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, int64_t stride, int32_t has_band_table) {
+    if (bh < 1 || n_rows < 1 || d < 1 || stride < 1 || bh > 65535 || n_rows > INT32_MAX || stride > 65535) return SPLAT_ERR_BAD_ARG;
+    return splat::band_kernel_choice(bh, n_rows, d, stride, has_band_table != 0);
+}
 
 #ifdef SPLAT_BAND_TRACE
 extern "C" void splat_debug_set_trace(void* device_buffer_4x1024_i64) {
