@@ -77,3 +77,23 @@ def test_tile_kernels_against_oracle(d, contiguous):
             assert rc == n.ERR_UNSUPPORTED_SHAPE
         else:
             assert rc == 0 and torch.equal(o2, tile), what
+
+
+@pytest.mark.parametrize("d", [32, 64])
+def test_sddmm_and_spmm_on_either_side_of_each_register_budget(d):
+    """CTAs of eight warps up to 148 and from there, of 32 and of 64 rows up to 470, to 614, to 888 and from there."""
+    import acsr_helpers as ah
+    import splat_native as n
+    for L, H in [(64, 74), (64, 75), (96, 156), (96, 157), (96, 204), (96, 205), (64, 470), (64, 471), (64, 614), (64, 615), (64, 888),
+                 (64, 889)]:
+        acsr = ah.create_acsr(ah.create_windowed_mask(L, 21), 16, 0)
+        meta = ao.metadata_from_pattern(ao.PATTERN_WINDOWED, L, 21, 0, 16)
+        T = acsr[5]
+        g = torch.Generator(device="cuda").manual_seed(L + H)
+        q, k, v = (torch.randn(1, H, L, d, device="cuda", generator=g) for _ in range(3))
+        s, o = torch.full((1, H, L, T), float("nan"), device="cuda"), torch.full_like(q, float("nan"))
+        n.sddmm(q, k.transpose(2, 3), s, acsr[2], acsr[3], acsr[4], T)
+        n.spmm(s, v, o, acsr[2], acsr[3], acsr[4], T)
+        assert_close(s, at.sddmm_acsr(q.cpu(), k.cpu().transpose(2, 3), meta, T), torch.float32, f"sddmm {L} {H}")
+        # sums of 43 products of normal values: 2^-24 of some 43 sqrt(d) each, well under the tolerance
+        assert_close(o / d ** 0.5, at.spmm_acsr(s.cpu(), v.cpu(), meta) / d ** 0.5, torch.float32, f"spmm {L} {H}")

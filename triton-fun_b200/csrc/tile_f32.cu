@@ -103,8 +103,10 @@ template <int D, int RW, int KW, Op OP> struct Layout {
     static constexpr int kPart = 32 * D + 64;           // a warp's partial result: O[32][D], maxima, sums
     static constexpr int kMain = kQ + kGroups * kGroupFloats;
     static constexpr int kFloats = OP == Op::kSddmm || kMain > kWarps * kPart ? kMain : kWarps * kPart;
-    static constexpr int kPerSm = KW == 8 ? (D == 128 || OP == Op::kFused ? 1 : 2) : (D == 128 ? 2 : 3);     // CTAs per SM the registers are budgeted for ...
-    static constexpr int kPerSmFull = D != 128 ? 4 : OP == Op::kSddmm ? 3 : 2;    // ... where there are more to run than kPerSm (SDDMM, SpMM)
+    // CTAs per SM the registers are budgeted for: usually, and where run() wants more.  (The same where a smaller budget
+    // changes nothing: D = 128 for lack of shared memory, SpMM at D = 32 needs 114 registers anyway.)
+    static constexpr int kPerSm = KW == 8 ? 1 : (D == 128 ? 2 : 3);
+    static constexpr int kPerSmMore = OP == Op::kFused || D == 128 || (OP == Op::kSpmm && D == 32) ? kPerSm : kPerSm + 1;
 };
 
 // acc[8 rows][NP pairs of columns] += a[8] x b[NP]
@@ -592,24 +594,29 @@ static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
 // six steps leave some of the eight groups without any): d64 fused 33.9 / 24.7, SDDMM 16.5 / 16.3, SpMM 16.9 / 14.1;
 // d128 42.1 / 43.7, 29.1 / 28.9, 19.8 / 21.5; d32 16.8 / 16.9, 12.0 / 10.9, 8.2 / 8.8; +-400, d64: 98 / 67, 55 / 53, 50 / 35.
 // At 192 CTAs +-64 fused d64 30.3 / 24.5, SpMM 11.0 / 13.9.
-// SDDMM and SpMM at d <= 64: four CTAs per SM instead of three where there are more than three to run, with 128 registers: H16
-// L1024 d64 +-64 (512 CTAs of 32 rows) 22.9 / 22.4 -> 20.0 / 20.4, B2 H16 L4096 window 256 161 / 155 -> 149 / 146; 384 CTAs
-// are one wave either way and slower with fewer registers, 16.7 / 16.4 against 19.5 / 19.7.  Eight warps: two CTAs per
-// SM, SpMM at 256 CTAs 14.2 -> 12.5.
+// SDDMM and SpMM at d <= 64, four CTAs per SM (two of eight warps) instead of three (one), with fewer registers: a wave of
+// them takes longer, so it is taken where it saves one.  Three / four, us, SDDMM then SpMM, L1024 d64 +-255: at 448 CTAs of
+// 32 rows (those at the ends of a head are short and make room for the few that are left) 48.2 / 60.7, 35.5 / 43.1; 480 57.3 / 60.9,
+// 41.6 / 43.6; 512 64.9 / 60.8, 45.0 / 43.5; 576 75.4 / 60.9, 49.3 / 43.9; 608 76.5 / 67.8, 50.2 / 48.7; 736 81.8 / 87.2,
+// 57.8 / 58.3; 864 86.1 / 93.5, 62.6 / 64.4; of 64 rows 448 86.8 / 92.3, 67.2 / 76.3; 512 105.6 / 93.1, 84.9 / 77.0; 736
+// 130.8 / 136.8, 103.4 / 104.7; 1024 169.0 / 163.3, 133.8 / 131.2; 1536 234.5 / 225.8, 185.5 / 179.9.  With +-64 the lines
+// are the same, but for 480 (27.8 / 25.9, 22.2 / 20.4).  Eight warps, one / two, +-64: 128 CTAs 8.7 / 8.9, 7.4 / 7.6; 160 14.9 /
+// 14.3, 12.0 / 12.0; 256 16.1 / 14.5, 13.7 / 12.1; SDDMM at d32 +-64 160 11.1 / 9.2.
+template <int D, int RW, int KW, Op OP>
+static int32_t launch_for(const Params& p, int64_t bh, int64_t blocks, cudaStream_t st) {
+    using L = Layout<D, RW, KW, OP>;
+    if constexpr (L::kPerSmMore != L::kPerSm)
+        if (KW == 8 ? blocks > 148 : (blocks > 470 && blocks <= 614) || blocks > 888)
+            return launch<D, RW, KW, OP, L::kPerSmMore>(p, bh, st);
+    return launch<D, RW, KW, OP>(p, bh, st);
+}
 template <int D, Op OP>
 static int32_t run(const Params& p, int64_t bh, cudaStream_t st) {
     const int64_t rows = ((int64_t)p.n_rows + p.stride - 1) / p.stride, classes = p.stride * bh;
-    if ((rows + 63) / 64 * classes >= 3 * 148) {
-        if constexpr (OP == Op::kFused) return launch<D, 2, 2, OP>(p, bh, st);
-        else return launch<D, 2, 2, OP, Layout<D, 2, 2, OP>::kPerSmFull>(p, bh, st);
-    }
-    if ((rows + 31) / 32 * classes >= 2 * 148) {
-        using L = Layout<D, 1, 4, OP>;
-        if constexpr (OP != Op::kFused && L::kPerSmFull != L::kPerSm)
-            if ((rows + 31) / 32 * classes > L::kPerSm * 148) return launch<D, 1, 4, OP, L::kPerSmFull>(p, bh, st);
-        return launch<D, 1, 4, OP>(p, bh, st);
-    }
-    return launch<D, 1, 8, OP>(p, bh, st);
+    const int64_t of64 = (rows + 63) / 64 * classes, of32 = (rows + 31) / 32 * classes;
+    if (of64 >= 3 * 148) return launch_for<D, 2, 2, OP>(p, bh, of64, st);
+    if (of32 >= 2 * 148) return launch_for<D, 1, 4, OP>(p, bh, of32, st);
+    return launch_for<D, 1, 8, OP>(p, bh, of32, st);
 }
 
 }  // namespace tile
