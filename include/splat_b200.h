@@ -258,11 +258,11 @@ int32_t splat_attention_fused_table(const void* q, const void* k, int64_t k_stri
                                     int32_t path, const int32_t* plan_i32, const int32_t* band_table,
                                     int32_t* status_word, int32_t* path_ran, void* stream);
 
-/* The kernel that splat_attention_fused* starts for a problem that SPLAT_PATH_BAND takes, rows with more than one
- * non-zero of this stride, as the library is set now: 1 = a Q tile per CTA, 2 = two per CTA, 3 = CTA pairs, 4 = the
- * persistent two-tile kernel (the values of SPLAT_B200_BAND_TILES; 3 may still hand a problem over to 2).  Negative
- * status: the forced kernel does not take it.  Host only. */
-int32_t splat_band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, int64_t stride, int32_t has_band_table);
+/* The kernel that splat_attention_fused* starts for a problem that SPLAT_PATH_BAND takes (plan_i32 as there), as the
+ * library is set now: 1 = a Q tile per CTA, 2 = two per CTA, 3 = CTA pairs, 4 = the persistent two-tile kernel (the
+ * values of SPLAT_B200_BAND_TILES; 3 may still hand a problem over to 2).  Negative status: the forced kernel does not
+ * take it.  Host only. */
+int32_t splat_band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, const int32_t* plan_i32, int32_t has_band_table);
 
 /* The five row vectors, the two span vectors and the largest row count of an explicit uint8 mask in one pass
  * (what splat_mask_row_summary_u8 and splat_acsr_from_row_summary compute together, same values bit for

@@ -1,4 +1,4 @@
-"""GPU: the persistent two-tile kernel of d = 128, which takes over at 592 to 1184 tiles of 128 rows.  It multiplies and sums in the
+"""GPU: the persistent two-tile kernel of d = 128, which takes over at 592 to 1776 tiles of 128 rows.  It multiplies and sums in the
 order of the kernel with a tile per CTA, so the results of the two agree bit for bit (and so do shards of a problem on either
 side of the line; the log-sum-exp of a row with one non-zero is summed in another order); the first and last head are
 also compared with the CPU oracle."""
@@ -14,21 +14,21 @@ pytestmark = pytest.mark.gpu
 #        kind, L, p0, p1, batch * heads
 PATTERNS = [
     (ao.PATTERN_CAUSAL_WINDOWED, 128, 40, 0, 740),     # one tile per head: neighbours never share keys; the fewest tiles
-    (ao.PATTERN_CAUSAL_WINDOWED, 384, 200, 0, 397),    # odd number of tiles per head and in all: items across heads, half an item
     (ao.PATTERN_CAUSAL_WINDOWED, 1000, 255, 0, 96),    # a short last tile
     (ao.PATTERN_CAUSAL_WINDOWED, 2048, 0, 0, 48),      # single-element rows only: nothing to multiply
-    (ao.PATTERN_CAUSAL_WINDOWED, 2048, 1500, 0, 49),   # ranges that grow with the row
     (ao.PATTERN_WINDOWED, 1536, 300, 0, 65),
-    (ao.PATTERN_BLOCKED, 2560, 777, 0, 40),            # neighbours whose ranges jump by more than the ring holds
     (ao.PATTERN_BLOCKED, 2048, 64, 0, 75),             # half steps at both ends
     (ao.PATTERN_STRIDED, 1024, 64, 0, 12),             # classes of 16 rows
-    (ao.PATTERN_STRIDED, 4096, 4, 0, 37),              # triangular classes of eight tiles
     (ao.PATTERN_DILATED, 3072, 300, 2, 33),
 ]
 
 
-# Too small for the kernel to be chosen: forced.
-SMALL = [
+# Left to the other kernel, too small or of too uneven tiles: forced.
+FORCED = [
+    (ao.PATTERN_CAUSAL_WINDOWED, 384, 200, 0, 397),    # odd number of tiles per head and in all: items across heads, half an item
+    (ao.PATTERN_CAUSAL_WINDOWED, 2048, 1500, 0, 49),   # ranges that grow with the row
+    (ao.PATTERN_BLOCKED, 2560, 777, 0, 40),            # neighbours whose ranges jump by more than the ring holds
+    (ao.PATTERN_STRIDED, 4096, 4, 0, 37),              # triangular classes of eight tiles
     (ao.PATTERN_CAUSAL_WINDOWED, 128, 127, 0, 1),      # one tile
     (ao.PATTERN_CAUSAL_WINDOWED, 64, 9, 0, 1),         # half a tile
     (ao.PATTERN_CAUSAL_WINDOWED, 256, 255, 0, 1),      # two, an item each
@@ -57,7 +57,7 @@ def test_where_it_does_not_apply_it_refuses(monkeypatch):
 
 
 @pytest.mark.parametrize("contiguous,dtype", [(False, torch.bfloat16), (True, torch.bfloat16), (False, torch.float16)])
-@pytest.mark.parametrize("kind,L,p0,p1,H", PATTERNS + SMALL)
+@pytest.mark.parametrize("kind,L,p0,p1,H", PATTERNS + FORCED)
 def test_duo_patterns(kind, L, p0, p1, H, contiguous, dtype, monkeypatch):
     import acsr_helpers as ah
     import splat_native as n
@@ -76,14 +76,13 @@ def test_duo_patterns(kind, L, p0, p1, H, contiguous, dtype, monkeypatch):
         n.check_status_word(0)
         return out
 
-    stride = {ao.PATTERN_STRIDED: p0, ao.PATTERN_DILATED: p1}.get(kind, 1)
-    if (kind, L, p0, p1, H) in SMALL:
+    if (kind, L, p0, p1, H) in FORCED:
         monkeypatch.setenv("SPLAT_B200_BAND_TILES", "4")
     else:
         monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
-        n.classify(acsr[2], acsr[3], acsr[4])
+        plan = n.classify(acsr[2], acsr[3], acsr[4])
         assert n.band_table(acsr[2], acsr[3], acsr[4], L) is not None
-        assert n._lib.splat_band_kernel_choice(H, L, d, stride, 1) == 4, "this kernel is not the one that runs"
+        assert n.band_kernel_choice(H, L, d, plan) == 4, "this kernel is not the one that runs"
     lse, lse_one = (torch.full((1, H, L), float("nan"), device="cuda") for _ in range(2))
     out, plain = run(lse), run(None)
     monkeypatch.setenv("SPLAT_B200_BAND_TILES", "1")
@@ -111,7 +110,7 @@ def test_duo_unscaled_scores_need_the_running_max(monkeypatch):
             monkeypatch.setenv("SPLAT_B200_BAND_TILES", variant)
         else:
             monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
-            assert n._lib.splat_band_kernel_choice(B * H, L, d, 1, 1) == 4
+            assert n.band_kernel_choice(B * H, L, d, n.classify(acsr[2], acsr[3], acsr[4])) == 4
         outs.append(torch.full_like(q, float("nan")))
         n.attention_fused(q, k.transpose(2, 3), v, outs[-1], acsr[2], acsr[3], acsr[4], 1.0, n.PATH_BAND)
         n.check_status_word(0)

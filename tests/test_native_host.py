@@ -145,20 +145,32 @@ def test_kernels_wait_through_the_tested_functions_only():
 
 def test_choice_of_the_fused_band_kernel(monkeypatch):
     import splat_native as n
-    choice = n._lib.splat_band_kernel_choice
+
+    def choice(bh, L, d, most, stride=1, single=0, table=True):      # most: longest row
+        return n.band_kernel_choice(bh, L, d, (most, stride, stride, 0, single, L, 0, L - single), table)
+
     monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
-    assert choice(64, 2048, 128, 1, 1) == 1                       # 1024 tiles: the last wave of 296 is less than half full
-    assert choice(70, 2048, 128, 1, 1) == 4                       # 1120
-    assert choice(512, 32768, 128, 1, 1) == 4
-    assert choice(512, 32768, 128, 1, 0) == 1                     # without a band table
-    assert choice(512, 32768, 64, 1, 1) == 1
-    assert choice(512, 32767, 128, 2, 1) == 1                     # classes of unequal length
-    assert choice(65535, 2147483647, 128, 1, 1) == 1              # more tiles than a grid has
-    assert choice(1, 128, 128, 1, 1) == 1
-    assert choice(0, 128, 128, 1, 1) < 0
+    # waves of 296 tiles: two, two and a bit, two and a half, three, three and a half, four
+    assert [choice(t // 16, 2048, 128, 401) for t in (576, 592, 608, 720, 736, 768, 880, 1024, 1040, 1168, 1184, 1216)] == \
+        [1, 4, 1, 1, 1, 4, 4, 1, 4, 4, 4, 4]
+    # bands of half the class and more: from four waves; bands that grow to that: from six
+    assert [choice(t // 16, 2048, 128, 1024) for t in (592, 768, 1040, 1184)] == [1, 1, 1, 4]
+    assert [choice(t // 16, 2048, 128, 2048) for t in (592, 768, 1040, 1184)] == [1, 1, 1, 4]
+    assert [choice(t // 16, 2048, 128, 1024, single=1) for t in (768, 1184)] == [1, 4]
+    assert [choice(t // 16, 2048, 128, 2048, single=1) for t in (592, 768, 1184, 1760, 1776)] == [1, 1, 1, 1, 4]
+    assert [choice(t // 64, 8192, 128, 1024, 8, 8) for t in (768, 1216, 1792)] == [1, 1, 4]
+    assert [choice(t // 64, 8192, 128, 256, 32, 32) for t in (640, 768, 1216)] == [1, 4, 4]      # classes of two tiles
+    assert [choice(t, 128, 128, 128, single=1) for t in (740, 800, 1184)] == [4, 4, 4]           # ... and of one
+    assert choice(512, 32768, 128, 1024) == 4
+    assert choice(512, 32768, 128, 1024, table=False) == 1
+    assert choice(512, 32768, 64, 1024) == 1
+    assert choice(512, 32767, 128, 1024, 2) == 1                  # classes of unequal length
+    assert choice(65535, 2147483647, 128, 3) == 1                 # more tiles than a grid has
+    assert choice(1, 128, 128, 128) == 1
+    assert choice(0, 128, 128, 128) < 0
     for forced, d, stride, expected in (("4", 128, 1, 4), ("4", 64, 1, -6), ("4", 128, 3, -6), ("1", 128, 1, 1), ("2", 128, 1, 2),
                                         ("3", 128, 1, 3), ("3", 64, 1, 2), ("2", 32, 1, 1), ("2", 128, 3, 1), ("7", 128, 1, 1)):
         monkeypatch.setenv("SPLAT_B200_BAND_TILES", forced)
-        assert choice(1, 256, d, stride, 1) == expected, (forced, d, stride)
+        assert choice(1, 256, d, 31, stride) == expected, (forced, d, stride)
     monkeypatch.setenv("SPLAT_B200_BAND_TILES", "4")
-    assert choice(1, 256, 128, 1, 0) == -6
+    assert choice(1, 256, 128, 31, table=False) == -6

@@ -65,7 +65,7 @@ SIGNATURES = {
     "splat_acsr_from_mask_u8": [_vp, _i64, _i64, _i64, _i32] + [_vp] * 9 + [_vp],
     "splat_transpose_16": [_vp, _vp, _i64, _i64, _i64, _vp],
     "splat_attention_host": [_vp] * 5 + [_i64] + [_vp] * 3 + [_i64] * 3 + [_f32, _i32, _i32] + [_vp] * 8,
-    "splat_band_kernel_choice": [_i64, _i64, _i64, _i64, _i32],
+    "splat_band_kernel_choice": [_i64, _i64, _i64, _vp, _i32],
     "splat_band_table": [_vp, _vp, _vp, _i64, _i64, _vp, _vp],
     "splat_attention_fused_table": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64,
                                     _i64, _i64, _f32, _i32, _i32, _vp, _vp, _vp, _vp, _vp],
@@ -286,6 +286,11 @@ def band_table(sTod_lin, sTod_tr, nnzs, n_rows: int):
     if hit[5] != stream.cuda_stream:      # the table is nobody's tensor but ours: its use elsewhere is ours to record
         hit[4].record_stream(stream)
     return hit[4].data_ptr()
+
+
+def band_kernel_choice(bh: int, n_rows: int, d: int, plan, has_band_table: bool = True) -> int:
+    """``splat_band_kernel_choice`` for a plan of classify(): the fused kernel that a band problem gets."""
+    return _lib.splat_band_kernel_choice(bh, n_rows, d, ctypes.cast((ctypes.c_int32 * 8)(*plan), _vp), int(has_band_table))
 
 
 _STATUS_WORDS: dict = {}

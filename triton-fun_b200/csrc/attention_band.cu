@@ -758,22 +758,36 @@ int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v,
 // L2 -> SM traffic), below.  3: persistent CTA pairs (attention_pair.cu), d = 128 only.  4: two tiles per persistent CTA
 // (attention_duo.cu), d = 128 and a band table only.  SPLAT_B200_BAND_TILES=1|2|3|4 selects; where 2 or 3 does not apply,
 // another runs, and where 4 does not, none.
-// Unset: 4 for enough tiles, else 1.  The persistent kernel takes
-// 0.83 to 0.95 of the time where the waves of two tiles per SM are many or the last one is half full at least; a few
-// tiles beyond two or three whole waves cost it a wave of its own (us, a CTA per tile / persistent: +-566 at 500 / 600 /
-// 700 / 800 / 900 / 1200 tiles 58.1 / 58.2, 63.7 / 69.3, 81.0 / 71.9, 85.2 / 75.1, 89.6 / 94.2, 116 / 110; +-60 at 640 / 720 /
-// 800 / 1040 / 1184 31.5 / 30.3, 34.2 / 36.0, 35.8 / 33.1, 45.2 / 41.2, 48.9 / 41.1).  At d = 64 it is no faster
-// (+-200, 1024 tiles 47 / 51).
-static int band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, int64_t stride, bool has_table) {
+// Unset: 4 where it is the faster, else 1.  Two tiles per SM at a time are coarse pieces of work: it gains 5 to 20 % where
+// their waves are many or the last one is well filled, and loses as much where a few pairs are left over for a wave of
+// their own, or a few long ones.  So below four waves of 296 tiles it asks for exactly two of them or a last one half full, and for
+// bands short against their class, which make most tiles alike (a class of two tiles does anyway); and
+// bands that grow with the row over most of the class (rows with one key beside such with half the class) have to wait
+// for six.  us, bf16, a CTA per tile / persistent, at tiles:
+//   +-200, L 1024           592 40.7 / 35.7   736 49.2 / 44.6   800 52.9 / 45.2    888 51.8 / 49.7   1040 59.3 / 54.7   1184 65.5 / 56.0
+//   window 1024, L 8192     576 55.1 / 48.6   704 72.3 / 65.4   832 76.6 / 67.9    960 91.2 / 84.8   1024 96.4 / 86.9   1152 102.6 / 88.5
+//   blocks of 200, L 1024   592 35.9 / 33.8   736 48.6 / 47.0   800 46.3 / 45.4    888 49.4 / 55.2   1040 56.8 / 56.9   1184 61.9 / 57.4
+//   blocks of 384, L 1536   600 40.7 / 49.6   804 51.0 / 56.2   888 52.6 / 63.3   1044 60.6 / 62.7   1188 68.9 / 67.9   1488 85.9 / 85.6
+//   +-400, L 1024           592 55.7 / 49.4   736 60.1 / 67.5   888 63.4 / 65.9    960 70.9 / 70.1   1184 84.3 / 74.8   1480 106 / 93
+//   dense causal, L 2048    592 70.7 / 66.9   800 79.3 / 88.5   896 85.5 / 104.5  1040 96.4 / 110.8  1184 107 / 117    1480 136 / 141
+//                          1776 163 / 164    2400 215 / 210    4736 422 / 376
+//   strided 8, L 8192       768 47.9 / 53.3   832 50.0 / 59.6  1152 63.9 / 66.1   1472 81.8 / 82.5   1776 101 / 98      2400 133 / 124
+//   strided 32, L 8192      768 27.2 / 26.6   832 28.8 / 27.0  1152 35.4 / 33.2   1280 39.7 / 37.2   1472 44.2 / 39.6
+// At d = 64 it is no faster (+-200, 1024 tiles 47 / 51).
+static int band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, const int32_t* plan, bool has_table) {
     int forced = 0;
     if (const char* e = getenv("SPLAT_B200_BAND_TILES"))
         if (e[0] >= '1' && e[0] <= '4') forced = e[0] - '0';
-    const int64_t tiles = bh * stride * ((n_rows / stride + 127) / 128);
+    const int64_t stride = plan[7] > 0 ? plan[1] : 1, rows = n_rows / stride, tiles = bh * stride * ((rows + 127) / 128);
     const bool duo_takes = d == 128 && n_rows % stride == 0 && has_table && tiles <= INT32_MAX;
     if (forced == 4) return duo_takes ? 4 : SPLAT_ERR_UNSUPPORTED_SHAPE;
     if ((d != 64 && d != 128) || n_rows % stride != 0) return 1;
-    if (forced == 0) return duo_takes && (tiles >= 8 * 148 || (tiles >= 4 * 148 && tiles % (2 * 148) >= 148)) ? 4 : 1;
-    return forced == 3 && d != 128 ? 2 : forced;
+    if (forced != 0) return forced == 3 && d != 128 ? 2 : forced;
+    constexpr int kWave = 2 * 148;
+    const bool alike = rows <= 256 || 2 * (int64_t)plan[0] < rows, grow = !alike && plan[4] > 0 && 2 * (int64_t)plan[0] > rows;
+    const bool faster = tiles >= 4 * kWave ? !grow || tiles >= 6 * kWave
+                                           : alike && (tiles == 2 * kWave || (tiles > 2 * kWave && tiles % kWave >= kWave / 2));
+    return duo_takes && faster ? 4 : 1;
 }
 
 int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, int64_t ksk,
@@ -804,7 +818,7 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
     if (!k_major && (stride != 1 || n_cols % 8 != 0)) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return SPLAT_ERR_MISALIGNED;
 
-    const int variant = band_kernel_choice(bh, n_rows, d, stride, band_table != nullptr);
+    const int variant = band_kernel_choice(bh, n_rows, d, plan, band_table != nullptr);
     if (variant < 0) return variant;
     if (variant == 4)
         return attention_duo(q, k, kt_major ? 1 : 0, v, o, bh, n_rows, d, stride, scale, dtype, status_word, band_table, lse, st);
@@ -840,9 +854,10 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
 
 }  // namespace splat
 
-extern "C" int32_t splat_band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, int64_t stride, int32_t has_band_table) {
-    if (bh < 1 || n_rows < 1 || d < 1 || stride < 1 || bh > 65535 || n_rows > INT32_MAX || stride > 65535) return SPLAT_ERR_BAD_ARG;
-    return splat::band_kernel_choice(bh, n_rows, d, stride, has_band_table != 0);
+extern "C" int32_t splat_band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, const int32_t* plan_i32, int32_t has_band_table) {
+    if (bh < 1 || n_rows < 1 || d < 1 || bh > 65535 || n_rows > INT32_MAX || !plan_i32) return SPLAT_ERR_BAD_ARG;
+    if (plan_i32[7] > 0 && (plan_i32[1] < 1 || plan_i32[1] > 65535)) return SPLAT_ERR_BAD_ARG;
+    return splat::band_kernel_choice(bh, n_rows, d, plan_i32, has_band_table != 0);
 }
 
 #ifdef SPLAT_BAND_TRACE
