@@ -749,9 +749,8 @@ int32_t attention_pair(const void* q, const void* k, int kt_major, const void* v
 int32_t attention_wide(const void* q, const void* k, int kt_major, const void* v, void* o, const float* lin, const float* tr,
                        const float* nnzs, int64_t bh, int64_t n_rows, int64_t d, int64_t stride, float scale, int32_t dtype,
                        int32_t* status_word, const int32_t* band_table, float* lse, cudaStream_t st);
-int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v, void* o, int64_t bh, int64_t n_rows, int64_t d,
-                      int64_t stride, float scale, int32_t dtype, int32_t* status_word, const int32_t* band_table, float* lse,
-                      cudaStream_t st);
+int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v, void* o, int64_t bh, int64_t n_rows, int64_t stride,
+                      float scale, int32_t dtype, int32_t* status_word, const int32_t* band_table, float* lse, cudaStream_t st);
 
 // Kernel of a band problem (see attention_band() for what one is).  1: one Q tile per CTA, two CTAs per SM (attention_wide.cu),
 // the only one that takes any d and classes of unequal length.  2: two Q tiles per CTA sharing every K/V tile (half the
@@ -821,7 +820,7 @@ int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, i
     const int variant = band_kernel_choice(bh, n_rows, d, plan, band_table != nullptr);
     if (variant < 0) return variant;
     if (variant == 4)
-        return attention_duo(q, k, kt_major ? 1 : 0, v, o, bh, n_rows, d, stride, scale, dtype, status_word, band_table, lse, st);
+        return attention_duo(q, k, kt_major ? 1 : 0, v, o, bh, n_rows, stride, scale, dtype, status_word, band_table, lse, st);
     if (variant == 1)
         return attention_wide(q, k, kt_major ? 1 : 0, v, o, lin, tr, nnzs, bh, n_rows, d, stride, scale, dtype, status_word,
                               band_table, lse, st);

@@ -1,6 +1,6 @@
 // Fused band attention for d = 128: a persistent CTA per SM with two 128-row Q tiles ("pipes") side by
 // side.  Problem, regrouping by residue class and operand layouts: see attention_band.cu; a step's arithmetic: see
-// attention_wide.cu, which has the other problems.
+// attention_wide.cu, which has the other problems (other d, classes of unequal length, no band table).
 //
 // What bounds a tile is its own chain S -> softmax -> P -> PV -> S: with the exponentials left out the kernel gains 10 %,
 // with the MMAs left out 18 %.  So there are two independent tiles per SM here as in attention_wide.cu, but
@@ -50,7 +50,7 @@ using sm::fmax3;
 using sm::mul2;
 using sm::pack2;
 
-constexpr int kD = 128;                  // columns of a tile (those past d are zero)
+constexpr int kD = 128;                  // columns of a tile
 constexpr int kTile = 128;               // rows of a Q tile, keys of a block
 constexpr int kChunk = 32;               // columns of a tensor-memory load
 constexpr int kChunks = kTile / kChunk;
@@ -82,23 +82,24 @@ constexpr int kSmemBytes = kStageOff + 8 * 2048 + 1024;   // + alignment slack
 enum : int { kErrOrder = 59, kErrV = 60, kErrQFree = 61, kErrKFree = 62, kErrVFree = 63, kErrItem = 64, kErrItemFree = 65, kErrClc = 66,
              kErrS = 67, kErrP = 68, kErrO = 69, kErrSFree = 70, kErrPv = 74, kErrIdle = 75 };
 
+struct Maps3 { CUtensorMap m[3]; };       // Q, K, V
+
 struct Params {
     const void* q;     // raw operands: rows with one non-zero are handled through them
     const void* k;
     const void* v;
     void* o;
-    const int2* rows;  // band table (see acsr_meta.cu): rows in class order, tiles' key ranges
+    const int2* bands; // band table (see acsr_meta.cu): of the rows in class order, tiles' key ranges
     const int2* tiles;
     float* lse;        // (BH, L) or null
     int32_t* status;
     int32_t* mirror;   // host copy of the status word, or null
     int64_t n_rows;    // L
-    Classes cls;
-    uint32_t classes;  // ... their number
+    int stride;        // classes of a head
+    int rows;          // ... rows of each
+    uint32_t pitch;    // ... tiles of each
     uint32_t total;    // tiles of all heads and classes
     uint32_t pairs;    // items of two tiles; the rest have one
-    int stride;
-    int d;             // head dimension, <= kD and a multiple of 8
     int kt_major;
     float scale_log2;
 };
@@ -170,12 +171,12 @@ constexpr int kSingle = -1, kEmpty = INT_MIN / 2;
 // Log-sum-exp of a row with one non-zero: its score.
 template <typename T>
 __device__ __forceinline__ float single_lse(const Params& p, int64_t head, int64_t row, int start) {
-    const T* q = reinterpret_cast<const T*>(p.q) + (head + row) * p.d;
-    const T* k = reinterpret_cast<const T*>(p.k) + head * p.d + (p.kt_major ? start : (int64_t)start * p.d);
+    const T* q = reinterpret_cast<const T*>(p.q) + (head + row) * kD;
+    const T* k = reinterpret_cast<const T*>(p.k) + head * kD + (p.kt_major ? start : (int64_t)start * kD);
     const int64_t step = p.kt_major ? p.n_rows : 1;
     float acc = 0.f;
 #pragma unroll 1
-    for (int c = 0; c < p.d; ++c) acc = fmaf(DT<T>::to_f(q[c]), DT<T>::to_f(k[c * step]), acc);
+    for (int c = 0; c < kD; ++c) acc = fmaf(DT<T>::to_f(q[c]), DT<T>::to_f(k[c * step]), acc);
     return acc * p.scale_log2 * kLn2;
 }
 
@@ -183,14 +184,12 @@ __device__ __forceinline__ float single_lse(const Params& p, int64_t head, int64
 __device__ __forceinline__ Tile tile_of(const Params& p, uint32_t n) {
     Tile t = {-1, 0, 0, 0, 0};
     if (n >= p.total) return t;
-    const uint32_t pitch = (uint32_t)p.cls.tile_pitch, rest = n / pitch, tile = n - rest * pitch;
-    t.bh = (int)(rest / p.classes);
-    t.res = (int)(rest - (uint32_t)t.bh * p.classes);
-    const int rows_v = p.cls.rows_of(t.res), u0 = (int)tile * kTile;
-    if (u0 >= rows_v) return t;              // (a class one tile shorter than the longest)
-    t.u0 = u0;
-    const int2 range = __ldg(p.tiles + t.res * p.cls.tile_pitch + tile);
-    const int hi = min(range.y, rows_v);
+    const uint32_t rest = n / p.pitch, tile = n - rest * p.pitch;
+    t.bh = (int)(rest / (uint32_t)p.stride);
+    t.res = (int)(rest - (uint32_t)t.bh * (uint32_t)p.stride);
+    t.u0 = (int)tile * kTile;
+    const int2 range = __ldg(p.tiles + t.res * (int64_t)p.pitch + tile);
+    const int hi = min(range.y, p.rows);
     if (hi > 0) { t.lo = range.x / 64; t.hi = (hi + 63) / 64; }
     return t;
 }
@@ -219,7 +218,7 @@ __device__ __forceinline__ int64_t clc_answer(const uint4* answer) {
 
 template <typename T, bool kLse>
 __global__ void __launch_bounds__(kThreads, 1)
-attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
+attention_duo_kernel(const __grid_constant__ Maps3 maps, const Params p) {
     constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + (((smem_u32(smem_raw) + 1023) & ~1023u) - smem_u32(smem_raw));
@@ -234,7 +233,7 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
     } else if (warp == kTmaWarp) {
         if (lane == 0) {
 #pragma unroll 1
-            for (int i = 0; i < 3; ++i) tma_prefetch_desc(maps.part[p.cls.longer > 0 ? 0 : 1] + i);
+            for (int i = 0; i < 3; ++i) tma_prefetch_desc(&maps.m[i]);
 #pragma unroll 1
             for (int i = 0; i < 2; ++i) {
                 mbar_init(&ctrl->q_full[i], 1);
@@ -323,7 +322,7 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                 auto load_q = [&](const Tile& t, int x, int& asked) {
                     if (asked > 0) ok = wait_bar(&ctrl->q_free[x], ((uint32_t)asked & 1u) ^ 1u, &ctrl->gave_up, kErrQFree);
                     if (!ok) return;
-                    load(&ctrl->q_full[x], smem + x * kTileBytes, maps.part[p.cls.part(t.res)], p.cls.in_part(t.res), t.u0, t.bh);
+                    load(&ctrl->q_full[x], smem + x * kTileBytes, &maps.m[0], t.res, t.u0, t.bh);
                     ++asked;
                 };
                 for (int n = 0; ok; ++n) {
@@ -349,10 +348,8 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                         if (q0) load_q(a, 0, q0_asked);
                         if (q1 && ok) load_q(b, 1, q1_asked);
                         if (!ok) break;
-                        const int real_res = x ? b.res : a.res, bh = x ? b.bh : a.bh, st = entry % kSlots;
-                        const int res = p.cls.in_part(real_res);
+                        const int res = x ? b.res : a.res, bh = x ? b.bh : a.bh, st = entry % kSlots;
                         const uint32_t parity = ((uint32_t)(entry / kSlots) & 1u) ^ 1u;
-                        const CUtensorMap* map = maps.part[p.cls.part(real_res)];
                         uint8_t* dst = smem + kKOff + st * kTileBytes;
                         if (entry >= kSlots) ok = wait_bar(&ctrl->k_free[st], parity, &ctrl->gave_up, kErrKFree);
                         if (!ok) break;
@@ -360,14 +357,14 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                             mbar_arrive_expect_tx(&ctrl->k_full[st], kTileBytes);
 #pragma unroll 1
                             for (int ch = 0; ch < kTile / 64; ++ch)       // 64-key chunks of [d][64 keys]
-                                tma_load_4d(dst + ch * (kD * 128), map + 1, &ctrl->k_full[st], block * kTile + ch * 64, 0, bh, 0);
+                                tma_load_4d(dst + ch * (kD * 128), &maps.m[1], &ctrl->k_full[st], block * kTile + ch * 64, 0, bh, 0);
                         } else {
-                            load(&ctrl->k_full[st], dst, map + 1, res, block * kTile, bh);
+                            load(&ctrl->k_full[st], dst, &maps.m[1], res, block * kTile, bh);
                         }
                         ++k_asked;
                         if (entry >= kSlots) ok = wait_bar(&ctrl->v_free[st], parity, &ctrl->gave_up, kErrVFree);
                         if (!ok) break;
-                        load(&ctrl->v_full[st], smem + kVOff + st * kTileBytes, map + 2, res, block * kTile, bh);
+                        load(&ctrl->v_full[st], smem + kVOff + st * kTileBytes, &maps.m[2], res, block * kTile, bh);
                         ++entry;
                     }
                 }
@@ -642,8 +639,8 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
             if (lane == 0) mbar_arrive(&ctrl->item_free[n % kItems]);
             begin = 0; end = kEmpty;
             const int u = now.u0 + w4 * 32 + lane;
-            if (more && now.u0 >= 0 && u < p.cls.rows_of(now.res)) {
-                const int2 band = __ldg(p.rows + p.cls.first_row(now.res) + u);
+            if (more && now.u0 >= 0 && u < p.rows) {
+                const int2 band = __ldg(p.bands + (int64_t)now.res * p.rows + u);
                 begin = band.x; end = band.y;
             }
             if (was.u0 < 0) continue;
@@ -657,9 +654,9 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
             // (all scores of a row -inf: zeros)
             const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
             const int64_t head = was.bh * p.n_rows;
-            const int u_warp = was.u0 + w4 * 32, rows_v = p.cls.rows_of(was.res);
+            const int u_warp = was.u0 + w4 * 32;
             const int64_t row_real = (int64_t)(u_warp + lane) * p.stride + was.res;
-            const bool exists = u_warp + lane < rows_v;
+            const bool exists = u_warp + lane < p.rows;
             if (kLse && exists) {
                 float e = -INFINITY;
                 if (row_end > 0) e = lse_from_log2(m_used, l_sum);
@@ -671,8 +668,8 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
             if (in_band != 0) {
                 const float2 inv2 = make_float2(inv, inv);
                 const int piece = lane & 3;
-                char* to = reinterpret_cast<char*>(p.o) + ((head + (int64_t)(u_warp + (lane >> 2)) * p.stride + was.res) * p.d + piece * 8) * 2;
-                const int64_t to_step = (int64_t)8 * p.stride * p.d * 2;
+                char* to = reinterpret_cast<char*>(p.o) + ((head + (int64_t)(u_warp + (lane >> 2)) * p.stride + was.res) * kD + piece * 8) * 2;
+                const int64_t to_step = (int64_t)8 * p.stride * kD * 2;
 #pragma unroll 1
                 for (int c = 0; c < kD; c += 32) {
                     uint32_t r[32];
@@ -695,7 +692,7 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                     for (int i = 0; i < 4; ++i) {
                         const int row = 8 * i + (lane >> 2);
                         const uint4 v = *reinterpret_cast<const uint4*>(stage + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
-                        if (((in_band >> row) & 1u) && c + piece * 8 < p.d) *reinterpret_cast<uint4*>(to + i * to_step + c * 2) = v;
+                        if ((in_band >> row) & 1u) *reinterpret_cast<uint4*>(to + i * to_step + c * 2) = v;
                     }
                     __syncwarp();
                 }
@@ -709,11 +706,9 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
                 left &= left - 1;
                 const int at = lane < 16 ? r0 : r1, c = (lane & 15) * 8;
                 const int start = __shfl_sync(0xffffffffu, row_start, at), kind = __shfl_sync(0xffffffffu, row_end, at);
-                if (c < p.d) {
-                    uint4 v = make_uint4(0, 0, 0, 0);
-                    if (kind == kSingle) v = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v) + (head + start) * p.d + c);
-                    *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.o) + (head + (int64_t)(u_warp + at) * p.stride + was.res) * p.d + c) = v;
-                }
+                uint4 v = make_uint4(0, 0, 0, 0);
+                if (kind == kSingle) v = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v) + (head + start) * kD + c);
+                *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.o) + (head + (int64_t)(u_warp + at) * p.stride + was.res) * kD + c) = v;
             }
         }
     }
@@ -728,7 +723,7 @@ attention_duo_kernel(const __grid_constant__ Maps<3> maps, const Params p) {
 }
 
 template <typename T>
-static int32_t launch(const Maps<3>& maps, const Params& prm, cudaStream_t st) {
+static int32_t launch(const Maps3& maps, const Params& prm, cudaStream_t st) {
     auto kern = prm.lse != nullptr ? attention_duo_kernel<T, true> : attention_duo_kernel<T, false>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes)) return SPLAT_ERR_LAUNCH;
     return launch_kernel(kern, prm.pairs + (prm.total > 2 * prm.pairs ? prm.total - 2 * prm.pairs : 0), kThreads, kSmemBytes, st, maps, prm);
@@ -737,34 +732,30 @@ static int32_t launch(const Maps<3>& maps, const Params& prm, cudaStream_t st) {
 }  // namespace duo
 }  // namespace band
 
-// Operands checked by attention_band().  band_table: not null.
-int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v, void* o, int64_t bh, int64_t n_rows, int64_t d,
-                      int64_t stride, float scale, int32_t dtype, int32_t* status_word, const int32_t* band_table, float* lse,
-                      cudaStream_t st) {
+// Operands checked by attention_band(): d = 128, a stride that divides n_rows, a band table, and the tiles of all heads
+// and classes fit 31 bits.
+int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v, void* o, int64_t bh, int64_t n_rows, int64_t stride,
+                      float scale, int32_t dtype, int32_t* status_word, const int32_t* band_table, float* lse, cudaStream_t st) {
     using namespace band;
     duo::Params p;
     p.q = q; p.k = k; p.v = v; p.o = o; p.lse = lse;
     p.status = status_word; p.mirror = status_mirror(status_word);
-    p.n_rows = n_rows; p.stride = (int)stride; p.d = (int)d;
+    p.n_rows = n_rows; p.stride = (int)stride; p.rows = (int)(n_rows / stride);
+    p.pitch = (uint32_t)((p.rows + duo::kTile - 1) / duo::kTile);
     p.kt_major = kt_major; p.scale_log2 = scale * kLog2e;
-    p.cls = Classes(n_rows, stride, duo::kTile);
-    p.classes = (uint32_t)(p.cls.rows > 0 ? stride : p.cls.longer);
-    p.rows = reinterpret_cast<const int2*>(band_table);
-    p.tiles = p.rows + n_rows;
-    p.total = (uint32_t)(bh * p.classes * p.cls.tile_pitch);     // (the caller has seen that it fits)
+    p.bands = reinterpret_cast<const int2*>(band_table);
+    p.tiles = p.bands + n_rows;
+    p.total = (uint32_t)(bh * stride * p.pitch);
     // A last wave of no more tiles than SMs goes one tile to an SM: alone a tile takes two thirds of the time of two.
     const uint32_t rest = p.total % (2 * 148);
     p.pairs = rest <= 148 ? (p.total - rest) / 2 : (p.total + 1) / 2;
-    Maps<3> maps;
-    for (int part = 0; part < 2; ++part) {
-        if (!p.cls.has(part)) continue;
-        CUtensorMap* m = maps.part[part];
-        if (!p.cls.view(m, q, dtype, bh, n_rows, d, stride, part, duo::kTile) ||
-            !(kt_major ? make_map_kt(m + 1, k, dtype, bh, n_rows, d, 128)
-                       : p.cls.view(m + 1, k, dtype, bh, n_rows, d, stride, part, duo::kTile)) ||
-            !p.cls.view(m + 2, v, dtype, bh, n_rows, d, stride, part, duo::kTile))
-            return SPLAT_ERR_DRIVER;
-    }
+    duo::Maps3 maps;
+    auto view = [&](CUtensorMap* m, const void* base) {
+        return make_map_view(m, base, dtype, bh, n_rows, duo::kD, stride, 0, stride, p.rows, duo::kTile);
+    };
+    if (!view(&maps.m[0], q) || !(kt_major ? make_map_kt(&maps.m[1], k, dtype, bh, n_rows, duo::kD, 128) : view(&maps.m[1], k)) ||
+        !view(&maps.m[2], v))
+        return SPLAT_ERR_DRIVER;
     return dtype == SPLAT_BF16 ? duo::launch<__nv_bfloat16>(maps, p, st) : duo::launch<__half>(maps, p, st);
 }
 
