@@ -53,9 +53,9 @@ def test_config1_full():
 @pytest.mark.parametrize("cfg", [2, 3, 4, 5])
 def test_config_sampled_heads_against_oracle(cfg, monkeypatch):
     """Full sequence length and pattern, two heads, every row compared with the CPU oracle -- for
-    the kernel the library picks at this size and for each of the three band kernels forced
-    (1: one Q tile per CTA, 2: two Q tiles per CTA, the kernel the full-size benchmark of
-    configuration 5 runs, 3: CTA pairs)."""
+    the kernel the library picks at this size and for each of the band kernels forced
+    (1: one Q tile per CTA, 2: two Q tiles per CTA, 3: CTA pairs, 4: persistent CTAs with two tiles, d = 128 only:
+    the kernel that configurations 3 to 5 get at full size)."""
     import splat_native as n
     B, H, L, d, dtype, kind, p0, p1, spread, seed = CONFIGS[cfg]
     heads = 2
@@ -63,7 +63,7 @@ def test_config_sampled_heads_against_oracle(cfg, monkeypatch):
     meta = ao.metadata_from_pattern(kind, L, p0, p1, 16)
     ref = at.attention_acsr(q.cpu(), k.cpu().transpose(2, 3), v.cpu(), meta, meta["trailing_dim"],
                             d ** -0.5)
-    for variant in (None, "1", "2", "3"):
+    for variant in (None, "1", "2", "3") + (("4",) if d == 128 else ()):
         if variant is None:
             monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
         else:
@@ -87,6 +87,7 @@ def test_config_full_size_properties(cfg):
     heads = B * H
     q, k, v = _inputs(cfg, heads)
     attn = _module(cfg, heads, path=n.PATH_BAND)
+    assert n.band_kernel_choice(heads, L, d, attn.plan) == (4 if d == 128 else 1)
     out = attn([q, k.transpose(2, 3), v]).clone()
     attn.check_status()
     assert torch.isfinite(out.float()).all()
