@@ -207,19 +207,23 @@ def torch_dense_masked_baseline(cfgs=(1, 2), budget_s=12.0):
     return out
 
 
-# fused band kernel by the library's SPLAT_B200_BAND_TILES switch (default: one Q tile per CTA)
-BAND_KERNELS = {"1": "attention_wide_kernel", "2": "attention_band_kernel", "3": "attention_pair_kernel"}
+# the library's fused band kernels, by the numbers of splat_band_kernel_choice
+BAND_KERNELS = {1: "attention_wide_kernel", 2: "attention_band_kernel", 3: "attention_pair_kernel", 4: "attention_duo_kernel"}
 
 
-def ncu_traffic(cfg, heads, path):
+def band_kernel(attn, heads, L, d):
+    """Name of the fused band kernel that the library picks for a module of `heads` heads."""
+    import splat_native as n
+    return BAND_KERNELS.get(n.band_kernel_choice(heads, L, d, attn.plan), "none")
+
+
+def ncu_traffic(cfg, heads, path, kernel):
     """DRAM bytes per launch of the fused kernel from the ncu captures summarised under
     profiles/ (dram__bytes_read.sum + dram__bytes_write.sum), scaled by the head count, with the
-    capture it came from.  None if the kernel sources changed after the capture."""
+    capture it came from.  None if the kernel sources changed after the capture or it is of another kernel."""
     meta_path = os.path.join(ROOT, "profiles", "dram_traffic.md")
     if path != "band" or not os.path.exists(meta_path):
         return None, None
-    if os.environ.get("SPLAT_B200_BAND_TILES", "1")[:1] != "1":
-        return None, "the traffic record covers the default kernel only"
     with open(meta_path) as f:
         text = f.read()
     try:
@@ -229,6 +233,8 @@ def ncu_traffic(cfg, heads, path):
     entry = rec["configs"].get(str(cfg))
     if entry is None:
         return None, None
+    if entry["kernel"] != kernel:
+        return None, f"the capture is of {entry['kernel']}"
     import hashlib
     h = hashlib.sha1()
     for name in rec["kernel_sources"]:
@@ -283,14 +289,15 @@ def time_config(cfg, dev, min_seconds=0.5, max_launches=20000):
     flops = 4.0 * nnz * d * heads
     bytes_alg = 4.0 * L * d * q.element_size() * heads
     t_flop, t_hbm = flops / (peaks["tflops"] * 1e12), bytes_alg / (peaks["hbm_gbs"] * 1e9)
-    traffic, prov = ncu_traffic(cfg, heads, "band")
+    kernel = band_kernel(attn, heads, L, d)
+    traffic, prov = ncu_traffic(cfg, heads, "band", kernel)
     if t_flop >= t_hbm:
         ach = flops / (mean_ms * 1e-3) / 1e12
         roof = {"bound": "tensor", "achieved": ach, "peak": peaks["tflops"], "unit": "TFLOP/s", "frac": ach / peaks["tflops"]}
     else:
         ach = bytes_alg / (mean_ms * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": ach / peaks["hbm_gbs"]}
-    roof.update({"traffic": traffic, "traffic_source": prov, "peak_source": peaks["source"]})
+    roof.update({"kernel": kernel, "traffic": traffic, "traffic_source": prov, "peak_source": peaks["source"]})
     out = {"workload": label, "dtype": dt, "launches": launches, "ms": mean_ms, "ms_median": per[len(per) // 2],
            "ms_best": per[0], "value": flops / (mean_ms * 1e-3) / 1e12, "unit": UNIT, "roofline": roof,
            "clocks": clocks.summary(), "l2": "L2 flushed by the launch itself: inputs + outputs = %.0f MB per launch"
@@ -548,13 +555,13 @@ def run_ours(args):
             gbs = bytes_alg / (launch_ms * 1e-3) / 1e9
             roof = {"bound": "hbm", "achieved": gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                     "frac": gbs / peaks["hbm_gbs"]}
-        traffic, traffic_source = ncu_traffic(cfg, heads, args.path)
+        kernel = ("sddmm + softmax + spmm (three launches)" if unfused else
+                  band_kernel(attn, heads, L, d) if args.path == "band" else "attention_rows_kernel")
+        traffic, traffic_source = ncu_traffic(cfg, heads, args.path, kernel)
         roof.update({"traffic": traffic, "traffic_unit": "bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum, "
                                                          "ncu capture scaled by heads)",
                      "traffic_source": traffic_source,
-                     "kernel": "sddmm + softmax + spmm (three launches)" if unfused else
-                               (BAND_KERNELS.get(os.environ.get("SPLAT_B200_BAND_TILES", "1")[:1], "attention_wide_kernel")
-                                if args.path == "band" else "attention_rows_kernel"),
+                     "kernel": kernel,
                      "peak_source": peaks["source"],
                      "peak_kind": "burst", "launch_ms": launch_ms, "launch_ms_median": launch_ms_median,
                      "launch_ms_best": launch_ms_best,

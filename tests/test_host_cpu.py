@@ -120,3 +120,15 @@ def test_two_rank_gloo_sharding(tmp_path):
     out = subprocess.run(cmd, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stdout + out.stderr
     assert out.stdout.count("ok") == 2
+
+
+def test_bench_names_the_kernel_that_the_library_picks(monkeypatch):
+    import types
+    import bench
+    monkeypatch.delenv("SPLAT_B200_BAND_TILES", raising=False)
+    window = types.SimpleNamespace(plan=(1024, 1, 1, 0, 1, 32768, 0, 32767))
+    assert bench.band_kernel(window, 512, 32768, 128) == "attention_duo_kernel"
+    assert bench.band_kernel(window, 1, 32768, 128) == "attention_wide_kernel"
+    assert bench.ncu_traffic(5, 512, "band", "attention_pair_kernel")[0] is None
+    monkeypatch.setenv("SPLAT_B200_BAND_TILES", "3")
+    assert bench.band_kernel(window, 512, 32768, 128) == "attention_pair_kernel"

@@ -6,8 +6,8 @@
 // with the MMAs left out 18 %.  So there are two independent tiles per SM here as in attention_wide.cu, but
 //   * the next tile's Q, K and V are on their way, and its first S is computed, while a tile ends.  A CTA per tile spent
 //     9.3 of 28.7 thousand cycles (five steps) on launch, prologue, first copies, epilogue and exit;
-//   * two tiles of one class share every K and V block of the union of their key ranges: half the L2 -> SM traffic, which
-//     came to 8 TB/s (B1 H37 L16384 window 1024);
+//   * two tiles of one class share every K and V block of the union of their key ranges: 1.84 GB read from L2 instead of
+//     2.94 (B1 H16 L32768 window 1024), which had come to 8 TB/s;
 //   * S(j + 1) does not wait for PV(j): P has columns of its own, and the 128 columns that are left hold one S, that of either
 //     tile in turn.  It is read into registers within some 200 cycles of its completion.
 // Tensor memory: P of pipe 0 (64 columns), S (128), P of pipe 1 (64), O of pipe 0 and of pipe 1 (128 each).

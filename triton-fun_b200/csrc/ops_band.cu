@@ -45,6 +45,8 @@ constexpr int kTile = 128;
 constexpr int kStep = 64;
 constexpr int kSubBytes = kTile * 128;          // 128 rows x 128 bytes
 constexpr int kStepBytesPerSub = kStep * 128;   // 64 keys x 128 bytes
+// What these kernels are bound by is instructions: with waits of a few of them (tc_ptx.cuh) and the control block at
+// constant addresses SDDMM at d = 128 went from 70.1 to 66.2 us, SpMM from 70.1 to 68.7 (B4 H16 L4096 window 256).
 constexpr int kThreads = 192;
 constexpr int kTmaWarp = 4;
 constexpr int kMmaWarp = 5;
