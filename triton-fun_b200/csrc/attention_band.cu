@@ -771,8 +771,9 @@ int32_t attention_duo(const void* q, const void* k, int kt_major, const void* v,
 //   dense causal, L 2048    592 70.7 / 66.9   800 79.3 / 88.5   896 85.5 / 104.5  1040 96.4 / 110.8  1184 107 / 117    1480 136 / 141
 //                          1776 163 / 164    2400 215 / 210    4736 422 / 376
 //   strided 8, L 8192       768 47.9 / 53.3   832 50.0 / 59.6  1152 63.9 / 66.1   1472 81.8 / 82.5   1776 101 / 98      2400 133 / 124
+//   documents of 50 - 500   576 44.1 / 41.1   800 53.6 / 56.8  1056 64.0 / 67.4   1184 69.4 / 67.9   1504 84.0 / 82.4   2368 124 / 117
 //   strided 32, L 8192      768 27.2 / 26.6   832 28.8 / 27.0  1152 35.4 / 33.2   1280 39.7 / 37.2   1472 44.2 / 39.6
-// At d = 64 it is no faster (+-200, 1024 tiles 47 / 51).
+// (The plan does not tell blocks and documents from windows.)  At d = 64 it is no faster (+-200, 1024 tiles 47 / 51).
 static int band_kernel_choice(int64_t bh, int64_t n_rows, int64_t d, const int32_t* plan, bool has_table) {
     int forced = 0;
     if (const char* e = getenv("SPLAT_B200_BAND_TILES"))
