@@ -43,10 +43,7 @@ using namespace tc;
 
 namespace duo {
 
-using sm::add2;
 using sm::ex2;
-using sm::fma2;
-using sm::fmax3;
 using sm::mul2;
 using sm::pack2;
 
@@ -587,23 +584,8 @@ attention_duo_kernel(const __grid_constant__ Maps3 maps, const Params p) {
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&ctrl->s_free);
-                if (!__all_sync(0xffffffffu, v_lo <= 0 && v_hi >= kTile)) {
-                    // band edge: keys outside [v_lo, v_hi) become -inf (exp2 -> 0)
-#pragma unroll
-                    for (int ch = 0; ch < kChunks; ++ch) {
-                        const int lo = min(max(v_lo - ch * kChunk, 0), kChunk), hi = min(max(v_hi - ch * kChunk, 0), kChunk);
-                        const uint32_t valid = (hi >= 32 ? ~0u : (1u << hi) - 1) & ~(lo >= 32 ? ~0u : (1u << lo) - 1);
-#pragma unroll
-                        for (int j = 0; j < kChunk; ++j) r[ch * kChunk + j] = (valid & (1u << j)) ? r[ch * kChunk + j] : 0xff800000u;
-                    }
-                }
-                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                for (int j = 0; j < kTile; j += 8)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        mx[i] = fmax3(mx[i], __uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
-                const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc);
+                if (!__all_sync(0xffffffffu, v_lo <= 0 && v_hi >= kTile)) sm::mask_scores(r, v_lo, v_hi);
+                const float m_new = fmaxf(m_used, sm::max_score(r) * sc);
                 // lazy rescale: only when a row's maximum has grown by more than 2^8 (false when both are -inf)
                 const bool need = (m_new - m_used) > kRescaleThreshold;
                 // before a rescale of O or the first store of P, the PV before has to be complete (it usually is)
@@ -625,18 +607,8 @@ attention_duo_kernel(const __grid_constant__ Maps3 maps, const Params p) {
                 float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    uint32_t* c = r + half * (kTile / 2);
                     uint32_t* pk = r + half * (kTile / 4);
-#pragma unroll
-                    for (int j = 0; j < kTile / 2; j += 4) {
-                        float2 a0 = fma2(make_float2(__uint_as_float(c[j]), __uint_as_float(c[j + 1])), sc2, nm2);
-                        float2 a1 = fma2(make_float2(__uint_as_float(c[j + 2]), __uint_as_float(c[j + 3])), sc2, nm2);
-                        a0.x = ex2(a0.x); a0.y = ex2(a0.y); a1.x = ex2(a1.x); a1.y = ex2(a1.y);
-                        acc0 = add2(acc0, a0);
-                        acc1 = add2(acc1, a1);
-                        pk[j >> 1] = pack2<T>(a0.x, a0.y);
-                        pk[(j >> 1) + 1] = pack2<T>(a1.x, a1.y);
-                    }
+                    sm::exp_scores<T, kTile / 2>(r + half * (kTile / 2), pk, sc2, nm2, acc0, acc1);
                     if (half == 0) pv_wait();
                     tmem_st32(p_addr + half * 32, pk);
                     tmem_st_wait();

@@ -47,5 +47,41 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// The pieces of a softmax step over a row's N scores in registers (attention_wide.cu, attention_duo.cu).
+// Band edge: keys outside [lo, hi) become -inf (exp2 -> 0), 32 at a time.
+template <int N>
+__device__ __forceinline__ void mask_scores(uint32_t (&r)[N], int lo, int hi) {
+#pragma unroll
+    for (int c = 0; c < N; c += 32) {
+        const int a = min(max(lo - c, 0), 32), b = min(max(hi - c, 0), 32);
+        const uint32_t valid = (b >= 32 ? ~0u : (1u << b) - 1) & ~(a >= 32 ? ~0u : (1u << a) - 1);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[c + j] = (valid & (1u << j)) ? r[c + j] : 0xff800000u;
+    }
+}
+template <int N>
+__device__ __forceinline__ float max_score(const uint32_t (&r)[N]) {
+    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < N; j += 8)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mx[i] = fmax3(mx[i], __uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
+    return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+}
+// N scores c -> probabilities exp2(c scale + offset), packed into p (which may be c's own front), and two halves of their sum.
+template <typename T, int N>
+__device__ __forceinline__ void exp_scores(const uint32_t* c, uint32_t* p, float2 scale, float2 offset, float2& sum0, float2& sum1) {
+#pragma unroll
+    for (int j = 0; j < N; j += 4) {
+        float2 a0 = fma2(make_float2(__uint_as_float(c[j]), __uint_as_float(c[j + 1])), scale, offset);
+        float2 a1 = fma2(make_float2(__uint_as_float(c[j + 2]), __uint_as_float(c[j + 3])), scale, offset);
+        a0.x = ex2(a0.x); a0.y = ex2(a0.y); a1.x = ex2(a1.x); a1.y = ex2(a1.y);
+        sum0 = add2(sum0, a0);
+        sum1 = add2(sum1, a1);
+        p[j >> 1] = pack2<T>(a0.x, a0.y);
+        p[(j >> 1) + 1] = pack2<T>(a1.x, a1.y);
+    }
+}
+
 }  // namespace sm
 }  // namespace splat
