@@ -121,7 +121,9 @@ int32_t splat_acsr_classify(const float* sTod_lin, const float* sTod_tr, const f
  * K[bh][col][k] = k_ptr[bh*k_stride_bh + col*k_stride_col + k*k_stride_k] (element strides), which
  * covers both a contiguous (BH, d, L) K^T (stride_col = 1, stride_k = L) and the transposed view
  * of a (BH, L, d) tensor (stride_col = d, stride_k = 1).  S and P are (BH, L, trailing_dim).
- * Inputs and outputs share one dtype; accumulation is fp32 (true fp32 FMA for SPLAT_F32).
+ * Inputs and outputs share one dtype; accumulation is fp32.  SPLAT_F32 operands are multiplied with all of their 24 bits: by
+ * fp32 FMA, or, in the fused call, on the tensor cores as three bf16 numbers each (never TF32); there an operand whose
+ * magnitude is below 2^-110 loses precision relative to itself.
  * Slots >= nnz_i of S and P rows are written as zero.
  * ------------------------------------------------------------------------------------------- */
 
@@ -153,7 +155,7 @@ int32_t splat_spmm(const void* p, const void* v, void* o, const float* sTod_lin,
  *   plan_i32 .... HOST pointer to a copy of the 8 ints of splat_acsr_classify, or NULL (then only
  *                 the generic kernel can run)
  *   status_word . device int32 the band kernel sets non-zero if one of its bounded waits gives up;
- *                 may be NULL for the generic path.  The caller clears and reads it.  WHILE THE WORD
+ *                 may be NULL for the generic path (fp32 bands then run on the CUDA cores).  The caller clears and reads it.  WHILE THE WORD
  *                 IS NON-ZERO EVERY TENSOR-CORE KERNEL THAT IS GIVEN IT RETURNS AT ENTRY WITHOUT
  *                 WRITING ITS OUTPUT (the entry point still returns SPLAT_OK: nothing is known at
  *                 enqueue time).  Read the word wherever the stream is synchronised anyway; a

@@ -1,0 +1,124 @@
+"""GPU: the fused fp32 kernel on the tensor cores (operands split into three bf16 numbers) at the edges of its tiles of 128 rows
+and steps of 64 keys, against 64 bits: it must not be further off than the kernel that sums with FMAs."""
+import ctypes
+
+import pytest
+import torch
+
+import acsr_helpers as ah
+import splat_native as n
+
+pytestmark = pytest.mark.gpu
+
+#        mask, L, heads (more than 148 tiles of 32 rows together: below, the register tiles run at d = 32 and 64)
+PATTERNS = [
+    (lambda L: ah.create_causal_windowed_mask(L, L - 1), 128, 38),      # one whole tile
+    (lambda L: ah.create_causal_windowed_mask(L, 63), 129, 31),         # one row in the second tile
+    (lambda L: ah.create_windowed_mask(L, 3), 70, 50),                  # a tile of 70 rows
+    (lambda L: ah.create_windowed_mask(L, 100), 1004, 5),               # K^T in loads of four
+    (lambda L: ah.create_windowed_mask(L, 40), 389, 13),                # K^T key by key
+    (lambda L: ah.create_blocked_mask(L, 48), 200, 22),
+    (lambda L: ah.create_strided_mask(L, 8), 203, 20),                  # classes of 26 and 25 rows, rows with one key
+    (lambda L: ah.create_dilated_mask(L, 40, 3), 301, 13),              # classes of 101 and 100 rows
+    ("documents", 1000, 5),                                             # ragged bands, rows with one key and with none
+]
+
+
+def _mask(mask, L):
+    if mask != "documents":
+        return mask(L)
+    g = torch.Generator().manual_seed(L)
+    row = torch.arange(L)
+    lo, hi = (row - torch.randint(0, 90, (L,), generator=g)).clamp(min=0), row + torch.randint(0, 30, (L,), generator=g)
+    m = (row[None] >= lo[:, None]) & (row[None] <= hi[:, None])
+    m[::17] = False
+    m[5::31] = row[None] == row[5::31, None]
+    return m.to(torch.uint8).cuda()
+
+
+def _exact(q, kt, v, acsr, scale):
+    """Output and log-sum-exp in 64 bits, from the row metadata."""
+    lin, tr, nnz = (t.double() for t in acsr[2:5])
+    stride, start = lin.round().clamp(min=1), (lin * tr).round()
+    off = torch.arange(q.shape[2], device="cuda").double()[None] - start[:, None]
+    on = (off >= 0) & (off < nnz[:, None] * stride[:, None]) & (torch.remainder(off, stride[:, None]) == 0)
+    s = (q.double() @ kt.double() * scale).masked_fill(~on, float("-inf"))
+    return torch.nan_to_num(torch.softmax(s, -1)) @ v.double(), torch.logsumexp(s, -1)
+
+
+def _call(q, kt, v, acsr, scale, status=True):
+    """(output, log-sum-exp); without a status word the register tiles run."""
+    H, L, d = q.shape[1:]
+    o, lse = torch.full_like(q, float("nan")), torch.full((1, H, L), float("nan"), device="cuda")
+    if status:
+        n.attention_fused(q, kt, v, o, acsr[2], acsr[3], acsr[4], scale, lse=lse)
+        n.check_status_word(0)
+        return o, lse
+    plan = (ctypes.c_int32 * 8)(*n.classify(*acsr[2:5]))
+    _bh, ksb, ksk, ksc = n._flat_bh(kt, "kt")
+    assert n._lib.splat_attention_fused_table(
+        q.data_ptr(), kt.data_ptr(), ksb, ksc, ksk, v.data_ptr(), o.data_ptr(), lse.data_ptr(), acsr[2].data_ptr(),
+        acsr[3].data_ptr(), acsr[4].data_ptr(), H, L, L, d, scale, n.dtype_code(q.dtype), n.PATH_AUTO,
+        ctypes.cast(plan, ctypes.c_void_p), None, None, None, n._stream(q.device)) == 0
+    return o, lse
+
+
+def _off(x, ref):
+    ok = torch.isfinite(ref)
+    assert torch.equal(torch.isfinite(x), ok)
+    return ((x.double() - ref)[ok].norm() / ref[ok].norm()).item()
+
+
+def _operands(H, L, d, contiguous, shift=0):
+    g = torch.Generator(device="cuda").manual_seed(L * d + H)
+    q, k, v = (torch.empty(H * L * d + 4, device="cuda").normal_(generator=g)[shift:shift + H * L * d].view(1, H, L, d) for _ in range(3))
+    kt = k.transpose(2, 3)
+    return q, kt.contiguous() if contiguous else kt, v
+
+
+@pytest.mark.parametrize("contiguous", [False, True])
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_no_further_off_than_fma_sums(d, contiguous):
+    for mask, L, H in PATTERNS:
+        acsr = ah.create_acsr(_mask(mask, L), 16, 0)
+        q, kt, v = _operands(H, L, d, contiguous)
+        for scale in (d ** -0.5, -1.0):
+            ref_o, ref_lse = _exact(q, kt, v, acsr, scale)
+            o, lse = _call(q, kt, v, acsr, scale)
+            tile_o, tile_lse = _call(q, kt, v, acsr, scale, status=False)
+            assert not torch.equal(o, tile_o), "the register tiles ran"
+            assert _off(o, ref_o) <= _off(tile_o, ref_o), (L, H, scale)
+            # both end in a value rounded to fp32 (2^-25 of it on average), of which the sums' errors are a part
+            assert _off(lse, ref_lse) <= max(_off(tile_lse, ref_lse), 2 ** -24), (L, H, scale)
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_operands_on_16_bytes_give_the_same_bits(d):
+    """Loads of 32 bytes where the operands allow them, of 16 elsewhere."""
+    L, H = 520, 9
+    acsr = ah.create_acsr(ah.create_windowed_mask(L, 70), 16, 0)
+    for contiguous in (False, True):
+        q, kt, v = _operands(H, L, d, contiguous)
+        o, lse = _call(q, kt, v, acsr, 0.2)
+        q4, k4, v4 = (torch.empty(t.numel() + 4, device="cuda")[4:].view(1, H, L, d).copy_(t) for t in (q, kt.transpose(2, 3), v))
+        kt4 = k4.transpose(2, 3)
+        if contiguous:
+            kt4 = torch.empty(kt.numel() + 4, device="cuda")[4:].view(1, H, d, L).copy_(kt)
+        o4, lse4 = _call(q4, kt4, v4, acsr, 0.2)
+        assert torch.equal(o, o4) and torch.equal(lse, lse4)
+
+
+def test_nothing_is_written_while_the_status_word_is_set():
+    acsr = ah.create_acsr(ah.create_windowed_mask(300, 40), 16, 0)
+    q, kt, v = _operands(40, 300, 64, False)
+    out = torch.full_like(q, 3.0)
+    launch = lambda: n.attention_fused(q, kt, v, out, acsr[2], acsr[3], acsr[4], 0.125)
+    n.status_word(q.device).fill_(7)
+    launch()
+    torch.cuda.synchronize()
+    assert (out == 3.0).all()
+    with pytest.raises(RuntimeError):      # the launcher looks at the host copy of the word
+        launch()
+    launch()
+    n.check_status_word(0)
+    assert torch.isfinite(out).all() and not (out == 3.0).any()

@@ -607,8 +607,9 @@ def attention_fused(q, kt, v, output, sTod_lin, sTod_tr, nnzs, scale: float = 1.
         if plan is None:
             plan = classify(sTod_lin, sTod_tr, nnzs)
         plan_arr = (ctypes.c_int32 * 8)(*plan)
-    if tensor_core:
+    if tensor_core or (path == PATH_AUTO and q.dtype == torch.float32):       # (fp32 bands: attention_split.cu)
         _raise_if_gave_up(dev)
+    if tensor_core:
         rows = _rows_of_k(kt, plan, L) if path == PATH_AUTO else None
         if rows is not None:
             kt, ksb, ksk, ksc = rows, n_cols * d, 1, d

@@ -14,7 +14,7 @@ int32_t attention_generic(const void* q, const void* k, int64_t ksb, int64_t ksc
 int32_t attention_tile_f32(const void* q, const void* k, int64_t ksb, int64_t ksc, int64_t ksk,
                            const void* v, void* o, const float* lin, const float* tr,
                            const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
-                           float scale, const int32_t* plan, float* lse, cudaStream_t st);
+                           float scale, const int32_t* plan, int32_t* status_word, float* lse, cudaStream_t st);
 // Returns SPLAT_ERR_UNSUPPORTED_SHAPE (and launches nothing) when the problem does not qualify.
 int32_t attention_band(const void* q, const void* k, int64_t ksb, int64_t ksc, int64_t ksk,
                        const void* v, void* o, const float* lin, const float* tr,
@@ -132,7 +132,7 @@ extern "C" int32_t splat_attention_fused_table(const void* q, const void* k, int
     int32_t rc = SPLAT_ERR_UNSUPPORTED_SHAPE;
     if (path == SPLAT_PATH_AUTO && dtype == SPLAT_F32)   // register tiles wherever the plan shows bands
         rc = splat::attention_tile_f32(q, k, k_stride_bh, k_stride_col, k_stride_k, v, o, sTod_lin, sTod_tr,
-                                       nnzs, bh, n_rows, n_cols, d, scale, plan_i32, lse, st);
+                                       nnzs, bh, n_rows, n_cols, d, scale, plan_i32, status_word, lse, st);
     if (rc == SPLAT_ERR_UNSUPPORTED_SHAPE)
         rc = splat::attention_generic(q, k, k_stride_bh, k_stride_col, k_stride_k, v, o, sTod_lin, sTod_tr,
                                       nnzs, bh, n_rows, n_cols, d, scale, dtype, lse, st);

@@ -1,4 +1,5 @@
-// fp32 SDDMM, SpMM and fused attention over ACSR on register tiles (CUDA cores, true fp32 FMA).
+// fp32 SDDMM, SpMM and fused attention over ACSR on register tiles (CUDA cores, true fp32 FMA).  Fused attention of more than
+// a wave of these tiles runs on the tensor cores (attention_split.cu).
 //
 // Applies to patterns whose rows, regrouped by residue class, are contiguous bands: one stride s for
 // all rows with more than one non-zero and start_i == i (mod s), as the plan of splat_acsr_classify
@@ -621,6 +622,10 @@ static int32_t run(const Params& p, int64_t bh, cudaStream_t st) {
 
 }  // namespace tile
 
+int32_t attention_split_f32(const void* q, const void* k, int kt, const void* v, void* o, const float* lin, const float* tr,
+                            const float* nnzs, int64_t bh, int64_t n_rows, int64_t d, int64_t stride, float scale,
+                            int32_t* status_word, float* lse, cudaStream_t st);    // attention_split.cu
+
 // Fills p and says whether the tile kernels take the problem (SPLAT_ERR_UNSUPPORTED_SHAPE if not).
 // plan: {max_nnz, stride_min, stride_max, misaligned, n_single, max_col+1, n_empty, n_multi}
 static int32_t tile_setup(tile::Params& p, const int32_t* plan, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
@@ -656,12 +661,21 @@ static int32_t tile_launch(const tile::Params& p, int64_t d, int64_t bh, cudaStr
 
 int32_t attention_tile_f32(const void* q, const void* k, int64_t ksb, int64_t ksc, int64_t ksk, const void* v, void* o,
                            const float* lin, const float* tr, const float* nnzs, int64_t bh, int64_t n_rows,
-                           int64_t n_cols, int64_t d, float scale, const int32_t* plan, float* lse, cudaStream_t st) {
+                           int64_t n_cols, int64_t d, float scale, const int32_t* plan, int32_t* status_word, float* lse,
+                           cudaStream_t st) {
     tile::Params p{};
     if (!q || !k || !v || !o || !lin || !tr || !nnzs) return SPLAT_ERR_UNSUPPORTED_SHAPE;   // left to the row kernel
     const int32_t rc = tile_setup(p, plan, bh, n_rows, n_cols, d, ksb, ksc, ksk, true, 24);
     if (rc != SPLAT_OK) return rc;
     if (!aligned16(k) || !aligned16(v) || !aligned16(o)) return SPLAT_ERR_UNSUPPORTED_SHAPE;
+    // The tensor cores take what is more than a wave of the tiles here: 128 rows to a CTA are coarser pieces of work.  us, here /
+    // there, at 128 and 160 CTAs of 32 rows: +-64 of L1024 d32 9.0 / 9.9, 14.9 / 9.9; d64 12.9 / 15.3, 21.2 / 15.4; d128 22.2 /
+    // 17.8, 36.7 / 17.9; window 32 of L200, 147 and 154: d32 7.3 / 7.4, 12.5 / 7.4; d64 9.7 / 11.5, 17.2 / 11.6; d128 15.5 /
+    // 13.8, 28.1 / 13.8.  At d = 128 they are the faster for less as well (window 32 of L256, 16 CTAs 15.3 / 14.7), but for a
+    // K^T that has to be gathered key by key (strided 16 of L2048, 64 CTAs 21.1 / 21.4).
+    const int64_t of32 = ((n_rows + p.stride - 1) / p.stride + 31) / 32 * p.stride * bh;
+    if (status_word != nullptr && aligned16(q) && scale != 0.f && (of32 > 148 || (d == 128 && (!p.kt || p.stride == 1))))
+        return attention_split_f32(q, k, p.kt, v, o, lin, tr, nnzs, bh, n_rows, d, p.stride, scale, status_word, lse, st);
     p.q = (const float*)q; p.k = (const float*)k; p.v = (const float*)v; p.o = (float*)o; p.lse = lse;
     p.lin = lin; p.tr = tr; p.nnzs = nnzs; p.scale_log2 = scale * kLog2e;
     return tile_launch<tile::Op::kFused>(p, d, bh, st);
