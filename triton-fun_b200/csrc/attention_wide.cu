@@ -23,6 +23,12 @@
 //     30 000 at stride 1 and 3 800 at stride 64; it remains for callers without a table.
 //   * Any d that is a multiple of 8 up to 128 runs: the copies fill a tile's columns past d with zeros, and
 //     the store clips them.  Any L: see band_classes.cuh.
+//   * Classes of up to 64 rows (strided patterns as a rule) have one step of 64 keys at most.  At d <= 64 they have a kernel of
+//     their own with half of the tensor memory, 80 registers a thread and four CTAs per SM.  us, 128-key steps -> this, at
+//     tiles, bf16 d64 strided 64 of L4096 64 4.68 -> 4.43, 256 5.73 -> 5.08, 512 10.07 -> 6.72, 1024 20.1 -> 11.4; strided 64
+//     of L1024 1024 18.4 -> 9.8; L64 causal 1000 19.7 -> 11.0; the same bits.  With two steps it depends on the number of tiles
+//     (class of 128 rows 256 5.97 -> 6.72, 512 12.2 -> 9.5), and with more of them the running maximum is another than
+//     with 128-key steps, so that shards of a problem would not agree bit for bit.
 //   * Few instructions where they are not the point: waits are a try and a counter (looking at the status word, a clock and an
 //     atomic in each of 15 of them were a quarter of the code), the control block has constant addresses, an MMA's
 //     descriptor is an addition.  us, before -> after: fp16 B4 H16 L4096 d64 window 256 64.1 -> 60.7; bf16 B4 H16 L4096
@@ -51,14 +57,12 @@ namespace wide {
 using sm::ex2;
 using sm::pack2;
 
-constexpr int kTile = 128;               // rows of a Q tile, keys of a step
+constexpr int kTile = 128;               // rows of a Q tile
 constexpr int kChunk = 32;               // columns of a tensor-memory load
-constexpr int kChunks = kTile / kChunk;
-constexpr int kSubBytes = kTile * 128;   // one 64-element (128-byte) column chunk of a tile
+constexpr int kSubBytes = kTile * 128;   // one 64-element (128-byte) column chunk of a Q tile
 constexpr int kTmaWarp = 4;
 constexpr int kMmaWarp = 5;
 constexpr int kThreads = 192;            // warps 0-3 softmax and epilogue, 4 TMA, 5 MMA issuer and tensor-memory owner
-constexpr int kTmemCols = 256;
 constexpr float kRescaleThreshold = 8.0f;   // log2 domain: P stays below 2^8 between rescales
 
 // status-word codes (which wait gave up)
@@ -91,7 +95,7 @@ struct Control {
     uint64_t k_full[2], k_free[2], v_full[2], v_free[2];
     uint64_t s_full;           // MMA -> softmax: scores ready (D = 128: and every earlier PV complete)
     uint64_t p_full[2];        // softmax -> MMA: probabilities of keys 0-63 / 64-127 stored (4 warp arrivals)
-    uint64_t s_free, pv_done;  // D = 64.  softmax -> MMA: scores read (4 warp arrivals); MMA -> softmax: PV complete
+    uint64_t s_free, pv_done;  // D = 64, 128-key steps.  softmax -> MMA: scores read (4 warp arrivals); MMA -> softmax: PV complete
     uint32_t tmem_base;
     int32_t abort_at_entry;
     int32_t gave_up;           // code of a wait that ran out
@@ -100,14 +104,24 @@ struct Control {
     alignas(16) uint32_t single[4];  // rows with one non-zero; later those of them whose score is not finite
 };
 
-template <int D> struct Layout {
+// kKeys: keys of a step; with 64 there is one step (classes of up to 64 rows)
+template <int D, int kKeys> struct Layout {
     static constexpr int kSub = D / 64;
-    static constexpr int kTileBytes = kSub * kSubBytes;
-    static constexpr int kSlots = D == 128 ? 1 : 2;         // K tiles, and V tiles, in shared memory
-    static constexpr int kKOff = kTileBytes;                // behind the Q tile
-    static constexpr int kVOff = kKOff + kSlots * kTileBytes;
-    static constexpr int kSmemBytes = kVOff + kSlots * kTileBytes + 1024;   // + alignment slack
+    static constexpr int kQBytes = kSub * kSubBytes;
+    static constexpr int kKeySub = kKeys * 128;             // one 64-element column chunk of a step's K or V
+    static constexpr int kKeyBytes = kSub * kKeySub;
+    static constexpr int kSlots = D == 128 || kKeys == 64 ? 1 : 2;      // steps of K, and of V, in shared memory
+    static constexpr int kKOff = kQBytes;                   // behind the Q tile
+    static constexpr int kVOff = kKOff + kSlots * kKeyBytes;
+    static constexpr int kSmemBytes = kVOff + kSlots * kKeyBytes + 1024;    // + alignment slack
+    static constexpr int kTmemCols = kKeys == 128 ? 256 : 128;
+    static constexpr int kPerSm = kKeys == 128 ? 2 : 4;
 };
+
+// Descriptors of operands in shared memory by their low words (smem_desc_sw128), so that an MMA's is one 32-bit addition.
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(const void* p, uint32_t lbo_bytes) { return ((smem_u32(p) & 0x3ffffu) >> 4) | (lbo_bytes >> 4) << 16; }
+__device__ __forceinline__ uint64_t desc_sw128(uint32_t lo) { return (uint64_t)kDescHi << 32 | lo; }
 
 // O of the warp's rows (n pieces of 16 columns) times corr.  Rare, and kept out of the main loop.
 __device__ __forceinline__ void rescale_o(uint32_t o_addr, int n, float corr) {
@@ -193,13 +207,14 @@ __device__ __forceinline__ uint4 odd_singles(const Params& p, uint4 single, int6
     return make_uint4(rows[0], rows[1], rows[2], rows[3]);
 }
 
-template <typename T, int D, bool kLse, bool kOwn>
-__global__ void __launch_bounds__(kThreads, 2)
+template <typename T, int D, int kKeys, bool kLse, bool kOwn>
+__global__ void __launch_bounds__(kThreads, Layout<D, kKeys>::kPerSm)
 attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
-    using L = Layout<D>;
-    constexpr int kSlots = L::kSlots;
-    constexpr bool kOwnP = D == 64;              // P has tensor-memory columns of its own
-    constexpr uint32_t kPCol = kOwnP ? kTile + D : 0;
+    using L = Layout<D, kKeys>;
+    constexpr int kSlots = L::kSlots, kTmemCols = L::kTmemCols;
+    constexpr bool kOwnP = D == 64 && kKeys == 128;              // P has tensor-memory columns of its own
+    constexpr uint32_t kPCol = kOwnP ? kKeys + D : 0;
+    constexpr int kHalves = kKeys / 64;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + (((smem_u32(smem_raw) + 1023) & ~1023u) - smem_u32(smem_raw));
     __shared__ Control ctrl_mem;             // (static: constant addresses)
@@ -216,16 +231,16 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     int jk = 0, jv = 0;                // TMA warp: K and V tiles requested
     int klo = 0;                       // first 128-key step
     auto load_k = [&]() {
-        const int st = jk % kSlots, row = (klo + jk) * kTile;
+        const int st = jk % kSlots, row = (klo + jk) * kKeys;
         if (jk >= kSlots && !wait_bar(&ctrl->k_free[st], ((uint32_t)(jk / kSlots) & 1u) ^ 1u, &ctrl->gave_up, kErrKFree)) return false;
-        mbar_arrive_expect_tx(&ctrl->k_full[st], L::kTileBytes);
-        uint8_t* dst = smem + L::kKOff + st * L::kTileBytes;
+        mbar_arrive_expect_tx(&ctrl->k_full[st], L::kKeyBytes);
+        uint8_t* dst = smem + L::kKOff + st * L::kKeyBytes;
         if (p.kt_major) {
-            for (int ch = 0; ch < kTile / 64; ++ch)       // 64-key chunks of [d][64 keys]
+            for (int ch = 0; ch < kHalves; ++ch)       // 64-key chunks of [d][64 keys]
                 tma_load_4d(dst + ch * (D * 128), map + 1, &ctrl->k_full[st], row + ch * 64, 0, (int)bh, 0);
         } else {
             for (int sub = 0; sub < L::kSub; ++sub)
-                tma_load_4d(dst + sub * kSubBytes, map + 1, &ctrl->k_full[st], sub * 64, res, row, (int)bh);
+                tma_load_4d(dst + sub * L::kKeySub, map + 1, &ctrl->k_full[st], sub * 64, res, row, (int)bh);
         }
         ++jk;
         return true;
@@ -233,10 +248,10 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     auto load_v = [&]() {
         const int st = jv % kSlots;
         if (jv >= kSlots && !wait_bar(&ctrl->v_free[st], ((uint32_t)(jv / kSlots) & 1u) ^ 1u, &ctrl->gave_up, kErrVFree)) return false;
-        mbar_arrive_expect_tx(&ctrl->v_full[st], L::kTileBytes);
+        mbar_arrive_expect_tx(&ctrl->v_full[st], L::kKeyBytes);
         for (int sub = 0; sub < L::kSub; ++sub)
-            tma_load_4d(smem + L::kVOff + st * L::kTileBytes + sub * kSubBytes, map + 2, &ctrl->v_full[st], sub * 64, res,
-                        (klo + jv) * kTile, (int)bh);
+            tma_load_4d(smem + L::kVOff + st * L::kKeyBytes + sub * L::kKeySub, map + 2, &ctrl->v_full[st], sub * 64, res,
+                        (klo + jv) * kKeys, (int)bh);
         ++jv;
         return true;
     };
@@ -269,11 +284,11 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
             ctrl->abort_at_entry = stop;
             ctrl->gave_up = 0;
             if (stop == 0) {
-                mbar_arrive_expect_tx(&ctrl->q_full, L::kTileBytes);
+                mbar_arrive_expect_tx(&ctrl->q_full, L::kQBytes);
                 for (int sub = 0; sub < L::kSub; ++sub)
                     tma_load_4d(smem + sub * kSubBytes, map, &ctrl->q_full, sub * 64, res, u0, (int)bh);
                 if (range.y > 0) {
-                    klo = range.x / kTile;
+                    klo = range.x / kKeys;
                     load_k();
                     load_v();
                 }
@@ -317,8 +332,8 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     if (hi64 <= 0) lo64 = 0;
     lo64 = lo64 / 64;          // in 64-key units from here
     hi64 = (hi64 + 63) / 64;
-    klo = lo64 >> 1;
-    const int steps = ((hi64 + 1) >> 1) - klo;   // 128-key steps
+    klo = lo64 / kHalves;
+    const int steps = (hi64 + kHalves - 1) / kHalves - klo;
     auto wait_all = [&](uint64_t* bar, uint32_t parity, int code) { return tc::wait_all(bar, parity, &ctrl->gave_up, code); };
 
     if (warp == kTmaWarp) {
@@ -349,59 +364,61 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
         if (steps > 0) {
             const bool lead = elect_one();
             constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-            const uint32_t idesc_qk = instr_desc_f16(fmt, kTile, kTile, p.kt_major ? 1u : 0u);
+            const uint32_t idesc_qk = instr_desc_f16(fmt, kTile, kKeys, p.kt_major ? 1u : 0u);
             const uint32_t idesc_qk_half = instr_desc_f16(fmt, kTile, 64, p.kt_major ? 1u : 0u);
             constexpr uint32_t idesc_pv = instr_desc_f16(fmt, kTile, D, 1);
-            const uint64_t q_desc = smem_desc_sw128(smem_u32(smem), 16, 1024);
-            const uint64_t k_desc = smem_desc_sw128(smem_u32(smem + L::kKOff), p.kt_major ? D * 128 : 16, 1024);
-            const uint64_t v_desc = smem_desc_sw128(smem_u32(smem + L::kVOff), kSubBytes, 1024);
-            const uint32_t k_step = (p.kt_major ? 2048 : 32) >> 4, k_sub = (p.kt_major ? 4 * 2048 : kSubBytes) >> 4;
-            const uint32_t o_tmem = tmem_base + kTile;
+            const uint32_t q_lo = desc_lo(smem, 16), k_lo = desc_lo(smem + L::kKOff, p.kt_major ? D * 128 : 16);
+            const uint32_t v_lo = desc_lo(smem + L::kVOff, L::kKeySub);
+            const uint32_t k_step = (p.kt_major ? 2048 : 32) >> 4, k_sub = (p.kt_major ? 4 * 2048 : L::kKeySub) >> 4;
+            const uint32_t o_tmem = tmem_base + kKeys;
             auto commit = [&](uint64_t* bar) { if (lead) mma_commit(bar); };
-            auto in_range = [&](int j, int half) { const int i = 2 * (klo + j) + half; return i >= lo64 && i < hi64; };
+            auto in_range = [&](int j, int half) { const int i = 2 * (klo + j) + half; return kHalves == 1 || (i >= lo64 && i < hi64); };
             bool ok = wait_all(&ctrl->q_full, 0, kErrQ);
             bool first_pv = true;
+            auto k_here = [&](int j) { return wait_all(&ctrl->k_full[j % kSlots], (uint32_t)(j / kSlots) & 1u, kErrKFull); };
             auto issue_s = [&](int j) {                // S(j); half steps outside the range are left out
                 const int st = j % kSlots;
-                ok = wait_all(&ctrl->k_full[st], (uint32_t)(j / kSlots) & 1u, kErrKFull);
-                if (!ok) return;
                 tc_fence_after_sync();
                 const bool h0 = in_range(j, 0), both = h0 && in_range(j, 1);
-                const uint32_t idesc = both ? idesc_qk : idesc_qk_half;
+                const uint32_t idesc = kHalves == 1 || both ? idesc_qk : idesc_qk_half;
                 const uint32_t skip = h0 ? 0u : 1u;
-                const uint32_t b_base = st * L::kTileBytes + skip * (p.kt_major ? D * 128 : 64 * 128);
                 if (lead) {
-                    uint64_t da = q_desc, db = k_desc + (b_base >> 4);
-#pragma unroll 1
-                    for (int sub = 0; sub < L::kSub; ++sub, da += kSubBytes >> 4, db += k_sub)
+                    const uint32_t to = tmem_base + skip * 64;
+                    uint32_t b = k_lo + ((st * L::kKeyBytes + skip * (p.kt_major ? D * 128 : 64 * 128)) >> 4);
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) mma_ss(tmem_base + skip * 64, da + kk * 2, db + kk * k_step, idesc, sub + kk > 0);
+                    for (int sub = 0; sub < L::kSub; ++sub, b += k_sub)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            mma_ss(to, desc_sw128(q_lo + ((sub * kSubBytes + kk * 32) >> 4)), desc_sw128(b + kk * k_step), idesc, sub + kk > 0);
                     mma_commit(&ctrl->s_full);
                     mma_commit(&ctrl->k_free[st]);
                 }
                 __syncwarp();
             };
+            if (ok) ok = k_here(0);
             if (ok) issue_s(0);
             for (int j = 0; j < steps && ok; ++j) {
                 if (kOwnP && j + 1 < steps) {          // the next scores as soon as these have been read
-                    ok = wait_all(&ctrl->s_free, (uint32_t)j & 1u, kErrSFree);
-                    if (ok) issue_s(j + 1);
+                    ok = k_here(j + 1) && wait_all(&ctrl->s_free, (uint32_t)j & 1u, kErrSFree);
                     if (!ok) break;
+                    issue_s(j + 1);
                 }
                 const int st = j % kSlots;
                 ok = wait_all(&ctrl->v_full[st], (uint32_t)(j / kSlots) & 1u, kErrVFull);
                 if (!ok) break;
 #pragma unroll 1
-                for (int half = 0; half < 2; ++half) {
-                    ok = wait_all(&ctrl->p_full[half], (uint32_t)j & 1u, kErrP);
+                for (int half = 0; half < kHalves; ++half) {
+                    // (the next K, which S(j + 1) takes right behind this, first: it is there as a rule)
+                    if (!kOwnP && half == kHalves - 1 && j + 1 < steps) ok = k_here(j + 1);
+                    if (ok) ok = wait_all(&ctrl->p_full[half], (uint32_t)j & 1u, kErrP);
                     if (!ok) break;
                     tc_fence_after_sync();
                     if (in_range(j, half)) {
                         if (lead) {
-                            const uint64_t db = v_desc + (uint32_t)((st * L::kTileBytes >> 4) + half * 512);
+                            const uint32_t b = v_lo + (uint32_t)(st * L::kKeyBytes >> 4) + half * 512;
 #pragma unroll
                             for (int kk = 0; kk < 4; ++kk)
-                                mma_ts(o_tmem, tmem_base + kPCol + half * 32 + kk * 8, db + kk * 128, idesc_pv, (!first_pv || kk > 0) ? 1u : 0u);
+                                mma_ts(o_tmem, tmem_base + kPCol + half * 32 + kk * 8, desc_sw128(b + kk * 128), idesc_pv, (!first_pv || kk > 0) ? 1u : 0u);
                         }
                         __syncwarp();
                         first_pv = false;
@@ -420,7 +437,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     } else {
         // ------------------------------------------------------------------ softmax + epilogue
         const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
-        const uint32_t s_addr = lane_addr, o_addr = lane_addr + kTile, p_addr = lane_addr + kPCol;
+        const uint32_t s_addr = lane_addr, o_addr = lane_addr + kKeys, p_addr = lane_addr + kPCol;
         const float sc = p.scale_log2;
         const float2 sc2 = make_float2(sc, sc);
         float m_used = -INFINITY, l_sum = 0.f;
@@ -429,51 +446,95 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
             ok = wait_all(&ctrl->s_full, (uint32_t)k & 1u, kErrS);
             if (!ok) break;
             tc_fence_after_sync();
-            const int c0 = (klo + k) * kTile;
+            const int c0 = (klo + k) * kKeys;
             const int v_lo = my_begin - c0, v_hi = my_end - c0;  // valid keys of this step: [v_lo, v_hi)
-            // D = 64: before the first store of P or a rescale of O, PV(k-1) has to be complete (it usually is)
+            // P with columns of its own: before the first store of P or a rescale of O, PV(k-1) has to be complete (it usually is)
             auto pv_wait = [&]() {
                 if (!kOwnP || k == 0) return true;
                 const bool r = wait_all(&ctrl->pv_done, (uint32_t)(k - 1) & 1u, kErrPv);
                 tc_fence_after_sync();
                 return r;
             };
-            auto scores_read = [&]() {
-                if (!kOwnP) return;
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&ctrl->s_free);
-            };
-            uint32_t r[kTile];
-#pragma unroll
-            for (int ch = 0; ch < kChunks; ++ch) tmem_ld32(s_addr + ch * kChunk, r + ch * kChunk);
-            tmem_ld_wait();
-            scores_read();
-            if (!__all_sync(0xffffffffu, v_lo <= 0 && v_hi >= kTile)) sm::mask_scores(r, v_lo, v_hi);
-            const float m_new = fmaxf(m_used, sm::max_score(r) * sc);
-            // lazy rescale: only when a row's maximum has grown by more than 2^8 (false when both are -inf)
-            const bool need = (m_new - m_used) > kRescaleThreshold;
-            if (__any_sync(0xffffffffu, need)) {
-                ok = pv_wait();
-                if (!ok) break;
-                const float corr = need ? ex2(m_used - m_new) : 1.f;
+            // Lazy rescale: only when a row's maximum has grown by more than 2^8 (false when both are -inf).
+            float corr = 1.f;
+            auto grown = [&](float mx) {
+                const float m_new = fmaxf(m_used, mx * sc);
+                const bool need = (m_new - m_used) > kRescaleThreshold;
+                corr = need ? ex2(m_used - m_new) : 1.f;
                 if (need) m_used = m_new;
-                l_sum *= corr;
-                if (k > 0) rescale_o(o_addr, D / 16, corr);
-            }
-            const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
-            const float2 nm2 = make_float2(-m_eff, -m_eff);
-            float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t* pk = r + half * (kTile / 4);
-                sm::exp_scores<T, kTile / 2>(r + half * (kTile / 2), pk, sc2, nm2, acc0, acc1);
-                if (kOwnP && half == 0) ok = pv_wait();
-                tmem_st32(p_addr + half * 32, pk);
+                const bool any = __any_sync(0xffffffffu, need);
+                if (any) l_sum *= corr;
+                return any;
+            };
+            auto offset = [&]() {
+                const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
+                return make_float2(-m_eff, -m_eff);
+            };
+            auto p_stored = [&](int half) {           // on its way to the tensor core
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&ctrl->p_full[half]);      // half 0: on its way to the tensor core
+                if (lane == 0) mbar_arrive(&ctrl->p_full[half]);
+            };
+            float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+            if constexpr (kKeys == 64) {
+                // The scores are fetched twice, 32 at a time, for four CTAs per SM (80 registers a thread).  Pieces outside all of
+                // a warp's bands are not fetched (their P is 0), pieces inside all of them not masked.
+                uint32_t r[32];
+                bool none[2], whole[2];
+                float mx = -INFINITY;
+#pragma unroll
+                for (int ch = 0; ch < 2; ++ch) {
+                    const int a = v_lo - ch * 32, b = v_hi - ch * 32;
+                    none[ch] = __all_sync(0xffffffffu, a >= 32 || b <= 0);
+                    whole[ch] = __all_sync(0xffffffffu, a <= 0 && b >= 32);
+                    if (none[ch]) continue;
+                    tmem_ld32(s_addr + ch * 32, r);
+                    tmem_ld_wait();
+                    if (!whole[ch]) sm::mask_scores(r, a, b);
+                    mx = fmaxf(mx, sm::max_score(r));
+                }
+                m_used = mx * sc;          // (the only step)
+                const float2 nm2 = offset();
+#pragma unroll
+                for (int ch = 0; ch < 2; ++ch) {
+                    if (none[ch]) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) r[i] = 0u;
+                    } else {
+                        tmem_ld32(s_addr + ch * 32, r);
+                        tmem_ld_wait();
+                        if (!whole[ch]) sm::mask_scores(r, v_lo - ch * 32, v_hi - ch * 32);
+                        sm::exp_scores<T, 32>(r, r, sc2, nm2, acc0, acc1);
+                    }
+                    tmem_st16(p_addr + ch * 16, r);
+                }
+                p_stored(0);
+            } else {
+                uint32_t r[kKeys];
+#pragma unroll
+                for (int ch = 0; ch < kKeys / kChunk; ++ch) tmem_ld32(s_addr + ch * kChunk, r + ch * kChunk);
+                tmem_ld_wait();
+                if (kOwnP) {                       // the next scores may be formed
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctrl->s_free);
+                }
+                if (!__all_sync(0xffffffffu, v_lo <= 0 && v_hi >= kKeys)) sm::mask_scores(r, v_lo, v_hi);
+                if (grown(sm::max_score(r)) && k > 0) {
+                    ok = pv_wait();
+                    if (!ok) break;
+                    rescale_o(o_addr, D / 16, corr);
+                }
+                const float2 nm2 = offset();
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t* pk = r + half * 32;
+                    sm::exp_scores<T, 64>(r + half * 64, pk, sc2, nm2, acc0, acc1);
+                    if (kOwnP && half == 0) ok = pv_wait();
+                    tmem_st32(p_addr + half * 32, pk);
+                    p_stored(half);
+                }
             }
             l_sum += (acc0.x + acc0.y) + (acc1.x + acc1.y);
             if (!ok) break;
@@ -509,23 +570,24 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
         }
         const T* vrow = reinterpret_cast<const T*>(p.v) + (head + row_start) * p.d;
         const int t = warp * 32 + lane;
-        uint32_t o_raw[D];
+        constexpr int kRead = kKeys == 64 ? 32 : D;             // columns of O in registers at a time
+        uint32_t o_raw[kRead];
         float2 odd0 = make_float2(0.f, 0.f), odd1 = odd0;       // not finite: nor is the row
-        if (have_o && ok) {
-#pragma unroll
-            for (int ch = 0; ch < D / 32; ++ch) tmem_ld32(o_addr + ch * 32, o_raw + ch * 32);
-            tmem_ld_wait();
-            if constexpr (kOwn) {
-#pragma unroll
-                for (int j = 0; j < D; j += 8) {
-                    odd0 = note_nonfinite(odd0, o_raw + j);
-                    odd1 = note_nonfinite(odd1, o_raw + j + 4);
-                }
-            }
-        }
 #pragma unroll
         for (int ch = 0; ch < D / 32; ++ch) {
-            const uint32_t* r = o_raw + ch * 32;
+            if (ch * 32 % kRead == 0 && have_o && ok) {
+#pragma unroll
+                for (int i = 0; i < kRead; i += 32) tmem_ld32(o_addr + ch * 32 + i, o_raw + i);
+                tmem_ld_wait();
+                if constexpr (kOwn) {
+#pragma unroll
+                    for (int j = 0; j < kRead; j += 8) {
+                        odd0 = note_nonfinite(odd0, o_raw + j);
+                        odd1 = note_nonfinite(odd1, o_raw + j + 4);
+                    }
+                }
+            }
+            const uint32_t* r = o_raw + ch * 32 % kRead;
             uint4 out[4];
             uint32_t* o32 = reinterpret_cast<uint32_t*>(out);
             if (row_nnz > 1 && have_o && ok) {
@@ -581,13 +643,13 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
 // B8 H64 L32768 d128 window 1024 11.71 -> 12.12 ms).  Problems with d = 64 or 128 and classes of one length do without:
 // they have only ever run on tensor cores, with finite V as a condition (splat_b200.h); the others came from the row
 // kernels, which read nothing but a row's own keys.
-template <typename T, int D>
+template <typename T, int D, int kKeys>
 static int32_t launch(const Maps<4>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
     const bool own = (prm.d != 64 && prm.d != 128) || prm.cls.longer != 0;
-    auto kern = own ? (prm.lse != nullptr ? attention_wide_kernel<T, D, true, true> : attention_wide_kernel<T, D, false, true>)
-                    : (prm.lse != nullptr ? attention_wide_kernel<T, D, true, false> : attention_wide_kernel<T, D, false, false>);
-    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), Layout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
-    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, Layout<D>::kSmemBytes, st, maps, prm);
+    auto kern = own ? (prm.lse != nullptr ? attention_wide_kernel<T, D, kKeys, true, true> : attention_wide_kernel<T, D, kKeys, false, true>)
+                    : (prm.lse != nullptr ? attention_wide_kernel<T, D, kKeys, true, false> : attention_wide_kernel<T, D, kKeys, false, false>);
+    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), Layout<D, kKeys>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
+    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, Layout<D, kKeys>::kSmemBytes, st, maps, prm);
 }
 
 }  // namespace wide
@@ -606,20 +668,26 @@ int32_t attention_wide(const void* q, const void* k, int kt_major, const void* v
     p.cls = Classes(n_rows, stride, wide::kTile);
     p.rows = reinterpret_cast<const int2*>(band_table);
     p.tiles = band_table != nullptr ? p.rows + n_rows : nullptr;
+    // Classes of up to 64 rows at d <= 64: the kernel with 64-key steps, see above.
+    const bool one_step = d <= 64 && p.cls.rows + (p.cls.longer > 0 ? 1 : 0) <= 64;
+    const int keys = one_step ? 64 : 128;
     Maps<4> maps;
     for (int part = 0; part < 2; ++part) {
         if (!p.cls.has(part)) continue;
         CUtensorMap* m = maps.part[part];
         if (!p.cls.view(m, q, dtype, bh, n_rows, d, stride, part, wide::kTile) ||
             !(kt_major ? make_map_kt(m + 1, k, dtype, bh, n_rows, d, d > 64 ? 128 : 64)
-                       : p.cls.view(m + 1, k, dtype, bh, n_rows, d, stride, part, wide::kTile)) ||
-            !p.cls.view(m + 2, v, dtype, bh, n_rows, d, stride, part, wide::kTile) ||
+                       : p.cls.view(m + 1, k, dtype, bh, n_rows, d, stride, part, keys)) ||
+            !p.cls.view(m + 2, v, dtype, bh, n_rows, d, stride, part, keys) ||
             !p.cls.view(m + 3, o, dtype, bh, n_rows, d, stride, part, 32))
             return SPLAT_ERR_DRIVER;
     }
-    return dtype == SPLAT_BF16
-        ? (d > 64 ? wide::launch<__nv_bfloat16, 128>(maps, p, bh, st) : wide::launch<__nv_bfloat16, 64>(maps, p, bh, st))
-        : (d > 64 ? wide::launch<__half, 128>(maps, p, bh, st) : wide::launch<__half, 64>(maps, p, bh, st));
+    auto launch = [&](auto element) {
+        using T = decltype(element);
+        if (d > 64) return wide::launch<T, 128, 128>(maps, p, bh, st);
+        return one_step ? wide::launch<T, 64, 64>(maps, p, bh, st) : wide::launch<T, 64, 128>(maps, p, bh, st);
+    };
+    return dtype == SPLAT_BF16 ? launch(__nv_bfloat16()) : launch(__half());
 }
 
 }  // namespace splat
