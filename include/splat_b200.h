@@ -122,8 +122,8 @@ int32_t splat_acsr_classify(const float* sTod_lin, const float* sTod_tr, const f
  * covers both a contiguous (BH, d, L) K^T (stride_col = 1, stride_k = L) and the transposed view
  * of a (BH, L, d) tensor (stride_col = d, stride_k = 1).  S and P are (BH, L, trailing_dim).
  * Inputs and outputs share one dtype; accumulation is fp32.  SPLAT_F32 operands are multiplied with all of their 24 bits: by
- * fp32 FMA, or, in the fused call, on the tensor cores as three bf16 numbers each (never TF32); there an operand whose
- * magnitude is below 2^-110 loses precision relative to itself.
+ * fp32 FMA, or on the tensor cores as three bf16 numbers each (never TF32); there an operand whose magnitude is below
+ * 2^-110 loses precision relative to itself.
  * Slots >= nnz_i of S and P rows are written as zero.
  * ------------------------------------------------------------------------------------------- */
 
@@ -232,7 +232,9 @@ int32_t splat_spmm_band(const void* p, const void* v, void* o, const float* sTod
                         int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
                         const int32_t* plan_i32, int32_t* status_word, void* stream);
 
-/* SDDMM / SpMM of fp32 operands on register tiles (true fp32 FMA), for patterns whose rows are bands
+/* SDDMM / SpMM of fp32 operands, for patterns whose rows are bands: on register tiles (true fp32 FMA), or, from one or two waves of
+ * them on and if the current device has a status word with a host copy (splat_set_status_mirror), on the tensor cores, which then
+ * work with that word as the band kernels do with theirs.  Rows are bands
  * of one stride (plan_i32 as from splat_acsr_classify); n_rows need not be a multiple of the stride.
  * d = 32, 64 or 128, K as rows of d or as a contiguous (BH, d, n_cols) array.  Otherwise
  * SPLAT_ERR_UNSUPPORTED_SHAPE / SPLAT_ERR_MISALIGNED without a launch: use splat_sddmm / splat_spmm. */

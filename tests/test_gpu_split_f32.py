@@ -122,3 +122,70 @@ def test_nothing_is_written_while_the_status_word_is_set():
     launch()
     n.check_status_word(0)
     assert torch.isfinite(out).all() and not (out == 3.0).any()
+
+
+#        mask, L, heads: more than two waves of tiles of 32 rows
+OPS = [
+    (lambda L: ah.create_causal_windowed_mask(L, L - 1), 128, 75),
+    (lambda L: ah.create_windowed_mask(L, 33), 129, 60),
+    (lambda L: ah.create_windowed_mask(L, 100), 1004, 10),
+    (lambda L: ah.create_windowed_mask(L, 40), 389, 23),
+    (lambda L: ah.create_strided_mask(L, 8), 330, 19),                  # classes of 42 and 41 rows
+    (lambda L: ah.create_dilated_mask(L, 40, 3), 301, 25),
+    ("documents", 1000, 10),
+]
+
+
+def _slots(acsr, L, T):
+    """Column of every slot (clamped) and whether it holds a non-zero."""
+    lin, tr, nnz = (t.double() for t in acsr[2:5])
+    stride, start = lin.round().clamp(min=1), (lin * tr).round()
+    j = torch.arange(T, device="cuda").double()
+    return (start[:, None] + j[None] * stride[:, None]).long().clamp(0, L - 1), j[None] < nnz[:, None]
+
+
+@pytest.mark.parametrize("contiguous", [False, True])
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_sddmm_and_spmm(d, contiguous):
+    for mask, L, H in OPS:
+        acsr = ah.create_acsr(_mask(mask, L), 16, 0)
+        meta, T = acsr[2:5], acsr[5]
+        cols, on = _slots(acsr, L, T)
+        q, kt, v = _operands(H, L, d, contiguous)
+        s = torch.full((1, H, L, T), float("nan"), device="cuda")
+        n.sddmm(q, kt, s, *meta, T)
+        n.check_status_word(0)
+        full = q.double() @ kt.double()
+        ref = torch.gather(full, 3, cols[None, None].expand(1, H, L, T)) * on
+        assert torch.count_nonzero(s * ~on) == 0, "padding slots must be zero"
+        # what a chain of d fp32 additions, rounded to nearest, is off by on average: 0.5 sqrt(d / 3) 2^-24 of the result
+        assert _off(s, ref) <= 0.5 * (d / 3) ** 0.5 * 2 ** -24, (L, H)
+        # SpMM of probabilities; padding slots are not read
+        p = torch.softmax(torch.where(on, ref * d ** -0.5, torch.tensor(float("-inf"), device="cuda").double()), -1)
+        p = torch.where(on, torch.nan_to_num(p), torch.tensor(float("nan"), device="cuda").double()).float()
+        o = torch.full((1, H, L, d), float("nan"), device="cuda")
+        n.spmm(p, v, o, *meta, T)
+        n.check_status_word(0)
+        dense = torch.zeros(1, H, L, L, device="cuda", dtype=torch.double)
+        dense.scatter_add_(3, cols[None, None].expand(1, H, L, T), torch.where(on, p, torch.zeros((), device="cuda")).double())
+        # a rounded result is off by 2^-25 of itself on average, a few additions by as much
+        assert _off(o, dense @ v.double()) <= 2 ** -23, (L, H)
+
+
+def test_sddmm_scores_that_are_not_finite():
+    """An infinity is no sum of three bf16 numbers: such rows are computed again, as the row kernels give them."""
+    L, H, d = 300, 40, 64
+    acsr = ah.create_acsr(ah.create_windowed_mask(L, 20), 16, 0)
+    meta, T = acsr[2:5], acsr[5]
+    q, kt, _v = _operands(H, L, d, False)
+    k = kt.transpose(2, 3)
+    k[:, :, 50, 3], k[:, :, 120, 5], q[:, :, 200, 7] = float("inf"), float("nan"), float("-inf")
+    q[:, :, 250, 0], k[:, :, 250, 0] = 3.4e38, 1e-30      # rounds to infinity in bf16
+    s, rows = torch.empty(1, H, L, T, device="cuda"), torch.empty(1, H, L, T, device="cuda")
+    n.sddmm(q, kt, s, *meta, T)
+    n.sddmm(q, kt, rows, *meta, T, n.PATH_GENERIC)
+    n.check_status_word(0)
+    ok = torch.isfinite(rows)
+    assert not ok.all() and torch.equal(torch.isfinite(s), ok)
+    assert torch.equal(torch.isnan(s), torch.isnan(rows)) and torch.equal(s[torch.isinf(s)], rows[torch.isinf(rows)])
+    assert (s[ok] - rows[ok]).abs().max() <= 1e-5 * rows[ok].abs().max()

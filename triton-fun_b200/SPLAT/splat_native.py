@@ -499,6 +499,7 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
     if x.dtype == torch.float32 and path == PATH_AUTO and x.numel() > 0:
         plan = _plan_unless_captured(sTod_lin, sTod_tr, nnzs)
     if plan is not None:
+        _raise_if_gave_up(dev)             # (a tensor-core kernel may run: ops_split.cu)
         plan_arr = (ctypes.c_int32 * 8)(*plan)
         with _on(dev):
             rc = _lib.splat_sddmm_tile(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
@@ -566,6 +567,7 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
     if x.dtype == torch.float32 and path == PATH_AUTO and x.numel() > 0:
         plan = _plan_unless_captured(sTod_lin, sTod_tr, nnzs)
     if plan is not None:
+        _raise_if_gave_up(dev)             # (a tensor-core kernel may run: ops_split.cu)
         plan_arr = (ctypes.c_int32 * 8)(*plan)
         with _on(dev):
             rc = _lib.splat_spmm_tile(x.data_ptr(), y.data_ptr(), output.data_ptr(),

@@ -31,10 +31,8 @@
 // d32 and d128, where there is room, 64 against 70 and 171 against 189).
 #include <limits.h>
 
-#include "common.cuh"
 #include "row_exact.cuh"
-#include "softmax_math.cuh"
-#include "tc_ptx.cuh"
+#include "split_f32.cuh"
 
 namespace splat {
 namespace band {
@@ -43,19 +41,10 @@ bool allow_dynamic_smem(const void* kernel, int bytes);   // attention_band.cu
 
 namespace split {
 
-using namespace tc;
-using sm::add2;
 using sm::ex2;
-using sm::fma2;
 using sm::mul2;
 
-constexpr int kTile = 128;               // rows of a tile
-constexpr int kKeys = 64;                // keys of a step
-constexpr int kWorkers = 256;            // warps 0-7: copies, softmax, epilogue; thread = (row, half of the columns)
-constexpr int kMmaWarp = 8;
 constexpr int kThreads = kWorkers + 128;   // (a warpgroup more: registers are handed from it to the others)
-constexpr int kSubBytes = kKeys * 128;   // 64 rows x 64 bf16
-
 // status-word codes (which wait gave up)
 enum : int { kErrK = 81, kErrP = 82, kErrS = 83, kErrO = 84, kErrMax = 85 };
 
@@ -95,8 +84,7 @@ struct Control {
 };
 
 template <int D> struct Layout {
-    static constexpr int kSub = D == 128 ? 2 : 1;
-    static constexpr int kPiece = kSub * kSubBytes;       // one of three of a step's K or V
+    static constexpr int kPiece = kPieceBytes<D>;
     static constexpr int kOperand = 3 * kPiece;
     // Q's pieces m and l in shared memory where tensor memory has no room for them beside two CTAs' other operands
     static constexpr bool kQSmem = D == 64;
@@ -110,51 +98,11 @@ template <int D> struct Layout {
     static constexpr int kO = kP + 3 * kKeys / 2;
     static constexpr int kTmemCols = D == 128 ? 512 : 256;
     static_assert(kO + D <= kTmemCols, "tensor memory");
-    static constexpr int kUnits = kKeys * D / 8 / kWorkers;   // pieces of 8 elements of a step's K or V per thread
     // Scores are fetched again for their exponentials where the registers of two CTAs do not hold them beside the rest; their
     // place is free, and the next S can begin, the later for it.
     static constexpr bool kAgain = D == 64;
     static constexpr int kWorkerRegs = D == 128 ? 232 : 104, kOtherRegs = D == 128 ? 40 : 32;   // of 168, 80 at the launch
 };
-
-__device__ __forceinline__ void load8(float (&x)[8], const float* p, int vec) {
-    if (vec == 8) {
-        asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7]) : "l"(p));
-    } else {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-        x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-    }
-}
-// two numbers -> their three bf16 pieces, packed
-__device__ __forceinline__ void split2(float2 x, uint32_t& h, uint32_t& m, uint32_t& l) {
-    const float2 minus = make_float2(-1.f, -1.f);
-    h = sm::pack2<__nv_bfloat16>(x.x, x.y);
-    x = fma2(make_float2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus, x);
-    m = sm::pack2<__nv_bfloat16>(x.x, x.y);
-    x = fma2(make_float2(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u)), minus, x);
-    l = sm::pack2<__nv_bfloat16>(x.x, x.y);
-}
-__device__ __forceinline__ void split8(const float (&x)[8], uint4& h, uint4& m, uint4& l) {
-    split2(make_float2(x[0], x[1]), h.x, m.x, l.x);
-    split2(make_float2(x[2], x[3]), h.y, m.y, l.y);
-    split2(make_float2(x[4], x[5]), h.z, m.z, l.z);
-    split2(make_float2(x[6], x[7]), h.w, m.w, l.w);
-}
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, uint4 r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
-                 : "memory");
-}
-// D[tmem] (+)= A * B with the operands' descriptors given by their low words.  (`lo` is hidden from the compiler where it is
-// formed, which otherwise keeps the sums of all 48 MMAs of a step in registers.)
-constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);     // groups of 8 rows 1024 bytes apart, version 1, 128-byte swizzle
-__device__ __forceinline__ uint32_t desc_lo(const void* p, uint32_t lbo_bytes) { return ((smem_u32(p) & 0x3ffffu) >> 4) | (lbo_bytes >> 4) << 16; }
-__device__ __forceinline__ uint32_t hidden(uint32_t x) {
-    asm volatile("" : "+r"(x));
-    return x;
-}
-__device__ __forceinline__ uint64_t desc(uint32_t lo) { return (uint64_t)kDescHi << 32 | lo; }
 
 // Columns outside [lo, hi) become -inf.
 __device__ __forceinline__ void mask16(uint32_t (&r)[16], int lo, int hi) {
@@ -163,10 +111,6 @@ __device__ __forceinline__ void mask16(uint32_t (&r)[16], int lo, int hi) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) r[j] = (valid & (1u << j)) ? r[j] : 0xff800000u;
 }
-
-// The six products: piece (0 h, 1 m, 2 l) of A and of B, the largest product last.
-__host__ __device__ constexpr int piece_a(int i) { return (0x001102 >> (4 * i)) & 15; }
-__host__ __device__ constexpr int piece_b(int i) { return (0x010120 >> (4 * i)) & 15; }
 
 template <int D, bool kKt, bool kLse>
 __global__ void __launch_bounds__(kThreads, Layout<D>::kPerSm)
@@ -310,50 +254,11 @@ attention_split_kernel(const __grid_constant__ Params p) {
         const int my_a = banded ? (about.x - res) / p.stride : 0, my_n = banded ? about.y : 0;     // the row's band, in class coordinates
         const float* kbase = kKt ? p.k + head * D : p.k + (head + res) * D;
         const float* vbase = p.v + (head + res) * D;
-        float x[L::kUnits][8];           // K or V on its way
-        auto ask_rows = [&](const float* base, int j, int vec) {
-#pragma unroll
-            for (int i = 0; i < L::kUnits; ++i) {
-                const int unit = threadIdx.x + i * kWorkers, u = lo + j * kKeys + unit / (D / 8), c = unit % (D / 8) * 8;
-                if (u < rows_v) {
-                    load8(x[i], base + (int64_t)u * pitch + c, vec);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) x[i][e] = 0.f;
-                }
-            }
-        };
+        float x[kUnits<D>][8];           // K or V on its way
+        auto ask_v = [&](int j) { ask_rows<D>(x, vbase, pitch, lo + j * kKeys, rows_v, p.vec_v); };
         auto ask_k = [&](int j) {
-            if constexpr (!kKt) {
-                ask_rows(kbase, j, p.vec_k);
-            } else {
-#pragma unroll
-                for (int i = 0; i < L::kUnits; ++i) {
-                    const int unit = threadIdx.x + i * kWorkers, c = unit / (kKeys / 8), key = lo + j * kKeys + unit % (kKeys / 8) * 8;
-                    const float* src = kbase + (int64_t)c * p.n_rows;
-                    if (p.vec_k > 1 && key + 8 <= rows_v) {
-                        load8(x[i], src + key, p.vec_k);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) x[i][e] = key + e < rows_v ? __ldg(src + (int64_t)(key + e) * p.stride + res) : 0.f;
-                    }
-                }
-            }
-        };
-        auto put = [&](uint8_t* dst, bool kt) {
-#pragma unroll
-            for (int i = 0; i < L::kUnits; ++i) {
-                const int unit = threadIdx.x + i * kWorkers;
-                const int per_row = kt ? kKeys / 8 : D / 8, row = unit / per_row, piece = unit % per_row;
-                // (columns past 64: the second half of the piece)
-                uint8_t* to = dst + (kt ? 0 : (piece >> 3) * kSubBytes) + row * 128 + (((piece & 7) ^ (row & 7)) << 4);
-                uint4 h, m, l;
-                split8(x[i], h, m, l);
-                *reinterpret_cast<uint4*>(to) = h;
-                *reinterpret_cast<uint4*>(to + L::kPiece) = m;
-                *reinterpret_cast<uint4*>(to + 2 * L::kPiece) = l;
-            }
-            fence_proxy_async_smem();
+            if constexpr (kKt) ask_kt<D>(x, kbase, p.n_rows, p.stride, res, lo + j * kKeys, rows_v, p.vec_k);
+            else ask_rows<D>(x, kbase, pitch, lo + j * kKeys, rows_v, p.vec_k);
         };
         auto arrive = [&](uint64_t* bar) {
             tc_fence_before_sync();
@@ -383,7 +288,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
                     tmem_st4(lane_addr + D + c / 2, l);
                 }
             }
-            put(smem + L::kKOff, kKt);
+            put<D, kKt>(x, smem + L::kKOff);
             tmem_st_wait();
             arrive(&ctrl->k_full);
             if (steps > 1) ask_k(1);
@@ -409,12 +314,12 @@ attention_split_kernel(const __grid_constant__ Params p) {
             tc_fence_after_sync();
             uint32_t r[32];
             if (!L::kAgain) tmem_ld32(s_addr, r);
-            if (j + 1 < steps) put(smem + L::kKOff, kKt);       // (S(j) is complete: K(j) has been read)
+            if (j + 1 < steps) put<D, kKt>(x, smem + L::kKOff);       // (S(j) is complete: K(j) has been read)
             if (!L::kAgain) {
                 tmem_ld_wait();
                 if (j + 1 < steps) arrive(&ctrl->k_full);
             }
-            ask_rows(vbase, j, p.vec_v);
+            ask_v(j);
             if (L::kAgain) {
                 tmem_ld32(s_addr, r);
                 tmem_ld_wait();
@@ -456,7 +361,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
                 }
             };
             auto next_v = [&] {
-                put(smem + L::kVOff + (j & 1) * L::kOperand, false);       // (P V(j - 2) is complete)
+                put<D, false>(x, smem + L::kVOff + (j & 1) * L::kOperand);       // (P V(j - 2) is complete)
                 if (j + 2 < steps) ask_k(j + 2);
             };
             if (!L::kAgain) {
@@ -625,9 +530,7 @@ int32_t attention_split_f32(const void* q, const void* k, int kt, const void* v,
     p.q = (const float*)q; p.k = (const float*)k; p.v = (const float*)v; p.o = (float*)o; p.lse = lse;
     p.lin = lin; p.tr = tr; p.nnzs = nnzs; p.status = status_word; p.mirror = status_mirror(status_word);
     p.n_rows = (int)n_rows; p.stride = (int)stride; p.kt = kt; p.sign = scale < 0.f ? -1.f : 1.f; p.scale_log2 = p.sign * scale * kLog2e;
-    auto vec = [](const void* base) { return (reinterpret_cast<uintptr_t>(base) & 31u) == 0 ? 8 : 4; };
-    p.vec_q = vec(q); p.vec_v = vec(v);
-    p.vec_k = !kt ? vec(k) : stride != 1 || n_rows % 4 != 0 ? 1 : n_rows % 8 != 0 ? 4 : vec(k);
+    p.vec_q = split::vec_of(q); p.vec_v = split::vec_of(v); p.vec_k = split::vec_of_k(k, kt, stride, n_rows);
     if (d == 32) return split::launch<32>(p, bh, st);
     if (d == 64) return split::launch<64>(p, bh, st);
     return split::launch<128>(p, bh, st);

@@ -1,5 +1,5 @@
-// fp32 SDDMM, SpMM and fused attention over ACSR on register tiles (CUDA cores, true fp32 FMA).  Fused attention of more than
-// a wave of these tiles runs on the tensor cores (attention_split.cu).
+// fp32 SDDMM, SpMM and fused attention over ACSR on register tiles (CUDA cores, true fp32 FMA).  What is more than a wave or two
+// of these tiles runs on the tensor cores (attention_split.cu, ops_split.cu).
 //
 // Applies to patterns whose rows, regrouped by residue class, are contiguous bands: one stride s for
 // all rows with more than one non-zero and start_i == i (mod s), as the plan of splat_acsr_classify
@@ -625,6 +625,10 @@ static int32_t run(const Params& p, int64_t bh, cudaStream_t st) {
 int32_t attention_split_f32(const void* q, const void* k, int kt, const void* v, void* o, const float* lin, const float* tr,
                             const float* nnzs, int64_t bh, int64_t n_rows, int64_t d, int64_t stride, float scale,
                             int32_t* status_word, float* lse, cudaStream_t st);    // attention_split.cu
+int32_t sddmm_split_f32(const void* q, const void* k, int kt, void* s, const float* lin, const float* tr, const float* nnzs, int64_t bh,
+                        int64_t n_rows, int64_t d, int64_t stride, int64_t trailing, int32_t* status_word, cudaStream_t st);
+int32_t spmm_split_f32(const void* p_in, const void* v, void* o, const float* lin, const float* tr, const float* nnzs, int64_t bh,
+                       int64_t n_rows, int64_t d, int64_t stride, int64_t trailing, int32_t* status_word, cudaStream_t st);    // ops_split.cu
 
 // Fills p and says whether the tile kernels take the problem (SPLAT_ERR_UNSUPPORTED_SHAPE if not).
 // plan: {max_nnz, stride_min, stride_max, misaligned, n_single, max_col+1, n_empty, n_multi}
@@ -652,6 +656,9 @@ static int32_t tile_setup(tile::Params& p, const int32_t* plan, int64_t bh, int6
     return SPLAT_OK;
 }
 
+// Tiles of 32 rows.
+static int64_t rows32(int64_t n_rows, int64_t stride, int64_t bh) { return ((n_rows + stride - 1) / stride + 31) / 32 * stride * bh; }
+
 template <tile::Op OP>
 static int32_t tile_launch(const tile::Params& p, int64_t d, int64_t bh, cudaStream_t st) {
     if (d == 32) return tile::run<32, OP>(p, bh, st);
@@ -673,8 +680,7 @@ int32_t attention_tile_f32(const void* q, const void* k, int64_t ksb, int64_t ks
     // 17.8, 36.7 / 17.9; window 32 of L200, 147 and 154: d32 7.3 / 7.4, 12.5 / 7.4; d64 9.7 / 11.5, 17.2 / 11.6; d128 15.5 /
     // 13.8, 28.1 / 13.8.  At d = 128 they are the faster for less as well (window 32 of L256, 16 CTAs 15.3 / 14.7), but for a
     // K^T that has to be gathered key by key (strided 16 of L2048, 64 CTAs 21.1 / 21.4).
-    const int64_t of32 = ((n_rows + p.stride - 1) / p.stride + 31) / 32 * p.stride * bh;
-    if (status_word != nullptr && aligned16(q) && scale != 0.f && (of32 > 148 || (d == 128 && (!p.kt || p.stride == 1))))
+    if (status_word != nullptr && aligned16(q) && scale != 0.f && (rows32(n_rows, p.stride, bh) > 148 || (d == 128 && (!p.kt || p.stride == 1))))
         return attention_split_f32(q, k, p.kt, v, o, lin, tr, nnzs, bh, n_rows, d, p.stride, scale, status_word, lse, st);
     p.q = (const float*)q; p.k = (const float*)k; p.v = (const float*)v; p.o = (float*)o; p.lse = lse;
     p.lin = lin; p.tr = tr; p.nnzs = nnzs; p.scale_log2 = scale * kLog2e;
@@ -697,6 +703,13 @@ extern "C" int32_t splat_sddmm_tile(const void* q, const void* k, int64_t k_stri
     if (!q || !k || !s_out || !sTod_lin || !sTod_tr || !nnzs) return SPLAT_ERR_BAD_ARG;
     if (plan_i32[0] > trailing_dim) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     if (!aligned16(k)) return SPLAT_ERR_MISALIGNED;
+    // The tensor cores (ops_split.cu) where there is more than a wave of the tiles here, at d = 32 more than two.  us, here / there,
+    // at CTAs of 32 rows: +-64 of L1024 d32 128 6.1 / 8.8, 256 9.2 / 8.9 (contiguous K^T 8.0 / 9.1), 320 11.3 / 9.2; d64 128
+    // 8.6 / 9.8, 160 14.3 / 9.8 (11.2 / 9.9); d128 128 13.7 / 13.8 (10.6 / 13.6), 160 22.9 / 13.8; causal 32 of L256 d64 152 9.2 / 8.5;
+    // 64 taps by 4 of L1000 d64 160 10.0 / 8.6, d32 256 7.2 / 7.8, 320 9.3 / 7.8.
+    int32_t* const word = registered_status_word();
+    if (word != nullptr && aligned16(q) && rows32(n_rows, p.stride, bh) > (d == 32 ? 296 : 148))
+        return sddmm_split_f32(q, k, p.kt, s_out, sTod_lin, sTod_tr, nnzs, bh, n_rows, d, p.stride, trailing_dim, word, (cudaStream_t)stream);
     p.q = (const float*)q; p.k = (const float*)k; p.sparse = (float*)s_out;
     p.lin = sTod_lin; p.tr = sTod_tr; p.nnzs = nnzs; p.trailing = (int)trailing_dim;
     return tile_launch<tile::Op::kSddmm>(p, d, bh, (cudaStream_t)stream);
@@ -713,6 +726,12 @@ extern "C" int32_t splat_spmm_tile(const void* p_in, const void* v, void* o, con
     if (!p_in || !v || !o || !sTod_lin || !sTod_tr || !nnzs) return SPLAT_ERR_BAD_ARG;
     if (plan_i32[0] > trailing_dim) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     if (!aligned16(v) || !aligned16(o)) return SPLAT_ERR_MISALIGNED;
+    // As above, but its steps wait for one another: more than two waves at d <= 64.  us: +-64 of L1024 d64 128 7.3 / 11.5, 256
+    // 12.1 / 11.6, 320 16.4 / 11.6; +-500 of L2048 d64 256 41.8 / 46.9, 512 76.9 / 47.6; d32 +-64 256 8.2 / 9.5, 320 12.8 / 9.5; 64 taps by 4
+    // of L1000 d64 288 8.5 / 9.2, 320 10.3 / 9.2; d128 +-64 128 11.3 / 14.7, 160 18.5 / 14.8; +-500 128 38.4 / 52.7, 192 62.7 / 53.0.
+    int32_t* const word = registered_status_word();
+    if (word != nullptr && rows32(n_rows, p.stride, bh) > (d == 128 ? 148 : 296))
+        return spmm_split_f32(p_in, v, o, sTod_lin, sTod_tr, nnzs, bh, n_rows, d, p.stride, trailing_dim, word, (cudaStream_t)stream);
     p.sparse = (float*)const_cast<void*>(p_in); p.v = (const float*)v; p.o = (float*)o;
     p.lin = sTod_lin; p.tr = sTod_tr; p.nnzs = nnzs; p.trailing = (int)trailing_dim;
     return tile_launch<tile::Op::kSpmm>(p, d, bh, (cudaStream_t)stream);
