@@ -33,6 +33,7 @@ struct Classes {
     dim3 grid(int64_t stride, int64_t bh) const {
         return dim3((unsigned)tile_pitch, (unsigned)(rows > 0 ? stride : longer), (unsigned)bh);
     }
+    int64_t tiles(int64_t stride, int64_t bh) const { return (int64_t)tile_pitch * (rows > 0 ? stride : longer) * bh; }     // of the grid
     bool has(int part) const { return part == 0 ? longer > 0 : rows > 0; }
     // view of a (BH, L, d) array: rows of `part`'s classes
     bool view(CUtensorMap* map, const void* base, int32_t dtype, int64_t bh, int64_t n_rows, int64_t d, int64_t stride,

@@ -9,14 +9,16 @@
 //   spmm_band_kernel    O[i] = sum_j' P[i, j'] V[start_i + j' stride]   (SPLAT/r_spmm.py:14-164)
 //       cp.async brings the 16-byte pieces of P that a 64-key step needs; a thread takes its row's pieces,
 //       shifts them into place and stores them in tensor memory as the A operand of O += P(k) V(k).
-// One CTA = one 128-row tile of one (bh, class).  Warps 0-3: thread = row = tensor-memory lane; 4 TMA; 5 MMA.
+// One CTA = one 128-row tile of one (bh, class).  Row warps: thread = row = tensor-memory lane, one warp to 32 rows or two that
+// share a step's columns (see two_warps()); then a TMA and an MMA warp.
 //
 // The sparse layout shifts every row by its own number of elements against the dense columns, so a row's 64
 // columns of a step begin anywhere in a 16-byte piece of the sparse array.  They begin at the SAME place in
 // every step (64 elements are eight pieces): with e the element index of the step's first column and
 // sft = e mod 8, a step of a row is eight whole pieces made of the last sft elements of the step before and
-// the first 64 - sft of this one.  The thread forms them in registers (barrel()), and a warp moves them through a
-// swizzled staging tile so that global memory sees 128 contiguous bytes per row.  The kernels before did this
+// the first 64 - sft of this one (with two warps to the rows four pieces of 32 columns, and the columns in front read with
+// the warp's own).  The thread forms them in registers (barrel()), and a warp moves them through a swizzled staging tile
+// so that global memory sees 128 or 64 contiguous bytes per row.  The kernels before did this
 // with 2-byte accesses, or 16-byte ones of 32 different rows per instruction: 70 % of the L1 wavefronts, a
 // third of the memory bandwidth.  B4 H16 L4096 d64 fp16 window 256: SDDMM 102 -> 59 us, SpMM 114 -> 65.
 // Pieces that a row's band only partly covers (its ends, if trailing_dim is no multiple of 8) are stored element
@@ -47,11 +49,7 @@ constexpr int kSubBytes = kTile * 128;          // 128 rows x 128 bytes
 constexpr int kStepBytesPerSub = kStep * 128;   // 64 keys x 128 bytes
 // What these kernels are bound by is instructions: with waits of a few of them (tc_ptx.cuh) and the control block at
 // constant addresses SDDMM at d = 128 went from 70.1 to 66.2 us, SpMM from 70.1 to 68.7 (B4 H16 L4096 window 256).
-constexpr int kThreads = 192;
-constexpr int kTmaWarp = 4;
-constexpr int kMmaWarp = 5;
 constexpr int kStages = 3;                      // K / V ring
-constexpr int kPPitch = 144;                    // bytes of a row's nine pieces: conflict-free 16-byte reads
 constexpr int kSingle = -1, kEmpty = INT_MIN / 2;   // row kinds, as in the band table (acsr_meta.cu)
 enum : int { kErrQ = 11, kErrFull = 12, kErrEmpty = 13, kErrReady = 14, kErrFree = 15 };
 
@@ -92,7 +90,7 @@ struct Control {
     int32_t gave_up;     // code of a wait that ran out
     int32_t lo[4];
     int32_t hi[4];
-    int4 about[kTile];   // sddmm: what a lane knows of its row, for the lanes that store it
+    uint32_t again[4];   // spmm: rows whose result is not finite
 };
 
 // The row warps' share of the prologue: this thread's band, and without a table the warp's key range.
@@ -111,7 +109,7 @@ __device__ __forceinline__ int2 load_band(const Params& p, Control* ctrl, int re
             }
         }
     }
-    if (p.rows == nullptr) {
+    if (p.rows == nullptr && warp < 4) {
         const int lo = warp_min_i(band.y > 0 ? band.x : INT_MAX), hi = warp_max_i(max(band.y, 0));
         if (lane == 0) { ctrl->lo[warp] = lo; ctrl->hi[warp] = hi; }
     }
@@ -125,50 +123,59 @@ __device__ __forceinline__ void key_range(int rows_v, const Control* ctrl, int* 
     *khi = (hi + kStep - 1) / kStep;
 }
 
-// out[0..31] = 64 elements (two per word) of the 72 in x[0..35] from element t on, 0 <= t <= kMax.
-template <int kMax>
-__device__ __forceinline__ void barrel(uint32_t (&x)[36], int t, uint32_t (&out)[32]) {
+// out = 2 kWords elements (two per word) of the eight more in x from element t on, 0 <= t <= kMax.
+template <int kMax, int kWords>
+__device__ __forceinline__ void barrel(uint32_t (&x)[kWords + 4], int t, uint32_t (&out)[kWords]) {
     const int s = t >> 1;
     if (kMax == 8 && (s & 4)) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = x[i + 4];
+        for (int i = 0; i < kWords; ++i) x[i] = x[i + 4];
     }
     if (s & 2) {
 #pragma unroll
-        for (int i = 0; i < 34; ++i) x[i] = x[i + 2];
+        for (int i = 0; i < kWords + 2; ++i) x[i] = x[i + 2];
     }
     if (s & 1) {
 #pragma unroll
-        for (int i = 0; i < 35; ++i) x[i] = x[i + 1];
+        for (int i = 0; i < kWords + 3; ++i) x[i] = x[i + 1];
     }
     const uint32_t shift = (t & 1) * 16;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) out[i] = __funnelshift_r(x[i], x[i + 1], shift);
+    for (int i = 0; i < kWords; ++i) out[i] = __funnelshift_r(x[i], x[i + 1], shift);
+}
+// 32 bit, 8 consecutive columns of tensor memory
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------
 // SDDMM
 // ---------------------------------------------------------------------------------------------
-template <int D> struct SddmmLayout {
+template <int D, int kRowWarps> struct SddmmLayout {
     static constexpr int kSub = D / 64;
     static constexpr int kQBytes = kSub * kSubBytes;
     static constexpr int kItemBytes = kSub * kStepBytesPerSub;
     static constexpr int kRingOff = kQBytes;
     static constexpr int kStageOff = kRingOff + kStages * kItemBytes;
     static constexpr int kSmemBytes = kStageOff + kTile * 128 + 1024;   // + alignment slack
-    static constexpr int kPerSm = D == 128 ? 2 : 3;
+    static constexpr int kPerSm = D == 128 || kRowWarps == 8 ? 2 : 3;
+    static constexpr int kThreads = (kRowWarps + 2) * 32;
 };
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kThreads, SddmmLayout<D>::kPerSm)
+template <typename T, int D, int kRowWarps>
+__global__ void __launch_bounds__(SddmmLayout<D, kRowWarps>::kThreads, SddmmLayout<D, kRowWarps>::kPerSm)
 sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
-    using L = SddmmLayout<D>;
+    using L = SddmmLayout<D, kRowWarps>;
+    constexpr int kTmaWarp = kRowWarps, kMmaWarp = kRowWarps + 1;
+    constexpr int kHalves = kRowWarps / 4, kCols = kStep / kHalves;      // warps that share 32 rows, columns of a step of each
     constexpr int kTmemCols = 128;   // two 64-column score buffers
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + (((smem_u32(smem_raw) + 1023) & ~1023u) - smem_u32(smem_raw));
     uint8_t* s_ring = smem + L::kRingOff;
     __shared__ Control ctrl_mem;             // (static: constant addresses)
     Control* const ctrl = &ctrl_mem;
+    __shared__ int4 about_mem[kRowWarps * 32];      // what a lane knows of its row, for the lanes that store it
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int real_res = blockIdx.y, res = p.cls.in_part(real_res), rows_v = p.cls.rows_of(real_res);
@@ -207,7 +214,7 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             }
             for (int b = 0; b < 2; ++b) {
                 mbar_init(&ctrl->ready[b], 1);
-                mbar_init(&ctrl->freed[b], 4);
+                mbar_init(&ctrl->freed[b], kRowWarps);
             }
             mbar_init(&ctrl->drain, 1);
             mbar_fence_init();
@@ -232,7 +239,7 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         }
     } else {
         depend_wait();
-        band = load_band(p, ctrl, real_res, u0 + warp * 32 + lane, warp, lane);
+        band = load_band(p, ctrl, real_res, u0 + (warp & 3) * 32 + lane, warp, lane);
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -290,54 +297,76 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         }
     } else {
         // ------------------------------------------------------------------ row warps
-        const uint32_t s_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
-        uint8_t* stage = smem + L::kStageOff + warp * 32 * 128;
+        const int rw = warp & 3, half = warp >> 2;
+        const uint32_t s_addr = tmem_base + ((uint32_t)(rw * 32) << 16);
+        uint8_t* stage = smem + L::kStageOff + warp * 32 * (kCols * 2);
         const int64_t head = bh * p.n_rows;
         // element index (in p.sparse) of class column 0 of this row, were its band to reach that far
-        const int64_t e_row = p.lead + (head + (int64_t)(u0 + warp * 32 + lane) * p.stride + real_res) * p.trailing_dim - band.x;
+        const int64_t e_row = p.lead + (head + (int64_t)(u0 + rw * 32 + lane) * p.stride + real_res) * p.trailing_dim - band.x;
         const int sft = (int)(e_row & 7);
-        // The rows whose pieces this lane stores: row 4 i + lane / 8, piece lane mod 8.  Byte offset of the piece of
+        constexpr int kPieces = kCols / 8, kRows = 32 / kPieces;       // 16-byte pieces of a row, rows of a warp's store
+        // The rows whose pieces this lane stores: row kRows i + lane / kPieces, piece lane mod kPieces.  Byte offset of the piece of
         // class column 0's step, and the column range in which the piece's first column is inside the band.
         // (what a lane knows of its row reaches the others through shared memory: five shuffles per row took 1 300 cycles)
         const int64_t e_base = __shfl_sync(0xffffffffu, e_row + band.x, 0) & ~(int64_t)7;
         uint8_t* base = reinterpret_cast<uint8_t*>(p.sparse + e_base);
         const int e_rel = (int)(e_row - e_base);
-        int4* about = ctrl->about + warp * 32;
-        about[lane] = make_int4(e_rel, u0 + warp * 32 + lane < rows_v ? 1 : 0, band.x, max(band.y, -64));     // (-64, below every step: no band)
+        int4* about = about_mem + warp * 32;
+        about[lane] = make_int4(e_rel, u0 + rw * 32 + lane < rows_v ? 1 : 0, band.x, max(band.y, -64));     // (-64, below every step: no band)
         __syncwarp();
-        int32_t off[8];
-        int lo8[8], hi8[8];
+        int32_t off[kPieces];
+        int lo8[kPieces], hi8[kPieces];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int4 r = about[4 * i + (lane >> 3)];
-            const int behind = (lane & 7) * 8 - (r.x & 7);       // first column - step's
+        for (int i = 0; i < kPieces; ++i) {
+            const int4 r = about[kRows * i + lane / kPieces];
+            const int behind = lane % kPieces * 8 - (r.x & 7);       // first column - the warp's first of the step
             off[i] = (r.x + behind) * 2;
             lo8[i] = r.z - behind;
             hi8[i] = r.w - behind;
         }
-        // this warp's first and last step with columns of its rows' bands
+        // this warp's first and last columns of its rows' bands
         const int w_lo = warp_min_i(band.y > 0 ? band.x : INT_MAX), w_hi = warp_max_i(band.y > 0 ? band.y + sft : 0);
-        uint32_t tail[4] = {0, 0, 0, 0};       // the last eight elements of the step before
+        uint32_t tail[4] = {0, 0, 0, 0};       // the eight elements before the warp's columns of the step
         bool ok = true;
         for (int k = klo; k <= khi && khi > klo; ++k) {      // khi: what is left of the last step
-            const int it = k - klo, b = it & 1, c0 = k * kStep;
-            const bool active = c0 < w_hi && c0 + kStep > w_lo;
+            const int it = k - klo, b = it & 1, c0 = k * kStep + half * kCols;
+            const bool active = c0 < w_hi && c0 + kCols > w_lo;
             if (k < khi) {
                 ok = wait_all(&ctrl->ready[b], (uint32_t)(it >> 1) & 1u, &ctrl->gave_up, kErrReady);
                 if (!ok) break;
                 tc_fence_after_sync();
             }
-            uint32_t x[36], out[32];
+            const uint32_t from = s_addr + b * kStep + half * kCols;
+            uint32_t x[kCols / 2 + 4], out[kCols / 2];
             if (active && k < khi) {
-                uint32_t r[64];
-                tmem_ld32(s_addr + b * kStep, r);
-                tmem_ld32(s_addr + b * kStep + 32, r + 32);
+                uint32_t r[kCols];
+#pragma unroll
+                for (int c = 0; c < kCols; c += 32) tmem_ld32(from + c, r + c);
                 tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 32; ++i) x[4 + i] = pack2<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                for (int i = 0; i < kCols / 2; ++i) x[4 + i] = pack2<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
             } else {
 #pragma unroll
-                for (int i = 4; i < 36; ++i) x[i] = 0u;
+                for (int i = 4; i < kCols / 2 + 4; ++i) x[i] = 0u;
+            }
+            // The eight columns in front: the warp's own last ones, or, of two warps that share the rows, columns 24-31 for the
+            // second one's 32, and columns 56-63 for the first one's of the next step.
+            if constexpr (kHalves == 2) {
+                if (!half) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[i] = tail[i];
+                }
+                if (k < khi) {
+                    uint32_t t[8];
+                    tmem_ld8(s_addr + b * kStep + (half ? kCols : kStep) - 8, t);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) tail[i] = pack2<T>(__uint_as_float(t[2 * i]), __uint_as_float(t[2 * i + 1]));
+                }
+                if (half) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[i] = tail[i];
+                }
             }
             if (k < khi) {
                 tc_fence_before_sync();
@@ -345,21 +374,24 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
                 if (lane == 0) mbar_arrive(&ctrl->freed[b]);   // the buffer may take the scores of step k + 2
             }
             if (!active) continue;
+            if constexpr (kHalves == 1) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = tail[i];
+                for (int i = 0; i < 4; ++i) x[i] = tail[i];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) tail[i] = x[32 + i];
+                for (int i = 0; i < 4; ++i) tail[i] = x[kCols / 2 + i];
+            }
             barrel<8>(x, 8 - sft, out);
 #pragma unroll
-            for (int q4 = 0; q4 < 8; ++q4)
-                *reinterpret_cast<uint4*>(stage + lane * 128 + ((q4 ^ (lane & 7)) << 4)) =
+            for (int q4 = 0; q4 < kPieces; ++q4)
+                *reinterpret_cast<uint4*>(stage + lane * (kCols * 2) + ((q4 ^ (kHalves == 2 ? (lane >> 1) & 3 : lane & 7)) << 4)) =
                     make_uint4(out[4 * q4], out[4 * q4 + 1], out[4 * q4 + 2], out[4 * q4 + 3]);
             __syncwarp();
             uint8_t* to = base + (int64_t)c0 * 2;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int row = 4 * i + (lane >> 3);
-                const uint4 v = *reinterpret_cast<const uint4*>(stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
+            for (int i = 0; i < kPieces; ++i) {
+                const int row = kRows * i + lane / kPieces;
+                const uint4 v = *reinterpret_cast<const uint4*>(
+                    stage + row * (kCols * 2) + ((lane % kPieces ^ (kHalves == 2 ? (row >> 1) & 3 : row & 7)) << 4));
                 if (c0 >= lo8[i] && c0 + 8 <= hi8[i]) {
                     *reinterpret_cast<uint4*>(to + off[i]) = v;
                 } else if (c0 + 8 > lo8[i] && c0 < hi8[i]) {
@@ -373,13 +405,13 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         }
         // padding slots, rows with one non-zero (a dot product by hand) and rows with none
         // (eight lanes per row: one element each of the pieces at either end, 16-byte stores between; a warp per row,
-        // element by element, took 2 to 3 us of a small call)
+        // element by element, took 2 to 3 us of a small call; either warp of the rows has half of them)
         const int4 mine = about[lane];
         const int nnz = mine.w > 0 ? mine.w - mine.z : (mine.w == kSingle ? 1 : 0);
         if (__any_sync(0xffffffffu, mine.y != 0 && nnz < p.trailing_dim)) {
             uint16_t* to = reinterpret_cast<uint16_t*>(base);
 #pragma unroll 1
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 8 / kHalves * half; i < 8 / kHalves * (half + 1); ++i) {
                 const int4 r = about[4 * i + (lane >> 3)];
                 const int l = lane & 7, slot0 = r.x + r.z, end = slot0 + p.trailing_dim;
                 const int from = r.y == 0 ? end : slot0 + (r.w > 0 ? r.w - r.z : (r.w == kSingle ? 1 : 0));
@@ -389,14 +421,14 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
                 if (last >= first && last + l < end) to[last + l] = 0;
             }
         }
-        unsigned todo = __ballot_sync(0xffffffffu, mine.y != 0 && mine.w == kSingle);
+        unsigned todo = half == 0 ? __ballot_sync(0xffffffffu, mine.y != 0 && mine.w == kSingle) : 0;
         const T* qg = reinterpret_cast<const T*>(p.q);
         const T* kg = reinterpret_cast<const T*>(p.kv);
         while (todo) {
             const int rr = __ffs(todo) - 1;
             todo &= todo - 1;
             const int start = about[rr].z;
-            const int64_t row_real = head + (int64_t)(u0 + warp * 32 + rr) * p.stride + real_res;
+            const int64_t row_real = head + (int64_t)(u0 + rw * 32 + rr) * p.stride + real_res;
             uint16_t* row = p.sparse + p.lead + row_real * p.trailing_dim;
             float acc = 0.f;
             const T* qr = qg + row_real * p.d;
@@ -422,12 +454,15 @@ sddmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
 // SpMM
 // ---------------------------------------------------------------------------------------------
 // kPerSm CTAs share an SM: two with three steps of P on their way, or, at D = 64 and with more than two CTAs per SM to
-// run, three with two steps each (96 registers and some spills): B3 H44 L7680 +-224 294 -> 270 us, B2 H116 L4032
+// run, three with two steps each (with one warp to 32 rows 112 registers and some spills): B3 H44 L7680 +-224 294 -> 270 us, B2 H116 L4032
 // +-17 165 -> 144 us; a single wave (H8 L1024) is faster with two, 7.5 against 8.3 us.
-template <int D, int kPerSm> struct SpmmLayout {
+template <int D, int kPerSm, int kRowWarps> struct SpmmLayout {
+    static constexpr int kThreads = (kRowWarps + 2) * 32;
+    static constexpr int kPieces = kStep * 4 / kRowWarps / 8 + 1;      // 16-byte pieces of a row's columns of a step (of one warp)
+    static constexpr int kPPitch = kPieces * 16;                  // (an odd number of pieces: conflict-free 16-byte reads)
     static constexpr int kSub = D / 64;
     static constexpr int kItemBytes = kSub * kStepBytesPerSub;    // 64 keys of V
-    static constexpr int kPBytes = kTile * kPPitch;               // a step's pieces of P
+    static constexpr int kPBytes = kRowWarps * 32 * kPPitch;      // a step's pieces of P
     static constexpr int kPStages = kPerSm == 2 ? 3 : 2;          // steps of P on their way
     static constexpr int kPOff = 0;                               // later reused as the output's staging
     static constexpr int kFront = (kPStages * kPBytes + 1023) / 1024 * 1024;
@@ -436,11 +471,12 @@ template <int D, int kPerSm> struct SpmmLayout {
     static_assert(kFront >= kSub * kSubBytes, "output staging");
 };
 
-template <typename T, int D, int kPerSm>
-__global__ void __launch_bounds__(kThreads, kPerSm)
+template <typename T, int D, int kPerSm, int kRowWarps>
+__global__ void __launch_bounds__((kRowWarps + 2) * 32, kPerSm)
 spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
-    using L = SpmmLayout<D, kPerSm>;
-    constexpr int kPStages = L::kPStages;
+    using L = SpmmLayout<D, kPerSm, kRowWarps>;
+    constexpr int kPStages = L::kPStages, kPPitch = L::kPPitch, kPieces = L::kPieces, kTmaWarp = kRowWarps, kMmaWarp = kRowWarps + 1;
+    constexpr int kHalves = kRowWarps / 4, kCols = kStep / kHalves;      // warps that share 32 rows, columns of a step of each
     constexpr int kTmemCols = D == 128 ? 256 : 128;   // the output accumulator, two steps of P (32 columns each)
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + (((smem_u32(smem_raw) + 1023) & ~1023u) - smem_u32(smem_raw));
@@ -479,7 +515,7 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
                 mbar_init(&ctrl->empty[i], 1);
             }
             for (int b = 0; b < 2; ++b) {
-                mbar_init(&ctrl->ready[b], 4);
+                mbar_init(&ctrl->ready[b], kRowWarps);
                 mbar_init(&ctrl->freed[b], 1);
             }
             mbar_init(&ctrl->drain, 1);
@@ -490,6 +526,7 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             const int32_t stop = entry_status(p.status, p.mirror);
             ctrl->abort_at_entry = stop;
             ctrl->gave_up = 0;
+            for (int w = 0; w < 4; ++w) ctrl->again[w] = 0;
             if (stop == 0 && range.y > 0) {
                 klo = range.x / kStep;
                 khi = (range.y + kStep - 1) / kStep;
@@ -500,7 +537,7 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         }
     } else {
         depend_wait();
-        band = load_band(p, ctrl, real_res, u0 + warp * 32 + lane, warp, lane);
+        band = load_band(p, ctrl, real_res, u0 + (warp & 3) * 32 + lane, warp, lane);
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -553,22 +590,23 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         }
     } else {
         // ------------------------------------------------------------------ P loaders + epilogue
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
+        const int rw = warp & 3, half = warp >> 2;
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(rw * 32) << 16);
         const int64_t head = bh * p.n_rows;
-        const int64_t e_row = p.lead + (head + (int64_t)(u0 + warp * 32 + lane) * p.stride + real_res) * p.trailing_dim - band.x;
+        const int64_t e_row = p.lead + (head + (int64_t)(u0 + rw * 32 + lane) * p.stride + real_res) * p.trailing_dim - band.x;
         const int sft = (int)((e_row + (int64_t)klo * kStep) & 7);
-        // Pieces of a step: nine per row, 288 per warp, piece idx = lane + 32 i of row idx / 9: byte offset of the
-        // piece in class column 0's step, and the range of a step's first column in which it holds some of the band.
+        // Pieces of a step: kPieces per row, piece idx = lane + 32 i of row idx / kPieces: byte offset of the
+        // piece in class column 0's step, and the range of the warp's first column in which it holds some of the band.
         const int64_t e_base = __shfl_sync(0xffffffffu, e_row + band.x, 0) & ~(int64_t)7;
         const uint8_t* base = reinterpret_cast<const uint8_t*>(p.sparse + e_base);
         int4* about = reinterpret_cast<int4*>(smem + L::kPOff + warp * 32 * kPPitch);      // (as in SDDMM)
         about[lane] = make_int4((int)(e_row - e_base), sft, band.x, band.y);
         __syncwarp();
-        int32_t off[9];
-        int first[9], last[9];
+        int32_t off[kPieces];
+        int first[kPieces], last[kPieces];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            const int idx = lane + 32 * i, row = idx / 9, piece = idx - row * 9;
+        for (int i = 0; i < kPieces; ++i) {
+            const int idx = lane + 32 * i, row = idx / kPieces, piece = idx - row * kPieces;
             const int4 r = about[row];
             const int behind = piece * 8 - r.y;
             off[i] = ((r.x & ~7) + piece * 8) * 2;
@@ -579,10 +617,10 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
         auto fetch = [&](int it) {
             if (klo + it < khi) {
                 const uint32_t dst = smem_u32(smem + L::kPOff) + (it % kPStages) * L::kPBytes + warp * 32 * kPPitch + lane * 16;
-                const int c0 = (klo + it) * kStep;
+                const int c0 = (klo + it) * kStep + half * kCols;
                 const uint8_t* from = base + (int64_t)c0 * 2;
 #pragma unroll
-                for (int i = 0; i < 9; ++i)
+                for (int i = 0; i < kPieces; ++i)
                     if (c0 >= first[i] && c0 < last[i])
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 512), "l"(from + off[i]) : "memory");
             }
@@ -595,33 +633,34 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             const int it = k - klo, b = it & 1;
             asm volatile("cp.async.wait_group %0;" ::"n"(kPStages - 1) : "memory");
             __syncwarp();
-            const int c0 = k * kStep;
-            const int lo = band.x - c0, hi = band.y - c0;       // valid columns of this step: [lo, hi)
-            uint32_t out[32];
-            if (c0 < w_hi && c0 + kStep > w_lo) {
+            const int c0 = k * kStep + half * kCols;
+            const int lo = band.x - c0, hi = band.y - c0;       // valid columns of the warp's: [lo, hi)
+            uint32_t out[kCols / 2];
+            if (c0 < w_hi && c0 + kCols > w_lo) {
                 const uint8_t* mine = smem + L::kPOff + (it % kPStages) * L::kPBytes + (warp * 32 + lane) * kPPitch;
-                uint32_t x[36];
+                uint32_t x[kCols / 2 + 4];
 #pragma unroll
-                for (int i = 0; i < 9; ++i) {
+                for (int i = 0; i < kPieces; ++i) {
                     const uint4 v = *reinterpret_cast<const uint4*>(mine + i * 16);
                     x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
                 }
-                barrel<7>(x, sft, out);          // the step's columns begin sft elements into the pieces
-                if (!__all_sync(0xffffffffu, lo <= 0 && hi >= kStep)) {
-                    // pairs of columns: 64 mask bits, two per word
-                    const int l = min(max(lo, 0), 64), h = min(max(hi, 0), 64);
-                    const uint64_t valid = (h >= 64 ? ~0ull : (1ull << h) - 1) & ~(l >= 64 ? ~0ull : (1ull << l) - 1);
-                    const uint32_t v0 = (uint32_t)valid, v1 = (uint32_t)(valid >> 32);
+                barrel<7>(x, sft, out);          // the warp's columns begin sft elements into the pieces
+                if (!__all_sync(0xffffffffu, lo <= 0 && hi >= kCols)) {
+                    // pairs of columns: a mask bit per column, two per word
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const uint32_t w = i < 16 ? v0 : v1;
-                        const int j = (2 * i) & 31;
-                        out[i] = ((w >> j) & 1u ? out[i] & 0xffffu : 0u) | ((w >> (j + 1)) & 1u ? out[i] & 0xffff0000u : 0u);
+                    for (int c = 0; c < kCols; c += 32) {
+                        const int l = min(max(lo - c, 0), 32), h = min(max(hi - c, 0), 32);
+                        const uint32_t valid = (h >= 32 ? ~0u : (1u << h) - 1) & ~(l >= 32 ? ~0u : (1u << l) - 1);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            uint32_t& w = out[c / 2 + i];
+                            w = ((valid >> (2 * i)) & 1u ? w & 0xffffu : 0u) | ((valid >> (2 * i + 1)) & 1u ? w & 0xffff0000u : 0u);
+                        }
                     }
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) out[i] = 0u;
+                for (int i = 0; i < kCols / 2; ++i) out[i] = 0u;
             }
             __syncwarp();
             fetch(it + kPStages);
@@ -630,7 +669,8 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
                 if (!ok) break;
                 tc_fence_after_sync();
             }
-            tmem_st32(lane_addr + p_col + b * 32, out);
+            if constexpr (kHalves == 1) tmem_st32(lane_addr + p_col + b * 32, out);
+            else tmem_st16(lane_addr + p_col + b * 32 + half * 16, out);
             tmem_st_wait();
             tc_fence_before_sync();
             __syncwarp();
@@ -643,16 +683,17 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             tc_fence_after_sync();
         }
         // every warp is through with its pieces of P before their memory becomes the staging of the output
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(kRowWarps * 32) : "memory");
         // epilogue: O for band rows, P[i,0] * V[start] for single-element rows, zero otherwise, staged in the
-        // 128-byte-swizzled tile layout, one TMA store per 64 columns and warp
-        const int t = warp * 32 + lane;
+        // 128-byte-swizzled tile layout (either warp of the rows half of the columns), one TMA store per 64 columns and 32 rows
+        const int t = rw * 32 + lane;
         const bool single = band.y == kSingle;
         const T* vrow = reinterpret_cast<const T*>(p.kv) + (head + band.x) * p.d;
         const float p0 = single ? to_f<T>(*reinterpret_cast<const T*>(p.sparse + e_row + band.x)) : 0.f;
         float2 odd = make_float2(0.f, 0.f);       // not finite: nor is the row
 #pragma unroll
-        for (int ch = 0; ch < D / 32; ++ch) {
+        for (int n = 0; n < D / 32 / kHalves; ++n) {
+            const int ch = half * (D / 32 / kHalves) + n;
             uint32_t r[32];
             if (have_o && ok) {
                 tmem_ld32(lane_addr + ch * 32, r);
@@ -685,12 +726,19 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             for (int q4 = 0; q4 < 4; ++q4)
                 *reinterpret_cast<uint4*>(srow + ((((ch & 1) * 4 + q4) ^ (t & 7)) << 4)) = outv[q4];
         }
-        unsigned again = __ballot_sync(0xffffffffu, band.y > 0 && !isfinite(odd.x + odd.y));
+        const unsigned odd_rows = __ballot_sync(0xffffffffu, band.y > 0 && !isfinite(odd.x + odd.y));
+        unsigned again = odd_rows;
         fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0 && u0 + warp * 32 < rows_v) {
+        if constexpr (kHalves == 2) {          // the first warp of the rows stores them
+            if (odd_rows != 0 && lane == 0) atomicOr(&ctrl->again[rw], odd_rows);
+            asm volatile("bar.sync 1, %0;" ::"n"(kRowWarps * 32) : "memory");
+            again = half == 0 ? ctrl->again[rw] : 0;
+        } else {
+            __syncwarp();
+        }
+        if (half == 0 && lane == 0 && u0 + rw * 32 < rows_v) {
             for (int sub = 0; sub < L::kSub; ++sub)
-                tma_store_4d(map + 1, smem + sub * kSubBytes + warp * 32 * 128, sub * 64, res, u0 + warp * 32, (int)bh);
+                tma_store_4d(map + 1, smem + sub * kSubBytes + rw * 32 * 128, sub * 64, res, u0 + rw * 32, (int)bh);
             tma_store_commit();
             if (again == 0) tma_store_wait_read();
             else tma_store_wait_all();
@@ -700,7 +748,7 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
             const int rr = __ffs(again) - 1;
             again &= again - 1;
             const int begin = __shfl_sync(0xffffffffu, band.x, rr), end = min(__shfl_sync(0xffffffffu, band.y, rr), rows_v);
-            const int64_t row = head + (int64_t)(u0 + warp * 32 + rr) * p.stride + real_res;
+            const int64_t row = head + (int64_t)(u0 + rw * 32 + rr) * p.stride + real_res;
             const float4 x = spmm_row<T>(reinterpret_cast<const T*>(p.sparse + p.lead + row * p.trailing_dim),
                                          reinterpret_cast<const T*>(p.kv) + head * p.d, (int64_t)begin * p.stride + real_res,
                                          p.stride, end - begin, p.d);
@@ -720,24 +768,41 @@ spmm_band_kernel(const __grid_constant__ Maps<2> maps, const Params p) {
 // ---------------------------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------------------------
+template <typename T, int D, int kRowWarps>
+static int32_t launch_sddmm(const Maps<2>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
+    using L = SddmmLayout<D, kRowWarps>;
+    auto kern = sddmm_band_kernel<T, D, kRowWarps>;
+    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), L::kSmemBytes)) return SPLAT_ERR_LAUNCH;
+    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), L::kThreads, L::kSmemBytes, st, maps, prm);
+}
+// Two warps to 32 rows halve what a step costs the warp that is in the way of the next, and leave twice as many to hide one
+// another's latencies; a warp to 32 rows moves 128 bytes of a row at a time instead of 64.  So the latter where rows are long and
+// the GPU is full.  us, one / two, SDDMM then SpMM: fp16 B4 H16 L4096 d64 window 256 55.3 / 51.5, 56.2 / 52.1; bf16 H16 L4096 d128
+// +-100 22.5 / 20.1, 20.0 / 18.7; fp16 H8 L1024 d64 +-64 8.3 / 5.9, 5.9 / 5.6; bf16 H4 L2048 d64 window 512 12.9 / 8.7, 10.2 / 8.9; B2 H16 L8192
+// d128 strided 64 55.5 / 46.6, 52.7 / 51.9; d64, H1 L8192 +-1000 (64 tiles) 39.1 / 25.0, 24.2 / 21.0; H4 (256) 58.0 / 58.7, 33.2 / 36.2; H24 L2048
+// +-500 (384) 35.5 / 40.7, 30.8 / 32.0; d128, H1 L8192 +-1000 33.3 / 28.2, 25.1 / 22.8; H4 56.5 / 65.4, 35.8 / 39.7; H8 L4096 +-600 (256) 32.4 / 33.6,
+// 25.0 / 27.1; H24 L2048 +-500 48.6 / 48.7, 36.8 / 38.2.
+// SDDMM at d <= 64 up to two waves: H3 L8192 +-1000 (192) 50.1 / 42.3, H4 +-700 (256) 37.0 / 30.1.
+static bool two_warps(const Params& prm, int64_t bh, int64_t tiles) { return prm.trailing_dim <= 512 || prm.cls.tiles(prm.stride, bh) <= tiles; }
 template <typename T, int D>
 static int32_t launch_sddmm(const Maps<2>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
-    auto kern = sddmm_band_kernel<T, D>;
-    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), SddmmLayout<D>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
-    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, SddmmLayout<D>::kSmemBytes, st, maps, prm);
+    return two_warps(prm, bh, D == 64 ? 296 : 148) ? launch_sddmm<T, D, 8>(maps, prm, bh, st) : launch_sddmm<T, D, 4>(maps, prm, bh, st);
 }
-template <typename T, int D, int kPerSm>
+template <typename T, int D, int kPerSm, int kRowWarps>
 static int32_t launch_spmm(const Maps<2>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
-    auto kern = spmm_band_kernel<T, D, kPerSm>;
-    constexpr int bytes = SpmmLayout<D, kPerSm>::kSmemBytes;
-    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), bytes)) return SPLAT_ERR_LAUNCH;
-    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, bytes, st, maps, prm);
+    using L = SpmmLayout<D, kPerSm, kRowWarps>;
+    auto kern = spmm_band_kernel<T, D, kPerSm, kRowWarps>;
+    if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), L::kSmemBytes)) return SPLAT_ERR_LAUNCH;
+    return launch_kernel(kern, prm.cls.grid(prm.stride, bh), L::kThreads, L::kSmemBytes, st, maps, prm);
 }
 template <typename T>
 static int32_t launch_spmm(const Maps<2>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
-    if (prm.d > 64) return launch_spmm<T, 128, 2>(maps, prm, bh, st);
-    const dim3 grid = prm.cls.grid(prm.stride, bh);
-    return (int64_t)grid.x * grid.y * grid.z > 2 * 148 ? launch_spmm<T, 64, 3>(maps, prm, bh, st) : launch_spmm<T, 64, 2>(maps, prm, bh, st);
+    if (two_warps(prm, bh, 148)) {
+        if (prm.d > 64) return launch_spmm<T, 128, 2, 8>(maps, prm, bh, st);
+        return prm.cls.tiles(prm.stride, bh) > 2 * 148 ? launch_spmm<T, 64, 3, 8>(maps, prm, bh, st) : launch_spmm<T, 64, 2, 8>(maps, prm, bh, st);
+    }
+    if (prm.d > 64) return launch_spmm<T, 128, 2, 4>(maps, prm, bh, st);
+    return prm.cls.tiles(prm.stride, bh) > 2 * 148 ? launch_spmm<T, 64, 3, 4>(maps, prm, bh, st) : launch_spmm<T, 64, 2, 4>(maps, prm, bh, st);
 }
 
 // Checks shared by both operators; fills stride.  plan as written by splat_acsr_classify:
