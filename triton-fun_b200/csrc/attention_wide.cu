@@ -378,6 +378,8 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
             auto k_here = [&](int j) { return wait_all(&ctrl->k_full[j % kSlots], (uint32_t)(j / kSlots) & 1u, kErrKFull); };
             auto issue_s = [&](int j) {                // S(j); half steps outside the range are left out
                 const int st = j % kSlots;
+                if (!kOwnP) ok = k_here(j);
+                if (!ok) return;
                 tc_fence_after_sync();
                 const bool h0 = in_range(j, 0), both = h0 && in_range(j, 1);
                 const uint32_t idesc = kHalves == 1 || both ? idesc_qk : idesc_qk_half;
@@ -395,7 +397,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
                 }
                 __syncwarp();
             };
-            if (ok) ok = k_here(0);
+            if (ok && kOwnP) ok = k_here(0);
             if (ok) issue_s(0);
             for (int j = 0; j < steps && ok; ++j) {
                 if (kOwnP && j + 1 < steps) {          // the next scores as soon as these have been read
@@ -408,9 +410,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
                 if (!ok) break;
 #pragma unroll 1
                 for (int half = 0; half < kHalves; ++half) {
-                    // (the next K, which S(j + 1) takes right behind this, first: it is there as a rule)
-                    if (!kOwnP && half == kHalves - 1 && j + 1 < steps) ok = k_here(j + 1);
-                    if (ok) ok = wait_all(&ctrl->p_full[half], (uint32_t)j & 1u, kErrP);
+                    ok = wait_all(&ctrl->p_full[half], (uint32_t)j & 1u, kErrP);
                     if (!ok) break;
                     tc_fence_after_sync();
                     if (in_range(j, half)) {
@@ -454,17 +454,6 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
                 const bool r = wait_all(&ctrl->pv_done, (uint32_t)(k - 1) & 1u, kErrPv);
                 tc_fence_after_sync();
                 return r;
-            };
-            // Lazy rescale: only when a row's maximum has grown by more than 2^8 (false when both are -inf).
-            float corr = 1.f;
-            auto grown = [&](float mx) {
-                const float m_new = fmaxf(m_used, mx * sc);
-                const bool need = (m_new - m_used) > kRescaleThreshold;
-                corr = need ? ex2(m_used - m_new) : 1.f;
-                if (need) m_used = m_new;
-                const bool any = __any_sync(0xffffffffu, need);
-                if (any) l_sum *= corr;
-                return any;
             };
             auto offset = [&]() {
                 const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
@@ -521,10 +510,24 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
                     if (lane == 0) mbar_arrive(&ctrl->s_free);
                 }
                 if (!__all_sync(0xffffffffu, v_lo <= 0 && v_hi >= kKeys)) sm::mask_scores(r, v_lo, v_hi);
-                if (grown(sm::max_score(r)) && k > 0) {
+                // Lazy rescale: only when a row's maximum has grown by more than 2^8 (false when both are -inf).  At D = 128 the
+                // maximum and the sum change behind the vote, at D = 64 beside it.  us, behind / beside: d64 window 256 of
+                // B4 H16 L4096 60.6 / 59.9, L1024 4 heads 7.23 / 7.17; d128 +-58 of L149 6.93 / 7.02, +-127 of H32 L2048 25.7 / 26.0.
+                const float m_new = fmaxf(m_used, sm::max_score(r) * sc);
+                const bool need = (m_new - m_used) > kRescaleThreshold;
+                const bool any = __any_sync(0xffffffffu, need);
+                float corr = 1.f;
+                auto raise = [&]() {
+                    corr = need ? ex2(m_used - m_new) : 1.f;
+                    if (need) m_used = m_new;
+                    if (any) l_sum *= corr;
+                };
+                if (kOwnP) raise();
+                if (any && (!kOwnP || k > 0)) {
                     ok = pv_wait();
                     if (!ok) break;
-                    rescale_o(o_addr, D / 16, corr);
+                    if (!kOwnP) raise();
+                    if (k > 0) rescale_o(o_addr, D / 16, corr);
                 }
                 const float2 nm2 = offset();
 #pragma unroll
