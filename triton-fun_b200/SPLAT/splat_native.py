@@ -314,7 +314,7 @@ def status_word(dev: torch.device) -> torch.Tensor:
             torch.cuda.current_stream(dev).synchronize()
             host = torch.zeros(1, dtype=torch.int32).pin_memory()
             check(_lib.splat_set_status_mirror(t.data_ptr(), host.data_ptr()), "splat_set_status_mirror")
-        _STATUS_MIRRORS[key] = {"host": host}
+        _STATUS_MIRRORS[key] = {"host": host, "value": ctypes.c_int32.from_address(host.data_ptr())}
         _STATUS_WORDS[key] = t
         _host.set_status(dev.index, t.data_ptr(), host.data_ptr())
     return t
@@ -325,7 +325,7 @@ def _raise_if_gave_up(dev: torch.device) -> None:
     timed-out wait (the kernels do nothing while the word is set), clear the word and raise
     instead of silently returning stale outputs.  Costs one host memory read."""
     m = _STATUS_MIRRORS.get((dev.type, dev.index))
-    if m is None or int(m["host"][0]) == 0:
+    if m is None or m["value"].value == 0:
         return
     torch.cuda.synchronize(dev)
     code = int(status_word(dev).item())
