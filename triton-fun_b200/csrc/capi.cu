@@ -147,7 +147,7 @@ extern "C" int32_t splat_attention_fused_table(const void* q, const void* k, int
         return SPLAT_ERR_BAD_ARG;
     }
     int32_t rc = SPLAT_ERR_UNSUPPORTED_SHAPE;
-    if (path == SPLAT_PATH_AUTO && dtype == SPLAT_F32)   // register tiles wherever the plan shows bands
+    if (path == SPLAT_PATH_AUTO && dtype == SPLAT_F32)   // register tiles or tensor cores wherever the plan shows bands
         rc = splat::attention_tile_f32(q, k, k_stride_bh, k_stride_col, k_stride_k, v, o, sTod_lin, sTod_tr,
                                        nnzs, bh, n_rows, n_cols, d, scale, plan_i32, status_word, lse, st);
     if (rc == SPLAT_ERR_UNSUPPORTED_SHAPE)

@@ -1,5 +1,5 @@
 // fp32 SDDMM, SpMM and fused attention over ACSR on register tiles (CUDA cores, true fp32 FMA).  What is more than a wave or two
-// of these tiles runs on the tensor cores (attention_split.cu, ops_split.cu).
+// of these tiles runs on the tensor cores (attention_split.cu, ops_split.cu), given a status word.
 //
 // Applies to patterns whose rows, regrouped by residue class, are contiguous bands: one stride s for
 // all rows with more than one non-zero and start_i == i (mod s), as the plan of splat_acsr_classify
@@ -589,6 +589,7 @@ static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
     return launch_kernel(kern, (unsigned)blocks, 32 * RW * KW, bytes, st, p);
 }
 
+// (More than a wave or two of 32-row CTAs come here without a status word, with Q off a 16-byte boundary or with scale 0 only.)
 // 64-row CTAs unless they leave SMs without their three CTAs: then 32-row CTAs, whose four warps share the
 // keys of one row block, finish sooner, while with the GPU full they load every key twice as often; and with
 // less than two such CTAs per SM eight warps share them.  Four / eight warps, us, at 256 CTAs (L1024, +-64, where five or
