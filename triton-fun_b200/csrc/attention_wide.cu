@@ -29,6 +29,9 @@
 //     of L1024 1024 18.4 -> 9.8; L64 causal 1000 19.7 -> 11.0; the same bits.  With two steps it depends on the number of tiles
 //     (class of 128 rows 256 5.97 -> 6.72, 512 12.2 -> 9.5), and with more of them the running maximum is another than
 //     with 128-key steps, so that shards of a problem would not agree bit for bit.
+//   * With d up to 32 the MMAs and the epilogue take the first 32 of a tile's 64 columns (kCols; the others are zero).  us, 64 columns -> 32:
+//     bf16 H2 L300 window 32 6.11 -> 5.73; fp16 H16 L512 window 128 6.83 -> 6.31, B4 H16 L4096 window 256 59.9 -> 57.0; bf16 B3 H34
+//     L633 strided 19 20.3 -> 17.3, B2 H16 L4096 strided 64 28.0 -> 25.2, H32 L8192 window 1024 122.2 -> 118.9; the same bits.
 //   * Few instructions where they are not the point: waits are a try and a counter (looking at the status word, a clock and an
 //     atomic in each of 15 of them were a quarter of the code), the control block has constant addresses, an MMA's
 //     descriptor is an addition.  us, before -> after: fp16 B4 H16 L4096 d64 window 256 64.1 -> 60.7; bf16 B4 H16 L4096
@@ -104,7 +107,7 @@ struct Control {
     alignas(16) uint32_t single[4];  // rows with one non-zero; later those of them whose score is not finite
 };
 
-// kKeys: keys of a step; with 64 there is one step (classes of up to 64 rows)
+// D: columns of a tile.  kKeys: keys of a step; with 64 there is one step (classes of up to 64 rows)
 template <int D, int kKeys> struct Layout {
     static constexpr int kSub = D / 64;
     static constexpr int kQBytes = kSub * kSubBytes;
@@ -207,7 +210,7 @@ __device__ __forceinline__ uint4 odd_singles(const Params& p, uint4 single, int6
     return make_uint4(rows[0], rows[1], rows[2], rows[3]);
 }
 
-template <typename T, int D, int kKeys, bool kLse, bool kOwn>
+template <typename T, int D, int kCols, int kKeys, bool kLse, bool kOwn>
 __global__ void __launch_bounds__(kThreads, Layout<D, kKeys>::kPerSm)
 attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
     using L = Layout<D, kKeys>;
@@ -366,7 +369,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
             constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
             const uint32_t idesc_qk = instr_desc_f16(fmt, kTile, kKeys, p.kt_major ? 1u : 0u);
             const uint32_t idesc_qk_half = instr_desc_f16(fmt, kTile, 64, p.kt_major ? 1u : 0u);
-            constexpr uint32_t idesc_pv = instr_desc_f16(fmt, kTile, D, 1);
+            constexpr uint32_t idesc_pv = instr_desc_f16(fmt, kTile, kCols, 1);
             const uint32_t q_lo = desc_lo(smem, 16), k_lo = desc_lo(smem + L::kKOff, p.kt_major ? D * 128 : 16);
             const uint32_t v_lo = desc_lo(smem + L::kVOff, L::kKeySub);
             const uint32_t k_step = (p.kt_major ? 2048 : 32) >> 4, k_sub = (p.kt_major ? 4 * 2048 : L::kKeySub) >> 4;
@@ -390,7 +393,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
 #pragma unroll
                     for (int sub = 0; sub < L::kSub; ++sub, b += k_sub)
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
+                        for (int kk = 0; kk < (kCols < 64 ? kCols / 16 : 4); ++kk)
                             mma_ss(to, desc_sw128(q_lo + ((sub * kSubBytes + kk * 32) >> 4)), desc_sw128(b + kk * k_step), idesc, sub + kk > 0);
                     mma_commit(&ctrl->s_full);
                     mma_commit(&ctrl->k_free[st]);
@@ -527,7 +530,7 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
                     ok = pv_wait();
                     if (!ok) break;
                     if (!kOwnP) raise();
-                    if (k > 0) rescale_o(o_addr, D / 16, corr);
+                    if (k > 0) rescale_o(o_addr, kCols / 16, corr);
                 }
                 const float2 nm2 = offset();
 #pragma unroll
@@ -573,11 +576,11 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
         }
         const T* vrow = reinterpret_cast<const T*>(p.v) + (head + row_start) * p.d;
         const int t = warp * 32 + lane;
-        constexpr int kRead = kKeys == 64 ? 32 : D;             // columns of O in registers at a time
+        constexpr int kRead = kKeys == 64 ? 32 : kCols;             // columns of O in registers at a time
         uint32_t o_raw[kRead];
         float2 odd0 = make_float2(0.f, 0.f), odd1 = odd0;       // not finite: nor is the row
 #pragma unroll
-        for (int ch = 0; ch < D / 32; ++ch) {
+        for (int ch = 0; ch < kCols / 32; ++ch) {
             if (ch * 32 % kRead == 0 && have_o && ok) {
 #pragma unroll
                 for (int i = 0; i < kRead; i += 32) tmem_ld32(o_addr + ch * 32 + i, o_raw + i);
@@ -646,11 +649,12 @@ attention_wide_kernel(const __grid_constant__ Maps<4> maps, const Params p) {
 // B8 H64 L32768 d128 window 1024 11.71 -> 12.12 ms).  Problems with d = 64 or 128 and classes of one length do without:
 // they have only ever run on tensor cores, with finite V as a condition (splat_b200.h); the others came from the row
 // kernels, which read nothing but a row's own keys.
-template <typename T, int D, int kKeys>
+template <typename T, int D, int kCols, int kKeys>
 static int32_t launch(const Maps<4>& maps, const Params& prm, int64_t bh, cudaStream_t st) {
     const bool own = (prm.d != 64 && prm.d != 128) || prm.cls.longer != 0;
-    auto kern = own ? (prm.lse != nullptr ? attention_wide_kernel<T, D, kKeys, true, true> : attention_wide_kernel<T, D, kKeys, false, true>)
-                    : (prm.lse != nullptr ? attention_wide_kernel<T, D, kKeys, true, false> : attention_wide_kernel<T, D, kKeys, false, false>);
+    auto kern = prm.lse != nullptr ? attention_wide_kernel<T, D, kCols, kKeys, true, true> : attention_wide_kernel<T, D, kCols, kKeys, false, true>;
+    if constexpr (kCols == D)
+        if (!own) kern = prm.lse != nullptr ? attention_wide_kernel<T, D, D, kKeys, true, false> : attention_wide_kernel<T, D, D, kKeys, false, false>;
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(kern), Layout<D, kKeys>::kSmemBytes)) return SPLAT_ERR_LAUNCH;
     return launch_kernel(kern, prm.cls.grid(prm.stride, bh), kThreads, Layout<D, kKeys>::kSmemBytes, st, maps, prm);
 }
@@ -687,8 +691,9 @@ int32_t attention_wide(const void* q, const void* k, int kt_major, const void* v
     }
     auto launch = [&](auto element) {
         using T = decltype(element);
-        if (d > 64) return wide::launch<T, 128, 128>(maps, p, bh, st);
-        return one_step ? wide::launch<T, 64, 64>(maps, p, bh, st) : wide::launch<T, 64, 128>(maps, p, bh, st);
+        if (d > 64) return wide::launch<T, 128, 128, 128>(maps, p, bh, st);
+        if (d > 32) return one_step ? wide::launch<T, 64, 64, 64>(maps, p, bh, st) : wide::launch<T, 64, 64, 128>(maps, p, bh, st);
+        return one_step ? wide::launch<T, 64, 32, 64>(maps, p, bh, st) : wide::launch<T, 64, 32, 128>(maps, p, bh, st);
     };
     return dtype == SPLAT_BF16 ? launch(__nv_bfloat16()) : launch(__half());
 }
