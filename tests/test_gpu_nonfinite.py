@@ -107,3 +107,38 @@ def test_rows_without_a_finite_score(dtype, d):
     none[50 + p0:90] = True
     out = out.cpu()
     assert torch.isnan(out[:, :, none]).all() and (out[:, :, ~none] - 1).abs().max() < 1e-3
+
+
+#        dtype, d, heads: fp32 on register tiles, and enough of them, or d = 128, for the tensor cores
+LSE_FORMS = [(torch.float32, 32, 2), (torch.float32, 64, 2), (torch.float32, 32, 30), (torch.float32, 64, 30), (torch.float32, 128, 2),
+             (torch.float16, 32, 2)]
+
+
+@pytest.mark.parametrize("dtype,d,H", LSE_FORMS)
+def test_log_sum_exp_beside_scores_of_minus_infinity(dtype, d, H):
+    """A key whose score is minus infinity has no weight: output and log-sum-exp are those of the row's other keys."""
+    import acsr_helpers as ah
+    import splat_native as n
+    L = 300
+    for kind, p0, p1 in ((ao.PATTERN_WINDOWED, 20, 0), (ao.PATTERN_DILATED, 40, 3)):
+        acsr = ah.create_acsr(ah.PatternMask(kind, L, p0, p1), 16, 0)
+        meta = ao.metadata_from_pattern(kind, L, p0, p1, 16)
+        torch.manual_seed(d + H)
+        q, k, v = (torch.randn(1, H, L, d) for _ in range(3))
+        q[:, :, :, 3] = q[:, :, :, 3].abs() + 0.1
+        k[:, :, 50, 3] = k[:, :, 200, 3] = -INF
+        if dtype == torch.float32:
+            k[:, :, 120, 3] = -3.395e38                  # infinite in bf16
+        q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+        scale = d ** -0.5
+        scores = at.sddmm_acsr(q, k.transpose(2, 3), meta, acsr[5])
+        ref_o, ref_lse = _attention(q, k, v, meta, acsr[5], scale), at.lse_acsr(scores, meta, scale)
+        assert torch.isfinite(ref_o).all() and torch.isinf(scores).any()
+        for contiguous in (False, True):
+            kt = k.cuda().transpose(2, 3)
+            out = torch.full((1, H, L, d), 5.0, dtype=dtype, device="cuda")
+            lse = torch.full((1, H, L), 5.0, device="cuda")
+            n.attention_fused(q.cuda(), kt.contiguous() if contiguous else kt, v.cuda(), out, acsr[2], acsr[3], acsr[4], scale, lse=lse)
+            n.check_status_word(0)
+            _same(out, ref_o, dtype, f"{kind} {contiguous}")
+            _same(lse, ref_lse, torch.float32, f"lse {kind} {contiguous}")

@@ -9,8 +9,8 @@
 // (1.06e-7 / 1.46e-7), the same six products with hh first 7.5e-7, sums over 1024 on the tensor core alone 6.6e-6
 // (5.7e-7).  Of a whole call 0.53 to 0.76 of that of the register tiles, at every pattern and size tried.
 // A tiny number's last pieces are denormal: below 2^-110 in magnitude an operand loses precision relative to itself.  Numbers
-// that are not finite, or round to infinity in bf16, make their rows NaN; such rows are computed again from their own
-// keys (row_exact.cuh), as in the other tile kernels.
+// that are not finite, or round to infinity in bf16, make their rows NaN; such rows, and their log-sum-exps, are computed again
+// from their own keys (row_exact.cuh), as in the other tile kernels.
 //
 // One CTA = 128 rows of one (bh, class).  Warps 0-7: thread = (row, half of the columns).  A step of 64 keys:
 //     K(j + 1), V(j) from global memory through registers, split, to shared memory (128-byte swizzle; both layouts of K)
@@ -495,17 +495,22 @@ attention_split_kernel(const __grid_constant__ Params p) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, L::kTmemCols);
     }
-    // rows that are not finite, perhaps by keys outside their bands
+    // rows that are not finite, perhaps by keys outside their bands (by the warps that have the registers)
     const uint4 again = *reinterpret_cast<const uint4*>(ctrl->again);
-    if ((again.x | again.y | again.z | again.w) == 0) return;
+    if ((again.x | again.y | again.z | again.w) == 0 || warp >= kMmaWarp) return;
 #pragma unroll 1
-    for (int i = warp; i < kTile; i += kThreads / 32) {
+    for (int i = warp; i < kTile; i += kWorkers / 32) {
         if (((ctrl->again[i >> 5] >> (i & 31)) & 1u) == 0) continue;
         const int2 about = ctrl->row[i];
         const int64_t row = head + (int64_t)(u0 + i) * p.stride + res;
         const int own = min(about.y, (p.n_rows - 1 - about.x) / p.stride + 1);
-        store_row(p.o + row * D, D, attention_row<float>(p.q + row * D, p.k + head * D, kKt ? 1 : D, kKt ? p.n_rows : 1, p.v + head * D,
-                                                         about.x, p.stride, own, D, p.sign * p.scale_log2));
+        const float* k = p.k + head * D;
+        const int64_t ksc = kKt ? 1 : D, ksk = kKt ? p.n_rows : 1;
+        const float scale = p.sign * p.scale_log2;
+        float4 o;
+        if constexpr (kLse) o = attention_row_lse<float>(p.q + row * D, k, ksc, ksk, p.v + head * D, about.x, p.stride, own, D, scale, p.lse + row);
+        else o = attention_row<float>(p.q + row * D, k, ksc, ksk, p.v + head * D, about.x, p.stride, own, D, scale);
+        store_row(p.o + row * D, D, o);
     }
 }
 

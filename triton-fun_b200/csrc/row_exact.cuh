@@ -13,12 +13,14 @@
 namespace splat {
 
 // softmax(scale q . K) V over the columns first, first + step, ... (nnz of them).  q: the row; k, v: the head's arrays,
-// element (column, c) of K at column * ksc + c * ksk.  Lane l returns columns l, l + 32, l + 64 and l + 96.
+// element (column, c) of K at column * ksc + c * ksk.  Lane l returns columns l, l + 32, l + 64 and l + 96, and the
+// maximum and the sum (both in the log2 domain) in `m` and `sum`.
 template <typename T>
-__device__ __noinline__ float4 attention_row(const T* q, const T* k, int64_t ksc, int64_t ksk, const T* v, int64_t first,
-                                             int step, int nnz, int d, float scale_log2) {
+__device__ __forceinline__ float4 attention_row_sums(const T* q, const T* k, int64_t ksc, int64_t ksk, const T* v, int64_t first,
+                                                     int step, int nnz, int d, float scale_log2, float& m, float& sum) {
     const int lane = threadIdx.x & 31;
-    float m = -INFINITY, l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+    float l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+    m = -INFINITY;
     for (int j = lane; j < nnz; j += 32)
         m = fmaxf(m, dot_strided<T>(q, k + (first + (int64_t)j * step) * ksc, ksk, d) * scale_log2);
     m = warp_max(m);
@@ -34,8 +36,24 @@ __device__ __noinline__ float4 attention_row(const T* q, const T* k, int64_t ksc
                 if (lane + 32 * i < d) acc[i] = fmaf(pt, DT<T>::to_f(row[lane + 32 * i]), acc[i]);
         }
     }
-    const float inv = 1.f / warp_sum(l);
+    sum = warp_sum(l);
+    const float inv = 1.f / sum;
     return make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
+}
+template <typename T>
+__device__ __noinline__ float4 attention_row(const T* q, const T* k, int64_t ksc, int64_t ksk, const T* v, int64_t first,
+                                             int step, int nnz, int d, float scale_log2) {
+    float m, sum;
+    return attention_row_sums<T>(q, k, ksc, ksk, v, first, step, nnz, d, scale_log2, m, sum);
+}
+// ... and the row's log-sum-exp to *lse
+template <typename T>
+__device__ __noinline__ float4 attention_row_lse(const T* q, const T* k, int64_t ksc, int64_t ksk, const T* v, int64_t first,
+                                                 int step, int nnz, int d, float scale_log2, float* lse) {
+    float m, sum;
+    const float4 o = attention_row_sums<T>(q, k, ksc, ksk, v, first, step, nnz, d, scale_log2, m, sum);
+    if ((threadIdx.x & 31) == 0) *lse = lse_from_log2(m, sum);
+    return o;
 }
 
 // sum_j p[j] V[first + j step], as above.
