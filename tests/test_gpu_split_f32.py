@@ -124,6 +124,26 @@ def test_nothing_is_written_while_the_status_word_is_set():
     assert torch.isfinite(out).all() and not (out == 3.0).any()
 
 
+def test_host_operands_while_the_status_word_is_set():
+    """forward_host's results are never taken for good after a kernel gave up."""
+    import r_attention
+    H, L, d = 4, 300, 128
+    attn = r_attention.RegularAttention(1, L, H, d, ah.create_windowed_mask(L, 40), 16, 16, 0, torch.float32, scale=d ** -0.5)
+    q, k, v = (torch.randn(1, H, L, d).pin_memory() for _ in range(3))
+    ref, out = torch.zeros(1, H, L, d).pin_memory(), torch.zeros(1, H, L, d).pin_memory()
+    attn.forward_host(q, k, v, ref)
+    torch.cuda.synchronize()
+    n.status_word(attn.nnzs.device).fill_(7)
+    attn.forward_host(q, k, v, out)        # a kernel that is started now passes the word on
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError):
+        attn.forward_host(q, k, v, out)
+    attn.forward_host(q, k, v, out)
+    torch.cuda.synchronize()
+    attn.check_status()
+    assert torch.equal(out, ref) and ref.abs().sum() > 0
+
+
 #        mask, L, heads: more than two waves of tiles of 32 rows
 OPS = [
     (lambda L: ah.create_causal_windowed_mask(L, L - 1), 128, 75),

@@ -200,7 +200,7 @@ def attention_host(q, k, v, out, stage: dict, sTod_lin, sTod_tr, nnzs, scale: fl
     """Host tensors (B,H,L,d) through the device in chunks; stage as RegularAttention.forward_host keeps it."""
     dev = nnzs.device
     B, H, L, d = q.shape
-    if _band_candidate(q, path):
+    if _may_give_up(q, path):
         _raise_if_gave_up(dev)
     sw = status_word(dev)
     table = band_table(sTod_lin, sTod_tr, nnzs, L) if _band_candidate(q, path) else None
@@ -435,6 +435,11 @@ def _band_candidate(x: torch.Tensor, path: int) -> bool:
     return path != PATH_GENERIC and x.dtype in (torch.float16, torch.bfloat16) and x.numel() > 0
 
 
+def _may_give_up(x: torch.Tensor, path: int) -> bool:
+    """A tensor-core kernel may run: 16-bit operands, or fp32 bands (attention_split.cu, ops_split.cu)."""
+    return _band_candidate(x, path) or (path == PATH_AUTO and x.dtype == torch.float32)
+
+
 def _native_from_now_on(dev: torch.device) -> None:
     """The native path takes ordinary operands once the status word exists.  Setting it up synchronises, which a
     capture does not allow; the kernels without bounded waits need none."""
@@ -609,7 +614,7 @@ def attention_fused(q, kt, v, output, sTod_lin, sTod_tr, nnzs, scale: float = 1.
         if plan is None:
             plan = classify(sTod_lin, sTod_tr, nnzs)
         plan_arr = (ctypes.c_int32 * 8)(*plan)
-    if tensor_core or (path == PATH_AUTO and q.dtype == torch.float32):       # (fp32 bands: attention_split.cu)
+    if _may_give_up(q, path):
         _raise_if_gave_up(dev)
     if tensor_core:
         rows = _rows_of_k(kt, plan, L) if path == PATH_AUTO else None
