@@ -232,12 +232,12 @@ int32_t splat_spmm_band(const void* p, const void* v, void* o, const float* sTod
                         int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
                         const int32_t* plan_i32, int32_t* status_word, void* stream);
 
-/* SDDMM / SpMM of fp32 operands, for patterns whose rows are bands: on register tiles (true fp32 FMA), or, from one or two waves of
- * them on and if the current device has a status word with a host copy (splat_set_status_mirror), on the tensor cores, which then
- * work with that word as the band kernels do with theirs.  Rows are bands
+/* SDDMM / SpMM of fp32 operands on register tiles (true fp32 FMA), for patterns whose rows are bands
  * of one stride (plan_i32 as from splat_acsr_classify); n_rows need not be a multiple of the stride.
  * d = 32, 64 or 128, K as rows of d or as a contiguous (BH, d, n_cols) array.  Otherwise
- * SPLAT_ERR_UNSUPPORTED_SHAPE / SPLAT_ERR_MISALIGNED without a launch: use splat_sddmm / splat_spmm. */
+ * SPLAT_ERR_UNSUPPORTED_SHAPE / SPLAT_ERR_MISALIGNED without a launch: use splat_sddmm / splat_spmm.
+ * The forms with a status word run on the tensor cores from one or two waves of the register tiles on, and use the word as
+ * splat_sddmm_band / splat_spmm_band do; with NULL they are the same as the others. */
 int32_t splat_sddmm_tile(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
                          int64_t k_stride_k, void* s_out, const float* sTod_lin, const float* sTod_tr,
                          const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
@@ -246,6 +246,15 @@ int32_t splat_spmm_tile(const void* p, const void* v, void* o, const float* sTod
                         const float* sTod_tr, const float* nnzs, int64_t bh, int64_t n_rows,
                         int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
                         const int32_t* plan_i32, void* stream);
+int32_t splat_sddmm_tile_status(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
+                                int64_t k_stride_k, void* s_out, const float* sTod_lin, const float* sTod_tr,
+                                const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
+                                int64_t trailing_dim, int32_t dtype, const int32_t* plan_i32, int32_t* status_word,
+                                void* stream);
+int32_t splat_spmm_tile_status(const void* p, const void* v, void* o, const float* sTod_lin,
+                               const float* sTod_tr, const float* nnzs, int64_t bh, int64_t n_rows,
+                               int64_t n_cols, int64_t d, int64_t trailing_dim, int32_t dtype,
+                               const int32_t* plan_i32, int32_t* status_word, void* stream);
 
 /* Band table of metadata whose plan shows bands of one stride: 2 (n_rows + stride ceil(ceil(n_rows / stride) /
  * 128)) device int32, 8-byte aligned, holding every row's band and every 128-row tile's key range in the

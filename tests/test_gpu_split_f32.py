@@ -1,12 +1,16 @@
 """GPU: the fused fp32 kernel on the tensor cores (operands split into three bf16 numbers) at the edges of its tiles of 128 rows
 and steps of 64 keys, against 64 bits: it must not be further off than the kernel that sums with FMAs."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
 
 import acsr_helpers as ah
 import splat_native as n
+from conftest import ROOT, SPLAT_DIR
 
 pytestmark = pytest.mark.gpu
 
@@ -209,3 +213,28 @@ def test_sddmm_scores_that_are_not_finite():
     assert not ok.all() and torch.equal(torch.isfinite(s), ok)
     assert torch.equal(torch.isnan(s), torch.isnan(rows)) and torch.equal(s[torch.isinf(s)], rows[torch.isinf(rows)])
     assert (s[ok] - rows[ok]).abs().max() <= 1e-5 * rows[ok].abs().max()
+
+
+FOREIGN_WORD = """
+import torch
+import acsr_helpers as ah
+import splat_native as n
+word = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+host = torch.zeros(1, dtype=torch.int32).pin_memory()
+assert n._lib.splat_set_status_mirror(word.data_ptr(), host.data_ptr()) == 0
+acsr = ah.create_acsr(ah.create_windowed_mask(300, 20), 16, 0)
+q, k, v = (torch.randn(1, 40, 300, 64, device="cuda") for _ in range(3))
+s, o = torch.full((1, 40, 300, acsr[5]), float("nan"), device="cuda"), torch.full_like(q, float("nan"))
+for _ in range(2):        # (the first call takes the Python path)
+    n.sddmm(q, k.transpose(2, 3), s.fill_(float("nan")), *acsr[2:5], acsr[5])
+    n.spmm(s.nan_to_num(), v, o.fill_(float("nan")), *acsr[2:5], acsr[5])
+    torch.cuda.synchronize()
+    assert torch.isfinite(s).all() and torch.isfinite(o).all(), "not written"
+assert word.item() == 7 and host.item() == 0, "another's word was used"
+"""
+
+
+def test_a_status_word_that_others_registered_is_not_used():
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join((SPLAT_DIR, ROOT)))
+    done = subprocess.run([sys.executable, "-c", FOREIGN_WORD], env=env, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]

@@ -1,6 +1,7 @@
 """GPU: the fp32 register-tile kernels (fused, SDDMM, SpMM) against the CPU oracle at the edges of their
 tiles: lengths around multiples of 64, classes with a missing last row, both K layouts, rows with one or
-no non-zero."""
+no non-zero.  Without a status word the library runs them at any size; the launchers, which have one, hand what is more than
+a wave or two of their tiles to the tensor cores (test_gpu_split_f32.py)."""
 import ctypes
 
 import pytest
@@ -27,6 +28,40 @@ PATTERNS = [
 ]
 
 
+def _tiles(plan, L, H):
+    """Tiles of 32 rows."""
+    stride = plan[1] if plan[7] > 0 else 1
+    return -(-(-(-L // stride)) // 32) * stride * H
+
+
+class _Tiles:
+    """The three operators on the register tiles: the library's entry points without a status word."""
+
+    def __init__(self, acsr, L, H, d):
+        import splat_native as n
+        self.n, self.T, self.sizes = n, acsr[5], (H, L, L, d)
+        self.plan = n.classify(acsr[2], acsr[3], acsr[4])
+        assert self.plan[3] == 0 and (self.plan[7] == 0 or self.plan[1] == self.plan[2])     # a band pattern
+        self.plan_arr = ctypes.cast((ctypes.c_int32 * 8)(*self.plan), ctypes.c_void_p)
+        self.acsr, self.vectors = acsr, [t.data_ptr() for t in acsr[2:5]]
+        self.fp32 = n.dtype_code(torch.float32)
+
+    def fused(self, q, kt, v, o, lse, scale):
+        _bh, ksb, ksk, ksc = self.n._flat_bh(kt, "kt")
+        return self.n._lib.splat_attention_fused_table(
+            q.data_ptr(), kt.data_ptr(), ksb, ksc, ksk, v.data_ptr(), o.data_ptr(), lse.data_ptr(), *self.vectors, *self.sizes, scale,
+            self.fp32, self.n.PATH_AUTO, self.plan_arr, None, None, None, self.n._stream(q.device))
+
+    def sddmm(self, q, kt, s):
+        _bh, ksb, ksk, ksc = self.n._flat_bh(kt, "kt")
+        return self.n._lib.splat_sddmm_tile(q.data_ptr(), kt.data_ptr(), ksb, ksc, ksk, s.data_ptr(), *self.vectors, *self.sizes, self.T,
+                                            self.fp32, self.plan_arr, self.n._stream(q.device))
+
+    def spmm(self, p, v, o):
+        return self.n._lib.splat_spmm_tile(p.data_ptr(), v.data_ptr(), o.data_ptr(), *self.vectors, *self.sizes, self.T, self.fp32,
+                                           self.plan_arr, self.n._stream(p.device))
+
+
 @pytest.mark.parametrize("contiguous", [False, True])
 @pytest.mark.parametrize("d", [32, 64, 128])
 def test_tile_kernels_against_oracle(d, contiguous):
@@ -38,52 +73,50 @@ def test_tile_kernels_against_oracle(d, contiguous):
         meta = ao.metadata_from_pattern(kind, L, p0, p1, 16)
         T, what = acsr[5], f"{(kind, L, p0, p1)} d={d}"
         q, k, v = (torch.randn(1, H, L, d) for _ in range(3))
-        kt = k.cuda().transpose(2, 3)
+        qd, kt, vd = q.cuda(), k.cuda().transpose(2, 3), v.cuda()
         kt = kt.contiguous() if contiguous else kt
         scale = d ** -0.5
-        plan = n.classify(acsr[2], acsr[3], acsr[4])
-        assert plan[3] == 0 and (plan[7] == 0 or plan[1] == plan[2])     # a band pattern
-        plan_arr = ctypes.cast((ctypes.c_int32 * 8)(*plan), ctypes.c_void_p)
-        vectors = [t.data_ptr() for t in acsr[2:5]]
-        o = torch.full((1, H, L, d), float("nan"), device="cuda")
-        lse = torch.full((1, H, L), float("nan"), device="cuda")
-        n.attention_fused(q.cuda(), kt, v.cuda(), o, acsr[2], acsr[3], acsr[4], scale, n.PATH_AUTO, lse=lse)
+        tile, tiles = _Tiles(acsr, L, H, d), _tiles(n.classify(*acsr[2:5]), L, H)
         s_ref = at.sddmm_acsr(q, k.transpose(2, 3), meta, T)
-        assert_close(o, at.attention_acsr(q, k.transpose(2, 3), v, meta, T, scale), torch.float32, f"fused {what}")
-        assert_close(lse, at.lse_acsr(s_ref, meta, scale), torch.float32, f"lse {what}")
-        s = torch.full((1, H, L, T), float("nan"), device="cuda")
-        n.sddmm(q.cuda(), kt, s, acsr[2], acsr[3], acsr[4], T)
-        assert_close(s, s_ref, torch.float32, f"sddmm {what}")
-        # the tile kernels ran: asked for by name they take the call and give the same bits
-        qd, tile = q.cuda(), torch.full_like(s, float("nan"))
-        _bh, ksb, ksk, ksc = n._flat_bh(kt, "kt")
-        assert n._lib.splat_sddmm_tile(qd.data_ptr(), kt.data_ptr(), ksb, ksc, ksk, tile.data_ptr(), *vectors, H, L, L, d, T,
-                                       n.dtype_code(s.dtype), plan_arr, n._stream(s.device)) == 0 and torch.equal(s, tile), what
-        if L > 32:      # (row kernels sum in another order)
-            rows = torch.empty_like(o)
-            n.attention_fused(qd, kt, v.cuda(), rows, acsr[2], acsr[3], acsr[4], scale, n.PATH_GENERIC)
-            assert not torch.equal(o, rows), f"fused {what}: the row kernel"
         _cols, valid = at._cols(meta, T)
-        assert torch.count_nonzero(s.cpu() * (~valid)) == 0, "padding slots must be zero"
         p = torch.rand(1, H, L, T)
         p_dev = torch.where(valid, p, torch.full_like(p, float("nan"))).cuda()     # padding is not read
-        o2 = torch.full((1, H, L, d), float("nan"), device="cuda")
-        n.spmm(p_dev, v.cuda(), o2, acsr[2], acsr[3], acsr[4], T)
-        assert_close(o2, at.spmm_acsr(p, v, meta), torch.float32, f"spmm {what}")
-        vd, tile = v.cuda(), torch.full_like(o2, float("nan"))
-        rc = n._lib.splat_spmm_tile(p_dev.data_ptr(), vd.data_ptr(), tile.data_ptr(), *vectors, H, L, L, d, T,
-                                    n.dtype_code(p.dtype), plan_arr, n._stream(s.device))
+        nan = lambda *shape: torch.full(shape, float("nan"), device="cuda")
+        o, lse, s, o2 = nan(1, H, L, d), nan(1, H, L), nan(1, H, L, T), nan(1, H, L, d)
+        assert tile.fused(qd, kt, vd, o, lse, scale) == 0 and tile.sddmm(qd, kt, s) == 0, what
+        assert_close(o, at.attention_acsr(q, k.transpose(2, 3), v, meta, T, scale), torch.float32, f"fused {what}")
+        assert_close(lse, at.lse_acsr(s_ref, meta, scale), torch.float32, f"lse {what}")
+        assert_close(s, s_ref, torch.float32, f"sddmm {what}")
+        assert torch.count_nonzero(s.cpu() * (~valid)) == 0, "padding slots must be zero"
+        if L > 32:      # (row kernels sum in another order)
+            rows = torch.empty_like(o)
+            n.attention_fused(qd, kt, vd, rows, acsr[2], acsr[3], acsr[4], scale, n.PATH_GENERIC)
+            assert not torch.equal(o, rows), f"fused {what}: the row kernel"
+        rc = tile.spmm(p_dev, vd, o2)
         if kind == ao.PATTERN_STRIDED:      # classes of 26 rows: too short for SpMM, which the row kernel does
             assert rc == n.ERR_UNSUPPORTED_SHAPE
         else:
-            assert rc == 0 and torch.equal(o2, tile), what
+            assert rc == 0
+            assert_close(o2, at.spmm_acsr(p, v, meta), torch.float32, f"spmm {what}")
+        # the launchers: the same kernels, so the same bits, up to the lines behind which the tensor cores take over
+        lo, ls, lo2 = nan(1, H, L, d), nan(1, H, L, T), nan(1, H, L, d)
+        n.attention_fused(qd, kt, vd, lo, acsr[2], acsr[3], acsr[4], scale, n.PATH_AUTO)
+        n.sddmm(qd, kt, ls, acsr[2], acsr[3], acsr[4], T)
+        n.spmm(p_dev, vd, lo2, acsr[2], acsr[3], acsr[4], T)
+        assert_close(ls, s_ref, torch.float32, f"sddmm launcher {what}")
+        assert_close(lo2, at.spmm_acsr(p, v, meta), torch.float32, f"spmm launcher {what}")
+        if tiles <= 148 and d < 128:
+            assert torch.equal(lo, o), what
+        if tiles <= (296 if d == 32 else 148):
+            assert torch.equal(ls, s), what
+        if rc == 0 and tiles <= (148 if d == 128 else 296):
+            assert torch.equal(lo2, o2), what
 
 
 @pytest.mark.parametrize("d", [32, 64])
 def test_sddmm_and_spmm_on_either_side_of_each_register_budget(d):
     """CTAs of eight warps up to 148 and from there, of 32 and of 64 rows up to 470, to 614, to 888 and from there."""
     import acsr_helpers as ah
-    import splat_native as n
     for L, H in [(64, 74), (64, 75), (96, 156), (96, 157), (96, 204), (96, 205), (64, 470), (64, 471), (64, 614), (64, 615), (64, 888),
                  (64, 889)]:
         acsr = ah.create_acsr(ah.create_windowed_mask(L, 21), 16, 0)
@@ -92,8 +125,8 @@ def test_sddmm_and_spmm_on_either_side_of_each_register_budget(d):
         g = torch.Generator(device="cuda").manual_seed(L + H)
         q, k, v = (torch.randn(1, H, L, d, device="cuda", generator=g) for _ in range(3))
         s, o = torch.full((1, H, L, T), float("nan"), device="cuda"), torch.full_like(q, float("nan"))
-        n.sddmm(q, k.transpose(2, 3), s, acsr[2], acsr[3], acsr[4], T)
-        n.spmm(s, v, o, acsr[2], acsr[3], acsr[4], T)
+        tile = _Tiles(acsr, L, H, d)
+        assert tile.sddmm(q, k.transpose(2, 3), s) == 0 and tile.spmm(s, v, o) == 0
         assert_close(s, at.sddmm_acsr(q.cpu(), k.cpu().transpose(2, 3), meta, T), torch.float32, f"sddmm {L} {H}")
         # sums of 43 products of normal values: 2^-24 of some 43 sqrt(d) each, well under the tolerance
         assert_close(o / d ** 0.5, at.spmm_acsr(s.cpu(), v.cpu(), meta) / d ** 0.5, torch.float32, f"spmm {L} {H}")

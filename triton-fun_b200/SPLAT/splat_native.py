@@ -55,6 +55,9 @@ SIGNATURES = {
     "splat_sddmm_tile": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64,
                          _i32, _vp, _vp],
     "splat_spmm_tile": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp],
+    "splat_sddmm_tile_status": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64,
+                                _i32, _vp, _vp, _vp],
+    "splat_spmm_tile_status": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp, _vp],
     "splat_sddmm_band_table": [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64,
                                _i32, _vp, _vp, _vp, _vp],
     "splat_spmm_band_table": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _vp,
@@ -507,12 +510,13 @@ def sddmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = 
         _raise_if_gave_up(dev)             # (a tensor-core kernel may run: ops_split.cu)
         plan_arr = (ctypes.c_int32 * 8)(*plan)
         with _on(dev):
-            rc = _lib.splat_sddmm_tile(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
-                                       _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
-                                       _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, trailing_dim,
-                                       dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p), _stream(dev))
+            rc = _lib.splat_sddmm_tile_status(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
+                                              _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
+                                              _f32_vec(nnzs, L, "nnzs"), bh, L, n_cols, d, trailing_dim,
+                                              dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p),
+                                              status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE:
-            check(rc, "splat_sddmm_tile")
+            check(rc, "splat_sddmm_tile_status")
             return
     with _on(dev):
         check(_lib.splat_sddmm(x.data_ptr(), y.data_ptr(), ksb, ksc, ksk, output.data_ptr(),
@@ -575,12 +579,13 @@ def spmm(x, y, output, sTod_lin, sTod_tr, nnzs, trailing_dim: int, path: int = P
         _raise_if_gave_up(dev)             # (a tensor-core kernel may run: ops_split.cu)
         plan_arr = (ctypes.c_int32 * 8)(*plan)
         with _on(dev):
-            rc = _lib.splat_spmm_tile(x.data_ptr(), y.data_ptr(), output.data_ptr(),
-                                      _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
-                                      _f32_vec(nnzs, L, "nnzs"), B * H, L, n_cols, d, T,
-                                      dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p), _stream(dev))
+            rc = _lib.splat_spmm_tile_status(x.data_ptr(), y.data_ptr(), output.data_ptr(),
+                                             _f32_vec(sTod_lin, L, "sTod_lin"), _f32_vec(sTod_tr, L, "sTod_tr"),
+                                             _f32_vec(nnzs, L, "nnzs"), B * H, L, n_cols, d, T,
+                                             dtype_code(x.dtype), ctypes.cast(plan_arr, ctypes.c_void_p),
+                                             status_word(dev).data_ptr(), _stream(dev))
         if rc not in _BAND_NOT_APPLICABLE:
-            check(rc, "splat_spmm_tile")
+            check(rc, "splat_spmm_tile_status")
             return
     with _on(dev):
         check(_lib.splat_spmm(x.data_ptr(), y.data_ptr(), output.data_ptr(),
@@ -646,5 +651,6 @@ def module_forward(attributes: dict, x):
 
 
 _host.bind(*(ctypes.cast(getattr(_lib, name), _vp).value for name in (
-    "splat_attention_fused_table", "splat_sddmm_band_table", "splat_spmm_band_table", "splat_sddmm_tile", "splat_spmm_tile",
+    "splat_attention_fused_table", "splat_sddmm_band_table", "splat_spmm_band_table", "splat_sddmm_tile_status",
+    "splat_spmm_tile_status",
     "splat_softmax", "splat_acsr_from_mask_u8", "splat_transpose_16", "splat_sddmm", "splat_spmm")), _warn_cuda_core_16bit)

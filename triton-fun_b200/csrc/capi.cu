@@ -56,7 +56,7 @@ extern "C" int32_t splat_selftest_bounded_wait(int32_t* status_word, int64_t lim
 }
 
 namespace splat {
-static struct { std::atomic<const int32_t*> word; std::atomic<int32_t*> mirror; std::atomic<int> device; } g_mirrors[64];
+static struct { std::atomic<const int32_t*> word; std::atomic<int32_t*> mirror; } g_mirrors[64];
 static std::mutex g_mirrors_mutex;
 
 int32_t* status_mirror(const int32_t* status_word) {   // entries are only ever filled from the front
@@ -67,32 +67,15 @@ int32_t* status_mirror(const int32_t* status_word) {   // entries are only ever 
     }
     return nullptr;
 }
-
-int32_t* registered_status_word() {
-    int device = -1;
-    if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
-    for (auto& e : g_mirrors) {
-        const int32_t* w = e.word.load(std::memory_order_acquire);
-        if (w == nullptr) break;
-        if (e.device.load(std::memory_order_relaxed) == device && e.mirror.load(std::memory_order_relaxed) != nullptr)
-            return const_cast<int32_t*>(w);
-    }
-    return nullptr;
-}
 }  // namespace splat
 
 extern "C" int32_t splat_set_status_mirror(int32_t* status_word, int32_t* host_copy) {
     if (!status_word) return SPLAT_ERR_BAD_ARG;
-    cudaPointerAttributes about;
-    int device = -1;
-    if (cudaPointerGetAttributes(&about, status_word) == cudaSuccess && about.type == cudaMemoryTypeDevice) device = about.device;
-    else (void)cudaGetLastError();
     std::lock_guard<std::mutex> lock(splat::g_mirrors_mutex);
     for (auto& e : splat::g_mirrors) {
         const int32_t* w = e.word.load(std::memory_order_relaxed);
         if (w != nullptr && w != status_word) continue;
         e.mirror.store(host_copy, std::memory_order_relaxed);
-        e.device.store(device, std::memory_order_relaxed);
         e.word.store(status_word, std::memory_order_release);
         return SPLAT_OK;
     }

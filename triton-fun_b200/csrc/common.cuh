@@ -135,8 +135,6 @@ inline int32_t launch_status() {
 
 // Host copy registered for a status word (splat_set_status_mirror), or null.  Defined in capi.cu.
 int32_t* status_mirror(const int32_t* status_word);
-// A status word of the current device that has a host copy, or null: for the entry points that are given none.
-int32_t* registered_status_word();
 
 // First thing a tensor-core kernel does (one thread): the status word, passed on to its host copy if set.
 __device__ __forceinline__ int32_t entry_status(const int32_t* status_word, int32_t* mirror) {

@@ -41,9 +41,9 @@ using SddmmBandFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int6
 using SpmmBandFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
                                int64_t, int64_t, int64_t, int32_t, const int32_t*, const int32_t*, int32_t*, void*);
 using SddmmTileFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, void*, const float*, const float*,
-                                const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
+                                const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, const int32_t*, int32_t*, void*);
 using SpmmTileFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
-                               int64_t, int64_t, int64_t, int32_t, const int32_t*, void*);
+                               int64_t, int64_t, int64_t, int32_t, const int32_t*, int32_t*, void*);
 using SddmmFn = int32_t (*)(const void*, const void*, int64_t, int64_t, int64_t, void*, const float*, const float*,
                             const float*, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t, void*);
 using SpmmFn = int32_t (*)(const void*, const void*, void*, const float*, const float*, const float*, int64_t, int64_t,
@@ -336,7 +336,7 @@ PyObject* sddmm(PyObject* const* a, Py_ssize_t n) {
     if (copied) ksb = n_cols * d;
     int32_t rc =
         dtype == 0 ? g_api.sddmm_tile(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
-                                      L, n_cols, d, trailing, dtype, plan, st)
+                                      L, n_cols, d, trailing, dtype, plan, g_status[dev].word, st)
                    : g_api.sddmm_band(x->const_data_ptr(), yp, ksb, ksc, ksk, out->data_ptr(), pl, pt, pn, B * H,
                                       L, n_cols, d, trailing, dtype, plan, table, g_status[dev].word, st);
     if (not_applicable(rc)) {
@@ -369,7 +369,7 @@ PyObject* spmm(PyObject* const* a, Py_ssize_t n) {
         return yes_or_none(false);
     void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
     int32_t rc = dtype == 0 ? g_api.spmm_tile(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
-                                                    n_cols, d, T, dtype, plan, st)
+                                                    n_cols, d, T, dtype, plan, g_status[dev].word, st)
                                   : g_api.spmm_band(x->const_data_ptr(), y->const_data_ptr(), out->data_ptr(), pl, pt, pn, B * H, L,
                                                     n_cols, d, T, dtype, plan, table, g_status[dev].word, st);
     if (not_applicable(rc)) {
@@ -412,7 +412,7 @@ PyObject* rows_of_k(PyObject* const* a, Py_ssize_t n) {
     return rows.defined() ? THPVariable_Wrap(rows) : yes_or_none(false);
 }
 
-// bind(fused, sddmm_band, spmm_band, sddmm_tile, spmm_tile, softmax, mask, transpose, sddmm, spmm, warn): addresses of the C ABI entry points
+// bind(fused, sddmm_band, spmm_band, sddmm_tile_status, spmm_tile_status, softmax, mask, transpose, sddmm, spmm, warn): addresses of the C ABI entry points
 // and the function that warns of 16-bit operands on the CUDA-core kernels
 PyObject* bind(PyObject*, PyObject* args) {
     unsigned long long f[10];

@@ -541,7 +541,7 @@ static int32_t launch(const Params& p, bool sddmm, int64_t bh, int64_t d, cudaSt
 }  // namespace ops
 }  // namespace split
 
-// Operands checked by splat_sddmm_tile() / splat_spmm_tile().
+// Operands checked by splat_sddmm_tile_status() / splat_spmm_tile_status().
 int32_t sddmm_split_f32(const void* q, const void* k, int kt, void* s, const float* lin, const float* tr, const float* nnzs, int64_t bh,
                         int64_t n_rows, int64_t d, int64_t stride, int64_t trailing, int32_t* status_word, cudaStream_t st) {
     split::ops::Params p{};

@@ -692,10 +692,11 @@ int32_t attention_tile_f32(const void* q, const void* k, int64_t ksb, int64_t ks
 
 using namespace splat;
 
-extern "C" int32_t splat_sddmm_tile(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
-                                    int64_t k_stride_k, void* s_out, const float* sTod_lin, const float* sTod_tr,
-                                    const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
-                                    int64_t trailing_dim, int32_t dtype, const int32_t* plan_i32, void* stream) {
+extern "C" int32_t splat_sddmm_tile_status(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
+                                           int64_t k_stride_k, void* s_out, const float* sTod_lin, const float* sTod_tr,
+                                           const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
+                                           int64_t trailing_dim, int32_t dtype, const int32_t* plan_i32, int32_t* status_word,
+                                           void* stream) {
     if (bh < 0 || n_rows < 0 || trailing_dim < 0) return SPLAT_ERR_BAD_ARG;
     if (dtype != SPLAT_F32 || trailing_dim < 1 || trailing_dim > INT32_MAX) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     tile::Params p{};
@@ -708,17 +709,26 @@ extern "C" int32_t splat_sddmm_tile(const void* q, const void* k, int64_t k_stri
     // at CTAs of 32 rows: +-64 of L1024 d32 128 6.1 / 8.8, 256 9.2 / 8.9 (contiguous K^T 8.0 / 9.1), 320 11.3 / 9.2; d64 128
     // 8.6 / 9.8, 160 14.3 / 9.8 (11.2 / 9.9); d128 128 13.7 / 13.8 (10.6 / 13.6), 160 22.9 / 13.8; causal 32 of L256 d64 152 9.2 / 8.5;
     // 64 taps by 4 of L1000 d64 160 10.0 / 8.6, d32 256 7.2 / 7.8, 320 9.3 / 7.8.
-    int32_t* const word = registered_status_word();
-    if (word != nullptr && aligned16(q) && rows32(n_rows, p.stride, bh) > (d == 32 ? 296 : 148))
-        return sddmm_split_f32(q, k, p.kt, s_out, sTod_lin, sTod_tr, nnzs, bh, n_rows, d, p.stride, trailing_dim, word, (cudaStream_t)stream);
+    if (status_word != nullptr && aligned16(q) && rows32(n_rows, p.stride, bh) > (d == 32 ? 296 : 148))
+        return sddmm_split_f32(q, k, p.kt, s_out, sTod_lin, sTod_tr, nnzs, bh, n_rows, d, p.stride, trailing_dim, status_word,
+                               (cudaStream_t)stream);
     p.q = (const float*)q; p.k = (const float*)k; p.sparse = (float*)s_out;
     p.lin = sTod_lin; p.tr = sTod_tr; p.nnzs = nnzs; p.trailing = (int)trailing_dim;
     return tile_launch<tile::Op::kSddmm>(p, d, bh, (cudaStream_t)stream);
 }
 
-extern "C" int32_t splat_spmm_tile(const void* p_in, const void* v, void* o, const float* sTod_lin, const float* sTod_tr,
-                                   const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
-                                   int64_t trailing_dim, int32_t dtype, const int32_t* plan_i32, void* stream) {
+extern "C" int32_t splat_sddmm_tile(const void* q, const void* k, int64_t k_stride_bh, int64_t k_stride_col,
+                                    int64_t k_stride_k, void* s_out, const float* sTod_lin, const float* sTod_tr,
+                                    const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
+                                    int64_t trailing_dim, int32_t dtype, const int32_t* plan_i32, void* stream) {
+    return splat_sddmm_tile_status(q, k, k_stride_bh, k_stride_col, k_stride_k, s_out, sTod_lin, sTod_tr, nnzs, bh, n_rows, n_cols,
+                                   d, trailing_dim, dtype, plan_i32, nullptr, stream);
+}
+
+extern "C" int32_t splat_spmm_tile_status(const void* p_in, const void* v, void* o, const float* sTod_lin, const float* sTod_tr,
+                                          const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
+                                          int64_t trailing_dim, int32_t dtype, const int32_t* plan_i32, int32_t* status_word,
+                                          void* stream) {
     if (bh < 0 || n_rows < 0 || trailing_dim < 0) return SPLAT_ERR_BAD_ARG;
     if (dtype != SPLAT_F32 || trailing_dim < 1 || trailing_dim > INT32_MAX) return SPLAT_ERR_UNSUPPORTED_SHAPE;
     tile::Params p{};
@@ -730,10 +740,17 @@ extern "C" int32_t splat_spmm_tile(const void* p_in, const void* v, void* o, con
     // As above, but its steps wait for one another: more than two waves at d <= 64.  us: +-64 of L1024 d64 128 7.3 / 11.5, 256
     // 12.1 / 11.6, 320 16.4 / 11.6; +-500 of L2048 d64 256 41.8 / 46.9, 512 76.9 / 47.6; d32 +-64 256 8.2 / 9.5, 320 12.8 / 9.5; 64 taps by 4
     // of L1000 d64 288 8.5 / 9.2, 320 10.3 / 9.2; d128 +-64 128 11.3 / 14.7, 160 18.5 / 14.8; +-500 128 38.4 / 52.7, 192 62.7 / 53.0.
-    int32_t* const word = registered_status_word();
-    if (word != nullptr && rows32(n_rows, p.stride, bh) > (d == 128 ? 148 : 296))
-        return spmm_split_f32(p_in, v, o, sTod_lin, sTod_tr, nnzs, bh, n_rows, d, p.stride, trailing_dim, word, (cudaStream_t)stream);
+    if (status_word != nullptr && rows32(n_rows, p.stride, bh) > (d == 128 ? 148 : 296))
+        return spmm_split_f32(p_in, v, o, sTod_lin, sTod_tr, nnzs, bh, n_rows, d, p.stride, trailing_dim, status_word,
+                              (cudaStream_t)stream);
     p.sparse = (float*)const_cast<void*>(p_in); p.v = (const float*)v; p.o = (float*)o;
     p.lin = sTod_lin; p.tr = sTod_tr; p.nnzs = nnzs; p.trailing = (int)trailing_dim;
     return tile_launch<tile::Op::kSpmm>(p, d, bh, (cudaStream_t)stream);
+}
+
+extern "C" int32_t splat_spmm_tile(const void* p_in, const void* v, void* o, const float* sTod_lin, const float* sTod_tr,
+                                   const float* nnzs, int64_t bh, int64_t n_rows, int64_t n_cols, int64_t d,
+                                   int64_t trailing_dim, int32_t dtype, const int32_t* plan_i32, void* stream) {
+    return splat_spmm_tile_status(p_in, v, o, sTod_lin, sTod_tr, nnzs, bh, n_rows, n_cols, d, trailing_dim, dtype, plan_i32, nullptr,
+                                  stream);
 }
