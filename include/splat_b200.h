@@ -122,8 +122,7 @@ int32_t splat_acsr_classify(const float* sTod_lin, const float* sTod_tr, const f
  * covers both a contiguous (BH, d, L) K^T (stride_col = 1, stride_k = L) and the transposed view
  * of a (BH, L, d) tensor (stride_col = d, stride_k = 1).  S and P are (BH, L, trailing_dim).
  * Inputs and outputs share one dtype; accumulation is fp32.  SPLAT_F32 operands are multiplied with all of their 24 bits: by
- * fp32 FMA, or on the tensor cores as three bf16 numbers each (never TF32); there an operand whose magnitude is below
- * 2^-110 loses precision relative to itself.
+ * fp32 FMA, or on the tensor cores as three bf16 numbers each (never TF32).
  * Slots >= nnz_i of S and P rows are written as zero.
  * ------------------------------------------------------------------------------------------- */
 

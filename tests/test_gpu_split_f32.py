@@ -196,6 +196,59 @@ def test_sddmm_and_spmm(d, contiguous):
         assert _off(o, dense @ v.double()) <= 2 ** -23, (L, H)
 
 
+@pytest.mark.parametrize("power", [-140, -126, -118, 52, 100, 115])
+def test_operands_of_any_magnitude(power):
+    """All bits of a tiny operand count, down to fp32's denormal numbers, and one that is too large for its three pieces, or the sums of
+    such, is not lost: relative errors are those of operands around 1, or of FMA sums where rows are computed again."""
+    L, H, d = 129, 64, 64
+    acsr = ah.create_acsr(ah.create_windowed_mask(L, 33), 16, 0)
+    meta, T = acsr[2:5], acsr[5]
+    cols, on = _slots(acsr, L, T)
+    x, kt, v = _operands(H, L, d, False)
+    up = 2.0 ** min(power, 100) * 2.0 ** max(power - 100, 0)
+    big = x * up                           # (rounded to the denormals' spacing at 2^-140)
+    other = kt * 2.0 ** (50 if power == 52 else 0)
+    s = torch.full((1, H, L, T), float("nan"), device="cuda")
+    n.sddmm(big, other, s, *meta, T)
+    ref = torch.gather(big.double() @ other.double(), 3, cols[None, None].expand(1, H, L, T)) * on
+    denormal = 2.0 ** -149 * ref.numel() ** 0.5 / ref.norm().item()        # what rounding the result to fp32 may add
+    # a chain of d additions, each off by 2^-24 / sqrt(3) of a partial sum that grows with the root of their number
+    assert _off(s, ref) <= (d / 6) ** 0.5 * 2 ** -24 + denormal
+    p = torch.rand(1, H, L, T, device="cuda") * on
+    dense = torch.zeros(1, H, L, L, device="cuda", dtype=torch.double)
+    dense.scatter_add_(3, cols[None, None].expand(1, H, L, T), p.double())
+    # sums of 67 products, at most 2^-25 of the largest partial sum each
+    for pp, vv in ((p, v * up), (p * up, v)):
+        o = torch.full((1, H, L, d), float("nan"), device="cuda")
+        n.spmm(pp, vv, o, *meta, T)
+        ref = (dense if pp is p else torch.zeros_like(dense).scatter_add_(3, cols[None, None].expand(1, H, L, T), pp.double())) @ vv.double()
+        denormal = 2.0 ** -149 * 4 * ref.numel() ** 0.5 / ref.norm().item()      # ... at each of up to three steps
+        assert _off(o, ref) <= 2 ** -22 + denormal
+    # fused: V, and Q with a scale that makes up for it
+    vv = v * up
+    ref_o, ref_lse = _exact(x, kt, vv, acsr, 0.125)
+    o, lse = _call(x, kt, vv, acsr, 0.125)
+    denormal = 2.0 ** -149 * ref_o.numel() ** 0.5 / ref_o.norm().item()
+    # scores as above, sums of 67 keys likewise, the exponentials' 2^-22 -- where rows are computed again with a chain of FMAs each
+    bound = ((d / 6) ** 0.5 + (67 / 6) ** 0.5) * 2 ** -24 + 2 ** -22
+    assert _off(o, ref_o) <= bound + denormal and _off(lse, ref_lse) <= 2 ** -22
+    if -120 <= power <= 60:
+        ref_o, ref_lse = _exact(big, kt, v, acsr, 0.125 / up)
+        o, lse = _call(big, kt, v, acsr, 0.125 / up)
+        assert _off(o, ref_o) <= bound and _off(lse, ref_lse) <= 2 ** -22
+    n.check_status_word(0)
+
+
+def test_tiny_scales_stay_on_the_register_tiles():
+    acsr = ah.create_acsr(ah.create_windowed_mask(300, 40), 16, 0)
+    q, kt, v = _operands(40, 300, 64, False)
+    q, kt = q * 2.0 ** 35, kt * 2.0 ** 35
+    for scale, same in ((2.0 ** -72, True), (0.0, True), (2.0 ** -60, False)):
+        o, lse = _call(q, kt, v, acsr, scale)
+        tile_o, tile_lse = _call(q, kt, v, acsr, scale, status=False)
+        assert torch.equal(o, tile_o) == same and (not same or torch.equal(lse, tile_lse))
+
+
 def test_sddmm_scores_that_are_not_finite():
     """An infinity is no sum of three bf16 numbers: such rows are computed again, as the row kernels give them."""
     L, H, d = 300, 40, 64

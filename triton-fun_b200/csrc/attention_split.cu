@@ -8,8 +8,7 @@
 // Error against 64 bits (2-norm, normal operands; in brackets a chain of fp32 FMAs): sums over 32 / 64 5.8e-8 / 7.6e-8
 // (1.06e-7 / 1.46e-7), the same six products with hh first 7.5e-7, sums over 1024 on the tensor core alone 6.6e-6
 // (5.7e-7).  Of a whole call 0.53 to 0.76 of that of the register tiles, at every pattern and size tried.
-// A tiny number's last pieces are denormal: below 2^-110 in magnitude an operand loses precision relative to itself.  Numbers
-// that are not finite, or round to infinity in bf16, make their rows NaN; such rows, and their log-sum-exps, are computed again
+// Numbers that are not finite, or too large (split2()), make their rows NaN; such rows, and their log-sum-exps, are computed again
 // from their own keys (row_exact.cuh), as in the other tile kernels.
 //
 // One CTA = 128 rows of one (bh, class).  Warps 0-7: thread = (row, half of the columns).  A step of 64 keys:
@@ -43,7 +42,6 @@ bool allow_dynamic_smem(const void* kernel, int bytes);   // attention_band.cu
 namespace split {
 
 using sm::ex2;
-using sm::mul2;
 
 constexpr int kThreads = kWorkers + 128;   // (a warpgroup more: registers are handed from it to the others)
 // status-word codes (which wait gave up)
@@ -66,6 +64,7 @@ struct Params {
     int kt;               // K is a contiguous (BH, D, L) array
     int vec_q, vec_k, vec_v;   // elements that a load may take at a time: 8, 4 or 1
     float scale_log2;     // > 0
+    float score_scale;    // scale_log2 for scores as the tensor core gives them: times kDown
     float sign;           // of the scale: goes to Q
 };
 
@@ -296,7 +295,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
         }
 #pragma unroll
         for (int i = 0; i < kHalf / 2; ++i) acc[i] = make_float2(0.f, 0.f);
-        auto add_o = [&] {              // acc += P V of the last step
+        auto add_o = [&] {              // acc += P V of the last step (2^32 times too large, up to the end)
 #pragma unroll
             for (int c = 0; c < kHalf; c += 16) {
                 uint32_t y[16];
@@ -307,7 +306,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
                     acc[c / 2 + i] = add2(acc[c / 2 + i], make_float2(__uint_as_float(y[2 * i]), __uint_as_float(y[2 * i + 1])));
             }
         };
-        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
+        const float2 sc2 = make_float2(p.score_scale, p.score_scale);
 #pragma unroll 1
         for (int j = 0; j < steps; ++j) {
             ok = wait_all(&ctrl->s_full, (uint32_t)j & 1u, &ctrl->gave_up, kErrS);
@@ -342,7 +341,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
             arrive(&ctrl->max_full[warp & 3]);
             ok = wait_all(&ctrl->max_full[warp & 3], (uint32_t)j & 1u, &ctrl->gave_up, kErrMax);
             if (!ok) break;
-            const float m_new = fmaxf(m_run, fmaxf(mine, ctrl->half[j & 1][half ^ 1][t]) * p.scale_log2);
+            const float m_new = fmaxf(m_run, fmaxf(mine, ctrl->half[j & 1][half ^ 1][t]) * p.score_scale);
             const float corr = m_new > m_run ? ex2(m_run - m_new) : 1.f;
             const bool moved = __any_sync(0xffffffffu, m_new > m_run);
             m_run = m_new;
@@ -439,7 +438,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
         }
         if (steps > 0 && ok) {
             l_sum = ctrl->half[steps & 1][0][t] + ctrl->half[steps & 1][1][t];
-            const float inv = 1.f / l_sum;
+            const float inv = 1.f / l_sum * kDown;
             const float2 inv2 = make_float2(inv, inv);
             float2 odd = make_float2(0.f, 0.f);
             constexpr int kPitch = kHalf * 4, kPer = kHalf / 4, kRows = 32 / kPer;     // a warp's 32 half rows; float4 of one; rows of a store
@@ -536,6 +535,7 @@ int32_t attention_split_f32(const void* q, const void* k, int kt, const void* v,
     p.q = (const float*)q; p.k = (const float*)k; p.v = (const float*)v; p.o = (float*)o; p.lse = lse;
     p.lin = lin; p.tr = tr; p.nnzs = nnzs; p.status = status_word; p.mirror = status_mirror(status_word);
     p.n_rows = (int)n_rows; p.stride = (int)stride; p.kt = kt; p.sign = scale < 0.f ? -1.f : 1.f; p.scale_log2 = p.sign * scale * kLog2e;
+    p.score_scale = p.scale_log2 * split::kDown;
     p.vec_q = split::vec_of(q); p.vec_v = split::vec_of(v); p.vec_k = split::vec_of_k(k, kt, stride, n_rows);
     if (d == 32) return split::launch<32>(p, bh, st);
     if (d == 64) return split::launch<64>(p, bh, st);

@@ -250,9 +250,11 @@ sddmm_split_kernel(const __grid_constant__ Params p) {
             if (__all_sync(0xffffffffu, band.x >= c0 + 32 || band.x + band.y <= c0)) continue;     // in none of the warp's bands
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
-                odd = fma2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), make_float2(0.f, 0.f), odd);
-                odd = fma2(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), make_float2(0.f, 0.f), odd);
-                *reinterpret_cast<uint4*>(stage + lane * kPitch + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+                const float2 a = mul2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), make_float2(kDown, kDown));
+                const float2 b = mul2(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), make_float2(kDown, kDown));
+                odd = fma2(a, make_float2(0.f, 0.f), odd);
+                odd = fma2(b, make_float2(0.f, 0.f), odd);
+                *reinterpret_cast<float4*>(stage + lane * kPitch + i) = make_float4(a.x, a.y, b.x, b.y);
             }
             __syncwarp();
             float* mem = first;
@@ -419,7 +421,8 @@ spmm_split_kernel(const __grid_constant__ Params p) {
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    acc[c / 2 + i] = add2(acc[c / 2 + i], make_float2(__uint_as_float(y[2 * i]), __uint_as_float(y[2 * i + 1])));
+                    acc[c / 2 + i] = fma2(make_float2(__uint_as_float(y[2 * i]), __uint_as_float(y[2 * i + 1])), make_float2(kDown, kDown),
+                                          acc[c / 2 + i]);
             }
         };
         bool ok = true;

@@ -16,6 +16,7 @@ namespace split {
 using namespace tc;
 using sm::add2;
 using sm::fma2;
+using sm::mul2;
 
 constexpr int kTile = 128;               // rows of a tile
 constexpr int kKeys = 64;                // keys of a step
@@ -36,9 +37,13 @@ __device__ __forceinline__ void load8(float (&x)[8], const float* p, int vec) {
         x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
     }
 }
-// two numbers -> their three bf16 pieces, packed
+// Two numbers, times 2^16 -> their three bf16 pieces, packed.  fp32's smallest number is 2^-149, bf16's 2^-133: unscaled, an
+// operand below 2^-110 would lose its last bits.  A product is 2^32 times too large (kDown); operands above 2^111 and sums above
+// 2^96 become infinite by it, and their rows are computed again like those of other infinities.
+constexpr float kUp = 65536.f, kDown = 1.f / (65536.f * 65536.f);
 __device__ __forceinline__ void split2(float2 x, uint32_t& h, uint32_t& m, uint32_t& l) {
     const float2 minus = make_float2(-1.f, -1.f);
+    x = mul2(x, make_float2(kUp, kUp));
     h = sm::pack2<__nv_bfloat16>(x.x, x.y);
     x = fma2(make_float2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus, x);
     m = sm::pack2<__nv_bfloat16>(x.x, x.y);

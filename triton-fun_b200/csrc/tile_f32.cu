@@ -589,7 +589,7 @@ static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
     return launch_kernel(kern, (unsigned)blocks, 32 * RW * KW, bytes, st, p);
 }
 
-// (More than a wave or two of 32-row CTAs come here without a status word, with Q off a 16-byte boundary or with scale 0 only.)
+// (More than a wave or two of 32-row CTAs come here without a status word, with Q off a 16-byte boundary or with a scale below 2^-60 only.)
 // 64-row CTAs unless they leave SMs without their three CTAs: then 32-row CTAs, whose four warps share the
 // keys of one row block, finish sooner, while with the GPU full they load every key twice as often; and with
 // less than two such CTAs per SM eight warps share them.  Four / eight warps, us, at 256 CTAs (L1024, +-64, where five or
@@ -680,8 +680,9 @@ int32_t attention_tile_f32(const void* q, const void* k, int64_t ksb, int64_t ks
     // there, at 128 and 160 CTAs of 32 rows: +-64 of L1024 d32 9.0 / 9.9, 14.9 / 9.9; d64 12.9 / 15.3, 21.2 / 15.4; d128 22.2 /
     // 17.8, 36.7 / 17.9; window 32 of L200, 147 and 154: d32 7.3 / 7.4, 12.5 / 7.4; d64 9.7 / 11.5, 17.2 / 11.6; d128 15.5 /
     // 13.8, 28.1 / 13.8.  At d = 128 they are the faster for less as well (window 32 of L256, 16 CTAs 15.3 / 14.7), but for a
-    // K^T that has to be gathered key by key (strided 16 of L2048, 64 CTAs 21.1 / 21.4).
-    if (status_word != nullptr && aligned16(q) && scale != 0.f && (rows32(n_rows, p.stride, bh) > 148 || (d == 128 && (!p.kt || p.stride == 1))))
+    // K^T that has to be gathered key by key (strided 16 of L2048, 64 CTAs 21.1 / 21.4).  Scales below 2^-60, 0 among them, stay
+    // here: scaled down by another 2^-32 (split_f32.cuh) they would lose bits.
+    if (status_word != nullptr && aligned16(q) && fabsf(scale) >= 0x1p-60f && (rows32(n_rows, p.stride, bh) > 148 || (d == 128 && (!p.kt || p.stride == 1))))
         return attention_split_f32(q, k, p.kt, v, o, lin, tr, nnzs, bh, n_rows, d, p.stride, scale, status_word, lse, st);
     p.q = (const float*)q; p.k = (const float*)k; p.v = (const float*)v; p.o = (float*)o; p.lse = lse;
     p.lin = lin; p.tr = tr; p.nnzs = nnzs; p.scale_log2 = scale * kLog2e;
