@@ -196,6 +196,39 @@ def test_sddmm_and_spmm(d, contiguous):
         assert _off(o, dense @ v.double()) <= 2 ** -23, (L, H)
 
 
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("window", [15, 63, 255])
+def test_operands_of_one_sign(window, d):
+    """Sums of positive numbers, where rounding towards zero does not average out."""
+    from test_gpu_tile_f32 import _Tiles
+    L, H = 1024, 10
+    acsr = ah.create_acsr(ah.create_windowed_mask(L, window), 16, 0)
+    meta, T = acsr[2:5], acsr[5]
+    cols, on = _slots(acsr, L, T)
+    tile = _Tiles(acsr, L, H, d)
+    scale = d ** -0.5
+    for form in ("uniform", "normal"):
+        q, kt, v = (t.abs() if form == "normal" else torch.rand_like(t) for t in _operands(H, L, d, False))
+        kt = kt.transpose(2, 3).contiguous().transpose(2, 3)
+        nan = lambda *shape: torch.full(shape, float("nan"), device="cuda")
+        s, tile_s, o = nan(1, H, L, T), nan(1, H, L, T), nan(1, H, L, d)
+        n.sddmm(q, kt, s, *meta, T)
+        assert tile.sddmm(q, kt, tile_s) == 0
+        ref = torch.gather(q.double() @ kt.double(), 3, cols[None, None].expand(1, H, L, T)) * on
+        assert _off(s, ref) <= _off(tile_s, ref), form
+        # P V: each of the four additions of a step's 64 keys is short by half of 2^-23 of the sum so far on average, 2^-24 (1 + 3/4 + 1/2 + 1/4)
+        # at most in all, and less the larger the mantissa; the steps are added with rounding
+        p = torch.rand(1, H, L, T, device="cuda") * on
+        n.spmm(p, v, o, *meta, T)
+        dense = torch.zeros(1, H, L, L, device="cuda", dtype=torch.double).scatter_add_(3, cols[None, None].expand(1, H, L, T), p.double())
+        assert _off(o, dense @ v.double()) <= 2 ** -23, form
+        ref_o, ref_lse = _exact(q, kt, v, acsr, scale)
+        o, lse = _call(q, kt, v, acsr, scale)
+        assert _off(o, ref_o) <= 2 ** -23, form
+        # a score is short by half of 2^-23 of itself, once; as much again for every other rounding together
+        assert _off(lse, ref_lse) <= 1.5 * 2 ** -24, form
+
+
 @pytest.mark.parametrize("power", [-140, -126, -118, 52, 100, 115])
 def test_operands_of_any_magnitude(power):
     """All bits of a tiny operand count, down to fp32's denormal numbers, and one that is too large for its three pieces, or the sums of

@@ -1,13 +1,19 @@
 // Fused attention of fp32 operands on the tensor cores, band patterns (the same as in tile_f32.cu).
 //
 // An fp32 number is the sum of three bf16 numbers to 2^-26 of itself: h = bf16(x), m = bf16(x - h), l = bf16(x - h - m).  A
-// product of two of them is six products on the tensor cores (hh, hm, mh, mm, hl, lh; what is left out is 2^-25), with fp32
-// accumulators.  Those round towards zero at every addition, so the order of the additions matters:
+// product of two of them is six products on the tensor cores (hh, hm, mh, mm, hl, lh; what is left out is 2^-22 of it at most and
+// 2^-25 on average), with fp32 accumulators.  Those round towards zero at every addition, so the order of the additions matters:
 //   * the five small products of a score are summed before hh, over all of d: they meet a small accumulator;
+//   * Q's h has six bits (split2()), so that most of what hh adds needs no rounding;
 //   * P V is summed on the tensor core over one step of 64 keys only; the steps are added up in registers, rounded to nearest.
-// Error against 64 bits (2-norm, normal operands; in brackets a chain of fp32 FMAs): sums over 32 / 64 5.8e-8 / 7.6e-8
-// (1.06e-7 / 1.46e-7), the same six products with hh first 7.5e-7, sums over 1024 on the tensor core alone 6.6e-6
-// (5.7e-7).  Of a whole call 0.53 to 0.76 of that of the register tiles, at every pattern and size tried.
+// Error against 64 bits over that of the register tiles (2-norm; L1024, windows of 31 to 1001 keys, d 32 to 128, the three operators):
+//   normal operands of either sign     fused 0.43 to 0.58, log-sum-exp 0.67 to 0.88, SDDMM 0.44 to 0.56, SpMM 0.37 to 1.01
+//   all of one sign                    fused 0.42 to 1.25, log-sum-exp 0.73 to 1.8 (it is 8e-8 then), SDDMM 0.24 to 0.66, SpMM 0.68 to 1.39 (9e-8;
+//                                      1.25 and 1.39 at 127 keys: sums of so few numbers that FMAs have hardly rounded)
+//   ... weights e^N(0,4), unnormalised SpMM 1.2 to 2.3 (1.8e-7)
+// for a truncated sum of numbers with one sign is short by half a unit or so, whatever they are.  (Six bits of V as well: SpMM
+// 1.39 -> 1.17, 2.3 -> 1.8, fused 1.25 -> 1.1 for 1 to 2 % of the time; of Q: log-sum-exp 2.6 -> 1.8 for nothing.  hh first instead
+// of last 7.5e-7 at sums over 64, sums over 1024 on the tensor core alone 6.6e-6.)
 // Numbers that are not finite, or too large (split2()), make their rows NaN; such rows, and their log-sum-exps, are computed again
 // from their own keys (row_exact.cuh), as in the other tile kernels.
 //
@@ -277,7 +283,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
                 uint4 h, m, l;
 #pragma unroll
                 for (int e = 0; e < 8; ++e) xq[i][e] *= p.sign;
-                split8(xq[i], h, m, l);
+                split8<true, true>(xq[i], h, m, l);
                 tmem_st4(lane_addr + c / 2, h);
                 if constexpr (L::kQSmem) {
                     uint8_t* to = smem + t * 128 + (((c / 8) ^ (t & 7)) << 4);
@@ -295,7 +301,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
         }
 #pragma unroll
         for (int i = 0; i < kHalf / 2; ++i) acc[i] = make_float2(0.f, 0.f);
-        auto add_o = [&] {              // acc += P V of the last step (2^32 times too large, up to the end)
+        auto add_o = [&] {              // acc += P V of the last step (2^16 times too large, up to the end)
 #pragma unroll
             for (int c = 0; c < kHalf; c += 16) {
                 uint32_t y[16];
@@ -409,7 +415,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
                         for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(r[16 * c + e + i]);
                     }
                     uint4 h, m, l;
-                    split8(y, h, m, l);
+                    split8<false>(y, h, m, l);
                     const uint32_t to = p_addr + (16 * c + e) / 2;
                     tmem_st4(to, h);
                     tmem_st4(to + 32, m);
@@ -438,7 +444,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
         }
         if (steps > 0 && ok) {
             l_sum = ctrl->half[steps & 1][0][t] + ctrl->half[steps & 1][1][t];
-            const float inv = 1.f / l_sum * kDown;
+            const float inv = 1.f / l_sum * (1.f / kUp);
             const float2 inv2 = make_float2(inv, inv);
             float2 odd = make_float2(0.f, 0.f);
             constexpr int kPitch = kHalf * 4, kPer = kHalf / 4, kRows = 32 / kPer;     // a warp's 32 half rows; float4 of one; rows of a store

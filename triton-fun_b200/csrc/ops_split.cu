@@ -212,7 +212,7 @@ sddmm_split_kernel(const __grid_constant__ Params p) {
                     for (int e = 0; e < 8; ++e) xq[e] = 0.f;
                 }
                 uint4 h, m, l;
-                split8(xq, h, m, l);
+                split8<true, true>(xq, h, m, l);
                 const uint32_t to = lane_addr + (half * kHalf + c) / 2;
                 tmem_st4(to, h);
                 tmem_st4(to + D / 2, m);

@@ -40,21 +40,35 @@ __device__ __forceinline__ void load8(float (&x)[8], const float* p, int vec) {
 // Two numbers, times 2^16 -> their three bf16 pieces, packed.  fp32's smallest number is 2^-149, bf16's 2^-133: unscaled, an
 // operand below 2^-110 would lose its last bits.  A product is 2^32 times too large (kDown); operands above 2^111 and sums above
 // 2^96 become infinite by it, and their rows are computed again like those of other infinities.
+//   kScale  false for the weights of a softmax: beside their row's largest, 1, those below 2^-110 are known to 2^-17 at most
+//   kShort  the first piece has six bits instead of eight (6 + 8 + 8 and a sign for each are 24 all the same), so that the products
+//           of first pieces are of 14 bits and sums of them have room in 24: see attention_split.cu
 constexpr float kUp = 65536.f, kDown = 1.f / (65536.f * 65536.f);
+template <bool kScale, bool kShort>
 __device__ __forceinline__ void split2(float2 x, uint32_t& h, uint32_t& m, uint32_t& l) {
     const float2 minus = make_float2(-1.f, -1.f);
-    x = mul2(x, make_float2(kUp, kUp));
-    h = sm::pack2<__nv_bfloat16>(x.x, x.y);
-    x = fma2(make_float2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus, x);
+    if (kScale) x = mul2(x, make_float2(kUp, kUp));
+    uint32_t a, b;
+    if (kShort) {
+        a = (__float_as_uint(x.x) + 0x20000u) & 0xfffc0000u;
+        b = (__float_as_uint(x.y) + 0x20000u) & 0xfffc0000u;
+        h = __byte_perm(a, b, 0x7632);
+    } else {
+        h = sm::pack2<__nv_bfloat16>(x.x, x.y);
+        a = h << 16;
+        b = h & 0xffff0000u;
+    }
+    x = fma2(make_float2(__uint_as_float(a), __uint_as_float(b)), minus, x);
     m = sm::pack2<__nv_bfloat16>(x.x, x.y);
     x = fma2(make_float2(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u)), minus, x);
     l = sm::pack2<__nv_bfloat16>(x.x, x.y);
 }
+template <bool kScale = true, bool kShort = false>
 __device__ __forceinline__ void split8(const float (&x)[8], uint4& h, uint4& m, uint4& l) {
-    split2(make_float2(x[0], x[1]), h.x, m.x, l.x);
-    split2(make_float2(x[2], x[3]), h.y, m.y, l.y);
-    split2(make_float2(x[4], x[5]), h.z, m.z, l.z);
-    split2(make_float2(x[6], x[7]), h.w, m.w, l.w);
+    split2<kScale, kShort>(make_float2(x[0], x[1]), h.x, m.x, l.x);
+    split2<kScale, kShort>(make_float2(x[2], x[3]), h.y, m.y, l.y);
+    split2<kScale, kShort>(make_float2(x[4], x[5]), h.z, m.z, l.z);
+    split2<kScale, kShort>(make_float2(x[6], x[7]), h.w, m.w, l.w);
 }
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, uint4 r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
