@@ -214,10 +214,10 @@ attention_split_kernel(const __grid_constant__ Params p) {
                     for (int i = 0; i < 6; ++i)
 #pragma unroll
                         for (int kk = 0; kk < D / 16; ++kk) {
-                            const uint64_t b = desc(kl + ((piece_b(i) * L::kPiece + (kKt ? kk * 2048 : (kk >> 2) * kSubBytes + (kk & 3) * 32)) >> 4));
+                            const uint64_t b = desc_sw128(kl + ((piece_b(i) * L::kPiece + (kKt ? kk * 2048 : (kk >> 2) * kSubBytes + (kk & 3) * 32)) >> 4));
                             const uint32_t add = i > 0 || kk > 0 ? 1u : 0u;
                             if (L::kQSmem && piece_a(i) > 0)
-                                mma_ss(tm + L::kS, desc(ql + (((piece_a(i) - 1) * L::kQPiece + kk * 32) >> 4)), b, idesc_s, add);
+                                mma_ss(tm + L::kS, desc_sw128(ql + (((piece_a(i) - 1) * L::kQPiece + kk * 32) >> 4)), b, idesc_s, add);
                             else
                                 mma_ts(tm + L::kS, tm + piece_a(i) * (D / 2) + kk * 8, b, idesc_s, add);
                         }
@@ -239,7 +239,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
                     for (int i = 0; i < 6; ++i)
 #pragma unroll
                         for (int kk = 0; kk < kKeys / 16; ++kk)
-                            mma_ts(tm + L::kO, tm + L::kP + piece_a(i) * 32 + kk * 8, desc(vl + ((piece_b(i) * L::kPiece + kk * 2048) >> 4)), idesc_o,
+                            mma_ts(tm + L::kO, tm + L::kP + piece_a(i) * 32 + kk * 8, desc_sw128(vl + ((piece_b(i) * L::kPiece + kk * 2048) >> 4)), idesc_o,
                                    (i > 0 || kk > 0) ? 1u : 0u);
                     mma_commit(&ctrl->o_full);
                 }

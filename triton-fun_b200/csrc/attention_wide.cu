@@ -121,11 +121,6 @@ template <int D, int kKeys> struct Layout {
     static constexpr int kPerSm = kKeys == 128 ? 2 : 4;
 };
 
-// Descriptors of operands in shared memory by their low words (smem_desc_sw128), so that an MMA's is one 32-bit addition.
-constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t desc_lo(const void* p, uint32_t lbo_bytes) { return ((smem_u32(p) & 0x3ffffu) >> 4) | (lbo_bytes >> 4) << 16; }
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t lo) { return (uint64_t)kDescHi << 32 | lo; }
-
 // O of the warp's rows (n pieces of 16 columns) times corr.  Rare, and kept out of the main loop.
 __device__ __forceinline__ void rescale_o(uint32_t o_addr, int n, float corr) {
     uint32_t v[16];

@@ -179,7 +179,7 @@ sddmm_split_kernel(const __grid_constant__ Params p) {
 #pragma unroll
                         for (int kk = 0; kk < D / 16; ++kk)
                             mma_ts(to, tm + piece_a(i) * (D / 2) + kk * 8,
-                                   desc(kl + ((piece_b(i) * kPieceBytes<D> + (kKt ? kk * 2048 : (kk >> 2) * kSubBytes + (kk & 3) * 32)) >> 4)),
+                                   desc_sw128(kl + ((piece_b(i) * kPieceBytes<D> + (kKt ? kk * 2048 : (kk >> 2) * kSubBytes + (kk & 3) * 32)) >> 4)),
                                    idesc, i > 0 || kk > 0 ? 1u : 0u);
                     mma_commit(&ctrl->done[j & 1]);
                 }
@@ -369,7 +369,7 @@ spmm_split_kernel(const __grid_constant__ Params p) {
                     for (int i = 0; i < 6; ++i)
 #pragma unroll
                         for (int kk = 0; kk < kKeys / 16; ++kk)
-                            mma_ts(tm + L::kO, from + piece_a(i) * 32 + kk * 8, desc(vl + ((piece_b(i) * kPieceBytes<D> + kk * 2048) >> 4)), idesc,
+                            mma_ts(tm + L::kO, from + piece_a(i) * 32 + kk * 8, desc_sw128(vl + ((piece_b(i) * kPieceBytes<D> + kk * 2048) >> 4)), idesc,
                                    i > 0 || kk > 0 ? 1u : 0u);
                     mma_commit(&ctrl->done[j & 1]);
                 }

@@ -74,15 +74,12 @@ __device__ __forceinline__ void tmem_st4(uint32_t taddr, uint4 r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
                  : "memory");
 }
-// D[tmem] (+)= A * B with the operands' descriptors given by their low words.  (`lo` is hidden from the compiler where it is
-// formed, which otherwise keeps the sums of all 48 MMAs of a step in registers.)
-constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);     // groups of 8 rows 1024 bytes apart, version 1, 128-byte swizzle
-__device__ __forceinline__ uint32_t desc_lo(const void* p, uint32_t lbo_bytes) { return ((smem_u32(p) & 0x3ffffu) >> 4) | (lbo_bytes >> 4) << 16; }
+// Hides from the compiler where a descriptor's low word (desc_lo()) or a tensor-memory address comes from: it otherwise keeps the sums
+// of all 48 MMAs of a step in registers.
 __device__ __forceinline__ uint32_t hidden(uint32_t x) {
     asm volatile("" : "+r"(x));
     return x;
 }
-__device__ __forceinline__ uint64_t desc(uint32_t lo) { return (uint64_t)kDescHi << 32 | lo; }
 
 // The six products: piece (0 h, 1 m, 2 l) of A and of B, the largest product last.
 __host__ __device__ constexpr int piece_a(int i) { return (0x001102 >> (4 * i)) & 15; }

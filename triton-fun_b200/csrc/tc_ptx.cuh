@@ -416,6 +416,14 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr, uint32_t
     return d;
 }
 
+// The same by its low word (start address and LBO; the rest, SBO = 1024 among it, is constant): where it changes from MMA to MMA that
+// is one 32-bit addition.
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(const void* p, uint32_t lbo_bytes) {
+    return ((smem_u32(p) & 0x3ffffu) >> 4) | (lbo_bytes >> 4) << 16;
+}
+__device__ __forceinline__ uint64_t desc_sw128(uint32_t lo) { return (uint64_t)kDescHi << 32 | lo; }
+
 // Instruction descriptor for kind::f16 with fp32 accumulation.
 // fmt: 0 = fp16, 1 = bf16 (both operands).  b_mn_major: 1 when B is MN-major.
 __host__ __device__ constexpr uint32_t instr_desc_f16(uint32_t fmt, uint32_t m, uint32_t n,
