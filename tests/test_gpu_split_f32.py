@@ -1,5 +1,6 @@
-"""GPU: the fused fp32 kernel on the tensor cores (operands split into three bf16 numbers) at the edges of its tiles of 128 rows
-and steps of 64 keys, against 64 bits: it must not be further off than the kernel that sums with FMAs."""
+"""GPU: the fp32 kernels on the tensor cores (operands split into three bf16 numbers) at the edges of their tiles of 128 rows
+and steps of 64 keys, against 64 bits: with operands of either sign they must not be further off than the kernels that sum with
+FMAs."""
 import ctypes
 import os
 import subprocess
@@ -73,9 +74,9 @@ def _off(x, ref):
     return ((x.double() - ref)[ok].norm() / ref[ok].norm()).item()
 
 
-def _operands(H, L, d, contiguous, shift=0):
+def _operands(H, L, d, contiguous):
     g = torch.Generator(device="cuda").manual_seed(L * d + H)
-    q, k, v = (torch.empty(H * L * d + 4, device="cuda").normal_(generator=g)[shift:shift + H * L * d].view(1, H, L, d) for _ in range(3))
+    q, k, v = (torch.empty(1, H, L, d, device="cuda").normal_(generator=g) for _ in range(3))
     kt = k.transpose(2, 3)
     return q, kt.contiguous() if contiguous else kt, v
 
@@ -112,20 +113,39 @@ def test_operands_on_16_bytes_give_the_same_bits(d):
         assert torch.equal(o, o4) and torch.equal(lse, lse4)
 
 
-def test_nothing_is_written_while_the_status_word_is_set():
+def test_q_off_a_16_byte_boundary_stays_on_the_register_tiles():
+    from test_gpu_tile_f32 import _Tiles
+    L, H, d = 300, 40, 64
+    acsr = ah.create_acsr(ah.create_windowed_mask(L, 40), 16, 0)
+    q, kt, v = _operands(H, L, d, False)
+    off = torch.empty(q.numel() + 1, device="cuda")[1:].view_as(q).copy_(q)
+    tile_o, tile_lse = _call(q, kt, v, acsr, 0.125, status=False)
+    o, lse = _call(off, kt, v, acsr, 0.125)
+    s, tile_s = (torch.full((1, H, L, acsr[5]), float("nan"), device="cuda") for _ in range(2))
+    n.sddmm(off, kt, s, *acsr[2:5], acsr[5])
+    assert _Tiles(acsr, L, H, d).sddmm(q, kt, tile_s) == 0
+    assert torch.equal(o, tile_o) and torch.equal(lse, tile_lse) and torch.equal(s, tile_s)
+
+
+@pytest.mark.parametrize("op", ["fused", "sddmm", "spmm"])
+def test_nothing_is_written_while_the_status_word_is_set(op):
     acsr = ah.create_acsr(ah.create_windowed_mask(300, 40), 16, 0)
     q, kt, v = _operands(40, 300, 64, False)
-    out = torch.full_like(q, 3.0)
-    launch = lambda: n.attention_fused(q, kt, v, out, acsr[2], acsr[3], acsr[4], 0.125)
+    meta, T = acsr[2:5], acsr[5]
+    out = torch.full((1, 40, 300, T), 1e6, device="cuda") if op == "sddmm" else torch.full_like(q, 1e6)
+    p = torch.rand(1, 40, 300, T, device="cuda")
+    launch = {"fused": lambda: n.attention_fused(q, kt, v, out, *meta, 0.125), "sddmm": lambda: n.sddmm(q, kt, out, *meta, T),
+              "spmm": lambda: n.spmm(p, v, out, *meta, T)}[op]
+    n.classify(*meta)
     n.status_word(q.device).fill_(7)
     launch()
     torch.cuda.synchronize()
-    assert (out == 3.0).all()
+    assert (out == 1e6).all()
     with pytest.raises(RuntimeError):      # the launcher looks at the host copy of the word
         launch()
     launch()
     n.check_status_word(0)
-    assert torch.isfinite(out).all() and not (out == 3.0).any()
+    assert torch.isfinite(out).all() and not (out == 1e6).any()
 
 
 def test_host_operands_while_the_status_word_is_set():
@@ -171,6 +191,7 @@ def _slots(acsr, L, T):
 @pytest.mark.parametrize("contiguous", [False, True])
 @pytest.mark.parametrize("d", [32, 64, 128])
 def test_sddmm_and_spmm(d, contiguous):
+    from test_gpu_tile_f32 import _Tiles
     for mask, L, H in OPS:
         acsr = ah.create_acsr(_mask(mask, L), 16, 0)
         meta, T = acsr[2:5], acsr[5]
@@ -179,6 +200,8 @@ def test_sddmm_and_spmm(d, contiguous):
         s = torch.full((1, H, L, T), float("nan"), device="cuda")
         n.sddmm(q, kt, s, *meta, T)
         n.check_status_word(0)
+        tile, tile_s = _Tiles(acsr, L, H, d), torch.full_like(s, float("nan"))
+        assert tile.sddmm(q, kt, tile_s) == 0 and not torch.equal(s, tile_s), "the register tiles ran"
         full = q.double() @ kt.double()
         ref = torch.gather(full, 3, cols[None, None].expand(1, H, L, T)) * on
         assert torch.count_nonzero(s * ~on) == 0, "padding slots must be zero"
@@ -190,6 +213,8 @@ def test_sddmm_and_spmm(d, contiguous):
         o = torch.full((1, H, L, d), float("nan"), device="cuda")
         n.spmm(p, v, o, *meta, T)
         n.check_status_word(0)
+        tile_o = torch.full_like(o, float("nan"))
+        assert tile.spmm(p, v, tile_o) == 0 and not torch.equal(o, tile_o), "the register tiles ran"
         dense = torch.zeros(1, H, L, L, device="cuda", dtype=torch.double)
         dense.scatter_add_(3, cols[None, None].expand(1, H, L, T), torch.where(on, p, torch.zeros((), device="cuda")).double())
         # a rounded result is off by 2^-25 of itself on average, a few additions by as much
