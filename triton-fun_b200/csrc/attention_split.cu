@@ -263,7 +263,7 @@ attention_split_kernel(const __grid_constant__ Params p) {
         float x[kUnits<D>][8];           // K or V on its way
         auto ask_v = [&](int j) { ask_rows<D>(x, vbase, pitch, lo + j * kKeys, rows_v, p.vec_v); };
         auto ask_k = [&](int j) {
-            if constexpr (kKt) ask_kt<D>(x, kbase, p.n_rows, p.stride, res, lo + j * kKeys, rows_v, p.vec_k);
+            if constexpr (kKt) ask_kt<D, false>(x, kbase, p.n_rows, p.stride, res, lo + j * kKeys, rows_v, p.vec_k);
             else ask_rows<D>(x, kbase, pitch, lo + j * kKeys, rows_v, p.vec_k);
         };
         auto arrive = [&](uint64_t* bar) {

@@ -196,7 +196,7 @@ sddmm_split_kernel(const __grid_constant__ Params p) {
         const float* kbase = kKt ? p.k + at.head * D : p.k + (at.head + at.res) * D;
         float x[kUnits<D>][8];           // K on its way
         auto ask_k = [&](int j) {
-            if constexpr (kKt) ask_kt<D>(x, kbase, p.n_rows, p.stride, at.res, lo + j * kKeys, at.rows_v, p.vec_k);
+            if constexpr (kKt) ask_kt<D, true>(x, kbase, p.n_rows, p.stride, at.res, lo + j * kKeys, at.rows_v, p.vec_k);
             else ask_rows<D>(x, kbase, at.pitch, lo + j * kKeys, at.rows_v, p.vec_k);
         };
         if (steps > 0) {

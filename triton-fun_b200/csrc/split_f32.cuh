@@ -99,20 +99,28 @@ __device__ __forceinline__ void ask_rows(float (&x)[kUnits<D>][8], const float* 
         }
     }
 }
-// ... of a (D, n_rows) K^T, eight keys of a row at a time where they are contiguous and aligned (vec > 1)
-template <int D>
+// ... of a (D, n_rows) K^T, eight keys of a row at a time where they are contiguous and aligned (vec > 1).  One branch for all units of a
+// thread: with one for each the fused kernel at d = 128 spilled where it counted, us, each / one: H8 L21120 window 25 161 / 150,
+// L8606 +-318 48.8 / 43.6, H22 L1152 window 96 39.7 / 38.4; d64 104.1 / 103.5 (B2 H16 L4096 window 256).  kAnew: the row addresses are
+// formed at every step instead of kept, which SDDMM has no registers for (us, kept / anew: d128 H6 L2944 +-38 17.4 / 16.2).
+template <int D, bool kAnew>
 __device__ __forceinline__ void ask_kt(float (&x)[kUnits<D>][8], const float* base, int n_rows, int stride, int res, int u, int rows_v,
                                        int vec) {
+    // (a thread's units are at the same keys, kWorkers * 8 / kKeys rows apart)
+    const int key = u + (int)threadIdx.x % (kKeys / 8) * 8;
+    const int rows = kAnew ? (int)hidden((uint32_t)n_rows) : n_rows;
+    const float* src = base + (int64_t)(threadIdx.x / (kKeys / 8)) * rows;
+    const int64_t pitch = (int64_t)(kWorkers * 8 / kKeys) * rows;
+    if (vec > 1 && key + 8 <= rows_v) {
+        src += key;
 #pragma unroll
-    for (int i = 0; i < kUnits<D>; ++i) {
-        const int unit = threadIdx.x + i * kWorkers, c = unit / (kKeys / 8), key = u + unit % (kKeys / 8) * 8;
-        const float* src = base + (int64_t)c * n_rows;
-        if (vec > 1 && key + 8 <= rows_v) {
-            load8(x[i], src + key, vec);
-        } else {
+        for (int i = 0; i < kUnits<D>; ++i, src += pitch) load8(x[i], src, vec);
+    } else {
+        src += (int64_t)key * stride + res;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x[i][e] = key + e < rows_v ? __ldg(src + (int64_t)(key + e) * stride + res) : 0.f;
-        }
+        for (int i = 0; i < kUnits<D>; ++i, src += pitch)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[i][e] = key + e < rows_v ? __ldg(src + (int64_t)e * stride) : 0.f;
     }
 }
 // kKt: the block came from ask_kt()
