@@ -26,9 +26,9 @@
 // say all: k_full (K(j + 1) in its place and S(j) read), p_full (V(j), P(j) in their places and P V(j - 1) fetched).
 // Pieces of 16 columns outside all of a warp's bands are not exponentiated.
 //
-// Measured, us, register tiles -> this: B2 H16 L4096 window 256 d32 166 -> 64, d64 248 -> 104, d128 561 -> 171; B1 H8 L8192
-// d128 256 taps by 2 288 -> 98; B3 H8 L3001 d64 +-200 240 -> 81; B1 H2 L8192 d128 +-700 389 -> 69.  At d64 the tensor pipe is
-// busy 37 % of the time, issue slots 46 %, ALUs 33 % (the split is seven ALU instructions for two numbers): a CTA's chain S -> max
+// Measured, us, register tiles -> this: B2 H16 L4096 window 256 d32 166 -> 64, d64 248 -> 104, d128 561 -> 172; B1 H8 L8192
+// d128 256 taps by 2 288 -> 99; B3 H8 L3001 d64 +-200 240 -> 81; B1 H2 L8192 d128 +-700 389 -> 69.  At d64 the tensor pipe is
+// busy 37 % of the time, issue slots 47 %, ALUs 34 % (the split is seven ALU instructions for two numbers): a CTA's chain S -> max
 // -> P -> P V, two CTAs to an SM.  Its MMAs, edges of the bands included, are 41 us of
 // tensor time, six times the products themselves 30.
 // What lost, at the same d64 problem: softmax warps of a thread per row (four) beside four that copy and issue 120 to 135 us

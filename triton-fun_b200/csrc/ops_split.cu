@@ -5,8 +5,8 @@
 //       the warp's 32 x 32 block goes through shared memory to stores along the rows
 //   spmm_split_kernel    O += P(j) V(j): 32 x 32 blocks of P by cp.async, a row of the sparse operand at a time, then split and
 //       placed in tensor memory; P V of a step is added to the O in registers a step later
-// Measured, us, register tiles -> this: B2 H16 L4096 window 256, d32 / d64 / d128 SDDMM 112 / 176 / 326 -> 56 / 68 / 100, SpMM 100 / 146 /
-// 279 -> 72 / 87 / 142 (HBM, d64: 31); H64 L1024 +-64 d64 60 -> 26, 52 -> 31.  SDDMM is bound by the instructions that store a row's 32
+// Measured, us, register tiles -> this: B2 H16 L4096 window 256, d32 / d64 / d128 SDDMM 112 / 176 / 326 -> 57 / 69 / 105, SpMM 100 / 146 /
+// 279 -> 72 / 88 / 143 (HBM, d64: 31); H64 L1024 +-64 d64 60 -> 26, 52 -> 31.  SDDMM is bound by the instructions that store a row's 32
 // scores at a time (rows begin at any element), SpMM by the chain of a step, P V -> O, V -> P V, and the copies of P, 4 bytes at a
 // time.  Two places of K and of the scores, or of P, so that a step's MMAs do not wait for the stores or the split of the
 // step before: SDDMM of H8 L1024 +-64 10.5 -> 10.0, SpMM 12.7 -> 11.6.

@@ -22,7 +22,7 @@
 // The packed FMA (two results per instruction, two cycles of the pipe) leaves the issue slots that the
 // shared-memory reads and the operand duplication need; in a loop of nothing but such updates an
 // 8 x 8 block takes 75 to 78 cycles instead of 64 (packed) and 77 to 83 (scalar).
-// Measured on B2 H16 L4096 d64, causal window 256 (1862 us with the row kernel):
+// Measured on B2 H16 L4096 d64, causal window 256 (1862 us with the row kernel, 104 on the tensor cores, which take it given a word):
 //   64 rows per CTA, 64-key steps, 8 x 8 scores per lane, K and V prefetched    267 us (scalar FMAs 301)
 //   the same, 32 rows x 2 keys per lane, the rows read uniformly                 280 us
 //   RW = 2, KW = 1, six CTAs per SM                                              258 us
@@ -589,7 +589,9 @@ static int32_t launch(Params p, int64_t bh, cudaStream_t st) {
     return launch_kernel(kern, (unsigned)blocks, 32 * RW * KW, bytes, st, p);
 }
 
-// (More than a wave or two of 32-row CTAs come here without a status word, with Q off a 16-byte boundary or with a scale below 2^-60 only.)
+// More than a wave or two of 32-row CTAs come here only without a status word (splat_sddmm_tile, splat_spmm_tile, a null word of the fused
+// entry points), with Q off a 16-byte boundary or with a scale below 2^-60: for these the 64-row CTAs, four warps and the
+// smaller register budget of more than 296 CTAs are.
 // 64-row CTAs unless they leave SMs without their three CTAs: then 32-row CTAs, whose four warps share the
 // keys of one row block, finish sooner, while with the GPU full they load every key twice as often; and with
 // less than two such CTAs per SM eight warps share them.  Four / eight warps, us, at 256 CTAs (L1024, +-64, where five or
